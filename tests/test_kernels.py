@@ -164,6 +164,33 @@ def test_gemm_f32(ops, T, N, K):
     assert torch.equal(y1[0], y[T - 1])
 
 
+@pytest.mark.parametrize("T, N, K", [
+    (1, 17, 4), (3, 8, 260), (8, 33, 2048), (9, 2100, 68), (16, 40, 2052), (24, 300, 8196), (25, 2561, 64),    # streamed
+    (32, 2560, 1020), (2, 2400, 516),                                # several portions of tokens, rows of a second round
+    (33, 130, 2304), (65, 127, 1792), (40, 129, 6152), (64, 128, 31), (200, 260, 16640)])      # tiles, alone and in clusters
+def test_gemm_f32_order_of_sums(ops, T, N, K):
+    """An element's sum is the same whatever kernel makes it, at the edges of segments (64), units (256), ranges (an eighth
+    of K) and tiles; and within its bound: at most 32 products one after another (even and odd k of a segment), one sum
+    of the two, the segments of a range, eight ranges and what is accumulated, each rounded to half of 2^-23."""
+    g = torch.Generator().manual_seed(T * N + K)
+    x, w = torch.randn(T, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
+    base = torch.randn(T, N, generator=g).to(DEV)
+    y, y2 = torch.full((T, N), float("nan"), device=DEV), base.clone()
+    ops.gemm_f32(x, w, y)
+    ops.gemm_f32(x, w, y2, accumulate=True)
+    units = (K + 255) // 256
+    roundings = 32 + 1 + 4 * ((units + 7) // 8) + 8 + 1
+    size = x.double().abs() @ w.double().abs().T + base.double().abs()
+    ref = x.double() @ w.double().T
+    assert bool(((y.double() - ref).abs() <= roundings * 2.0 ** -24 * size).all())
+    assert bool(((y2.double() - ref - base.double()).abs() <= roundings * 2.0 ** -24 * size).all())
+    for rows in (slice(0, 1), slice(T // 2, T // 2 + 7), slice(max(0, T - 30), T)):       # other kernels, other portions
+        part, part2 = torch.empty_like(y[rows]), base[rows].clone()
+        ops.gemm_f32(x[rows].contiguous(), w, part)
+        ops.gemm_f32(x[rows].contiguous(), w, part2, accumulate=True)
+        assert torch.equal(part, y[rows]) and torch.equal(part2, y2[rows])
+
+
 # ---------------------------------------------------------------- paged attention
 def paged(k, v, dtype, n_extra_pages=3, seed=0):
     """Scatter dense per-sequence K/V ([len, nkv, hd] each) over shuffled pages.
