@@ -250,6 +250,34 @@ def test_attention_f32(ops, nh, nkv, hd, window):
     close(out, plain_attention_rows(qs, ks, vs, q_lens, window), 2e-5)
 
 
+@pytest.mark.parametrize("nh, nkv, hd", [(4, 2, 36), (3, 1, 260)])
+def test_attention_f32_warps_of_a_query(ops, nh, nkv, hd):
+    """Four warps share a query's keys in chunks of 32: lengths around a chunk, around four of them, with and without a
+    window that leaves warps without a chunk; against float64, and a query alone against itself among others, bit for bit."""
+    g = torch.Generator().manual_seed(hd)
+    lens = [1, 31, 32, 33, 64, 127, 128, 129, 300]
+    k = [torch.randn(n, nkv, hd, generator=g) for n in lens]
+    v = [torch.randn(n, nkv, hd, generator=g) for n in lens]
+    k_cache, v_cache, table = paged(k, v, torch.float32)
+    q = torch.randn(len(lens), nh * hd, generator=g).to(DEV)
+    pos = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=DEV)
+    seq = torch.arange(len(lens), dtype=torch.int32, device=DEV)
+    for window in (0, 1, 40):
+        out = torch.empty(len(lens), nh * hd, device=DEV)
+        ops.attention_f32(q, k_cache, v_cache, out, table, seq, pos, nh, nkv, hd, PAGE, window, hd ** -0.5)
+        for i, n in enumerate(lens):
+            first = max(0, n - window) if window else 0
+            for h in range(nh):
+                kk, vv = k[i][first:, h // (nh // nkv)].double(), v[i][first:, h // (nh // nkv)].double()
+                p = torch.softmax(kk @ q[i, h * hd:(h + 1) * hd].double().cpu() * hd ** -0.5, 0)
+                # hd products and as many keys a sum, scores of size one: a few hundred roundings of 2^-24 at most
+                close(out[i, h * hd:(h + 1) * hd], p @ vv, 3e-5)
+            one = torch.empty(1, nh * hd, device=DEV)
+            ops.attention_f32(q[i:i + 1].contiguous(), k_cache, v_cache, one, table, seq[i:i + 1].contiguous(),
+                              pos[i:i + 1].contiguous(), nh, nkv, hd, PAGE, window, hd ** -0.5)
+            assert torch.equal(one[0], out[i])
+
+
 @pytest.mark.parametrize("nh, nkv, hd, window", [(4, 2, 16, 0), (6, 2, 24, 0), (3, 1, 40, 0), (5, 5, 72, 70),
                                                  (32, 8, 128, 0), (8, 1, 64, 100), (40, 2, 32, 0), (4, 4, 256, 0)])
 def test_attention_bf16_prefill(ops, nh, nkv, hd, window):
