@@ -81,29 +81,45 @@ __device__ __forceinline__ float norm_block_sum(float v, float* scratch) {
   return t;
 }
 
+// A step of few rows (FEW: at most two a SM) is bound by the chain of latencies from the kernel before to the kernel
+// after: 512 threads a row, so that a thread has one or two loads to wait for, and the weight, which no kernel before
+// wrote, is in registers before the wait for that kernel ends (8 rows of 4,096: 4.8 -> 3.0 us in a decode step).
+
+constexpr int FEW_ROWS = 296, FEW_THREADS = 512;
+
 template <typename TG, typename TO, int THREADS, int NORM_CACHE>
-__global__ void __launch_bounds__(THREADS, NORM_CACHE == 4 ? 1280 / THREADS : 1) rmsnorm_vec_kernel(const float* __restrict__ x,
+__global__ void __launch_bounds__(THREADS, NORM_CACHE == 4 && THREADS != FEW_THREADS ? 1280 / THREADS : 1) rmsnorm_vec_kernel(const float* __restrict__ x,
                                                              const int* __restrict__ row_index,
                                                              const TG* __restrict__ gamma, float eps,
                                                              TO* __restrict__ out, int H,
                                                              float4* __restrict__ clear, size_t clear_n4) {
+  constexpr bool FEW = THREADS == FEW_THREADS;
   __shared__ float scratch[THREADS / 32];
   jb::pdl_launch_dependents();
+  const int n4 = H >> 2;
+  float4 g[FEW ? NORM_CACHE : 1];
+  if (FEW) {
+#pragma unroll
+    for (int c = 0; c < NORM_CACHE; ++c)
+      if (threadIdx.x + c * THREADS < n4) g[FEW ? c : 0] = load4(gamma + 4 * (threadIdx.x + c * THREADS));
+  }
   jb::pdl_wait();
-  clear_slice(clear, clear_n4);
+  if (!FEW) clear_slice(clear, clear_n4);
   const int r = blockIdx.x;
   const size_t src = row_index ? (size_t)row_index[r] : (size_t)r;
   const float* xr = x + src * H;
-  const int n4 = H >> 2;
   float4 cache[NORM_CACHE];
   float ss = 0.0f;
 #pragma unroll
   for (int c = 0; c < NORM_CACHE; ++c) {
     const int i = threadIdx.x + c * THREADS;
-    if (i < n4) {
-      cache[c] = load4(xr + 4 * i);
-      ss += cache[c].x * cache[c].x + cache[c].y * cache[c].y + cache[c].z * cache[c].z + cache[c].w * cache[c].w;
-    }
+    if (i < n4) cache[c] = load4(xr + 4 * i);
+  }
+  if (FEW) clear_slice(clear, clear_n4);         // while the row is on its way
+#pragma unroll
+  for (int c = 0; c < NORM_CACHE; ++c) {
+    const int i = threadIdx.x + c * THREADS;
+    if (i < n4) ss += cache[c].x * cache[c].x + cache[c].y * cache[c].y + cache[c].z * cache[c].z + cache[c].w * cache[c].w;
   }
   for (int i = threadIdx.x + NORM_CACHE * THREADS; i < n4; i += THREADS) {
     const float4 v = load4(xr + 4 * i);
@@ -116,13 +132,13 @@ __global__ void __launch_bounds__(THREADS, NORM_CACHE == 4 ? 1280 / THREADS : 1)
   for (int c = 0; c < NORM_CACHE; ++c) {
     const int i = threadIdx.x + c * THREADS;
     if (i < n4) {
-      const float4 g = load4(gamma + 4 * i), v = cache[c];
-      store4(o + 4 * i, make_float4((v.x / rms) * g.x, (v.y / rms) * g.y, (v.z / rms) * g.z, (v.w / rms) * g.w));
+      const float4 w = FEW ? g[FEW ? c : 0] : load4(gamma + 4 * i), v = cache[c];
+      store4(o + 4 * i, make_float4((v.x / rms) * w.x, (v.y / rms) * w.y, (v.z / rms) * w.z, (v.w / rms) * w.w));
     }
   }
   for (int i = threadIdx.x + NORM_CACHE * THREADS; i < n4; i += THREADS) {
-    const float4 g = load4(gamma + 4 * i), v = load4(xr + 4 * i);
-    store4(o + 4 * i, make_float4((v.x / rms) * g.x, (v.y / rms) * g.y, (v.z / rms) * g.z, (v.w / rms) * g.w));
+    const float4 w = load4(gamma + 4 * i), v = load4(xr + 4 * i);
+    store4(o + 4 * i, make_float4((v.x / rms) * w.x, (v.y / rms) * w.y, (v.z / rms) * w.z, (v.w / rms) * w.w));
   }
 }
 
@@ -236,11 +252,15 @@ JB_EXPORT int jb_rmsnorm(const float* x, const int* row_index, const void* gamma
             "rmsnorm: the buffer to clear is not made of whole 16-byte vectors");
   float4* clear4 = (float4*)clear;
   const size_t clear_n4 = clear ? (size_t)clear_n >> 2 : 0;
-  const bool vec = (H & 3) == 0, narrow = H <= 2048, wide = H > 4096;
-  jb::Launch cfg(dim3(rows), dim3(vec ? (narrow ? 128 : 256) : (H >= 512 ? 256 : 128)), 0, stream);
+  const bool vec = (H & 3) == 0, narrow = H <= 2048, wide = H > 4096, few = vec && rows <= FEW_ROWS && H >= 1024;
+  jb::Launch cfg(dim3(rows), dim3(few ? FEW_THREADS : vec ? (narrow ? 128 : 256) : (H >= 512 ? 256 : 128)), 0, stream);
   cudaError_t e;
 #define JB_LAUNCH_NORM(TG, TO)                                                                                          \
-  e = !vec     ? cudaLaunchKernelEx(&cfg.c, rmsnorm_kernel<TG, TO>, x, row_index, (const TG*)gamma, eps, (TO*)out, H,   \
+  e = few      ? cudaLaunchKernelEx(&cfg.c, narrow ? rmsnorm_vec_kernel<TG, TO, FEW_THREADS, 1>                         \
+                                            : wide ? rmsnorm_vec_kernel<TG, TO, FEW_THREADS, 4>                         \
+                                                   : rmsnorm_vec_kernel<TG, TO, FEW_THREADS, 2>,                        \
+                                    x, row_index, (const TG*)gamma, eps, (TO*)out, H, clear4, clear_n4)                 \
+      : !vec   ? cudaLaunchKernelEx(&cfg.c, rmsnorm_kernel<TG, TO>, x, row_index, (const TG*)gamma, eps, (TO*)out, H,   \
                                     clear4, clear_n4)                                                                   \
       : narrow ? cudaLaunchKernelEx(&cfg.c, rmsnorm_vec_kernel<TG, TO, 128, 4>, x, row_index, (const TG*)gamma, eps,    \
                                     (TO*)out, H, clear4, clear_n4)                                                      \
@@ -549,15 +569,22 @@ __global__ void __launch_bounds__(THREADS) sublayer_norm_add_vec_kernel(float* _
                                                                          TO* __restrict__ x_out, int H,
                                                                          float4* __restrict__ clear, size_t clear_n4,
                                                                          float4* __restrict__ clear2, size_t clear2_n4) {
+  constexpr bool FEW = THREADS == FEW_THREADS;
   __shared__ float scratch[THREADS / 32];
   jb::pdl_launch_dependents();
-  jb::pdl_wait();
-  clear_slice(clear, clear_n4);
-  clear_slice(clear2, clear2_n4);
   const size_t row = (size_t)blockIdx.x * H;
   float* res = residual + row;
   const int n4 = H >> 2;
+  float4 g[FEW ? CACHE : 1], r[FEW ? CACHE : 1];      // few rows: see the norm above
+  if (FEW && y != nullptr) {
+#pragma unroll
+    for (int c = 0; c < CACHE; ++c)
+      if (threadIdx.x + c * THREADS < n4) g[FEW ? c : 0] = load4(gamma + 4 * (threadIdx.x + c * THREADS));
+  }
+  jb::pdl_wait();
   if (y == nullptr) {
+    clear_slice(clear, clear_n4);
+    clear_slice(clear2, clear2_n4);
     for (int i = threadIdx.x; i < n4; i += THREADS) store4(x_out + row + 4 * i, load4(res + 4 * i));
     return;
   }
@@ -569,8 +596,15 @@ __global__ void __launch_bounds__(THREADS) sublayer_norm_add_vec_kernel(float* _
     const int i = threadIdx.x + c * THREADS;
     if (i < n4) {
       cache[c] = load4(yr + 4 * i);
-      ss += cache[c].x * cache[c].x + cache[c].y * cache[c].y + cache[c].z * cache[c].z + cache[c].w * cache[c].w;
+      if (FEW) r[FEW ? c : 0] = load4(res + 4 * i);
     }
+  }
+  clear_slice(clear, clear_n4);
+  clear_slice(clear2, clear2_n4);
+#pragma unroll
+  for (int c = 0; c < CACHE; ++c) {
+    const int i = threadIdx.x + c * THREADS;
+    if (i < n4) ss += cache[c].x * cache[c].x + cache[c].y * cache[c].y + cache[c].z * cache[c].z + cache[c].w * cache[c].w;
   }
   for (int i = threadIdx.x + CACHE * THREADS; i < n4; i += THREADS) {
     const float4 v = load4(yr + 4 * i);
@@ -579,10 +613,9 @@ __global__ void __launch_bounds__(THREADS) sublayer_norm_add_vec_kernel(float* _
   ss = norm_block_sum<THREADS>(ss, scratch);
   const float rms = sqrtf(ss / (float)H + eps);
   const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  auto finish = [&](int i, float4 v) {
-    const float4 g = load4(gamma + 4 * i), r = load4(res + 4 * i);
-    const float4 o = make_float4(r.x + mult * ((v.x / rms) * g.x), r.y + mult * ((v.y / rms) * g.y),
-                                 r.z + mult * ((v.z / rms) * g.z), r.w + mult * ((v.w / rms) * g.w));
+  auto finish = [&](int i, float4 v, float4 w, float4 old) {
+    const float4 o = make_float4(old.x + mult * ((v.x / rms) * w.x), old.y + mult * ((v.y / rms) * w.y),
+                                 old.z + mult * ((v.z / rms) * w.z), old.w + mult * ((v.w / rms) * w.w));
     store4(res + 4 * i, o);
     store4(yr + 4 * i, zero);
     if (x_out != nullptr) store4(x_out + row + 4 * i, o);
@@ -590,9 +623,10 @@ __global__ void __launch_bounds__(THREADS) sublayer_norm_add_vec_kernel(float* _
 #pragma unroll
   for (int c = 0; c < CACHE; ++c) {
     const int i = threadIdx.x + c * THREADS;
-    if (i < n4) finish(i, cache[c]);
+    if (i < n4) finish(i, cache[c], FEW ? g[FEW ? c : 0] : load4(gamma + 4 * i), FEW ? r[FEW ? c : 0] : load4(res + 4 * i));
   }
-  for (int i = threadIdx.x + CACHE * THREADS; i < n4; i += THREADS) finish(i, load4(yr + 4 * i));
+  for (int i = threadIdx.x + CACHE * THREADS; i < n4; i += THREADS)
+    finish(i, load4(yr + 4 * i), load4(gamma + 4 * i), load4(res + 4 * i));
 }
 }  // namespace
 
@@ -608,11 +642,15 @@ JB_EXPORT int jb_sublayer_norm_add(float* y, const void* gamma, int gamma_dtype,
   const size_t clear_n4 = clear ? (size_t)clear_n >> 2 : 0;
   float4* clear24 = (float4*)clear2;
   const size_t clear2_n4 = clear2 ? (size_t)clear2_n >> 2 : 0;
-  const bool vec = (H & 3) == 0, narrow = H <= 2048;
-  jb::Launch cfg(dim3(T), dim3(vec ? (narrow ? 128 : 256) : (H >= 1024 ? 256 : 128)), 0, stream);
+  const bool vec = (H & 3) == 0, narrow = H <= 2048, few = vec && T <= FEW_ROWS && H >= 1024 && H <= 4096;
+  jb::Launch cfg(dim3(T), dim3(few ? FEW_THREADS : vec ? (narrow ? 128 : 256) : (H >= 1024 ? 256 : 128)), 0, stream);
   cudaError_t e;
 #define JB_LAUNCH_SN(TG, TO)                                                                                        \
-  e = !vec     ? cudaLaunchKernelEx(&cfg.c, sublayer_norm_add_kernel<TG, TO>, y, (const TG*)gamma, eps, mult,      \
+  e = few      ? cudaLaunchKernelEx(&cfg.c, narrow ? sublayer_norm_add_vec_kernel<TG, TO, FEW_THREADS, 1>          \
+                                                   : sublayer_norm_add_vec_kernel<TG, TO, FEW_THREADS, 2>,         \
+                                    y, (const TG*)gamma, eps, mult, residual, (TO*)x_out, H, clear4, clear_n4,     \
+                                    clear24, clear2_n4)                                                            \
+      : !vec   ? cudaLaunchKernelEx(&cfg.c, sublayer_norm_add_kernel<TG, TO>, y, (const TG*)gamma, eps, mult,      \
                                     residual, (TO*)x_out, H, clear4, clear_n4, clear24, clear2_n4)                 \
       : narrow ? cudaLaunchKernelEx(&cfg.c, sublayer_norm_add_vec_kernel<TG, TO, 128, 4>, y, (const TG*)gamma, eps, \
                                     mult, residual, (TO*)x_out, H, clear4, clear_n4, clear24, clear2_n4)           \

@@ -29,6 +29,131 @@ __device__ __forceinline__ void clear_slice(float4* __restrict__ p, size_t n4) {
     p[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const bf16* p) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&raw.x), b = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
+  return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
+}
+__device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store4(bf16* p, float4 v) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+  *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+__device__ __forceinline__ void fma4(float4& y, float a, float4 x) {
+  y.x = fmaf(a, x.x, y.x), y.y = fmaf(a, x.y, y.y), y.z = fmaf(a, x.z, y.z), y.w = fmaf(a, x.w, y.w);
+}
+
+// Both reads for rows of whole 16-byte vectors and two to four streams, y null: a read alone.  A thread keeps CACHE
+// float4 of u in registers between the passes, all its loads are in flight at once, and the weight is asked for before
+// the wait for the kernel before (a decode step is bound by that chain: 4 rows 5.6 -> 2.4 us; a prompt by bytes: 2,623 rows of
+// 2 x 2,048 with a rewrite, 129 MB, 46 -> 22 us; before, u went through shared memory and the result left two bytes a
+// thread).
+template <typename TG, typename TO, int THREADS, int CACHE, int S>
+__global__ void __launch_bounds__(THREADS) streams_rows_kernel(float* __restrict__ x, float* __restrict__ y,
+                                                               const int* __restrict__ row_index, const float* __restrict__ M,
+                                                               const float* __restrict__ b, const float* __restrict__ a,
+                                                               const TG* __restrict__ gamma, float eps, TO* __restrict__ out,
+                                                               int H, float* __restrict__ clear, float4* __restrict__ clear2,
+                                                               size_t clear2_n4) {
+  __shared__ float scratch[THREADS / 32];
+  jb::pdl_launch_dependents();
+  const int n4 = H >> 2;
+  float mix[S][S], into[S], an[S];
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    an[s] = a != nullptr ? a[s] : 1.0f;
+    into[s] = y != nullptr ? b[s] : 0.0f;
+#pragma unroll
+    for (int to = 0; to < S; ++to) mix[s][to] = y != nullptr ? M[s * S + to] : 0.0f;
+  }
+  float4 g[CACHE];
+#pragma unroll
+  for (int c = 0; c < CACHE; ++c)
+    if (threadIdx.x + c * THREADS < n4) g[c] = load4(gamma + 4 * (threadIdx.x + c * THREADS));
+  jb::pdl_wait();
+  const size_t r = blockIdx.x, src = row_index != nullptr ? (size_t)row_index[r] : r;
+  float* xr = x + src * S * H;
+  float4 u[CACHE];
+  float ss = 0.0f;
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  float4 old[CACHE][S], yv[CACHE];
+#pragma unroll
+  for (int c = 0; c < CACHE; ++c) {
+    const int i = 4 * (threadIdx.x + c * THREADS);
+    if (i >= H) break;
+#pragma unroll
+    for (int s = 0; s < S; ++s) old[c][s] = load4(xr + (size_t)s * H + i);
+    if (y != nullptr) yv[c] = load4(y + r * H + i);
+  }
+  clear_slice(clear2, clear2_n4);
+#pragma unroll
+  for (int c = 0; c < CACHE; ++c) {
+    const int i = 4 * (threadIdx.x + c * THREADS);
+    if (i >= H) break;
+    u[c] = zero;
+#pragma unroll
+    for (int to = 0; to < S; ++to) {
+      float4 v = old[c][to];
+      if (y != nullptr) {
+        v = zero;
+#pragma unroll
+        for (int s = 0; s < S; ++s) fma4(v, mix[s][to], old[c][s]);
+        fma4(v, into[to], yv[c]);
+        store4(xr + (size_t)to * H + i, v);
+      }
+      fma4(u[c], an[to], v);
+    }
+    ss += u[c].x * u[c].x;
+    ss += u[c].y * u[c].y;
+    ss += u[c].z * u[c].z;
+    ss += u[c].w * u[c].w;
+    if (y != nullptr) store4(y + r * H + i, zero);
+    if (clear != nullptr) store4(clear + r * H + i, zero);
+  }
+  ss = jb::warp_sum(ss);
+  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  ss = 0.0f;
+#pragma unroll
+  for (int w = 0; w < THREADS / 32; ++w) ss += scratch[w];
+  const float rms = sqrtf(ss / (float)H + eps);
+#pragma unroll
+  for (int c = 0; c < CACHE; ++c) {
+    const int i = 4 * (threadIdx.x + c * THREADS);
+    if (i >= H) break;
+    store4(out + r * H + i, make_float4((u[c].x / rms) * g[c].x, (u[c].y / rms) * g[c].y, (u[c].z / rms) * g[c].z,
+                                        (u[c].w / rms) * g[c].w));
+  }
+}
+
+// The kernel above where it fits (`true`: launched, its status in *e): rows of at most 4,096 numbers, 512 threads for few
+// of them, else two float4 a thread (four at most).
+template <typename TG, typename TO>
+bool launch_streams_rows(float* x, float* y, const int* row_index, const float* M, const float* b, const float* a, int S,
+                         const TG* gamma, float eps, TO* out, int rows, int H, float* clear, float4* clear2, size_t clear2_n4,
+                         cudaStream_t stream, cudaError_t* e) {
+  const uintptr_t all = (uintptr_t)x | (uintptr_t)y | (uintptr_t)gamma | (uintptr_t)out | (uintptr_t)clear;
+  if (H % 4 != 0 || H > 4096 || H < 512 || S < 2 || S > 4 || (all & 15) != 0) return false;
+  const bool few = rows <= 296;
+  const int n4 = H >> 2, threads = few ? 512 : 256;
+  jb::Launch cfg(dim3(rows), dim3(threads), 0, stream);
+#define JB_GO(T, C, SS)                                                                                                  \
+  *e = cudaLaunchKernelEx(&cfg.c, streams_rows_kernel<TG, TO, T, C, SS>, x, y, row_index, M, b, a, gamma, eps, out, H,  \
+                          clear, clear2, clear2_n4)
+#define JB_GO_S(T, C)            \
+  if (S == 2) JB_GO(T, C, 2);    \
+  else if (S == 3) JB_GO(T, C, 3); \
+  else JB_GO(T, C, 4)
+  if (few && n4 <= 512) { JB_GO_S(512, 1); }
+  else if (few) { JB_GO_S(512, 2); }
+  else if (n4 <= 512) { JB_GO_S(256, 2); }
+  else { JB_GO_S(256, 4); }
+#undef JB_GO_S
+#undef JB_GO
+  return true;
+}
+
 template <typename TG, typename TO>
 __global__ void streams_rmsnorm_kernel(const float* __restrict__ x, const int* __restrict__ row_index,
                                        const float* __restrict__ a, int S, const TG* __restrict__ gamma, float eps,
@@ -198,6 +323,9 @@ JB_EXPORT int jb_streams_rmsnorm(const float* x, const int* row_index, const flo
   cudaError_t e = cudaSuccess;
 #define JB_LAUNCH_SN(TG, TO)                                                                                    \
   do {                                                                                                          \
+    if (launch_streams_rows<TG, TO>(const_cast<float*>(x), nullptr, row_index, nullptr, nullptr, a, S,          \
+                                    (const TG*)gamma, eps, (TO*)out, rows, H, clear, clear2_4, clear2_n4, stream, &e)) \
+      break;                                                                                                    \
     if (smem > 48 * 1024)                                                                                       \
       cudaFuncSetAttribute(streams_rmsnorm_kernel<TG, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
     e = cudaLaunchKernelEx(&cfg.c, streams_rmsnorm_kernel<TG, TO>, x, row_index, a, S, (const TG*)gamma, eps,   \
@@ -239,6 +367,9 @@ JB_EXPORT int jb_streams_mix_rmsnorm(float* x, float* y, const float* M, const f
   cudaError_t e = cudaSuccess;
 #define JB_LAUNCH_SMN(TG, TO)                                                                                       \
   do {                                                                                                              \
+    if (launch_streams_rows<TG, TO>(x, y, nullptr, M, b, a, S, (const TG*)gamma, eps, (TO*)out, T, H, nullptr,      \
+                                    clear2_4, clear2_n4, stream, &e))                                               \
+      break;                                                                                                        \
     if (smem > 48 * 1024)                                                                                           \
       cudaFuncSetAttribute(streams_mix_rmsnorm_kernel<TG, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
     e = cudaLaunchKernelEx(&cfg.c, streams_mix_rmsnorm_kernel<TG, TO>, x, y, M, b, a, S, (const TG*)gamma, eps,     \

@@ -53,6 +53,125 @@ __device__ __forceinline__ void store_out(bf16* p, const Vec<4>& x) {
   *reinterpret_cast<uint2*>(p) = u;
 }
 
+// One sum over the block with one barrier: `scratch` holds a float a warp, and no two sums of a launch share it.
+template <int THREADS>
+__device__ __forceinline__ float sum_once(float v, float* scratch) {
+  v = jb::warp_sum(v);
+  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
+  __syncthreads();
+  float t = 0.0f;
+#pragma unroll
+  for (int w = 0; w < THREADS / 32; ++w) t += scratch[w];
+  return t;
+}
+
+// The kernel below for rows of whole 16-byte vectors that THREADS threads hold CACHE float4 each of: every row is read
+// once, all its loads in flight together, into registers; the weights are asked for before the wait for the kernel
+// before.  (1,500 rows of 2,048 from two normed branches, 80 MB: 27 -> 11 us, one row 3.6 -> 1.9 us; before, the branches were
+// read twice and the row passed through shared memory four times.)
+template <typename TO, int THREADS, int CACHE>
+__global__ void __launch_bounds__(THREADS) join_norm_rows_kernel(
+    float* __restrict__ stream, float* __restrict__ ya, float* __restrict__ yb, const float* __restrict__ wa,
+    const float* __restrict__ wb, float mult, float mult_b, const float* __restrict__ scale, const float* __restrict__ extra,
+    const float* __restrict__ gamma, float eps, int center, TO* __restrict__ x_out, const int* __restrict__ row_index, int W,
+    float4* __restrict__ clear, size_t clear_n4, float4* __restrict__ clear2, size_t clear2_n4) {
+  __shared__ float scratch[4][THREADS / 32];
+  jb::pdl_launch_dependents();
+  const bool joins = ya != nullptr, branches = yb != nullptr, normed = wa != nullptr;
+  Vec<4> ga[CACHE], gb[CACHE], sc[CACHE], g[CACHE], v[CACHE], a[CACHE], b[CACHE];
+#pragma unroll
+  for (int c = 0; c < CACHE; ++c) {
+    const int i = 4 * ((int)threadIdx.x + c * THREADS);
+    if (i >= W) break;
+    if (normed) ga[c].load(wa + i), gb[c].load(wb + i);
+    if (scale != nullptr) sc[c].load(scale + i);
+    if (x_out != nullptr) g[c].load(gamma + i);
+  }
+  jb::pdl_wait();
+  const size_t src = row_index != nullptr ? (size_t)row_index[blockIdx.x] : (size_t)blockIdx.x, at = src * W;
+#pragma unroll
+  for (int c = 0; c < CACHE; ++c) {
+    const int i = 4 * ((int)threadIdx.x + c * THREADS);
+    if (i >= W) break;
+    v[c].load(stream + at + i);
+    if (joins) a[c].load(ya + at + i);
+    if (branches) b[c].load(yb + at + i);
+  }
+  clear_slice(clear, clear_n4);
+  clear_slice(clear2, clear2_n4);
+  float inv_a = 1.0f, inv_b = 1.0f;
+  if (normed) {
+    float sa = 0.0f, sb = 0.0f;
+#pragma unroll
+    for (int c = 0; c < CACHE; ++c) {
+      if (4 * ((int)threadIdx.x + c * THREADS) >= W) break;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sa = fmaf(a[c].v[j], a[c].v[j], sa), sb = fmaf(b[c].v[j], b[c].v[j], sb);
+    }
+    sa = jb::warp_sum(sa), sb = jb::warp_sum(sb);
+    if ((threadIdx.x & 31) == 0) scratch[0][threadIdx.x >> 5] = sa, scratch[1][threadIdx.x >> 5] = sb;
+    __syncthreads();
+    sa = sb = 0.0f;
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; ++w) sa += scratch[0][w], sb += scratch[1][w];
+    inv_a = 1.0f / sqrtf(sa / (float)W + eps);
+    inv_b = 1.0f / sqrtf(sb / (float)W + eps);
+  }
+  Vec<4> zero;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) zero.v[j] = 0.0f;
+  float sum = 0.0f;
+#pragma unroll
+  for (int c = 0; c < CACHE; ++c) {
+    const int i = 4 * ((int)threadIdx.x + c * THREADS);
+    if (i >= W) break;
+    if (joins) {
+      Vec<4> y = a[c];
+      zero.store(ya + at + i);
+      if (branches) {
+        zero.store(yb + at + i);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          y.v[j] = normed ? mult * ((y.v[j] * inv_a) * ga[c].v[j]) + mult_b * ((b[c].v[j] * inv_b) * gb[c].v[j])
+                          : mult * y.v[j] + mult_b * b[c].v[j];
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[c].v[j] = scale != nullptr ? fmaf(sc[c].v[j], y.v[j], v[c].v[j]) : v[c].v[j] + y.v[j];
+    }
+    if (extra != nullptr) {
+      Vec<4> x;
+      x.load(extra + at + i);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[c].v[j] += x.v[j];
+    }
+    if (joins || extra != nullptr) v[c].store(stream + at + i);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sum += v[c].v[j];
+  }
+  if (x_out == nullptr) return;
+  const float mean = center ? sum_once<THREADS>(sum, scratch[2]) / (float)W : 0.0f;
+  float sq = 0.0f;
+#pragma unroll
+  for (int c = 0; c < CACHE; ++c) {
+    if (4 * ((int)threadIdx.x + c * THREADS) >= W) break;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float d = v[c].v[j] - mean;
+      sq = fmaf(d, d, sq);
+    }
+  }
+  const float inv = 1.0f / sqrtf(sum_once<THREADS>(sq, scratch[3]) / (float)W + eps);
+  TO* x = x_out + (size_t)blockIdx.x * W;
+#pragma unroll
+  for (int c = 0; c < CACHE; ++c) {
+    const int i = 4 * ((int)threadIdx.x + c * THREADS);
+    if (i >= W) break;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[c].v[j] = ((v[c].v[j] - mean) * inv) * g[c].v[j];
+    store_out(x + i, v[c]);
+  }
+}
+
 template <typename TO, int V>
 __global__ void join_norm_kernel(float* __restrict__ stream, float* __restrict__ ya, float* __restrict__ yb,
                                  const float* __restrict__ wa, const float* __restrict__ wb, float mult,
@@ -269,8 +388,28 @@ JB_EXPORT int jb_join_norm(float* stream, float* ya, float* yb, const float* wa,
                         (uintptr_t)scale | (uintptr_t)extra | (uintptr_t)gamma | (uintptr_t)x_out;
   const bool vec = W % 4 == 0 && (all & 15) == 0;
   const int per = vec ? 4 : 1;
+  cudaError_t e = cudaSuccess;
+  if (vec && W >= 512 && W <= 4096) {
+    // few rows, at most two an SM: as many threads as a row has vectors; more: two or four vectors a thread
+    const bool few = T <= 296;
+    jb::Launch rows(dim3(T), dim3(few ? (W <= 2048 ? 512 : 1024) : 256), 0, stream_);
+#define JB_GO(TO, THREADS, C)                                                                                             \
+  e = cudaLaunchKernelEx(&rows.c, join_norm_rows_kernel<TO, THREADS, C>, stream, ya, yb, wa, wb, mult, mult_b, scale, extra, \
+                         gamma, eps, center, (TO*)x_out, row_index, W, (float4*)clear, clear ? (size_t)clear_n >> 2 : (size_t)0, \
+                         (float4*)clear2, clear2 ? (size_t)clear2_n >> 2 : (size_t)0)
+#define JB_GO_W(TO)                           \
+  if (few && W <= 2048) JB_GO(TO, 512, 1);    \
+  else if (few) JB_GO(TO, 1024, 1);           \
+  else if (W <= 2048) JB_GO(TO, 256, 2);      \
+  else JB_GO(TO, 256, 4)
+    if (out_dtype == JB_F32) { JB_GO_W(float); }
+    else if (out_dtype == JB_BF16) { JB_GO_W(bf16); }
+    else return JB_ERR_BAD_DTYPE;
+#undef JB_GO_W
+#undef JB_GO
+    return (int)e;
+  }
   jb::Launch cfg(dim3(T), dim3(W >= 2048 * per ? 512 : W >= 512 * per ? 256 : 128), smem, stream_);
-  cudaError_t e;
 #define JB_LAUNCH_JN(TO, V)                                                                                        \
   do {                                                                                                             \
     if (smem > 48 * 1024) {                                                                                        \
