@@ -336,6 +336,7 @@ __global__ void __launch_bounds__(DN_WARPS * 32) expert_down_kernel(
 // are two steps' fragments under a permutation of the columns that the pairs' fragments share (a dot product does not
 // mind the order), so the weights stream once, 16 bytes a lane, and the pairs' rows come from L2 the same way.
 constexpr int TC_WARPS = 8, NG = 2;
+constexpr int DEEP_BLOCKS = 4 * 148;           // blocks of the second product up to which one wave holds them all: DEEP
 
 __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                           uint32_t b1) {
@@ -366,8 +367,13 @@ __device__ __forceinline__ uint4 stream16(const bf16* p) {
 // MATS = 2: act[pair][f] = gated(Wg_e[f] . x, Wu_e[f] . x), bfloat16, x = h[token of the pair] (times its weight with
 // weigh_input), 16 f a block.  MATS = 1: out[token of the pair][c] += (weight of the pair) Wd_e[c] . act[pair], 16
 // c a block.  K: the rows' width (a multiple of 32), R: the number of rows.
-template <int MATS>
-__global__ void __launch_bounds__(TC_WARPS * 32, 2) expert_tc_kernel(
+// Bound by the weights' bytes, if enough of them are asked for.  DEEP: 256 bytes a lane at a time, two blocks an SM; else 64
+// bytes, and four blocks an SM, whose loads fill each other's waits for sums and stores.  The second product (few columns a
+// warp, then a sum and a store) gains from more blocks as soon as there are several an SM: 16 tokens, two of 8 experts,
+// 4096 -> 2048: 42.5 -> 27 us, 8 tokens 41 -> 32, 2 tokens of 7168 -> 4096: 64 -> 54; with one token (256 blocks) it takes
+// 17.7 us so and 13.5 DEEP.  The first product has enough in flight: 48.8, 46.3 and 82.7 us DEEP, 52.5, 52.9 and 92.3 else.
+template <int MATS, bool DEEP>
+__global__ void __launch_bounds__(TC_WARPS * 32, DEEP ? 2 : 4) expert_tc_kernel(
     const bf16* __restrict__ x, const int* __restrict__ sel_e, const float* __restrict__ sel_w, int top, int n_pairs,
     const bf16* __restrict__ wa, const bf16* __restrict__ wb, bf16* __restrict__ act, float* __restrict__ out, int K, int R,
     jb::Gate gate, int weigh) {
@@ -404,7 +410,7 @@ __global__ void __launch_bounds__(TC_WARPS * 32, 2) expert_tc_kernel(
       for (int m = 0; m < MATS; ++m)
 #pragma unroll
         for (int q = 0; q < NG; ++q) d[m][q][0] = d[m][q][1] = d[m][q][2] = d[m][q][3] = 0.0f;
-      constexpr int AHEAD = MATS == 2 ? 4 : 8;     // blocks of columns a warp has in flight
+      constexpr int AHEAD = DEEP ? 8 / MATS : 2;         // blocks of columns a warp has in flight
       // a warp's blocks come in neighbouring pairs (128 bytes of a row): pair p of the warp is pair p TC_WARPS + warp
       const auto block = [&](int i) { return ((i >> 1) * TC_WARPS + warp) * 2 + (i & 1); };
       for (int i0 = 0; block(i0) < blocks; i0 += AHEAD) {
@@ -668,12 +674,13 @@ JB_EXPORT int jb_experts_few_tokens_tc(const void* h, const int* sel_e, const fl
             "experts: operands must be 16-byte aligned");
   const jb::Gate gate{gate_limit, gate_alpha};
   jb::Launch c1(dim3((F + 15) / 16, E), dim3(TC_WARPS * 32), 0, stream);
-  cudaError_t e = cudaLaunchKernelEx(&c1.c, expert_tc_kernel<2>, (const bf16*)h, sel_e, sel_w, top, pairs,
+  cudaError_t e = cudaLaunchKernelEx(&c1.c, expert_tc_kernel<2, true>, (const bf16*)h, sel_e, sel_w, top, pairs,
                                      (const bf16*)w_gate, (const bf16*)w_up, (bf16*)act, (float*)nullptr, W, F, gate,
                                      weight_on_output ? 0 : 1);
   if (e != cudaSuccess) return (int)e;
+  const bool deep = (long long)(pairs < E ? pairs : E) * ((W + 15) / 16) <= DEEP_BLOCKS;    // at most so many have work
   jb::Launch c2(dim3((W + 15) / 16, E), dim3(TC_WARPS * 32), 0, stream);
-  return (int)cudaLaunchKernelEx(&c2.c, expert_tc_kernel<1>, (const bf16*)act, sel_e, sel_w, top, pairs,
+  return (int)cudaLaunchKernelEx(&c2.c, deep ? expert_tc_kernel<1, true> : expert_tc_kernel<1, false>, (const bf16*)act, sel_e, sel_w, top, pairs,
                                  (const bf16*)w_down, (const bf16*)nullptr, (bf16*)nullptr, out, F, W, gate,
                                  weight_on_output);
 }
