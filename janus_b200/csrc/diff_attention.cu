@@ -189,6 +189,105 @@ __global__ void conv_rope_cache_vec_kernel(const float* __restrict__ proj, int l
   }
 }
 
+// The same for prompts with up to four taps: a thread owns four channels (both halves of four rotated pairs) and walks
+// WALK_TOKENS tokens, its last three inputs in registers, so an input is read once instead of `taps` times, and its taps
+// once a walk; WALK_AHEAD tokens' inputs and places are in flight before the first is used.  (2,623 tokens x 3,072
+// channels, 59 MB: 87 us a token a thread, 37 so.)
+constexpr int WALK_TOKENS = 16, WALK_AHEAD = 4, WALK_TAPS = 4;
+
+template <typename TC>
+__global__ void __launch_bounds__(128) conv_rope_cache_walk_kernel(
+    const float* __restrict__ proj, int ld, const float* __restrict__ conv_w, int taps, const float* __restrict__ conv_state,
+    const int* __restrict__ token_seq, const int* __restrict__ q_start, const int* __restrict__ seq_slot,
+    const int* __restrict__ positions, const float* __restrict__ cos_sin, int rot, float* __restrict__ q_out,
+    const int* __restrict__ dest, TC* __restrict__ k_cache, TC* __restrict__ v_cache, int T, int H, int G, int d, int e,
+    int page_size) {
+  jb::pdl_launch_dependents();
+  const int Cq = H * 2 * d, Ck = G * 2 * d, Cv = G * e, C = Cq + Ck + Cv;
+  const int c = 4 * (blockIdx.y * blockDim.x + threadIdx.x);
+  if (c >= C) return;
+  const int half = rot >> 1, i = c < Cq ? c % d : c < Cq + Ck ? (c - Cq) % d : rot;
+  const bool turns = cos_sin != nullptr && i < rot;
+  if (turns && i >= half) return;                        // written with the pair's first member
+  const int parts = turns ? 2 : 1;
+  float w[2][WALK_TAPS][4];                              // [half][tokens back][channel]; taps that are not there weigh nothing
+#pragma unroll
+  for (int p = 0; p < 2; ++p)
+#pragma unroll
+    for (int b = 0; b < WALK_TAPS; ++b)
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        w[p][b][x] = p < parts && b < taps ? conv_w[(size_t)(c + p * half + x) * taps + taps - 1 - b] : 0.0f;
+  jb::pdl_wait();
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  float4 win[2][WALK_TAPS - 1];                          // win[.][b]: the input b + 1 tokens back
+  const int t0 = blockIdx.x * WALK_TOKENS, t1 = min(T, t0 + WALK_TOKENS);
+  const auto put = [&](int c0, float4 y, int t, size_t page, int off) {
+    if (c0 < Cq) {
+      *reinterpret_cast<float4*>(q_out + (size_t)t * Cq + c0) = y;
+    } else if (c0 < Cq + Ck) {
+      const int kc = c0 - Cq;
+      store4c<TC>(k_cache + ((page * 2 * G + kc / d) * page_size + off) * d + kc % d, y);
+    } else {
+      const int vc = c0 - Cq - Ck;
+      store4c<TC>(v_cache + ((page * G + vc / e) * page_size + off) * e + vc % e, y);
+    }
+  };
+  int before = -1;
+  for (int tb = t0; tb < t1; tb += WALK_AHEAD) {
+    float4 u[WALK_AHEAD][2];
+    int seqs[WALK_AHEAD], pos[WALK_AHEAD], dst[WALK_AHEAD];
+#pragma unroll
+    for (int k = 0; k < WALK_AHEAD; ++k) {
+      const int t = min(tb + k, t1 - 1);
+      seqs[k] = token_seq[t], pos[k] = turns ? positions[t] : 0, dst[k] = dest[t];
+#pragma unroll
+      for (int p = 0; p < 2; ++p)
+        u[k][p] = p < parts ? *reinterpret_cast<const float4*>(proj + (size_t)t * ld + c + p * half) : zero;
+    }
+#pragma unroll
+    for (int k = 0; k < WALK_AHEAD; ++k) {
+      const int t = tb + k;
+      if (t >= t1) break;
+      if (seqs[k] != before) {                           // the walk's first token, or a sequence's: fill the windows
+        before = seqs[k];
+        const int local = t - q_start[before];
+        const float* st = conv_state + (size_t)seq_slot[before] * (taps - 1) * C;
+#pragma unroll
+        for (int b = 0; b < WALK_TAPS - 1; ++b)
+#pragma unroll
+          for (int p = 0; p < 2; ++p)
+            win[p][b] = p >= parts || b + 1 >= taps ? zero
+                        : b + 1 <= local ? *reinterpret_cast<const float4*>(proj + (size_t)(t - b - 1) * ld + c + p * half)
+                                         : *reinterpret_cast<const float4*>(st + (size_t)(taps - 1 - (b + 1 - local)) * C + c + p * half);
+      }
+      float4 y[2] = {zero, zero};
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        if (p >= parts) break;
+#pragma unroll
+        for (int b = WALK_TAPS - 1; b >= 0; --b) {       // the oldest first
+          const float4 v = b > 0 ? win[p][b - 1] : u[k][p];
+          y[p].x = fmaf(w[p][b][0], v.x, y[p].x), y[p].y = fmaf(w[p][b][1], v.y, y[p].y);
+          y[p].z = fmaf(w[p][b][2], v.z, y[p].z), y[p].w = fmaf(w[p][b][3], v.w, y[p].w);
+        }
+        win[p][2] = win[p][1], win[p][1] = win[p][0], win[p][0] = u[k][p];
+      }
+      const size_t page = (size_t)(dst[k] / page_size);
+      const int off = dst[k] % page_size;
+      if (!turns) {
+        put(c, y[0], t, page, off);
+        continue;
+      }
+      const float* cs = cos_sin + (size_t)pos[k] * half * 2 + 2 * i;
+      const float4 a0 = *reinterpret_cast<const float4*>(cs), a1 = *reinterpret_cast<const float4*>(cs + 4);
+      const float4 a = y[0], b = y[1];
+      put(c, make_float4(a.x * a0.x - b.x * a0.y, a.y * a0.z - b.y * a0.w, a.z * a1.x - b.z * a1.y, a.w * a1.z - b.w * a1.w), t, page, off);
+      put(c + half, make_float4(b.x * a0.x + a.x * a0.y, b.y * a0.z + a.y * a0.w, b.z * a1.x + a.z * a1.y, b.w * a1.z + a.w * a1.w), t, page, off);
+    }
+  }
+}
+
 __global__ void conv_state_update_kernel(const float* __restrict__ proj, int ld, float* __restrict__ conv_state, int taps,
                                          const int* __restrict__ q_start, const int* __restrict__ seq_slot, int C) {
   jb::pdl_launch_dependents();
@@ -310,6 +409,166 @@ template <int EJ> struct Columns<bf16, EJ> {
 };
 
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// Few (token, query head) pairs over bfloat16 pages: single-token steps.  A block a pair; a warp takes a chunk of 32 keys
+// at a time, all of whose bytes are asked for at once: the value rows (neighbours in a page) by asynchronous copies into
+// shared memory, its lanes' key rows into registers, eight or sixteen 16-byte loads each, before the first of them is
+// used.  The warps' parts meet side by side.  What bounds it is the chain of memory latencies of one chunk, cold after a
+// step's weights have passed through L2 (4 sequences x 16 heads over 516 keys: 26.6 -> 14.9 us; before, a lane's value rows came
+// eight at a time after the scores, one warp added up sixteen parts one after another, and two warps had a second chunk).
+constexpr int STAGED_PAIRS = 4096;         // more of them than the SMs hold at once have other blocks' loads to wait under
+constexpr int STAGED_WARPS = 20;           // the chunks of a window of 512 keys and of kept keys that it has left behind
+
+template <int EJ>
+__global__ void __launch_bounds__(STAGED_WARPS * 32) diff_attention_staged_kernel(
+    const float* __restrict__ q, const bf16* __restrict__ k_cache, const bf16* __restrict__ v_cache, bf16* __restrict__ out,
+    const int* __restrict__ block_table, const int* __restrict__ token_seq, const int* __restrict__ positions, int H, int G,
+    int d, int e, int page_size, int max_pages, int window, int keep_first, float scale, float lambda, float eps,
+    float out_scale) {
+  constexpr int PART = 64 * EJ;
+  extern __shared__ __align__(16) unsigned char staged_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  bf16* vs = reinterpret_cast<bf16*>(staged_smem) + (size_t)warp * 32 * e;     // this warp's 32 value rows
+  float* qw = reinterpret_cast<float*>(staged_smem + (size_t)warps * 64 * e);  // q [2 d], parts [warp][2][32 EJ], then m, l
+  float* parts = qw + 2 * d;
+  float* ml = parts + warps * PART;                                            // [4][STAGED_WARPS]: m1, l1, m2, l2
+  jb::pdl_launch_dependents();
+  jb::pdl_wait();
+  const int t = blockIdx.x / H, h = blockIdx.x % H, g = h / (H / G);
+  const int pos = positions[t];
+  const int* pages = block_table + (size_t)token_seq[t] * max_pages;
+  const int kstart = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+  for (int i = threadIdx.x; i < 2 * d; i += blockDim.x) qw[i] = q[((size_t)t * H + h) * 2 * d + i];
+
+  // the chunks a query sees, numbered: the kept keys' that the window has left behind, then the window's
+  const int window_chunk = kstart / 32, kept = min(keep_first, kstart);
+  const int kept_chunks = min((kept + 31) / 32, window_chunk), chunks = kept_chunks + pos / 32 - window_chunk + 1;
+  const auto begin_of = [&](int n) { return 32 * (n < kept_chunks ? n : window_chunk + n - kept_chunks); };
+  const auto stage = [&](int c0) {
+    const bf16* src = v_cache + (((size_t)pages[c0 / page_size] * G + g) * page_size + c0 % page_size) * e;
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(vs);
+    for (int i = lane; i < 4 * e; i += 32)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * i), "l"(src + 8 * i));
+    asm volatile("cp.async.commit_group;");
+  };
+  if (warp < chunks) stage(begin_of(warp));
+  __syncthreads();                                                             // q is there
+
+  float m1 = -CUDART_INF_F, l1 = 0.0f, m2 = -CUDART_INF_F, l2 = 0.0f;
+  float a1[EJ], a2[EJ];
+#pragma unroll
+  for (int j = 0; j < EJ; ++j) a1[j] = a2[j] = 0.0f;
+  for (int n = warp; n < chunks; n += warps) {
+    const int c0 = begin_of(n), key = c0 + lane;
+    const bool valid = key <= pos && (key >= kstart || key < keep_first);
+    float s1 = -CUDART_INF_F, s2 = -CUDART_INF_F;
+    if (valid) {
+      const bf16* k1 = k_cache + (((size_t)pages[c0 / page_size] * 2 * G + 2 * g) * page_size + c0 % page_size + lane) * d;
+      const bf16* k2 = k1 + (size_t)page_size * d;
+      float d1 = 0.0f, d2 = 0.0f;
+#pragma unroll 1
+      for (int i0 = 0; i0 < d; i0 += 64) {                                     // as many loads in flight as d allows, 16 at most
+        uint4 ka[8], kb[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (i0 + 8 * u < d) {
+            ka[u] = *reinterpret_cast<const uint4*>(k1 + i0 + 8 * u);
+            kb[u] = *reinterpret_cast<const uint4*>(k2 + i0 + 8 * u);
+          }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          if (i0 + 8 * u >= d) break;
+          const __nv_bfloat162* ap = reinterpret_cast<const __nv_bfloat162*>(&ka[u]);
+          const __nv_bfloat162* bp = reinterpret_cast<const __nv_bfloat162*>(&kb[u]);
+          const float* qa = qw + i0 + 8 * u;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 af = __bfloat1622float2(ap[j]), bf = __bfloat1622float2(bp[j]);
+            d1 = fmaf(qa[2 * j], af.x, d1);
+            d1 = fmaf(qa[2 * j + 1], af.y, d1);
+            d2 = fmaf(qa[d + 2 * j], bf.x, d2);
+            d2 = fmaf(qa[d + 2 * j + 1], bf.y, d2);
+          }
+        }
+      }
+      s1 = d1 * scale;
+      s2 = d2 * scale;
+    }
+    const float n1 = fmaxf(m1, jb::warp_max(s1)), n2 = fmaxf(m2, jb::warp_max(s2));
+    const unsigned seen = __ballot_sync(0xffffffffu, valid);
+    // exp(-inf) = 0 before the first key; scores of -inf alone leave everything as it was
+    const float p1 = valid && n1 != -CUDART_INF_F ? expf(s1 - n1) : 0.0f, p2 = valid && n2 != -CUDART_INF_F ? expf(s2 - n2) : 0.0f;
+    const float c1 = n1 != -CUDART_INF_F ? expf(m1 - n1) : 1.0f, c2 = n2 != -CUDART_INF_F ? expf(m2 - n2) : 1.0f;
+    l1 = l1 * c1 + jb::warp_sum(p1);
+    l2 = l2 * c2 + jb::warp_sum(p2);
+    m1 = n1;
+    m2 = n2;
+#pragma unroll
+    for (int j = 0; j < EJ; ++j) {
+      a1[j] *= c1;
+      a2[j] *= c2;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+    const int lo = __ffs(seen) - 1, hi = 32 - __clz(seen);                     // every chunk has a key that is seen
+#pragma unroll 8
+    for (int kk = lo; kk < hi; ++kk) {
+      const float w1 = __shfl_sync(0xffffffffu, p1, kk), w2 = __shfl_sync(0xffffffffu, p2, kk);
+      if (!((seen >> kk) & 1u)) continue;                                      // uniform across the warp
+      float v[EJ];
+      Columns<bf16, EJ>::load(vs + (size_t)kk * e, EJ * lane, e, true, v);
+#pragma unroll
+      for (int j = 0; j < EJ; ++j) {
+        a1[j] = fmaf(w1, v[j], a1[j]);
+        a2[j] = fmaf(w2, v[j], a2[j]);
+      }
+    }
+    __syncwarp();                                                              // the rows have been read
+    if (n + warps < chunks) stage(begin_of(n + warps));
+  }
+
+  // the parts meet: lane w of every warp knows warp w's weights, in warp 0 a lane adds up its columns in warp order
+#pragma unroll
+  for (int j = 0; j < EJ; ++j) {
+    parts[warp * PART + 32 * j + lane] = a1[j];
+    parts[warp * PART + 32 * EJ + 32 * j + lane] = a2[j];
+  }
+  if (lane == 0) ml[warp] = m1, ml[STAGED_WARPS + warp] = l1, ml[2 * STAGED_WARPS + warp] = m2, ml[3 * STAGED_WARPS + warp] = l2;
+  __syncthreads();
+  if (warp != 0) return;
+  const bool there = lane < warps && lane < chunks;                            // a warp without a chunk weighs nothing
+  m1 = there ? ml[lane] : -CUDART_INF_F;
+  m2 = there ? ml[2 * STAGED_WARPS + lane] : -CUDART_INF_F;
+  const float top1 = jb::warp_max(m1), top2 = jb::warp_max(m2);
+  const float f1 = there && m1 != -CUDART_INF_F ? expf(m1 - top1) : 0.0f, f2 = there && m2 != -CUDART_INF_F ? expf(m2 - top2) : 0.0f;
+  l1 = jb::warp_sum(there ? ml[STAGED_WARPS + lane] * f1 : 0.0f);
+  l2 = jb::warp_sum(there ? ml[3 * STAGED_WARPS + lane] * f2 : 0.0f);
+#pragma unroll
+  for (int j = 0; j < EJ; ++j) a1[j] = a2[j] = 0.0f;
+#pragma unroll 4
+  for (int w = 0; w < min(warps, chunks); ++w) {
+    const float w1 = __shfl_sync(0xffffffffu, f1, w), w2 = __shfl_sync(0xffffffffu, f2, w);
+#pragma unroll
+    for (int j = 0; j < EJ; ++j) {
+      a1[j] = fmaf(parts[w * PART + 32 * j + lane], w1, a1[j]);
+      a2[j] = fmaf(parts[w * PART + 32 * EJ + 32 * j + lane], w2, a2[j]);
+    }
+  }
+  float o[EJ], ss = 0.0f;
+#pragma unroll
+  for (int j = 0; j < EJ; ++j) {
+    o[j] = a1[j] / l1 - lambda * (a2[j] / l2);
+    if (EJ * lane + j < e) ss += o[j] * o[j];
+  }
+  ss = jb::warp_sum(ss);
+  const float rms = sqrtf(ss / (float)e + eps);
+  bf16* orow = out + ((size_t)t * H + h) * e;
+#pragma unroll
+  for (int j = 0; j < EJ; ++j) {
+    const int c = EJ * lane + j;
+    if (c < e) orow[c] = __float2bfloat16_rn((o[j] / rms) * out_scale);
+  }
+}
 
 // One block per (token, query head); its warps take the chunks of 32 keys in turn (chunk n goes to warp
 // n mod warps) and their partial results (maximum, sum, weighted values of each map) meet in warp order.
@@ -495,6 +754,17 @@ JB_EXPORT int jb_conv_rope_cache(const float* proj, int ld, const float* conv_w,
   const bool vec = d % 4 == 0 && e % 4 == 0 && rot % 8 == 0 && ld % 4 == 0 &&
                    (((uintptr_t)proj | (uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)conv_state |
                      (uintptr_t)cos_sin) & 15) == 0;
+  if (vec && conv_w != nullptr && taps >= 2 && taps <= WALK_TAPS && !update_state && T >= 4 * WALK_TOKENS) {
+    jb::Launch wcfg(dim3((T + WALK_TOKENS - 1) / WALK_TOKENS, (C / 4 + 127) / 128), dim3(128), 0, stream);
+    if (cache_dtype == JB_F32)
+      return (int)cudaLaunchKernelEx(&wcfg.c, conv_rope_cache_walk_kernel<float>, proj, ld, conv_w, taps, (const float*)conv_state,
+                                     token_seq, q_start, seq_slot, positions, cos_sin, rot, q_out, dest, (float*)k_cache,
+                                     (float*)v_cache, T, H, G, d, e, page_size);
+    if (cache_dtype == JB_BF16)
+      return (int)cudaLaunchKernelEx(&wcfg.c, conv_rope_cache_walk_kernel<bf16>, proj, ld, conv_w, taps, (const float*)conv_state,
+                                     token_seq, q_start, seq_slot, positions, cos_sin, rot, q_out, dest, (bf16*)k_cache,
+                                     (bf16*)v_cache, T, H, G, d, e, page_size);
+  }
   if (vec) {
     const int vthreads = C / 4 >= 512 ? 256 : 128;
     jb::Launch vcfg(dim3(T, (C / 4 + vthreads - 1) / vthreads), dim3(vthreads), 0, stream);
@@ -557,8 +827,24 @@ JB_EXPORT int jb_diff_attention(const float* q, const void* k_cache, const void*
     forced = env ? atoi(env) : 0;
   }
   if (forced > 0) warps = forced < max_warps(EJ_) ? forced : max_warps(EJ_);
-  const size_t smem = (size_t)(2 * d + warps * (4 + 64 * EJ_)) * sizeof(float);
   const bool f32c = cache_dtype == JB_F32;
+  if (!f32c && out_dtype == JB_BF16 && forced == 0 && (long long)T * H <= STAGED_PAIRS && e <= 128 && e % 8 == 0 && d % 8 == 0 &&
+      page_size % 32 == 0 && (((uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0) {
+    const int chunks = (int)((keys + 62) / 32 + (window > 0 && keep_first > 0 ? 1 : 0));     // of a query at most
+    int w = warps;
+    if (w == max_warps(4) && (long long)T * H <= sms) w = STAGED_WARPS;        // one block an SM has room for all of them
+    if (w > STAGED_WARPS) w = STAGED_WARPS;
+    if (w > chunks) w = chunks;
+    const size_t bytes = (size_t)w * 64 * e + (size_t)(2 * d + w * 64 * EJ_ + 4 * STAGED_WARPS) * sizeof(float);
+    auto* fn = e <= 64 ? diff_attention_staged_kernel<2> : diff_attention_staged_kernel<4>;
+    cudaError_t se = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (se != cudaSuccess) return (int)se;
+    jb::Launch scfg(dim3((unsigned)(T * H)), dim3(w * 32), bytes, stream);
+    return (int)cudaLaunchKernelEx(&scfg.c, fn, q, (const bf16*)k_cache, (const bf16*)v_cache, (bf16*)out, block_table,
+                                   token_seq, positions, H, G, d, e, page_size, max_pages, window, keep_first, scale, lambda,
+                                   eps, out_scale);
+  }
+  const size_t smem = (size_t)(2 * d + warps * (4 + 64 * EJ_)) * sizeof(float);
   // bit 0: key rows in 16-byte loads; bit 1: the value cache is aligned for a lane's columns in one load; bit 2: prefetch
   static int prefetch_on = -1;             // JANUS_DIFF_PREFETCH=0: no prefetch of the rows a warp reads next (experiments)
   if (prefetch_on < 0) {

@@ -62,6 +62,88 @@ def picked(cache, dest):
     return cache[dest.long() // PAGE, :, dest.long() % PAGE]
 
 
+@pytest.mark.parametrize("H, G, d, e", [(4, 1, 64, 128), (4, 2, 16, 64), (2, 2, 72, 72), (3, 1, 128, 8)])
+@pytest.mark.parametrize("window, kept", [(0, 0), (40, 0), (512, 4), (512, 70), (1, 33)])
+@pytest.mark.parametrize("copies", [1, 60])
+def test_diff_attention_single_tokens(ops, H, G, d, e, window, kept, copies):
+    """One query of every sequence over bfloat16 pages, lengths at the edges of chunks (32) and pages (64), windows that
+    start inside a chunk, kept keys in their own chunk or in the window's, few pairs and many (fewer warps a pair)."""
+    lens = [1, 32, 33, 64, 97, 600, 745] * copies
+    B, n_pages = len(lens), sum((n + PAGE - 1) // PAGE for n in lens)
+    g = torch.Generator().manual_seed(d + e)
+    kc = torch.randn(n_pages, 2 * G, PAGE, d, generator=g).to(torch.bfloat16).to(DEV)
+    vc = torch.randn(n_pages, G, PAGE, e, generator=g).to(torch.bfloat16).to(DEV)
+    order, at = torch.randperm(n_pages, generator=g), 0
+    table = torch.full((B, 12), -1, dtype=torch.int32)
+    for b, n in enumerate(lens):
+        need = (n + PAGE - 1) // PAGE
+        table[b, :need] = order[at:at + need].int()
+        at += need
+    table = table.to(DEV)
+    q = rnd(B, H * 2 * d)
+    pos, seq = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=DEV), torch.arange(B, dtype=torch.int32, device=DEV)
+    out = torch.empty(B, H * e, dtype=torch.bfloat16, device=DEV)
+    lam, eps, scale = 0.4, 1e-5, d ** -0.5
+    ops.diff_attention(q, kc, vc, out, table, seq, pos, H, G, d, e, PAGE, window, kept, scale, lam, eps, 0.5)
+    for b in range(7):
+        n = lens[b]
+        pages = table[b, :(n + PAGE - 1) // PAGE].long()
+        k = kc[pages].double().permute(1, 0, 2, 3).reshape(G, 2, -1, d)[:, :, :n]
+        v = vc[pages].double().permute(1, 0, 2, 3).reshape(G, -1, e)[:, :n]
+        j = torch.arange(n, device=DEV)
+        seen = (n - 1 - j < window) | (j < kept) if window else torch.ones(n, dtype=torch.bool, device=DEV)
+        qq = q[b].double().view(H, 2, d)
+        s = torch.einsum("hmd,hmnd->hmn", qq, k.repeat_interleave(H // G, 0)) * scale
+        p = torch.softmax(s.masked_fill(~seen, -math.inf), -1)
+        maps = torch.einsum("hmn,hne->hme", p, v.repeat_interleave(H // G, 0))
+        want = unit(maps[:, 0] - lam * maps[:, 1], eps) * 0.5
+        # scores of size one from float32 sums of up to 128 products, then bfloat16; a difference that nearly cancels is
+        # divided by its own size, hence the room of a factor of four
+        assert worst(out[b].view(H, e), want) <= 4 * TOL[torch.bfloat16]
+    for b in range(7, B):
+        if b % 7 == 3:
+            assert bool(torch.isfinite(out[b].float()).all())
+
+
+def conv_reference(x, w, lens, states):
+    """x [T, C] float64 of sequences of the given lengths, w [C, taps], states [n, taps - 1, C]: the causal convolution."""
+    taps, out, at = w.shape[1], [], 0
+    for n, st in zip(lens, states):
+        full = torch.cat([st, x[at:at + n]])
+        out.append(sum(full[j:j + n] * w[:, j] for j in range(taps)))
+        at += n
+    return torch.cat(out)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("taps", [0, 2, 3, 4, 5])
+@pytest.mark.parametrize("H, G, d, e, rot", [(4, 2, 64, 128, 32), (2, 1, 16, 12, 16), (3, 3, 20, 8, 0), (2, 2, 12, 20, 8)])
+@pytest.mark.parametrize("lens", [[63], [1, 15, 2, 47, 16], [130, 1, 1, 1, 17]])
+def test_conv_rope_cache_prompts(ops, H, G, d, e, rot, taps, lens, dtype):
+    """Prompts of 64 tokens and more walk with their inputs in registers where there are two to four taps, others take a
+    token a thread; sequences that begin and end inside a walk, states that are not zero."""
+    T, n, C = sum(lens), len(lens), H * 2 * d + G * 2 * d + G * e
+    proj, w = rnd(T, C), rnd(C, max(taps, 1), seed=1) if taps else None
+    state = rnd(n + 1, max(taps - 1, 1), C, seed=3)
+    slots = torch.arange(n, 0, -1, dtype=torch.int32, device=DEV)
+    seq = torch.repeat_interleave(torch.arange(n), torch.tensor(lens)).int().to(DEV)
+    q_start = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    pos = torch.cat([torch.arange(k) + 3 for k in lens]).int().to(DEV)
+    table = table_of(200, rot // 2) if rot else None
+    k_cache, dest = pages_of(T, 2 * G, d, dtype)
+    v_cache, q = torch.zeros(k_cache.shape[0], G, PAGE, e, dtype=dtype, device=DEV), torch.empty(T, H * 2 * d, device=DEV)
+    ops.conv_rope_cache(proj, w, taps if taps else 1, state if taps else None, seq, q_start, slots, pos, table, rot, q, dest, k_cache,
+                        v_cache, H, G, d, e, PAGE)
+    x = proj.double()
+    if taps:
+        x = conv_reference(x, w.double(), lens, [state[s].double() for s in slots.tolist()])
+    want_q = turned(x[:, :H * 2 * d].view(T, 2 * H, d), pos, table, rot)
+    want_k = turned(x[:, H * 2 * d:(H + G) * 2 * d].view(T, 2 * G, d), pos, table, rot)
+    assert worst(q.view(T, 2 * H, d), want_q) <= TOL[torch.float32]
+    assert worst(picked(k_cache, dest), want_k) <= TOL[dtype]
+    assert worst(picked(v_cache, dest), x[:, (H + G) * 2 * d:].view(T, G, e)) <= TOL[dtype]
+
+
 @pytest.mark.parametrize("T, W, E", [(16, 1184, 8), (16, 1200, 8), (1, 2048, 4), (3, 4736, 4)])
 def test_expert_down_blocks(ops, T, W, E):
     """The second product of few pairs' experts on both sides of the line between few blocks and many."""
