@@ -62,6 +62,74 @@ def picked(cache, dest):
     return cache[dest.long() // PAGE, :, dest.long() % PAGE]
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("H, G, d, rot", [(4, 2, 16, 8), (32, 8, 128, 64), (3, 1, 20, 0), (16, 4, 128, 128), (5, 5, 132, 8),
+                                          (8, 2, 36, 12), (40, 8, 256, 128)])
+@pytest.mark.parametrize("off", [0, 1])
+def test_qk_norm_rope_cache(ops, H, G, d, rot, dtype, off):
+    T, eps = 5, 1e-5
+    wide = rnd(T, (H + G) * d + 4 + off)                     # off = 1: rows that are no whole vectors take the general kernel
+    bq, bk, wq, wk = rnd(H * d, seed=1), rnd(G * d, seed=2), rnd(H * d, seed=3), rnd(G * d, seed=4)
+    pos, table = ints(0, 7, 3, 90, 41), table_of(100, max(rot // 2, 1)) if rot else None
+    k_cache, dest = pages_of(T, G, d, dtype)
+    v_cache, q = torch.zeros_like(k_cache), torch.empty(T, H * d, dtype=dtype, device=DEV)
+    ops.qk_norm_rope_cache(wide, bq, bk, wq, wk, eps, table, rot, pos, q, dest, k_cache, v_cache, H, G, d, PAGE)
+    x = wide.double()
+    qd, kd = x[:, :H * d] + bq.double(), x[:, H * d:(H + G) * d] + bk.double()
+    want_q = turned((unit(qd, eps) * wq.double()).view(T, H, d), pos, table, rot)
+    want_k = turned((unit(kd, eps) * wk.double()).view(T, G, d), pos, table, rot)
+    assert worst(q.view(T, H, d), want_q) <= TOL[dtype]
+    assert worst(picked(k_cache, dest), want_k) <= TOL[dtype]
+    assert worst(picked(v_cache, dest), kd.view(T, G, d)) <= TOL[dtype]
+    assert int((k_cache != 0).any(-1).sum()) == T * G
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T", [3, 300])
+@pytest.mark.parametrize("H, G, d, e, dp, rot", [(16, 4, 128, 128, 128, 64), (4, 2, 20, 12, 24, 16), (3, 3, 128, 132, 128, 128),
+                                                 (33, 1, 64, 64, 64, 0), (4, 1, 128, 64, 136, 8), (2, 2, 132, 64, 136, 8),
+                                                 (4, 2, 12, 12, 16, 12)])
+@pytest.mark.parametrize("form", ["weights", "unit", "mixed"])
+def test_head_norm_rope_cache(ops, T, H, G, d, e, dp, rot, form, dtype):
+    eps, ep = 1e-5, (e + 7) // 8 * 8
+    proj = rnd(T, (H + G) * d + G * e + 4)
+    pos = torch.randint(0, 500, (T,), generator=torch.Generator().manual_seed(T), dtype=torch.int32).to(DEV)
+    table = table_of(500, max(rot // 2, 1)) if rot else None
+    wq, wk = (rnd(d, seed=1), rnd(d, seed=2)) if form != "unit" else (None, None)
+    first = rnd(T, G * e, seed=3) if form == "mixed" else None
+    k_cache, dest = pages_of(T, G, dp, dtype)
+    v_cache, q = torch.zeros(k_cache.shape[0], G, PAGE, ep, dtype=dtype, device=DEV), torch.full((T, H * dp), 9.0, dtype=dtype, device=DEV)
+    every = 0 if form == "mixed" else 128
+    ops.head_norm_rope_cache(proj, wq, wk, eps, table, rot, pos, q, dest, k_cache, v_cache, H, G, d, e, dp, PAGE,
+                             unit_norm=form == "unit", temp_coef=0.1, temp_every=every, stored_vdim=ep, first=first, mix=0.3)
+    x = proj.double()
+    qd, kd = unit(x[:, :H * d].view(T, H, d), eps), unit(x[:, H * d:(H + G) * d].view(T, G, d), eps)
+    if wq is not None:
+        qd, kd = qd * wq.double(), kd * wk.double()
+    vd = x[:, (H + G) * d:(H + G) * d + G * e].view(T, G, e)
+    if first is not None:
+        vd = 0.7 * vd + 0.3 * first.double().view(T, G, e)
+    qd, kd = turned(qd, pos, table, rot), turned(kd, pos, table, rot)
+    if every:
+        qd = qd * (1.0 + 0.1 * torch.log(((pos.double() + 1) / every).floor() + 1.0))[:, None, None]
+    got = q.view(T, H, dp)
+    assert worst(got[..., :d], qd) <= TOL[dtype] and not bool(got[..., d:].any())
+    assert worst(picked(k_cache, dest)[..., :d], kd) <= TOL[dtype]
+    assert worst(picked(v_cache, dest)[..., :e], vd) <= TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T, Q, r, rp", [(1, 8192, 256, 256), (5, 4096, 20, 24), (3, 4100, 1024, 1024), (2, 64, 1028, 1028),
+                                         (2, 61, 16, 16)])
+def test_latent_prep(ops, T, Q, r, rp, dtype):
+    proj, w, eps = rnd(T, Q + r), rnd(r, seed=1), 1e-5
+    cache, dest = pages_of(T, 1, rp, dtype)
+    q = torch.empty(T, Q, dtype=dtype, device=DEV)
+    ops.latent_prep(proj, Q, r, w, eps, q, dest, cache, stored_rank=rp)
+    assert torch.equal(q, proj[:, :Q].to(dtype))
+    assert worst(picked(cache, dest)[:, 0, :r], unit(proj[:, Q:].double(), eps) * w.double()) <= TOL[dtype]
+
+
 @pytest.mark.parametrize("H, G, d, e", [(4, 1, 64, 128), (4, 2, 16, 64), (2, 2, 72, 72), (3, 1, 128, 8)])
 @pytest.mark.parametrize("window, kept", [(0, 0), (40, 0), (512, 4), (512, 70), (1, 33)])
 @pytest.mark.parametrize("copies", [1, 60])
