@@ -29,7 +29,7 @@
 #include <math_constants.h>
 #include <stdio.h>
 
-#include "common.cuh"
+#include "state_step.cuh"
 
 namespace {
 
@@ -53,15 +53,28 @@ __global__ void __launch_bounds__(128) gla_decay_kernel(const float* __restrict_
                                                         float inv_tau, float* __restrict__ alpha, int C, int T) {
   extern __shared__ __align__(16) float low_s[];               // [TB][rank4]
   jb::pdl_launch_dependents();
-  jb::pdl_wait();
   const int rank4 = (rank + 3) & ~3;
   const int t0 = blockIdx.x * TB, n = min(TB, T - t0);
+  // STEP rows of the matrix are in flight at once, the first ones before the wait (four at a time, a step of 8 tokens x
+  // 2,048 channels of rank 64 took 13.4 us: sixteen rounds of latency; now 11.7)
+  constexpr int STEP = 16;
+  float w[CPT][STEP];
+  const auto load = [&](int c0, int j0) {
+#pragma unroll
+    for (int q = 0; q < CPT; ++q)
+#pragma unroll
+      for (int i = 0; i < STEP; ++i) w[q][i] = (j0 + i < rank && c0 + q < C) ? a2t[(size_t)(j0 + i) * C + c0 + q] : 0.0f;
+  };
+  int c0 = (blockIdx.y * blockDim.x + threadIdx.x) * CPT;
+  load(c0, 0);
+  jb::pdl_wait();
   for (int i = threadIdx.x; i < TB * rank4; i += blockDim.x) {
     const int u = i / rank4, j = i % rank4;
     low_s[i] = (u < n && j < rank) ? proj[(size_t)(t0 + u) * ld + low_col + j] : 0.0f;
   }
   __syncthreads();
-  for (int c0 = (blockIdx.y * blockDim.x + threadIdx.x) * CPT; c0 < C; c0 += gridDim.y * blockDim.x * CPT) {
+  for (bool first = true; c0 < C; c0 += gridDim.y * blockDim.x * CPT, first = false) {
+    if (!first) load(c0, 0);
     float z[CPT][TB];
 #pragma unroll
     for (int q = 0; q < CPT; ++q) {
@@ -69,18 +82,18 @@ __global__ void __launch_bounds__(128) gla_decay_kernel(const float* __restrict_
 #pragma unroll
       for (int u = 0; u < TB; ++u) z[q][u] = b;
     }
-    for (int j = 0; j < rank4; j += 4) {
-      float w[CPT][4];
+    for (int j0 = 0; j0 < rank4; j0 += STEP) {
+      if (j0 > 0) load(c0, j0);
 #pragma unroll
-      for (int q = 0; q < CPT; ++q)
+      for (int i = 0; i < STEP; i += 4) {
+        if (j0 + i >= rank4) break;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) w[q][i] = (j + i < rank && c0 + q < C) ? a2t[(size_t)(j + i) * C + c0 + q] : 0.0f;
+        for (int u = 0; u < TB; ++u) {
+          const float4 l = *reinterpret_cast<const float4*>(low_s + u * rank4 + j0 + i);
 #pragma unroll
-      for (int u = 0; u < TB; ++u) {
-        const float4 l = *reinterpret_cast<const float4*>(low_s + u * rank4 + j);
-#pragma unroll
-        for (int q = 0; q < CPT; ++q)
-          z[q][u] = fmaf(w[q][3], l.w, fmaf(w[q][2], l.z, fmaf(w[q][1], l.y, fmaf(w[q][0], l.x, z[q][u]))));
+          for (int q = 0; q < CPT; ++q)
+            z[q][u] = fmaf(w[q][i + 3], l.w, fmaf(w[q][i + 2], l.z, fmaf(w[q][i + 1], l.y, fmaf(w[q][i], l.x, z[q][u]))));
+        }
       }
     }
 #pragma unroll
@@ -164,6 +177,64 @@ __device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.com
 __device__ __forceinline__ void copy_async_wait_all_but_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 constexpr int VEC_QK = 1, VEC_V = 2;   // which rows of a token are whole, aligned 16-byte vectors in global memory
+
+// One token of every sequence (state_step.cuh); the first column block of a head carries the normalizer.  (8 sequences of
+// 16 heads of 128 x 128, 17 MB of state: 8.6 us as a walk over one token, 4.3 so.)
+template <int RI, bool SCALAR>
+__global__ void __launch_bounds__(jb::STEP_THREADS, RI <= 8 ? 3 : 1) gated_linear_step_kernel(
+    const float* __restrict__ proj, int ld, int q_col, int k_col, int v_col, float q_scale, const float* __restrict__ dec,
+    int dec_ld, float* __restrict__ out, float* __restrict__ den, float* __restrict__ state, long long state_ld,
+    const int* __restrict__ q_start, const int* __restrict__ seq_slot, int H, int d, int e) {
+  __shared__ float4 sums[jb::STEP_THREADS / 32][jb::STEP_COLS / 4];
+  __shared__ float norm_s[jb::STEP_ROWS];
+  jb::pdl_launch_dependents();
+  const int seq = blockIdx.x, h = blockIdx.y, col = threadIdx.x & 15, row = threadIdx.x >> 4;
+  const int j = (int)blockIdx.z * jb::STEP_COLS + 4 * col, ex = e + (SCALAR ? 1 : 0);
+  const bool in = j < e;
+  jb::pdl_wait();
+  const size_t t = (size_t)q_start[seq];
+  float* st = state + (size_t)seq_slot[seq] * state_ld + (size_t)h * d * ex;
+  const float* q = proj + t * ld + q_col + (size_t)h * d;
+  const float* k = proj + t * ld + k_col + (size_t)h * d;
+  const float* gates = dec + (t * H + h) * 4;                  // SCALAR: keep, take, exp(-m)
+  const float* a = dec + t * dec_ld + (size_t)h * d;           // else: a decay per key channel
+  const float keep = SCALAR ? gates[0] : 0.0f, take = SCALAR ? gates[1] : 1.0f;
+  float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (in) {
+    const float* p = proj + t * ld + v_col + (size_t)h * e + j;
+    v = make_float4(p[0] * take, p[1] * take, p[2] * take, p[3] * take);
+  }
+  if (SCALAR && blockIdx.z == 0 && col == 0) {                 // n <- keep n + take k, and its product with q
+    float* n = st + (size_t)d * e;
+    float nr[RI], kr[RI], qr[RI], nq = 0.0f;
+#pragma unroll
+    for (int i = 0; i < RI; ++i) {
+      const int r = row + jb::STEP_ROWS * i;
+      if (r < d) nr[i] = n[r], kr[i] = k[r], qr[i] = q[r];
+    }
+#pragma unroll
+    for (int i = 0; i < RI; ++i) {
+      const int r = row + jb::STEP_ROWS * i;
+      if (r < d) {
+        nr[i] = fmaf(keep, nr[i], kr[i] * take);
+        n[r] = nr[i];
+        nq = fmaf(nr[i], qr[i], nq);
+      }
+    }
+    norm_s[row] = nq;
+  }
+  const float4 y = jb::state_step<RI>(st + j, e, in, d, row, v, [&](int r) { return SCALAR ? keep : a[r]; },
+                                      [&](int r) { return k[r]; }, [&](int r) { return q[r]; });
+  const float total = jb::step_columns(y, sums);
+  const int at = (int)blockIdx.z * jb::STEP_COLS + threadIdx.x;
+  if (threadIdx.x < jb::STEP_COLS && at < e) out[t * H * e + (size_t)h * e + at] = total * q_scale;
+  if (SCALAR && blockIdx.z == 0 && threadIdx.x == 0) {
+    float nq = 0.0f;
+#pragma unroll
+    for (int i = 0; i < jb::STEP_ROWS; ++i) nq += norm_s[i];
+    den[t * H + h] = fmaxf(fabsf(nq * q_scale), gates[2]) + DEN_FLOOR;
+  }
+}
 
 // RMAX: rows of S a thread holds (a multiple of 4, 4 RMAX >= d); shared rows are padded to 4 RMAX with zeros.
 // SCALAR: one decay and one input scale per head and token (`dec` is the float4 gates [T][H]); else `dec` holds a decay
@@ -519,6 +590,16 @@ JB_EXPORT int jb_gated_linear_scan(const float* proj, int ld, int q_col, int k_c
   JB_REFUSE(d < 1 || d > 256 || e < 1, "gated_linear_scan: key size %d is outside [1, 256]", d);
   JB_REFUSE(seg_len > 0 && (scratch == nullptr || seg_decay == nullptr), "gated_linear_scan: segments need scratch");
   JB_REFUSE(scalar && den == nullptr, "gated_linear_scan: the normalizer needs a place for the divisors");
+  const int ex = e + (scalar ? 1 : 0);
+  if (seg_len < 0 && e % 4 == 0 && state_ld % 4 == 0 && d * ex % 4 == 0 && ((uintptr_t)state & 15) == 0) {
+    jb::Launch cfg(dim3(n_seqs, H, (e + jb::STEP_COLS - 1) / jb::STEP_COLS), dim3(jb::STEP_THREADS), 0, stream);
+    auto* fn = scalar ? (d <= 64 ? gated_linear_step_kernel<4, true> : d <= 128 ? gated_linear_step_kernel<8, true>
+                                                                                : gated_linear_step_kernel<16, true>)
+                      : (d <= 64 ? gated_linear_step_kernel<4, false> : d <= 128 ? gated_linear_step_kernel<8, false>
+                                                                                 : gated_linear_step_kernel<16, false>);
+    return (int)cudaLaunchKernelEx(&cfg.c, fn, proj, ld, q_col, k_col, v_col, q_scale, dec, dec_ld, out, den, state, state_ld,
+                                   q_start, seq_slot, H, d, e);
+  }
   if (scalar)
     return scan_all<true, true>(proj, ld, q_col, k_col, v_col, q_scale, dec, dec_ld, out, den, state, state_ld, q_start,
                                 seq_slot, n_seqs, H, d, e, max_q_len, seg_len, scratch, seg_decay, stream);

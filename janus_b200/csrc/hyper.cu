@@ -396,6 +396,13 @@ __global__ void embed_streams_kernel(const TT* __restrict__ table, const int* __
   if (id < 0) id = feedback[token_slot[t]];
   const TT* row = table + (size_t)id * H;
   float* o = out + (size_t)t * S * H;
+  if ((H & 3) == 0 && (((uintptr_t)table | (uintptr_t)out) & 15) == 0) {      // four columns a thread
+    for (int i = 4 * threadIdx.x; i < H; i += 4 * blockDim.x) {
+      const float4 v = load4(row + i);
+      for (int s = 0; s < S; ++s) store4(o + (size_t)s * H + i, v);
+    }
+    return;
+  }
   for (int i = threadIdx.x; i < H; i += blockDim.x) {
     const float v = jb::to_f32(row[i]);
     for (int s = 0; s < S; ++s) o[(size_t)s * H + i] = v;
@@ -408,7 +415,7 @@ JB_EXPORT int jb_embed_streams(const void* table, int table_dtype, const int* id
                                const int* feedback, const int* token_slot, cudaStream_t stream) {
   if (T <= 0) return 0;
   JB_REFUSE(S < 1 || S > MAX_STREAMS, "embed_streams: %d streams are outside [1, %d]", S, MAX_STREAMS);
-  jb::Launch cfg(dim3(T), dim3(H >= 1024 ? 256 : 128), 0, stream);
+  jb::Launch cfg(dim3(T), dim3(T <= 296 && H >= 2048 ? 512 : H >= 1024 ? 256 : 128), 0, stream);
   if (table_dtype == JB_F32)
     return (int)cudaLaunchKernelEx(&cfg.c, embed_streams_kernel<float>, (const float*)table, ids, out, H, S, feedback, token_slot);
   if (table_dtype == JB_BF16)

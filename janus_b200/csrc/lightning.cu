@@ -207,6 +207,59 @@ __global__ void lightning_prefix_kernel(float* __restrict__ scratch, const float
   }
 }
 
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&raw.x), b = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
+  return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
+}
+__device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+  *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+
+// gated_rmsnorm with the row in registers, CACHE vectors a thread, row and gate in flight together, the weight asked for
+// before the wait (4 rows of 2,048 in a decode step: 7.8 us with two scalar passes, 1.9 so; 2,623 rows, 54 MB: 31 and 12 us).
+template <typename TG, typename TO, int THREADS_N, int CACHE>
+__global__ void __launch_bounds__(THREADS_N) gated_rmsnorm_rows_kernel(const float* __restrict__ o, const TG* __restrict__ w,
+                                                                       const float* __restrict__ gate, int gate_ld, float eps,
+                                                                       TO* __restrict__ out, int N) {
+  __shared__ float scratch[THREADS_N / 32];
+  jb::pdl_launch_dependents();
+  const size_t t = blockIdx.x;
+  float4 x[CACHE], g[CACHE], ww[CACHE];
+#pragma unroll
+  for (int c = 0; c < CACHE; ++c) {
+    const int i = 4 * ((int)threadIdx.x + c * THREADS_N);
+    if (i < N) ww[c] = load4(w + i);
+  }
+  jb::pdl_wait();
+#pragma unroll
+  for (int c = 0; c < CACHE; ++c) {
+    const int i = 4 * ((int)threadIdx.x + c * THREADS_N);
+    if (i < N) x[c] = load4(o + t * N + i), g[c] = load4(gate + t * gate_ld + i);
+  }
+  float ss = 0.0f;
+#pragma unroll
+  for (int c = 0; c < CACHE; ++c)
+    if (4 * ((int)threadIdx.x + c * THREADS_N) < N) ss += x[c].x * x[c].x + x[c].y * x[c].y + x[c].z * x[c].z + x[c].w * x[c].w;
+  ss = jb::warp_sum(ss);
+  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  ss = 0.0f;
+#pragma unroll
+  for (int i = 0; i < THREADS_N / 32; ++i) ss += scratch[i];
+  const float rms = sqrtf(ss / (float)N + eps);
+  const auto one = [&](float v, float weight, float z) { return (v / rms) * weight * (1.0f / (1.0f + expf(-z))); };
+#pragma unroll
+  for (int c = 0; c < CACHE; ++c) {
+    const int i = 4 * ((int)threadIdx.x + c * THREADS_N);
+    if (i < N) store4(out + t * N + i, make_float4(one(x[c].x, ww[c].x, g[c].x), one(x[c].y, ww[c].y, g[c].y),
+                                                   one(x[c].z, ww[c].z, g[c].z), one(x[c].w, ww[c].w, g[c].w)));
+  }
+}
+
 template <typename TG, typename TO>
 __global__ void gated_rmsnorm_kernel(const float* __restrict__ o, const TG* __restrict__ w, const float* __restrict__ gate,
                                      int gate_ld, float eps, TO* __restrict__ out, int N) {
@@ -278,10 +331,18 @@ JB_EXPORT int jb_lightning_scan(const float* proj, int ld, int q_col, int k_col,
 JB_EXPORT int jb_gated_rmsnorm(const float* o, const void* w, int w_dtype, const float* gate, int gate_ld, float eps,
                                void* out, int out_dtype, int T, int N, cudaStream_t stream) {
   if (T <= 0) return 0;
-  jb::Launch cfg(dim3(T), dim3(N >= 2048 ? 256 : 128), 0, stream);
+  const bool rows = ((N | gate_ld) & 3) == 0 && N >= 512 && N <= 4096 &&
+                    (((uintptr_t)o | (uintptr_t)w | (uintptr_t)gate | (uintptr_t)out) & 15) == 0;
+  const bool few = T <= 296;                 // at most two rows an SM: a thread a vector
+  jb::Launch cfg(dim3(T), dim3(rows ? (few ? (N <= 2048 ? 512 : 1024) : 256) : N >= 2048 ? 256 : 128), 0, stream);
   cudaError_t e;
 #define JB_LAUNCH_GN(TG, TO) \
-  e = cudaLaunchKernelEx(&cfg.c, gated_rmsnorm_kernel<TG, TO>, o, (const TG*)w, gate, gate_ld, eps, (TO*)out, N)
+  e = cudaLaunchKernelEx(&cfg.c, !rows ? gated_rmsnorm_kernel<TG, TO>                                              \
+                                 : few ? (N <= 2048 ? gated_rmsnorm_rows_kernel<TG, TO, 512, 1>                    \
+                                                    : gated_rmsnorm_rows_kernel<TG, TO, 1024, 1>)                  \
+                                 : N <= 2048 ? gated_rmsnorm_rows_kernel<TG, TO, 256, 2>                           \
+                                             : gated_rmsnorm_rows_kernel<TG, TO, 256, 4>,                          \
+                         o, (const TG*)w, gate, gate_ld, eps, (TO*)out, N)
   if (w_dtype == JB_F32 && out_dtype == JB_F32) JB_LAUNCH_GN(float, float);
   else if (w_dtype == JB_F32 && out_dtype == JB_BF16) JB_LAUNCH_GN(float, bf16);
   else if (w_dtype == JB_BF16 && out_dtype == JB_F32) JB_LAUNCH_GN(bf16, float);

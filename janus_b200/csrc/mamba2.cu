@@ -24,7 +24,7 @@
 // sequence's state.
 #include <stdio.h>
 
-#include "common.cuh"
+#include "state_step.cuh"
 
 namespace {
 
@@ -89,6 +89,9 @@ __device__ __forceinline__ float4 silu4(float4 v) {
   return make_float4(silu_f(v.x), silu_f(v.y), silu_f(v.z), silu_f(v.w));
 }
 
+// MAX: taps at most (the loops over them are unrolled, the window stays in registers); AHEAD tokens' inputs are in flight
+// before the first is used (2,532 tokens x 8,448 channels, 171 MB: 103 us a token a time, 65 so).
+template <int MAX>
 __global__ void causal_conv_silu_vec_kernel(const float* __restrict__ proj, int ld, int col0, int C,
                                             const float* __restrict__ w, const float* __restrict__ bias, int taps,
                                             const float* __restrict__ state, long long slot_stride, long long state_off,
@@ -98,22 +101,35 @@ __global__ void causal_conv_silu_vec_kernel(const float* __restrict__ proj, int 
   jb::pdl_wait();
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
   if (c >= C) return;
-  float wr[4][CONV_MAX_TAPS];
+  float wr[4][MAX];
 #pragma unroll
   for (int k = 0; k < 4; ++k)
 #pragma unroll
-    for (int j = 0; j < CONV_MAX_TAPS; ++j) wr[k][j] = j < taps ? w[(size_t)(c + k) * taps + j] : 0.0f;
+    for (int j = 0; j < MAX; ++j) wr[k][j] = j < taps ? w[(size_t)(c + k) * taps + j] : 0.0f;
   const float4 b4 = bias != nullptr ? *reinterpret_cast<const float4*>(bias + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  float4 win[CONV_MAX_TAPS - 1];          // win[j]: the input taps - 1 - j tokens back (slots taps - 1 and up unused)
+  float4 win[MAX - 1];          // win[j]: the input taps - 1 - j tokens back (slots taps - 1 and up unused)
   const int t0 = blockIdx.x * CONV_TOKENS, t1 = min(T, t0 + CONV_TOKENS);
   int seq_before = -1;
-  for (int t = t0; t < t1; ++t) {
-    const int seq = token_seq[t];
+  constexpr int AHEAD = MAX <= 4 ? 8 : 4;
+  float4 next[AHEAD];
+  int next_seq[AHEAD];
+  for (int tb = t0; tb < t1; tb += AHEAD) {
+#pragma unroll
+  for (int k = 0; k < AHEAD; ++k) {
+    const int t = min(tb + k, t1 - 1);
+    next_seq[k] = token_seq[t];
+    next[k] = *reinterpret_cast<const float4*>(proj + (size_t)t * ld + col0 + c);
+  }
+#pragma unroll
+  for (int k = 0; k < AHEAD; ++k) {
+    const int t = tb + k;
+    if (t >= t1) break;
+    const int seq = next_seq[k];
     if (seq != seq_before) {               // the tile's first token, or a sequence's first: fill the window
       const int s0 = q_start[seq], li = t - s0;
       const float* st = state + (size_t)seq_slot[seq] * slot_stride + state_off;
 #pragma unroll
-      for (int j = 0; j < CONV_MAX_TAPS - 1; ++j) {
+      for (int j = 0; j < MAX - 1; ++j) {
         if (j < taps - 1) {
           const int src = li - (taps - 1) + j;
           win[j] = src >= 0 ? *reinterpret_cast<const float4*>(proj + (size_t)(s0 + src) * ld + col0 + c)
@@ -122,10 +138,10 @@ __global__ void causal_conv_silu_vec_kernel(const float* __restrict__ proj, int 
       }
       seq_before = seq;
     }
-    const float4 u = *reinterpret_cast<const float4*>(proj + (size_t)t * ld + col0 + c);
+    const float4 u = next[k];
     float4 acc = b4;
 #pragma unroll
-    for (int j = 0; j < CONV_MAX_TAPS - 1; ++j) {
+    for (int j = 0; j < MAX - 1; ++j) {
       if (j < taps - 1) {
         acc.x = fmaf(wr[0][j], win[j].x, acc.x);
         acc.y = fmaf(wr[1][j], win[j].y, acc.y);
@@ -134,7 +150,7 @@ __global__ void causal_conv_silu_vec_kernel(const float* __restrict__ proj, int 
       }
     }
 #pragma unroll
-    for (int j = 0; j < CONV_MAX_TAPS; ++j) {
+    for (int j = 0; j < MAX; ++j) {
       if (j == taps - 1) {
         acc.x = fmaf(wr[0][j], u.x, acc.x);
         acc.y = fmaf(wr[1][j], u.y, acc.y);
@@ -144,11 +160,12 @@ __global__ void causal_conv_silu_vec_kernel(const float* __restrict__ proj, int 
     }
     *reinterpret_cast<float4*>(out + (size_t)t * C + c) = silu4(acc);
 #pragma unroll
-    for (int j = 0; j < CONV_MAX_TAPS - 2; ++j)
+    for (int j = 0; j < MAX - 2; ++j)
       if (j < taps - 2) win[j] = win[j + 1];
 #pragma unroll
-    for (int j = 0; j < CONV_MAX_TAPS - 1; ++j)
+    for (int j = 0; j < MAX - 1; ++j)
       if (j == taps - 2) win[j] = u;
+  }
   }
 }
 
@@ -173,6 +190,37 @@ __global__ void conv_state_shift_kernel(const float* __restrict__ proj, int ld, 
 
 // ---- the recurrence -----------------------------------------------------------------------------------------
 enum { WHOLE = 0, LOCAL = 1, FROM_START = 3 };
+
+// One token of every sequence (state_step.cuh).  (8 sequences x 128 heads of 128 x 64, 67 MB of state: 25 -> 15 us; as a walk
+// over one token the loads follow one another in five rounds, 128 threads a block.)
+template <int RI>
+__global__ void __launch_bounds__(jb::STEP_THREADS, RI <= 4 ? 4 : RI <= 8 ? 3 : 1) mamba2_step_kernel(
+    const float* __restrict__ xbc, int ldx, int b_col, int c_col, const float* __restrict__ dt_raw, int ld_dt,
+    const float* __restrict__ dt_bias, const float* __restrict__ A_log, const float* __restrict__ Dskip,
+    float* __restrict__ out, float* __restrict__ state, long long slot_stride, long long state_off,
+    const int* __restrict__ q_start, const int* __restrict__ seq_slot, int H, int G, int N, int P) {
+  __shared__ float4 sums[jb::STEP_THREADS / 32][jb::STEP_COLS / 4];
+  jb::pdl_launch_dependents();
+  const int seq = blockIdx.x, h = blockIdx.y, g = h / (H / G), row = threadIdx.x >> 4;
+  const int j = (int)blockIdx.z * jb::STEP_COLS + 4 * ((int)threadIdx.x & 15);
+  const bool in = j < P;
+  const float neg_a = -expf(A_log[h]), bias = dt_bias[h], dskip = Dskip[h];
+  jb::pdl_wait();
+  const size_t t = (size_t)q_start[seq];
+  const float* xr = xbc + t * ldx;
+  const float dt = softplus_f(dt_raw[t * ld_dt + h] + bias), a = expf(neg_a * dt);
+  float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (in) {
+    const float* p = xr + (size_t)h * P + j;
+    v = make_float4(dt * p[0], dt * p[1], dt * p[2], dt * p[3]);
+  }
+  float* st = state + (size_t)seq_slot[seq] * slot_stride + state_off + (size_t)h * N * P + j;
+  const float4 y = jb::state_step<RI>(st, P, in, N, row, v, [&](int) { return a; }, [&](int r) { return xr[b_col + g * N + r]; },
+                                      [&](int r) { return xr[c_col + g * N + r]; });
+  const float total = jb::step_columns(y, sums);
+  const int at = (int)blockIdx.z * jb::STEP_COLS + threadIdx.x;
+  if (threadIdx.x < jb::STEP_COLS && at < P) out[t * H * P + (size_t)h * P + at] = fmaf(dskip, xr[(size_t)h * P + at], total);
+}
 
 // RMAX: rows of S a thread holds (a multiple of 4, PARTS * RMAX >= N); shared rows are padded to PARTS * RMAX with zeros
 template <int RMAX, int PHASE>
@@ -462,6 +510,51 @@ __device__ __forceinline__ void store4_out(bf16* p, float4 v) {
 
 // Pieces made of whole 16-byte vectors: the gated values stay in shared memory between the two passes (the piece is
 // read once), 16 bytes a thread.
+// gated_group_rmsnorm with a piece's values in registers, CACHE vectors a thread, all loads in flight together and the
+// weight asked for before the wait: few rows take 1,024 threads a piece (8 rows of 8,192: 12 us through shared memory with
+// 256, 3.8 so; 2,532 rows: 53 and 47 to 53), many 512.
+template <typename TO, int THREADS_G, int CACHE>
+__global__ void __launch_bounds__(THREADS_G) gated_group_rmsnorm_rows_kernel(const float* __restrict__ y,
+                                                                             const float* __restrict__ gate, int gate_ld,
+                                                                             const float* __restrict__ w, float eps,
+                                                                             TO* __restrict__ out, int N, int parts) {
+  __shared__ float scratch[THREADS_G / 32];
+  jb::pdl_launch_dependents();
+  const int t = blockIdx.x, n = N / parts, c0 = (int)blockIdx.y * n, n4 = n >> 2;
+  const float4* row = reinterpret_cast<const float4*>(y + (size_t)t * N + c0);
+  const float4* g = reinterpret_cast<const float4*>(gate + (size_t)t * gate_ld + c0);
+  const float4* w4 = reinterpret_cast<const float4*>(w + c0);
+  float4 a[CACHE], z[CACHE], ww[CACHE];
+#pragma unroll
+  for (int c = 0; c < CACHE; ++c)
+    if ((int)threadIdx.x + c * THREADS_G < n4) ww[c] = w4[threadIdx.x + c * THREADS_G];
+  jb::pdl_wait();
+#pragma unroll
+  for (int c = 0; c < CACHE; ++c)
+    if ((int)threadIdx.x + c * THREADS_G < n4) a[c] = row[threadIdx.x + c * THREADS_G], z[c] = g[threadIdx.x + c * THREADS_G];
+  float ss = 0.0f;
+#pragma unroll
+  for (int c = 0; c < CACHE; ++c) {
+    if ((int)threadIdx.x + c * THREADS_G >= n4) break;
+    a[c] = make_float4(a[c].x * silu_f(z[c].x), a[c].y * silu_f(z[c].y), a[c].z * silu_f(z[c].z), a[c].w * silu_f(z[c].w));
+    ss += a[c].x * a[c].x + a[c].y * a[c].y + a[c].z * a[c].z + a[c].w * a[c].w;
+  }
+  ss = jb::warp_sum(ss);
+  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  ss = 0.0f;
+#pragma unroll
+  for (int i = 0; i < THREADS_G / 32; ++i) ss += scratch[i];
+  const float rms = sqrtf(ss / (float)n + eps);
+#pragma unroll
+  for (int c = 0; c < CACHE; ++c) {
+    const int i = (int)threadIdx.x + c * THREADS_G;
+    if (i >= n4) break;
+    store4_out(out + (size_t)t * N + c0 + 4 * i, make_float4((a[c].x / rms) * ww[c].x, (a[c].y / rms) * ww[c].y,
+                                                             (a[c].z / rms) * ww[c].z, (a[c].w / rms) * ww[c].w));
+  }
+}
+
 template <typename TO>
 __global__ void gated_group_rmsnorm_vec_kernel(const float* __restrict__ y, const float* __restrict__ gate, int gate_ld,
                                                const float* __restrict__ w, float eps, TO* __restrict__ out, int N,
@@ -509,7 +602,7 @@ JB_EXPORT int jb_causal_conv_silu(const float* proj, int ld, int col0, int C, co
                        (((uintptr_t)proj | (uintptr_t)out | (uintptr_t)state | (uintptr_t)bias) & 15) == 0;
   if (!single_tokens && aligned && taps <= CONV_MAX_TAPS && T >= 4 * CONV_TOKENS) {
     jb::Launch cfg(dim3((T + CONV_TOKENS - 1) / CONV_TOKENS, (C / 4 + 127) / 128), dim3(128), 0, stream);
-    cudaError_t e = cudaLaunchKernelEx(&cfg.c, causal_conv_silu_vec_kernel, proj, ld, col0, C, w, bias, taps,
+    cudaError_t e = cudaLaunchKernelEx(&cfg.c, taps <= 4 ? causal_conv_silu_vec_kernel<4> : causal_conv_silu_vec_kernel<CONV_MAX_TAPS>, proj, ld, col0, C, w, bias, taps,
                                        (const float*)state, slot_stride, state_off, token_seq, q_start, seq_slot, out, T);
     if (e != cudaSuccess) return (int)e;
   } else {
@@ -534,7 +627,8 @@ JB_EXPORT int jb_causal_conv_silu(const float* proj, int ld, int col0, int C, co
 // ld_dt floats, head h in column h; dt_bias, A_log, Dskip: [H] float32; out: float32 [T, H P]; state: per slot
 // slot_stride floats, the recurrence's [H][N][P] at state_off.  seg_len > 0 with scratch (n_seqs *
 // ceil(max_q_len / seg_len) * H * N * P floats) and seg_decay (n_seqs * ceil(max_q_len / seg_len) * H floats)
-// runs the three passes over segments; seg_len = 0 walks every sequence in one block per column block.
+// runs the three passes over segments; seg_len = 0 walks every sequence in one block per column block; seg_len < 0 says
+// that every sequence brings one token.
 JB_EXPORT int jb_mamba2_scan(const float* xbc, int ldx, int b_col, int c_col, const float* dt_raw, int ld_dt,
                              const float* dt_bias, const float* A_log, const float* Dskip, float* out, float* state,
                              long long slot_stride, long long state_off, const int* q_start, const int* seq_slot,
@@ -544,6 +638,12 @@ JB_EXPORT int jb_mamba2_scan(const float* xbc, int ldx, int b_col, int c_col, co
   JB_REFUSE(N < 1 || N > 256 || P < 1, "mamba2_scan: state size %d is outside [1, 256]", N);
   JB_REFUSE(G < 1 || H % G != 0, "mamba2_scan: %d heads are not a multiple of %d groups", H, G);
   JB_REFUSE(seg_len > 0 && (scratch == nullptr || seg_decay == nullptr), "mamba2_scan: segments need scratch");
+  if (seg_len < 0 && P % 4 == 0 && slot_stride % 4 == 0 && state_off % 4 == 0 && ((uintptr_t)state & 15) == 0) {
+    jb::Launch step(dim3(n_seqs, H, (P + jb::STEP_COLS - 1) / jb::STEP_COLS), dim3(jb::STEP_THREADS), 0, stream);
+    auto* fn = N <= 64 ? mamba2_step_kernel<4> : N <= 128 ? mamba2_step_kernel<8> : mamba2_step_kernel<16>;
+    return (int)cudaLaunchKernelEx(&step.c, fn, xbc, ldx, b_col, c_col, dt_raw, ld_dt, dt_bias, A_log, Dskip, out, state,
+                                   slot_stride, state_off, q_start, seq_slot, H, G, N, P);
+  }
   const int rmax = N <= 64 ? 8 : N <= 128 ? 16 : 32;
   const size_t smem = (size_t)(2 * CT * PARTS * (rmax + 4) + CT * EB + 3 * CT + 4) * sizeof(float);
   const bool segmented = seg_len > 0;
@@ -591,6 +691,21 @@ JB_EXPORT int jb_gated_group_rmsnorm(const float* y, const float* gate, int gate
   const int n = N / parts;
   const bool aligned = ((n | N | gate_ld) & 3) == 0 && n * (int)sizeof(float) <= 48 * 1024 &&
                        (((uintptr_t)y | (uintptr_t)gate | (uintptr_t)w | (uintptr_t)out) & 15) == 0;
+  if (aligned && n >= 1024 && n <= 8192) {
+    const bool few = (long long)T * parts <= 148;
+    const int threads = few && n > 2048 ? 1024 : n <= 2048 ? 256 : 512;
+    jb::Launch cfg(dim3(T, parts), dim3(threads), 0, stream);
+#define JB_GO(TO)                                                                                                     \
+  return (int)cudaLaunchKernelEx(&cfg.c, threads == 1024 ? gated_group_rmsnorm_rows_kernel<TO, 1024, 2>               \
+                                         : threads == 256 ? gated_group_rmsnorm_rows_kernel<TO, 256, 2>               \
+                                         : n <= 4096 ? gated_group_rmsnorm_rows_kernel<TO, 512, 2>                    \
+                                                     : gated_group_rmsnorm_rows_kernel<TO, 512, 4>,                   \
+                                 y, gate, gate_ld, w, eps, (TO*)out, N, parts)
+    if (out_dtype == JB_F32) JB_GO(float);
+    if (out_dtype == JB_BF16) JB_GO(bf16);
+#undef JB_GO
+    return JB_ERR_BAD_DTYPE;
+  }
   if (aligned) {
     jb::Launch cfg(dim3(T, parts), dim3(n >= 2048 ? 256 : 128), (size_t)n * sizeof(float), stream);
     if (out_dtype == JB_F32)

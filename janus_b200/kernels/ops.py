@@ -1463,13 +1463,14 @@ def causal_conv_silu(proj: torch.Tensor, col0: int, channels: int, weight: torch
 def mamba2_scan(xbc: torch.Tensor, b_col: int, c_col: int, dt_raw: torch.Tensor, dt_bias: torch.Tensor,
                 a_log: torch.Tensor, d_skip: torch.Tensor, out: torch.Tensor, state: torch.Tensor, state_off: int,
                 q_start: torch.Tensor, seq_slot: torch.Tensor, n_seqs: int, heads: int, groups: int, n_state: int,
-                vdim: int, max_q_len: int = 1, workspace=None) -> None:
+                vdim: int, max_q_len: int = 1, workspace=None, single_tokens: bool = False) -> None:
     """Per sequence and head S <- a_t S + dt_t B_t x_t^T, out_t = S^T C_t + D x_t over the step's tokens in order, with
     dt_t = softplus(dt_raw_t + dt_bias) and a_t = exp(-exp(a_log) dt_t).  xbc float32 [T, ld]: x in columns
     [0, heads vdim), B at b_col and C at c_col ([groups][n_state]); dt_raw a float32 view [T, heads] of wider rows;
     state float32 [slots, n] with the recurrence's [heads, n_state, vdim] block at offset state_off of a slot's row.
     With a workspace, steps whose longest sequence brings more than two segments of tokens run in three passes over
-    segments (3 launches), else one launch."""
+    segments (3 launches), else one launch.  `single_tokens`: every sequence
+    brings one token (the state is read and written once)."""
     T = xbc.shape[0]
     _need(xbc, "convolved x, B, C", torch.float32)
     _need(out, "scan out", torch.float32, (T, heads * vdim))
@@ -1484,8 +1485,10 @@ def mamba2_scan(xbc: torch.Tensor, b_col: int, c_col: int, dt_raw: torch.Tensor,
     _need(seq_slot, "sequence slots", torch.int32, (n_seqs,))
     if max(heads * vdim, b_col + groups * n_state, c_col + groups * n_state) > xbc.shape[1]:
         raise KernelError("mamba2_scan: the columns reach past the rows")
-    seg, scratch, seg_decay = 0, None, None
-    if workspace is not None and max_q_len > 2 * MAMBA2_SEGMENT:
+    if single_tokens and T != n_seqs:
+        raise KernelError("mamba2_scan: single_tokens needs one token per sequence")
+    seg, scratch, seg_decay = -1 if single_tokens else 0, None, None
+    if workspace is not None and max_q_len > 2 * MAMBA2_SEGMENT and not single_tokens:
         seg = mamba2_segment_for(n_seqs, max_q_len, heads, n_state, vdim)
         tiles = (max_q_len + seg - 1) // seg
         scratch = workspace.get("mamba2_segments", (n_seqs * tiles * heads * n_state * vdim,), torch.float32)
@@ -1494,7 +1497,7 @@ def mamba2_scan(xbc: torch.Tensor, b_col: int, c_col: int, dt_raw: torch.Tensor,
         _ptr(xbc), xbc.shape[1], int(b_col), int(c_col), _ptr(dt_raw), dt_raw.stride(0), _ptr(dt_bias), _ptr(a_log),
         _ptr(d_skip), _ptr(out), _ptr(state), state.shape[1], int(state_off), _ptr(q_start), _ptr(seq_slot), n_seqs,
         heads, groups, n_state, vdim, int(max_q_len), seg, _ptr(scratch), _ptr(seg_decay), _stream()),
-        "mamba2_scan", kernels=3 if seg else 1)
+        "mamba2_scan", kernels=3 if seg > 0 else 1)
 
 
 def gated_group_rmsnorm(y: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, eps: float, parts: int,
@@ -1817,14 +1820,15 @@ def exp_gates(proj: torch.Tensor, i_col: int, f_col: int, bias_i: torch.Tensor, 
 def gated_linear_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, q_scale: float, decays: torch.Tensor,
                       out: torch.Tensor, state: torch.Tensor, q_start: torch.Tensor, seq_slot: torch.Tensor,
                       n_seqs: int, heads: int, dim: int, vdim: int, max_q_len: int = 1, workspace=None,
-                      divisors: Optional[torch.Tensor] = None) -> None:
+                      divisors: Optional[torch.Tensor] = None, single_tokens: bool = False) -> None:
     """Per sequence and head S <- diag(a_t) S + b_t k_t v_t^T, out_t = S^T (q_t q_scale) over the step's tokens in
     order; proj float32 [T, ld] holds q, k, v at the given columns.  Without `divisors`, `decays` is float32
     [T, heads dim], a decay per key channel, b = 1, and a slot's state row holds [heads, dim, vdim].  With `divisors`
     (float32 [T, heads], written), `decays` is what `exp_gates` left ([T, heads, 4]: a_t and b_t one number a head),
     a normalizer n <- a_t n + b_t k_t walks along, divisors[t, h] = max(|n . q|, exp(-m_t)) + 1e-6, and a slot's state
     row holds per head [dim, vdim] then [dim] of n.  With a workspace, steps whose longest sequence brings more than
-    256 tokens run in passes over segments of 64 to 256 tokens (4 launches); else one launch."""
+    256 tokens run in passes over segments of 64 to 256 tokens (4 launches); else one launch.  `single_tokens`: every
+    sequence brings one token (the state is read and written once)."""
     T = proj.shape[0]
     scalar = divisors is not None
     _need(proj, "projections", torch.float32)
@@ -1840,8 +1844,10 @@ def gated_linear_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, q_
     _need(seq_slot, "sequence slots", torch.int32, (n_seqs,))
     if max(q_col + heads * dim, k_col + heads * dim, v_col + heads * vdim) > proj.shape[1]:
         raise KernelError("gated_linear_scan: the projections' columns reach past the rows")
-    seg, scratch, seg_decay = 0, None, None
-    if workspace is not None and max_q_len > 2 * GATED_LINEAR_SEGMENT:
+    if single_tokens and T != n_seqs:
+        raise KernelError("gated_linear_scan: single_tokens needs one token per sequence")
+    seg, scratch, seg_decay = -1 if single_tokens else 0, None, None
+    if workspace is not None and max_q_len > 2 * GATED_LINEAR_SEGMENT and not single_tokens:
         # the blocks are laid out as the state-space recurrence's (a segment, a head, 64 value columns; four blocks an SM
         # up to 128 rows of state, else two): the segment length that fills the SMs in whole waves is picked the same way
         seg = mamba2_segment_for(n_seqs, max_q_len, heads, dim, vdim)
@@ -1853,7 +1859,7 @@ def gated_linear_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, q_
         _ptr(proj), proj.shape[1], int(q_col), int(k_col), int(v_col), float(q_scale), _ptr(decays),
         0 if scalar else heads * dim, int(scalar), _ptr(out), _ptr(divisors), _ptr(state), state.shape[1],
         _ptr(q_start), _ptr(seq_slot), n_seqs, heads, dim, vdim, int(max_q_len), seg, _ptr(scratch), _ptr(seg_decay),
-        _stream()), "gated_linear_scan", kernels=4 if seg else 1)
+        _stream()), "gated_linear_scan", kernels=4 if seg > 0 else 1)
 
 
 # -- dynamic tanh in the place of a norm -------------------------------------------------------------------------

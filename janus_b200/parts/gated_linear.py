@@ -107,7 +107,8 @@ class GatedLinearAttention(_GatedLinearBase):
         ops.gla_decay(proj, self.extra_col, self.rank, self.a2t, self.a2_bias, self.tau, decays)
         o = ws.get("gla_o", (T, self.v_width), torch.float32)
         ops.gated_linear_scan(proj, 0, self.k_col, self.v_col, self.q_scale, decays, o, cache_view.state, ctx.q_start,
-                              ctx.seq_slot, ctx.n_seqs, self.nh, self.dim, self.vdim, ctx.max_q_len, ws)
+                              ctx.seq_slot, ctx.n_seqs, self.nh, self.dim, self.vdim, ctx.max_q_len, ws,
+                              single_tokens=ctx.is_decode)
         gated = ws.get("gla_gated", (T, self.v_width), self.dtype)
         ops.head_norm_gate(o, proj[:, self.gate_col: self.gate_col + self.v_width], self.norm_weight, self.eps, gated,
                            self.nh, self.vdim)
@@ -160,7 +161,8 @@ class MatrixMemory(_GatedLinearBase):
         o = ws.get("matrix_memory_o", (T, self.v_width), torch.float32)
         divisors = ws.get("matrix_memory_divisors", (T, self.nh), torch.float32)
         ops.gated_linear_scan(proj, 0, self.k_col, self.v_col, self.q_scale, gates, o, state, ctx.q_start, ctx.seq_slot,
-                              ctx.n_seqs, self.nh, self.dim, self.vdim, ctx.max_q_len, ws, divisors=divisors)
+                              ctx.n_seqs, self.nh, self.dim, self.vdim, ctx.max_q_len, ws, divisors=divisors,
+                              single_tokens=ctx.is_decode)
         gated = ws.get("matrix_memory_gated", (T, self.v_width), self.dtype)
         ops.head_norm_gate(o, proj[:, self.gate_col: self.gate_col + self.v_width], self.norm_weight, self.eps, gated,
                            self.nh, self.vdim, sigmoid=True, denom=divisors)

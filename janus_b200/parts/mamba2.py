@@ -100,7 +100,7 @@ class Mamba2Mixer(Mixer):
         y = ws.get("mamba2_y", (T, self.inner), torch.float32)
         ops.mamba2_scan(xbc, self.inner, self.inner + self.bc_width, proj[:, self.inner + self.channels:],
                         self.dt_bias, self.a_log, self.d_skip, y, state, 0, ctx.q_start, ctx.seq_slot, ctx.n_seqs,
-                        self.nh, self.groups, self.n_state, self.vdim, ctx.max_q_len, ws)
+                        self.nh, self.groups, self.n_state, self.vdim, ctx.max_q_len, ws, single_tokens=ctx.is_decode)
         gated = ws.get("mamba2_gated", (T, self.inner), self.dtype)
         ops.gated_group_rmsnorm(y, proj[:, : self.inner], self.norm_weight, self.eps, self.norm_groups, gated)
         self.o.forward_add(gated, residual)

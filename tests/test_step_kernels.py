@@ -130,6 +130,47 @@ def test_latent_prep(ops, T, Q, r, rp, dtype):
     assert worst(picked(cache, dest)[:, 0, :r], unit(proj[:, Q:].double(), eps) * w.double()) <= TOL[dtype]
 
 
+@pytest.mark.parametrize("T", [1, 148, 149])
+@pytest.mark.parametrize("N, parts", [(1020, 1), (1024, 1), (2048, 1), (2052, 1), (4096, 2), (4100, 1), (8192, 1), (8196, 1), (16384, 4)])
+def test_gated_group_rmsnorm(ops, T, N, parts):
+    y, wide, w, eps = rnd(T, N), rnd(T, N + 4, seed=1), rnd(N, seed=2), 1e-5
+    out = torch.empty(T, N, dtype=torch.bfloat16, device=DEV)
+    ops.gated_group_rmsnorm(y, wide[:, :N], w, eps, parts, out)
+    z = wide[:, :N].double()
+    v = (y.double() * z * torch.sigmoid(z)).view(T, parts, -1)
+    assert worst(out, unit(v, eps).view(T, N) * w.double()) <= TOL[torch.bfloat16]
+
+
+@pytest.mark.parametrize("n_seqs, H, G, N, P", [(1, 2, 1, 16, 64), (3, 4, 2, 128, 64), (2, 2, 1, 100, 68), (2, 3, 3, 256, 12),
+                                                (2, 2, 1, 64, 10)])
+def test_mamba2_single_tokens(ops, n_seqs, H, G, N, P):
+    """One token of every sequence, slots out of order: the single-token kernel (P a multiple of 4) and the walk."""
+    ld = H * P + 2 * G * N
+    xbc, dt, bias, a_log, skip = rnd(n_seqs, ld), rnd(n_seqs, H, seed=1), rnd(H, seed=2), rnd(H, seed=3, s=0.5), rnd(H, seed=4)
+    before = rnd(n_seqs + 2, H * N * P + 8, seed=5)
+    slots, q_start = torch.arange(n_seqs - 1, -1, -1, dtype=torch.int32, device=DEV), torch.arange(n_seqs + 1, dtype=torch.int32, device=DEV)
+    out, state = torch.empty(n_seqs, H * P, device=DEV), before.clone()
+    ops.mamba2_scan(xbc, H * P, H * P + G * N, dt, bias, a_log, skip, out, state, 4, q_start, slots, n_seqs, H, G, N, P,
+                    single_tokens=True)
+    walked, state2 = torch.empty_like(out), before.clone()
+    ops.mamba2_scan(xbc, H * P, H * P + G * N, dt, bias, a_log, skip, walked, state2, 4, q_start, slots, n_seqs, H, G, N, P)
+    x = xbc.double()
+    v, b, c = x[:, :H * P].view(-1, H, P), x[:, H * P:H * P + G * N].view(-1, G, N), x[:, H * P + G * N:].view(-1, G, N)
+    b, c = b.repeat_interleave(H // G, 1), c.repeat_interleave(H // G, 1)
+    z = dt.double() + bias.double()
+    step = torch.logaddexp(z, torch.zeros_like(z))
+    old = before[slots.long(), 4:4 + H * N * P].double().view(n_seqs, H, N, P)
+    new = torch.exp(-torch.exp(a_log.double()) * step)[..., None, None] * old + (step[..., None] * b)[..., None] * v[:, :, None]
+    y = torch.einsum("shnp,shn->shp", new, c) + skip.double()[:, None] * v
+    # sums of N products of numbers of size one, decays from exponentials: a few hundred roundings of 2^-24
+    for got, st in ((out, state), (walked, state2)):
+        assert worst(got.view(n_seqs, H, P), y) <= 2e-5
+        assert worst(st[slots.long(), 4:4 + H * N * P].view(n_seqs, H, N, P), new) <= 2e-5
+        keep = torch.ones_like(before, dtype=torch.bool)
+        keep[slots.long(), 4:4 + H * N * P] = False
+        assert torch.equal(st[keep], before[keep])
+
+
 @pytest.mark.parametrize("H, G, d, e", [(4, 1, 64, 128), (4, 2, 16, 64), (2, 2, 72, 72), (3, 1, 128, 8)])
 @pytest.mark.parametrize("window, kept", [(0, 0), (40, 0), (512, 4), (512, 70), (1, 33)])
 @pytest.mark.parametrize("copies", [1, 60])
@@ -183,6 +224,24 @@ def conv_reference(x, w, lens, states):
     return torch.cat(out)
 
 
+@pytest.mark.parametrize("taps", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("C", [8, 516])
+@pytest.mark.parametrize("lens", [[64], [1, 15, 2, 47, 16], [130, 1, 1, 1, 17]])
+def test_causal_conv_silu_prompts(ops, taps, C, lens):
+    """Walks of sixteen tokens with eight (four taps) or four inputs in flight; sequences that begin and end inside a walk."""
+    T, n = sum(lens), len(lens)
+    x, w, bias = rnd(T, C + 4), rnd(C, taps, seed=1), rnd(C, seed=2)
+    state = rnd(n + 1, (taps - 1) * C + 4, seed=3)
+    slots = torch.arange(n, 0, -1, dtype=torch.int32, device=DEV)
+    seq = torch.repeat_interleave(torch.arange(n), torch.tensor(lens)).int().to(DEV)
+    q_start = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    before, out = state.double().clone(), torch.empty(T, C, device=DEV)
+    ops.causal_conv_silu(x, 4, C, w, bias, taps, state, 4, seq, q_start, slots, out, n)
+    states = [before[s, 4:].view(taps - 1, C) for s in slots.tolist()]
+    y = conv_reference(x[:, 4:].double(), w.double(), lens, states) + bias.double()
+    assert worst(out, y * torch.sigmoid(y)) <= TOL[torch.float32]
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("taps", [0, 2, 3, 4, 5])
 @pytest.mark.parametrize("H, G, d, e, rot", [(4, 2, 64, 128, 32), (2, 1, 16, 12, 16), (3, 3, 20, 8, 0), (2, 2, 12, 20, 8)])
@@ -210,6 +269,73 @@ def test_conv_rope_cache_prompts(ops, H, G, d, e, rot, taps, lens, dtype):
     assert worst(q.view(T, 2 * H, d), want_q) <= TOL[torch.float32]
     assert worst(picked(k_cache, dest), want_k) <= TOL[dtype]
     assert worst(picked(v_cache, dest), x[:, (H + G) * 2 * d:].view(T, G, e)) <= TOL[dtype]
+
+
+@pytest.mark.parametrize("T", [1, 296, 297])
+@pytest.mark.parametrize("N", [508, 512, 2048, 2052, 4096, 4100])
+def test_gated_rmsnorm(ops, T, N):
+    o, wide, w, eps = rnd(T, N), rnd(T, N + 4, seed=1), rnd(N, seed=2).to(torch.bfloat16), 1e-5
+    out = torch.empty(T, N, dtype=torch.bfloat16, device=DEV)
+    ops.gated_rmsnorm(o, w, wide[:, :N], eps, out)
+    assert worst(out, unit(o.double(), eps) * w.double() * torch.sigmoid(wide[:, :N].double())) <= TOL[torch.bfloat16]
+
+
+@pytest.mark.parametrize("rank", [1, 15, 16, 17, 64, 66])
+@pytest.mark.parametrize("T, C", [(1, 7), (8, 2048), (17, 515)])
+def test_gla_decay(ops, T, C, rank):
+    proj, a2, bias = rnd(T, rank + 5), rnd(C, rank, seed=1), rnd(C, seed=2)
+    alpha = torch.empty(T, C, device=DEV)
+    ops.gla_decay(proj, 5, rank, a2.t().contiguous(), bias, 16.0, alpha)
+    z = proj[:, 5:].double() @ a2.double().T + bias.double()
+    # the argument's error (rank roundings of a sum of the size sqrt(rank)) reaches a decay through a sixteenth of itself
+    assert worst(alpha, torch.sigmoid(z) ** (1 / 16.0)) <= TOL[torch.float32]
+
+
+@pytest.mark.parametrize("n_seqs, H, d, e", [(1, 2, 16, 64), (3, 4, 128, 128), (2, 2, 100, 68), (2, 3, 256, 12), (2, 2, 64, 10)])
+@pytest.mark.parametrize("kind", ["channels", "normalizer"])
+def test_state_steps(ops, n_seqs, H, d, e, kind):
+    """One token of every sequence, slots out of order: the single-token kernels (values a multiple of 4) and the walks."""
+    ld = H * (2 * d + e)
+    proj = rnd(n_seqs, ld)
+    slots, q_start = torch.arange(n_seqs - 1, -1, -1, dtype=torch.int32, device=DEV), torch.arange(n_seqs + 1, dtype=torch.int32, device=DEV)
+    per = d * (e + 1) if kind == "normalizer" else d * e
+    before = rnd(n_seqs + 1, H * per, seed=5)
+    q, k, v = proj[:, :H * d].double().view(-1, H, d), proj[:, H * d:2 * H * d].double().view(-1, H, d), proj[:, 2 * H * d:].double().view(-1, H, e)
+    old = before[slots.long()].double().view(n_seqs, H, per)
+    S, scale, den, gates = old[..., :d * e].view(n_seqs, H, d, e), d ** -0.5, None, None
+    if kind == "channels":
+        gates = torch.rand(n_seqs, H * d, generator=torch.Generator().manual_seed(2)).to(DEV)
+        a = gates.double().view(n_seqs, H, d)
+    else:
+        gates = torch.rand(n_seqs, H, 4, generator=torch.Generator().manual_seed(2)).to(DEV)
+        a, v = gates[..., 0:1].double(), v * gates[..., 1:2].double()
+        n = a * old[..., d * e:] + gates[..., 1:2].double() * k
+        den = torch.maximum((n * q).sum(-1).abs() * scale, gates[..., 2].double()) + 1e-6
+    new = a[..., None] * S + k[..., None] * v[:, :, None]
+    y = torch.einsum("shde,shd->she", new, q) * scale
+    for single in (True, False):
+        out, state = torch.empty(n_seqs, H * e, device=DEV), before.clone()
+        got_den = torch.empty(n_seqs, H, device=DEV) if den is not None else None
+        ops.gated_linear_scan(proj, 0, H * d, 2 * H * d, scale, gates, out, state, q_start, slots, n_seqs, H, d, e,
+                              divisors=got_den, single_tokens=single)
+        # sums of d products of numbers of size one: a few hundred roundings of 2^-24
+        got = state[slots.long()].view(n_seqs, H, per)
+        assert worst(out.view(n_seqs, H, e), y) <= 2e-5
+        assert worst(got[..., :d * e].reshape(n_seqs, H, d, e), new) <= 2e-5
+        if den is not None:
+            assert worst(got[..., d * e:], n) <= 2e-5 and worst(got_den, den) <= 2e-5
+        assert torch.equal(state[n_seqs], before[n_seqs])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("H", [6, 8, 2044, 2048])
+@pytest.mark.parametrize("T", [1, 297])
+def test_embed_streams(ops, T, H, dtype):
+    """Every stream starts as the token's row: a copy, number for number."""
+    table, ids = rnd(50, H).to(dtype), torch.randint(0, 50, (T,), dtype=torch.int32, device=DEV)
+    out = torch.full((T, 3 * H), float("nan"), device=DEV)
+    ops.embed_streams(table, ids, out, 3)
+    assert torch.equal(out.view(T, 3, H), table[ids.long()].float()[:, None].expand(T, 3, H))
 
 
 @pytest.mark.parametrize("T, W, E", [(16, 1184, 8), (16, 1200, 8), (1, 2048, 4), (3, 4736, 4)])
