@@ -100,9 +100,12 @@ class GatedDeltaRule(Mixer):
         ops.causal_conv_silu(proj, 0, self.channels, self.conv_w, None, self.taps, state, self.scan_floats,
                              ctx.token_seq, ctx.q_start, ctx.seq_slot, conv, ctx.n_seqs, single_tokens=ctx.is_decode)
         o = ws.get("delta_o", (T, self.v_width), torch.float32)
+        floats = 0 if ctx.is_decode else ops.delta_rule_scratch(ctx.n_seqs, self.nh, ctx.max_q_len, self.channels, 0,
+                                                                self.qk_width, self.dim)
+        scratch = ws.get("delta_scratch", (floats,), torch.float32) if floats else None
         ops.delta_rule(conv, 0, self.qk_width, 2 * self.qk_width, proj, self.b_col, self.a_col, self.a_log,
                        self.dt_bias, UNIT_EPS, o, state, 0, ctx.q_start, ctx.seq_slot, ctx.n_seqs, self.nh, self.nkv,
-                       self.dim, self.vdim)
+                       self.dim, self.vdim, scratch, ctx.max_q_len)
         gated = ws.get("delta_gated", (T, self.v_width), self.dtype)
         ops.head_norm_gate(o, proj[:, self.gate_col: self.gate_col + self.v_width], self.norm_weight, self.eps, gated,
                            self.nh, self.vdim)

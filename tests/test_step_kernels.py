@@ -171,6 +171,53 @@ def test_mamba2_single_tokens(ops, n_seqs, H, G, N, P):
         assert torch.equal(st[keep], before[keep])
 
 
+@pytest.mark.parametrize("H, G, d, e", [(2, 1, 128, 128), (4, 2, 64, 24), (2, 2, 20, 17), (3, 3, 4, 130)])
+@pytest.mark.parametrize("lens", [[64], [65, 1, 31, 32, 33], [200, 3]])
+@pytest.mark.parametrize("slab", [0, 2])
+def test_delta_rule_chunks(ops, H, G, d, e, lens, slab):
+    """Prompts by chunks of 32 against the recurrence in float64 and against the walk token by token, unequal lengths, slots
+    out of order, from a state that is not zero, with scratch for everything or for two chunks a sequence at a time."""
+    T, n = sum(lens), len(lens)
+    cols = 2 * G * d + H * e
+    ldc = (cols + 3) // 4 * 4
+    conv, raw = rnd(T, ldc), rnd(T, 2 * H + 3, seed=1)
+    a_log, bias = rnd(H, seed=2, mean=-1.0), rnd(H, seed=3)
+    before = rnd(n + 1, H * d * e + 4, seed=4, s=0.3)
+    q_start = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    slots = torch.arange(n, 0, -1, dtype=torch.int32, device=DEV)
+    floats = (slab or (max(lens) + 31) // 32) * n * H * ops._DELTA_CHUNK_FLOATS
+    asked = ops.delta_rule_scratch(n, H, max(lens), ldc, 0, G * d, d)
+    assert asked == (0 if d <= 64 or max(lens) < 192 else n * H * 7 * ops._DELTA_CHUNK_FLOATS)
+    results = []
+    for scratch in (torch.full((floats,), float("nan"), device=DEV), None):
+        out, state = torch.full((T, H * e), float("nan"), device=DEV), before.clone()
+        ops.delta_rule(conv, 0, G * d, 2 * G * d, raw, 0, H, a_log, bias, 1e-6, out, state, 4, q_start, slots, n, H, G, d, e,
+                       scratch, max(lens))
+        results.append((out, state))
+    x = conv.double()
+    q, k, v = x[:, :G * d].view(T, G, d), x[:, G * d:2 * G * d].view(T, G, d), x[:, 2 * G * d:cols].reshape(T, H, e)
+    norm = lambda t: (t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)).repeat_interleave(H // G, 1)      # noqa: E731
+    q, k = norm(q) * d ** -0.5, norm(k)
+    beta = torch.sigmoid(raw[:, :H].double())
+    z = raw[:, H:2 * H].double() + bias.double()
+    decay = torch.exp(-torch.exp(a_log.double()) * torch.logaddexp(z, torch.zeros_like(z)))
+    want, after = torch.zeros(T, H, e, dtype=torch.float64, device=DEV), before.double().clone()
+    at = 0
+    for s, length in enumerate(lens):
+        S = before[slots[s].long(), 4:].double().view(H, d, e)
+        for t in range(at, at + length):
+            S = decay[t][:, None, None] * S
+            w = beta[t][:, None] * (v[t] - torch.einsum("hde,hd->he", S, k[t]))
+            S = S + k[t][:, :, None] * w[:, None, :]
+            want[t] = torch.einsum("hde,hd->he", S, q[t])
+        after[slots[s].long(), 4:] = S.reshape(-1)
+        at += length
+    # sums of up to 128 products and a chain of 32 writes a chunk, decays that forget what lies far back: a few hundred
+    # roundings of 2^-24 against the mean size of a result; the walk's own error stands beside it
+    err = [max(worst(o.view(T, H, e), want), worst(s, after)) for o, s in results]
+    assert err[0] <= 4e-5 and err[0] <= 4 * err[1] + 4e-6, err
+
+
 @pytest.mark.parametrize("H, G, d, e", [(4, 1, 64, 128), (4, 2, 16, 64), (2, 2, 72, 72), (3, 1, 128, 8)])
 @pytest.mark.parametrize("window, kept", [(0, 0), (40, 0), (512, 4), (512, 70), (1, 33)])
 @pytest.mark.parametrize("copies", [1, 60])
