@@ -1,0 +1,458 @@
+// Recurrences with a matrix state per head and one decay a token and head, for prompts, by chunks of 32 tokens:
+//
+//   S_t = a_t S_(t-1) + b_t k_t v_t^T,   y_t = scale S_t^T q_t        (S [d][e], query/key head j = h / (H / G))
+//
+// With L_t the sum of log a up to token t of a chunk that starts from state S,
+//   y_t = scale (exp(L_t) S^T q_t + sum over s <= t of exp(L_t - L_s) b_s (q_t . k_s) v_s),
+//   S  <- exp(L_end) S + sum over t of exp(L_end - L_t) b_t k_t v_t^T,
+// so what a token-by-token walk does in d x e steps of its own are three small products a chunk.  `state_prepare_kernel`
+// (a block per chunk and key head, all chunks side by side) makes P[t][s] = scale exp(L_t - L_s) b_s (q_t . k_s), which knows
+// nothing of the state, and the tokens' scales; `state_chunks_kernel` (a block per sequence, head and 64 value columns, the
+// state in shared memory) walks the chunks: [exp(L) q, P] [S; v] is one product, whose sums two halves of the block share,
+// then the state's update.  A thread has four by four outputs and eight rows by four columns of the state; sums go in pairs
+// of neighbouring rows (packed multiply-adds).  Bound by what shared memory delivers (84% of its rate with all SMs full; the
+// multiply-adds, which would bound it next, 55%).  Eight sequences of 1,024 tokens, 128 heads of 128 x 64: 2,054 us as
+// segments walked token by token, 1,188 so; 16 heads of 128 x 128 with a matrix memory 1,342 and 421; with 16 columns a
+// block, for which every q and k is read four times as often, 1,689 and 552.
+// All float32 but for the sums L and their differences, which are float64: a sum that has passed a strong decay is large, and
+// a difference of two of them would keep few digits in 32 bits.  Decays only appear as exponentials of differences that are
+// not positive.
+// Kinds: MAMBA   q = C, k = B, v = x, a = exp(-exp(A_log) dt), b = dt = softplus(raw + bias), y + D x
+//        LIGHTNING q, k, v through SiLU, a one number a head, b = 1
+//        MEMORY  a, b and exp(-m) as `exp_gates` leaves them; values of one make the normalizer n (the first block of a
+//                head has it beside its columns), of which the divisor max(|scale n . q|, exp(-m)) + 1e-6 is kept
+#include <stdio.h>
+
+#include "common.cuh"
+
+namespace {
+
+constexpr int C = 32, DMAX = 128, LD = DMAX + 4, THREADS = 256;
+constexpr int P_FLOATS = C * C, SC_FLOATS = 4 * C, QK_FLOATS = 2 * C * DMAX;
+constexpr float DEN_FLOOR = 1e-6f;
+enum { MAMBA = 0, LIGHTNING = 1, MEMORY = 2 };
+// scratch of a chunk and head: P, the scales, and for LIGHTNING the activated q and k
+__host__ __device__ constexpr int scratch_floats(int kind) { return P_FLOATS + SC_FLOATS + (kind == LIGHTNING ? QK_FLOATS : 0); }
+
+__device__ __forceinline__ float silu(float z) { return z / (1.0f + expf(-z)); }
+__device__ __forceinline__ float4 silu4(float4 z) { return make_float4(silu(z.x), silu(z.y), silu(z.z), silu(z.w)); }
+
+struct Args {
+  const float* proj;      // rows of ld: q, k and v at their columns
+  int ld, q_col, k_col, v_col;
+  const float* gates;     // MAMBA: raw dt, rows of ld_gates; MEMORY: [T][H][4] of a, b, exp(-m)
+  int ld_gates;
+  const float* rate;      // MAMBA: A_log [H]; LIGHTNING: a [H]
+  const float* bias;      // MAMBA: dt_bias [H]
+  const float* skip;      // MAMBA: D [H]
+  float scale;
+  float* out;             // [T][H e]
+  float* den;             // MEMORY: [T][H]
+  float* state;
+  long long slot_stride, state_off;
+  const int* q_start;
+  const int* seq_slot;
+  int H, G, d, e;
+  float* scratch;
+  int first_tile, tiles, heads_here;
+};
+
+template <int KIND>
+__global__ void __launch_bounds__(THREADS) state_prepare_kernel(const Args a) {
+  __shared__ __align__(16) float q_s[C][LD], k_s[C][LD];
+  __shared__ float qk_s[C][C + 1];
+  jb::pdl_launch_dependents();
+  const int seq = blockIdx.x / a.tiles, tile = blockIdx.x % a.tiles, R = a.H / a.G, j = blockIdx.y;
+  const int h_begin = j * R + (int)blockIdx.z * a.heads_here, h_end = min((j + 1) * R, h_begin + a.heads_here);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  jb::pdl_wait();
+  const int t0 = a.q_start[seq] + (a.first_tile + tile) * C, n = min(C, a.q_start[seq + 1] - t0);
+  if (n <= 0) return;
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  float4 qv[4], kv[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int t = 4 * warp + u;
+    const bool in = t < n && 4 * lane < a.d;
+    const float* row = a.proj + (size_t)(t0 + (t < n ? t : 0)) * a.ld + (size_t)j * a.d + (in ? 4 * lane : 0);
+    qv[u] = in ? *reinterpret_cast<const float4*>(row + a.q_col) : zero;
+    kv[u] = in ? *reinterpret_cast<const float4*>(row + a.k_col) : zero;
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int t = 4 * warp + u;
+    if (KIND == LIGHTNING) {                                   // (silu(0) is 0)
+      qv[u] = silu4(qv[u]), kv[u] = silu4(kv[u]);
+      float* QK_g = a.scratch + ((size_t)blockIdx.x * a.H + j) * scratch_floats(KIND) + P_FLOATS + SC_FLOATS;   // G = H here
+      *reinterpret_cast<float4*>(QK_g + t * DMAX + 4 * lane) = qv[u];
+      *reinterpret_cast<float4*>(QK_g + (C + t) * DMAX + 4 * lane) = kv[u];
+    }
+    *reinterpret_cast<float4*>(&q_s[t][4 * lane]) = qv[u];
+    *reinterpret_cast<float4*>(&k_s[t][4 * lane]) = kv[u];
+  }
+  __syncthreads();
+  {
+    jb::Pair qk[2][2] = {{0, 0}, {0, 0}};                      // two by two entries a thread; above the diagonal nobody reads
+#pragma unroll 4
+    for (int r = 0; r < DMAX; r += 4) {
+      ulonglong2 b[2], c[2];
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        b[x] = *reinterpret_cast<const ulonglong2*>(&q_s[ty + 16 * x][r]);
+        c[x] = *reinterpret_cast<const ulonglong2*>(&k_s[tx + 16 * x][r]);
+      }
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y <= x; ++y) qk[x][y] = jb::fma2(b[x].y, c[y].y, jb::fma2(b[x].x, c[y].x, qk[x][y]));
+    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+      for (int y = 0; y < 2; ++y) qk_s[ty + 16 * x][tx + 16 * y] = jb::lo(qk[x][y]) + jb::hi(qk[x][y]);
+  }
+  __syncthreads();
+  for (int h = h_begin + warp; h < h_end; h += THREADS / 32) { // a head a warp, a token a lane
+    float log_a = 0.0f, b = 0.0f, floor = 0.0f;
+    if (lane < n) {
+      const size_t t = (size_t)(t0 + lane);
+      if (KIND == MAMBA) {
+        const float z = a.gates[t * a.ld_gates + h] + a.bias[h];
+        b = z > 20.0f ? z : log1pf(expf(z));
+        log_a = -expf(a.rate[h]) * b;
+      } else if (KIND == LIGHTNING) {
+        b = 1.0f;
+        log_a = logf(a.rate[h]);
+      } else {
+        const float* g = a.gates + (t * a.H + h) * 4;
+        log_a = logf(g[0]), b = g[1], floor = g[2];
+      }
+      log_a = fmaxf(log_a, -10000.0f);                         // a decay of zero; the sums stay finite
+    }
+    double L = log_a;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double before = __shfl_up_sync(0xffffffffu, L, o);
+      if (lane >= o) L += before;
+    }
+    const double end = __shfl_sync(0xffffffffu, L, 31);
+    float* P_g = a.scratch + ((size_t)blockIdx.x * a.H + h) * scratch_floats(KIND);
+    // per token: what multiplies q_t S, what multiplies k_t on its way into the state, the chunk's decay, exp(-m)
+    reinterpret_cast<float4*>(P_g + P_FLOATS)[lane] = make_float4(expf((float)L) * a.scale, expf((float)(end - L)) * b, expf((float)end), floor);
+#pragma unroll 8
+    for (int t = 0; t < C; ++t) {
+      const double Lt = __shfl_sync(0xffffffffu, L, t);
+      P_g[t * C + lane] = lane <= t ? expf((float)(Lt - L)) * b * a.scale * qk_s[t][lane] : 0.0f;
+    }
+  }
+}
+
+// copies 16 bytes, or zeros
+__device__ __forceinline__ void async16(float* dst, const float* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(in ? 16 : 0));
+}
+__device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;"); }
+
+constexpr int COLS = 64, SLD = 2 * COLS + 4;   // columns of a block; floats of a pair of the state's rows, and padding
+constexpr int VLD = COLS + 4;
+template <int KIND, int D>
+constexpr int chunk_smem() {
+  return (3 * C * (D + 4) + 2 * C * (C + 4) + 2 * SC_FLOATS + (D + C) / 2 * SLD + C * VLD + (KIND == MEMORY ? D : 0)) * 4;
+}
+
+// D: keys' numbers at most.  Eight warps: four of 16 columns, twice, for the two halves of the sums over keys and tokens.
+template <int KIND, int D>
+__global__ void __launch_bounds__(THREADS, 2) state_chunks_kernel(const Args a) {
+  constexpr int LDD = D + 4, RT = D / 16;      // RT: the state's rows a thread updates, of four columns
+  extern __shared__ __align__(16) float smem[];
+  float* q_b = smem;                           // two buffers of q [C][LDD]
+  float* k_s = q_b + 2 * C * LDD;              // k [C][LDD]
+  float* P_b = k_s + C * LDD;                  // two buffers of P [C][C + 4]
+  float4* sc_b = reinterpret_cast<float4*>(P_b + 2 * C * (C + 4));         // two buffers of the scales [C]
+  float* S_s = P_b + 2 * C * (C + 4) + 2 * SC_FLOATS;                      // [D / 2][SLD]: two rows of a column are neighbours
+  float* v_s = S_s + D / 2 * SLD;              // the values, laid out as more rows of the state
+  float* vk_s = v_s + C / 2 * SLD;             // the values as they join the state [C][VLD]
+  float* n_s = vk_s + C * VLD;                 // MEMORY: the normalizer [D], of the first column block
+  jb::pdl_launch_dependents();
+  const int seq = blockIdx.z, h = blockIdx.y, c0 = blockIdx.x * COLS, H = a.H, d = a.d, e = a.e, j = h / (H / a.G);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool pairs = ((e | a.v_col) & 1) == 0 && ((uintptr_t)a.out & 7) == 0;          // columns go two at a time
+  const bool has_n = KIND == MEMORY && blockIdx.x == 0;
+  jb::pdl_wait();
+  const int begin = a.q_start[seq] + a.first_tile * C, n_all = min(a.q_start[seq + 1] - begin, a.tiles * C);
+  if (n_all <= 0) return;
+  float* S_g = a.state + (size_t)a.seq_slot[seq] * a.slot_stride + a.state_off + (size_t)h * d * (e + (KIND == MEMORY ? 1 : 0));
+  const float* scratch_g = a.scratch + ((size_t)seq * a.tiles * H + h) * scratch_floats(KIND);
+  const size_t per_chunk = (size_t)H * scratch_floats(KIND);
+  const int chunks = (n_all + C - 1) / C;
+
+  auto load_rows = [&](float* dst, int chunk, int col, int which) {
+    const int t0 = begin + chunk * C, n = min(C, n_all - chunk * C);
+    for (int i = tid; i < C * D / 4; i += THREADS) {
+      const int t = i / (D / 4), r = (i % (D / 4)) * 4;
+      if (KIND == LIGHTNING) {
+        async16(dst + t * LDD + r, scratch_g + chunk * per_chunk + P_FLOATS + SC_FLOATS + (which * C + t) * DMAX + r, true);
+      } else {
+        const bool in = t < n && r < d;
+        async16(dst + t * LDD + r, a.proj + (size_t)(t0 + (in ? t : 0)) * a.ld + col + (size_t)j * d + (in ? r : 0), in);
+      }
+    }
+  };
+  auto load_qp = [&](int chunk) {
+    if (chunk < chunks) {
+      load_rows(q_b + (chunk & 1) * C * LDD, chunk, a.q_col, 0);
+      const float* P_g = scratch_g + chunk * per_chunk;
+      async16(P_b + (chunk & 1) * C * (C + 4) + (tid / 8) * (C + 4) + (tid % 8) * 4, P_g + tid * 4, true);     // 256 pieces
+      if (tid < C) async16(reinterpret_cast<float*>(sc_b + (chunk & 1) * C + tid), P_g + P_FLOATS + 4 * tid, true);
+    }
+    commit();
+  };
+  auto load_k = [&](int chunk) {
+    if (chunk < chunks) load_rows(k_s, chunk, a.k_col, 1);
+    commit();
+  };
+  // values: a thread two neighbouring columns of every 16 of a token, and what the token's key is worth, a chunk ahead
+  const int vt = tid >> 3, vc = (tid & 7) * 2;
+  float2 v[COLS / 16];
+  float v_scale;
+  auto fetch_v = [&](int chunk) {
+    const bool in = vt < n_all - chunk * C;
+    const float* row = a.proj + (size_t)(begin + chunk * C + (in ? vt : 0)) * a.ld + a.v_col + (size_t)h * e;
+    v_scale = chunk < chunks ? scratch_g[chunk * per_chunk + P_FLOATS + 4 * vt + 1] : 0.0f;
+#pragma unroll
+    for (int i = 0; i < COLS / 16; ++i) {
+      const int c = c0 + 16 * i + vc;
+      v[i] = make_float2(0.0f, 0.0f);
+      if (in && pairs && c < e) v[i] = *reinterpret_cast<const float2*>(row + c);
+      if (in && !pairs) v[i] = make_float2(c < e ? row[c] : 0.0f, c + 1 < e ? row[c + 1] : 0.0f);
+    }
+  };
+  auto store_v = [&] {
+#pragma unroll
+    for (int i = 0; i < COLS / 16; ++i) {
+      if (KIND == LIGHTNING) v[i] = make_float2(silu(v[i].x), silu(v[i].y));
+      float* at = v_s + (vt >> 1) * SLD + 2 * (16 * i + vc) + (vt & 1);
+      at[0] = v[i].x, at[2] = v[i].y;
+      *reinterpret_cast<float2*>(vk_s + vt * VLD + 16 * i + vc) = make_float2(v[i].x * v_scale, v[i].y * v_scale);
+    }
+  };
+  load_qp(0);
+  load_k(0);
+  fetch_v(0);
+  for (int i = tid; i < D * COLS; i += THREADS) {
+    const int r = i / COLS, c = i % COLS;
+    S_s[(r >> 1) * SLD + 2 * c + (r & 1)] = (r < d && c0 + c < e) ? S_g[(size_t)r * e + c0 + c] : 0.0f;
+  }
+  if (has_n && tid < D) n_s[tid] = tid < d ? S_g[(size_t)d * e + tid] : 0.0f;
+  store_v();
+
+  // outputs: a thread four tokens tg + 8 i and four columns, col[x] and the one after it, over one half of the sums
+  const int half = warp >> 2, tg = lane >> 2;
+  const int col[2] = {16 * (warp & 3) + 2 * (lane & 3), 16 * (warp & 3) + 8 + 2 * (lane & 3)};
+  // state's update: a thread RT rows, columns uc, uc + 1, uc + 16 and uc + 17
+  const int ur = ((warp >> 1) * 4 + (lane >> 3)) * RT, uc = (warp & 1) * 32 + 2 * (lane & 7);
+  const float skip = KIND == MAMBA ? a.skip[h] : 0.0f;
+
+  for (int chunk = 0; chunk < chunks; ++chunk) {
+    const int t0 = begin + chunk * C, n = min(C, n_all - chunk * C);
+    // copies in flight, oldest first: q and P of this chunk, k of it
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();                                                       // values and state are whole too
+    load_qp(chunk + 1);
+    fetch_v(chunk + 1);
+    float* q_s = q_b + (chunk & 1) * C * LDD;
+    const float* P_s = P_b + (chunk & 1) * C * (C + 4);
+    const float4* sc_s = sc_b + (chunk & 1) * C;
+    float o[4][4];
+    {
+      jb::Pair acc[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) acc[i][x] = 0;
+      // four numbers of the rows' left factors at L, of which the right ones lie at R
+      const auto step = [&](const float* L, int ld, const float* R) {
+        ulonglong2 l4[4], b[2][2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) l4[i] = *reinterpret_cast<const ulonglong2*>(L + (tg + 8 * i) * ld);
+#pragma unroll
+        for (int y = 0; y < 2; ++y)
+#pragma unroll
+          for (int x = 0; x < 2; ++x) b[y][x] = *reinterpret_cast<const ulonglong2*>(R + y * SLD + 2 * col[x]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            acc[i][2 * x] = jb::fma2(l4[i].y, b[1][x].x, jb::fma2(l4[i].x, b[0][x].x, acc[i][2 * x]));
+            acc[i][2 * x + 1] = jb::fma2(l4[i].y, b[1][x].y, jb::fma2(l4[i].x, b[0][x].y, acc[i][2 * x + 1]));
+          }
+      };
+#pragma unroll 2
+      for (int k = half * (D / 2); k < (half + 1) * (D / 2); k += 4) step(q_s + k, LDD, S_s + (k >> 1) * SLD);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float s = sc_s[tg + 8 * i].x;
+        const jb::Pair ss = jb::pair(s, s);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) acc[i][x] = jb::mul2(acc[i][x], ss);
+      }
+#pragma unroll 2
+      for (int s = half * (C / 2); s < (half + 1) * (C / 2); s += 4) step(P_s + s, C + 4, v_s + (s >> 1) * SLD);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) o[i][x] = jb::lo(acc[i][x]) + jb::hi(acc[i][x]);
+    }
+    if (KIND == MAMBA) {                                                   // D x, by the half that keeps the token
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if ((i >> 1) == half) {
+          const int t = tg + 8 * i;
+#pragma unroll
+          for (int x = 0; x < 4; ++x) o[i][x] = fmaf(skip, v_s[(t >> 1) * SLD + 2 * (col[x >> 1] + (x & 1)) + (t & 1)], o[i][x]);
+        }
+    }
+    if (has_n) {                                                           // divisors: eight lanes a token
+      const int l = tid & 7;
+      float dot = 0.0f, ones = 0.0f;
+#pragma unroll
+      for (int r = 4 * l; r < D; r += 32) {
+        const float4 x = *reinterpret_cast<const float4*>(q_s + vt * LDD + r), y = *reinterpret_cast<const float4*>(n_s + r);
+        dot = fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, fmaf(x.w, y.w, dot))));
+      }
+      const float4 p = *reinterpret_cast<const float4*>(P_s + vt * (C + 4) + 4 * l), sc = sc_s[vt];
+      ones = (p.x + p.y) + (p.z + p.w);
+      dot = fmaf(dot, sc.x, ones);
+      dot += __shfl_xor_sync(0xffffffffu, dot, 1);
+      dot += __shfl_xor_sync(0xffffffffu, dot, 2);
+      dot += __shfl_xor_sync(0xffffffffu, dot, 4);
+      if (l == 0 && vt < n) a.den[(size_t)(t0 + vt) * H + h] = fmaxf(fabsf(dot), sc.w) + DEN_FLOOR;
+    }
+    // in flight: k of this chunk, q and P of the next
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();                                                       // q, P, the values and the state have been read, k is there
+    // the halves meet: each keeps two tokens and hands the other its part of the rest, where q was
+    float4* hand = reinterpret_cast<float4*>(q_s) + (tid & 127);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if ((i >> 1) != half) hand[128 * i] = make_float4(o[i][0], o[i][1], o[i][2], o[i][3]);
+    {
+      jb::Pair S[RT / 2][4];
+      const float decay = sc_s[0].z;
+      const jb::Pair g = jb::pair(decay, decay);
+#pragma unroll
+      for (int p = 0; p < RT / 2; ++p)
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const ulonglong2 old = *reinterpret_cast<const ulonglong2*>(S_s + ((ur >> 1) + p) * SLD + 2 * (uc + 16 * x));
+          S[p][2 * x] = jb::mul2(old.x, g);
+          S[p][2 * x + 1] = jb::mul2(old.y, g);
+        }
+#pragma unroll 4
+      for (int t = 0; t < C; ++t) {
+        ulonglong2 k[RT / 4];
+#pragma unroll
+        for (int p = 0; p < RT / 4; ++p) k[p] = *reinterpret_cast<const ulonglong2*>(k_s + t * LDD + ur + 4 * p);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const float2 w = *reinterpret_cast<const float2*>(vk_s + t * VLD + uc + 16 * x);
+          const jb::Pair w0 = jb::pair(w.x, w.x), w1 = jb::pair(w.y, w.y);
+#pragma unroll
+          for (int p = 0; p < RT / 4; ++p) {
+            S[2 * p][2 * x] = jb::fma2(k[p].x, w0, S[2 * p][2 * x]);
+            S[2 * p][2 * x + 1] = jb::fma2(k[p].x, w1, S[2 * p][2 * x + 1]);
+            S[2 * p + 1][2 * x] = jb::fma2(k[p].y, w0, S[2 * p + 1][2 * x]);
+            S[2 * p + 1][2 * x + 1] = jb::fma2(k[p].y, w1, S[2 * p + 1][2 * x + 1]);
+          }
+        }
+      }
+#pragma unroll
+      for (int p = 0; p < RT / 2; ++p)
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+          *reinterpret_cast<ulonglong2*>(S_s + ((ur >> 1) + p) * SLD + 2 * (uc + 16 * x)) = make_ulonglong2(S[p][2 * x], S[p][2 * x + 1]);
+    }
+    if (has_n && tid < D) {                                                // n <- decay n + the sum of b k
+      float s = n_s[tid] * sc_s[0].z;
+#pragma unroll 8
+      for (int t = 0; t < C; ++t) s = fmaf(k_s[t * LDD + tid], sc_s[t].y, s);
+      n_s[tid] = s;
+    }
+    __syncthreads();                                                       // k has been read, the parts are there
+    load_k(chunk + 1);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if ((i >> 1) == half) {
+        const float4 part = hand[128 * i];
+        const int t = tg + 8 * i;
+        const float y[4] = {o[i][0] + part.x, o[i][1] + part.y, o[i][2] + part.z, o[i][3] + part.w};
+        if (t < n) {
+          float* dst = a.out + ((size_t)(t0 + t) * H + h) * e + c0;
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const int c = col[x];
+            if (pairs) {
+              if (c0 + c < e) *reinterpret_cast<float2*>(dst + c) = make_float2(y[2 * x], y[2 * x + 1]);
+            } else {
+              if (c0 + c < e) dst[c] = y[2 * x];
+              if (c0 + c + 1 < e) dst[c + 1] = y[2 * x + 1];
+            }
+          }
+        }
+      }
+    store_v();                                                             // the next chunk's
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  for (int i = tid; i < D * COLS; i += THREADS) {
+    const int r = i / COLS, c = i % COLS;
+    if (r < d && c0 + c < e) S_g[(size_t)r * e + c0 + c] = S_s[(r >> 1) * SLD + 2 * c + (r & 1)];
+  }
+  if (has_n && tid < d) S_g[(size_t)d * e + tid] = n_s[tid];
+}
+
+template <int KIND, int D>
+int launch(Args a, int n_seqs, int max_q_len, cudaStream_t stream) {
+  constexpr int smem = chunk_smem<KIND, D>();
+  cudaError_t e = cudaFuncSetAttribute(state_chunks_kernel<KIND, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return (int)e;
+  const int group = a.H / a.G;
+  // a block makes the products of a chunk and key head once for its group's heads, or for a share of them where that
+  // leaves SMs without a block
+  const long long chunks = (long long)n_seqs * a.tiles * a.G;
+  int parts = (int)((2 * 148 + chunks - 1) / chunks);
+  parts = parts < group ? parts : group;
+  a.heads_here = (group + parts - 1) / parts;
+  for (a.first_tile = 0; a.first_tile * C < max_q_len; a.first_tile += a.tiles) {
+    jb::Launch prepare(dim3(n_seqs * a.tiles, a.G, (group + a.heads_here - 1) / a.heads_here), dim3(THREADS), 0, stream);
+    e = cudaLaunchKernelEx(&prepare.c, state_prepare_kernel<KIND>, a);
+    if (e != cudaSuccess) return (int)e;
+    jb::Launch walk(dim3((a.e + COLS - 1) / COLS, a.H, n_seqs), dim3(THREADS), smem, stream);
+    e = cudaLaunchKernelEx(&walk.c, state_chunks_kernel<KIND, D>, a);
+    if (e != cudaSuccess) return (int)e;
+  }
+  return 0;
+}
+
+}  // namespace
+
+// kind: 0 state-space (MAMBA), 1 LIGHTNING, 2 matrix MEMORY, see the top.  d <= 128; d, ld, q_col and k_col multiples of 4,
+// proj and scratch 16-byte aligned.  `scratch` holds `tiles` chunks of every sequence (H * 1152 floats a chunk, LIGHTNING
+// H * 9344); longer prompts go in slabs of as many, one after another from the state the last left.
+JB_EXPORT int jb_state_chunks(int kind, const float* proj, int ld, int q_col, int k_col, int v_col, const float* gates,
+                              int ld_gates, const float* rate, const float* bias, const float* skip, float scale, float* out,
+                              float* den, float* state, long long slot_stride, long long state_off, const int* q_start,
+                              const int* seq_slot, int n_seqs, int H, int G, int d, int e, int max_q_len, float* scratch,
+                              int tiles, cudaStream_t stream) {
+  if (n_seqs <= 0 || max_q_len <= 0) return 0;
+  JB_REFUSE(d < 1 || d > DMAX || e < 1 || ((d | ld | q_col | k_col) & 3) != 0 || (((uintptr_t)proj | (uintptr_t)scratch) & 15) != 0,
+            "state_chunks: keys of %d numbers in rows of %d at columns %d and %d", d, ld, q_col, k_col);
+  JB_REFUSE(G < 1 || H % G != 0 || tiles < 1 || (kind == LIGHTNING && G != H), "state_chunks: %d heads, %d key heads, %d tiles", H, G, tiles);
+  const Args a{proj, ld, q_col, k_col, v_col, gates, ld_gates, rate, bias, skip, scale, out, den, state, slot_stride, state_off,
+               q_start, seq_slot, H, G, d, e, scratch, 0, tiles, 0};
+  const auto run = [&](auto small, auto large) { return (d <= 64 ? small : large)(a, n_seqs, max_q_len, stream); };
+  if (kind == MAMBA) return run(launch<MAMBA, 64>, launch<MAMBA, 128>);
+  if (kind == LIGHTNING) return run(launch<LIGHTNING, 64>, launch<LIGHTNING, 128>);
+  JB_REFUSE(kind != MEMORY, "state_chunks: kind %d", kind);
+  return run(launch<MEMORY, 64>, launch<MEMORY, 128>);
+}

@@ -70,6 +70,7 @@ _SIGNATURES = {
     "jb_delta_rule": "piiiipiiippfppllppiiiiip", "jb_delta_rule_chunks": "piiiipiiippfppllppiiiiiipip",
     "jb_route_topk": "piiippiiiipfip", "jb_experts_few_tokens": "pippipppippiiiiffip", "jb_expert_gather": "pippipiip", "jb_experts_few_tokens_tc": "pppipppppiiiiffip",
     "jb_expert_scatter": "pppipiip",
+    "jb_state_chunks": "ipiiiipipppfpppllppiiiiiipip",
     "jb_gla_decay": "piiippfpiip", "jb_exp_gates": "piiippfppllppiip",
     "jb_gated_linear_scan": "piiiifpiippplppiiiiiippp", "jb_scale_rows_sigmoid": "pipiiip",
     "jb_attention_tc_prefill": "pppppppiiiiiiiiiifpp", "jb_attention_tc_prefill_capped": "pppppppiiiiiiiiiiififfpppipp",
@@ -1133,13 +1134,59 @@ def streams_mix_rmsnorm(x: torch.Tensor, y: torch.Tensor, mix: torch.Tensor, out
 LIGHTNING_SEGMENT = 128       # tokens of a segment when a long prompt's recurrence runs in segments side by side
 
 
+# -- recurrences with a matrix state and one decay a token and head, by chunks of tokens -----------------------------
+STATE_CHUNK = 32
+STATE_CHUNKS_FROM = 128               # longest sequence's tokens from which chunks are taken
+STATE_WALK_TOKENS = 256               # ... and up to which the walks have no segments
+STATE_SCRATCH_BYTES = 64 << 20        # at most: longer prompts go through it slab by slab
+_STATE_KINDS = {"mamba": (0, STATE_CHUNK * (STATE_CHUNK + 4)),
+                "lightning": (1, STATE_CHUNK * (STATE_CHUNK + 4 + 256)),      # and the activated queries and keys
+                "memory": (2, STATE_CHUNK * (STATE_CHUNK + 4))}
+
+
+def state_chunks_pay(kind: str, n_seqs: int, heads: int, dim: int, vdim: int, max_q_len: int) -> bool:
+    """Whether chunks are the faster form.  A block (64 value columns of a head) walks its sequence's chunks, 5 to 9 us
+    each, so long prompts need blocks for all SMs; segments walked token by token make up for few sequences.  Walk and
+    chunks, microseconds: 16 heads of 128 x 128 with a matrix memory, one sequence, 128 tokens 82.7 and 49.9, 256 tokens 162
+    and 96, 1,024 tokens 151 and 349; four sequences of 1,024 tokens (128 blocks) 491 and 382, eight 1,342 and 421.
+    Lightning, the same heads, four sequences of 1,024 tokens 430 and 302, eight 817 and 461.  State space, 32 heads of 128
+    x 64, four sequences of 1,024 tokens (128 blocks) 317 and 328, eight 616 and 334; 128 heads, eight of 512 1,114 and 615.
+    At 64 tokens the two are even (24 and 21, 31 and 33)."""
+    if max_q_len < STATE_CHUNKS_FROM or dim > 128:
+        return False
+    blocks = n_seqs * heads * -(-vdim // 64)
+    return max_q_len <= STATE_WALK_TOKENS or blocks >= (128 if dim > 64 and kind != "mamba" else 148)
+
+
+def _state_chunks(kind: str, workspace, proj: torch.Tensor, q_col: int, k_col: int, v_col: int, gates, ld_gates: int, rate,
+                  bias, skip, scale: float, out, den, state, slot_stride: int, state_off: int, q_start, seq_slot, n_seqs: int,
+                  heads: int, kv_heads: int, dim: int, vdim: int, max_q_len: int) -> bool:
+    """Runs a prompt's recurrence by chunks of 32 tokens where that pays and is possible (scratch to be had, keys whose
+    rows are whole 16-byte vectors); False: it was not."""
+    if workspace is None or not state_chunks_pay(kind, n_seqs, heads, dim, vdim, max_q_len):
+        return False
+    if any(x % 4 for x in (dim, proj.shape[1], q_col, k_col)) or proj.data_ptr() % 16:
+        return False
+    code, per_head = _STATE_KINDS[kind]
+    tiles = (max_q_len + STATE_CHUNK - 1) // STATE_CHUNK
+    slab = max(1, min(tiles, STATE_SCRATCH_BYTES // (4 * per_head * n_seqs * heads)))
+    scratch = workspace.get("state_chunks", (per_head * n_seqs * heads * slab,), torch.float32)
+    _check(_lib("state_chunks").jb_state_chunks(
+        code, _ptr(proj), proj.shape[1], int(q_col), int(k_col), int(v_col), _ptr(gates), int(ld_gates), _ptr(rate), _ptr(bias),
+        _ptr(skip), float(scale), _ptr(out), _ptr(den), _ptr(state), int(slot_stride), int(state_off), _ptr(q_start),
+        _ptr(seq_slot), n_seqs, heads, kv_heads, dim, vdim, int(max_q_len), _ptr(scratch), slab, _stream()),
+        "state_chunks " + kind, kernels=2 * -(-tiles // slab))
+    return True
+
+
 def lightning_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, out: torch.Tensor, state: torch.Tensor,
                    q_start: torch.Tensor, seq_slot: torch.Tensor, decay: torch.Tensor, n_seqs: int, heads: int,
                    dim: int, vdim: int, max_q_len: int = 1, workspace=None) -> None:
     """Per sequence and head S <- decay S + silu(k_t) silu(v_t)^T, out_t = S^T silu(q_t) over the step's tokens in
     order; proj float32 [T, ld] holds the raw q, k, v at the given columns; state float32 [slots, heads, dim, vdim].
-    With a workspace, steps whose longest sequence brings more than two segments of tokens run in three passes over
-    segments (their states from zero, a prefix pass, the outputs), 3 launches; else one launch."""
+    With a workspace, prompts go by chunks of tokens where that pays; else steps whose longest sequence brings more than
+    two segments of tokens run in three passes over segments (their states from zero, a prefix pass, the outputs), 3
+    launches; else one launch."""
     T = proj.shape[0]
     _need(proj, "lightning projections", torch.float32)
     _need(out, "lightning out", torch.float32, (T, heads * vdim))
@@ -1151,6 +1198,9 @@ def lightning_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, out: 
     _need(decay, "decay", torch.float32, (heads,))
     if max(q_col + heads * dim, k_col + heads * dim, v_col + heads * vdim) > proj.shape[1]:
         raise KernelError("lightning_scan: the projections' columns reach past the rows")
+    if _state_chunks("lightning", workspace, proj, q_col, k_col, v_col, None, 0, decay, None, None, 1.0, out,
+                     None, state, heads * dim * vdim, 0, q_start, seq_slot, n_seqs, heads, heads, dim, vdim, max_q_len):
+        return
     seg, scratch = 0, None
     if workspace is not None and max_q_len > 2 * LIGHTNING_SEGMENT:
         seg = LIGHTNING_SEGMENT
@@ -1468,9 +1518,9 @@ def mamba2_scan(xbc: torch.Tensor, b_col: int, c_col: int, dt_raw: torch.Tensor,
     dt_t = softplus(dt_raw_t + dt_bias) and a_t = exp(-exp(a_log) dt_t).  xbc float32 [T, ld]: x in columns
     [0, heads vdim), B at b_col and C at c_col ([groups][n_state]); dt_raw a float32 view [T, heads] of wider rows;
     state float32 [slots, n] with the recurrence's [heads, n_state, vdim] block at offset state_off of a slot's row.
-    With a workspace, steps whose longest sequence brings more than two segments of tokens run in three passes over
-    segments (3 launches), else one launch.  `single_tokens`: every sequence
-    brings one token (the state is read and written once)."""
+    With a workspace, prompts go by chunks of tokens where that pays; else steps whose longest sequence brings more than
+    two segments of tokens run in three passes over segments (3 launches), else one launch.  `single_tokens`: every
+    sequence brings one token (the state is read and written once)."""
     T = xbc.shape[0]
     _need(xbc, "convolved x, B, C", torch.float32)
     _need(out, "scan out", torch.float32, (T, heads * vdim))
@@ -1487,6 +1537,10 @@ def mamba2_scan(xbc: torch.Tensor, b_col: int, c_col: int, dt_raw: torch.Tensor,
         raise KernelError("mamba2_scan: the columns reach past the rows")
     if single_tokens and T != n_seqs:
         raise KernelError("mamba2_scan: single_tokens needs one token per sequence")
+    if not single_tokens and _state_chunks("mamba", workspace, xbc, c_col, b_col, 0, dt_raw, dt_raw.stride(0), a_log, dt_bias,
+                                           d_skip, 1.0, out, None, state, state.shape[1], state_off, q_start, seq_slot, n_seqs,
+                                           heads, groups, n_state, vdim, max_q_len):
+        return
     seg, scratch, seg_decay = -1 if single_tokens else 0, None, None
     if workspace is not None and max_q_len > 2 * MAMBA2_SEGMENT and not single_tokens:
         seg = mamba2_segment_for(n_seqs, max_q_len, heads, n_state, vdim)
@@ -1859,8 +1913,9 @@ def gated_linear_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, q_
     [T, heads dim], a decay per key channel, b = 1, and a slot's state row holds [heads, dim, vdim].  With `divisors`
     (float32 [T, heads], written), `decays` is what `exp_gates` left ([T, heads, 4]: a_t and b_t one number a head),
     a normalizer n <- a_t n + b_t k_t walks along, divisors[t, h] = max(|n . q|, exp(-m_t)) + 1e-6, and a slot's state
-    row holds per head [dim, vdim] then [dim] of n.  With a workspace, steps whose longest sequence brings more than
-    256 tokens run in passes over segments of 64 to 256 tokens (4 launches); else one launch.  `single_tokens`: every
+    row holds per head [dim, vdim] then [dim] of n.  With a workspace, prompts with `divisors` go by chunks of tokens where
+    that pays; else steps whose longest sequence brings more than 256 tokens run in passes over segments of 64 to 256
+    tokens (4 launches); else one launch.  `single_tokens`: every
     sequence brings one token (the state is read and written once)."""
     T = proj.shape[0]
     scalar = divisors is not None
@@ -1879,6 +1934,10 @@ def gated_linear_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, q_
         raise KernelError("gated_linear_scan: the projections' columns reach past the rows")
     if single_tokens and T != n_seqs:
         raise KernelError("gated_linear_scan: single_tokens needs one token per sequence")
+    if scalar and not single_tokens and _state_chunks("memory", workspace, proj, q_col, k_col, v_col, decays, 0, None, None, None,
+                                                      q_scale, out, divisors, state, state.shape[1], 0, q_start, seq_slot,
+                                                      n_seqs, heads, heads, dim, vdim, max_q_len):
+        return
     seg, scratch, seg_decay = -1 if single_tokens else 0, None, None
     if workspace is not None and max_q_len > 2 * GATED_LINEAR_SEGMENT and not single_tokens:
         # the blocks are laid out as the state-space recurrence's (a segment, a head, 64 value columns; four blocks an SM

@@ -374,6 +374,86 @@ def test_state_steps(ops, n_seqs, H, d, e, kind):
         assert torch.equal(state[n_seqs], before[n_seqs])
 
 
+class Scratch:
+    def __init__(self):
+        self.asked = []
+
+    def get(self, name, shape, dtype):
+        self.asked.append(name)
+        return torch.full(shape, float("nan"), dtype=dtype, device=DEV)
+
+
+@pytest.mark.parametrize("H, G, d, e", [(2, 2, 128, 128), (4, 4, 64, 24), (3, 3, 20, 17), (2, 2, 4, 33), (6, 6, 128, 66), (2, 2, 68, 64), (2, 2, 64, 130)])
+@pytest.mark.parametrize("lens", [[64], [65, 1, 31, 32, 33], [300, 3]])
+@pytest.mark.parametrize("kind", ["mamba", "lightning", "memory"])
+@pytest.mark.parametrize("slab", [0, 2])
+def test_state_chunks(ops, monkeypatch, H, G, d, e, lens, kind, slab):
+    """Prompts by chunks of 32 tokens against the recurrences in float64 and against the walk token by token: unequal lengths,
+    slots out of order, states that are not zero, decays of zero and of one, scratch for everything or two chunks at a time."""
+    G = {"mamba": max(1, H // 2) if H % 2 == 0 else 1}.get(kind, H)
+    T, n = sum(lens), len(lens)
+    if slab:
+        monkeypatch.setattr(ops, "STATE_SCRATCH_BYTES", slab * n * H * 4 * ops._STATE_KINDS[kind][1])
+    monkeypatch.setattr(ops, "state_chunks_pay", lambda *_: True)
+    per = d * (e + 1) if kind == "memory" else d * e
+    before = rnd(n + 1, H * per + (4 if kind == "mamba" else 0), seed=4, s=0.3)
+    q_start = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    slots = torch.arange(n, 0, -1, dtype=torch.int32, device=DEV)
+    vw = (H * e + 3) // 4 * 4
+    proj = rnd(T, vw + 2 * G * d)
+    v, k, q = proj[:, :H * e].double().view(T, H, e), proj[:, vw:vw + G * d].double(), proj[:, vw + G * d:].double()
+    k, q = (t.view(T, G, d).repeat_interleave(H // G, 1) for t in (k, q))
+    silu = lambda z: z * torch.sigmoid(z)                                                                      # noqa: E731
+    scale, skip = 1.0, torch.zeros(H, device=DEV)
+    g = torch.Generator().manual_seed(7)
+    if kind == "mamba":
+        raw, bias, a_log, skip = rnd(T, H, seed=5), rnd(H, seed=6), rnd(H, seed=7, s=0.5), rnd(H, seed=8)
+        z = raw.double() + bias.double()
+        take = torch.logaddexp(z, torch.zeros_like(z))
+        keep = torch.exp(-torch.exp(a_log.double()) * take)
+    elif kind == "lightning":
+        decay = torch.tensor([[0.97, 1.0, 0.3, 0.999, 0.5, 0.0][h % 6] for h in range(H)], device=DEV)
+        keep, take = decay.double().expand(T, H), torch.ones(T, H, dtype=torch.float64, device=DEV)
+        q, k, v = silu(q), silu(k), silu(v)
+    else:
+        gates = torch.rand(T, H, 4, generator=g)
+        gates[:, :, 0] = gates[:, :, 0] ** 0.2
+        gates[3::17, :, 0] = 0.0
+        gates, scale = gates.to(DEV), d ** -0.5
+        keep, take = gates[..., 0].double(), gates[..., 1].double()
+    results = []
+    for workspace in (Scratch(), None):
+        out, state = torch.full((T, H * e), float("nan"), device=DEV), before.clone()
+        den = torch.full((T, H), float("nan"), device=DEV) if kind == "memory" else None
+        if kind == "mamba":
+            ops.mamba2_scan(proj, vw, vw + G * d, raw, bias, a_log, skip, out, state, 4, q_start, slots, n, H, G, d, e, max(lens), workspace)
+        elif kind == "lightning":
+            ops.lightning_scan(proj, vw + G * d, vw, 0, out, state.view(-1, H, d, e), q_start, slots, decay, n, H, d, e, max(lens), workspace)
+        else:
+            ops.gated_linear_scan(proj, vw + G * d, vw, 0, scale, gates, out, state, q_start, slots, n, H, d, e, max(lens), workspace,
+                                  divisors=den)
+        assert workspace is None or workspace.asked == ["state_chunks"]
+        results.append((out, state, den))
+    off = 4 if kind == "mamba" else 0
+    want, after, want_den = torch.zeros(T, H, e, dtype=torch.float64, device=DEV), before.double().clone(), torch.zeros(T, H, dtype=torch.float64, device=DEV)
+    at = 0
+    for s, length in enumerate(lens):
+        st = before[slots[s].long(), off:].double().view(H, per)
+        S, norm = st[:, :d * e].view(H, d, e), st[:, d * e:]
+        for t in range(at, at + length):
+            S = keep[t][:, None, None] * S + (take[t][:, None] * k[t])[:, :, None] * v[t][:, None, :]
+            want[t] = torch.einsum("hde,hd->he", S, q[t]) * scale + skip.double()[:, None] * v[t]
+            if kind == "memory":
+                norm = keep[t][:, None] * norm + take[t][:, None] * k[t]
+                want_den[t] = torch.maximum((norm * q[t]).sum(-1).abs() * scale, gates[t, :, 2].double()) + 1e-6
+        after[slots[s].long(), off:] = torch.cat([S.reshape(H, -1), norm], 1).reshape(-1)
+        at += length
+    # sums of up to 128 products, states that grow where nothing decays: some hundred roundings of 2^-24 against the mean size
+    # of a result; the walk's own error stands beside it
+    err = [max(worst(o.view(T, H, e), want), worst(st, after), worst(dn, want_den) if dn is not None else 0.0) for o, st, dn in results]
+    assert err[0] <= 6e-5 and err[0] <= 4 * err[1] + 4e-6, err
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("H", [6, 8, 2044, 2048])
 @pytest.mark.parametrize("T", [1, 297])
@@ -385,7 +465,7 @@ def test_embed_streams(ops, T, H, dtype):
     assert torch.equal(out.view(T, 3, H), table[ids.long()].float()[:, None].expand(T, 3, H))
 
 
-@pytest.mark.parametrize("T, W, E", [(16, 1184, 8), (16, 1200, 8), (1, 2048, 4), (3, 4736, 4)])
+@pytest.mark.parametrize("T, W, E", [(16, 1184, 8), (16, 1216, 8), (1, 2048, 4), (3, 4736, 4)])
 def test_expert_down_blocks(ops, T, W, E):
     """The second product of few pairs' experts on both sides of the line between few blocks and many."""
     F, top = 96, 2
