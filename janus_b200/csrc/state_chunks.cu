@@ -156,15 +156,21 @@ __device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;"
 
 constexpr int COLS = 64, SLD = 2 * COLS + 4;   // columns of a block; floats of a pair of the state's rows, and padding
 constexpr int VLD = COLS + 4;
-template <int KIND, int D>
+constexpr int HAND_FLOATS = 4 * 3 * 128 * 4;   // what four parts of a block hand one another
+template <int KIND, int D, int SPLIT>
 constexpr int chunk_smem() {
-  return (3 * C * (D + 4) + 2 * C * (C + 4) + 2 * SC_FLOATS + (D + C) / 2 * SLD + C * VLD + (KIND == MEMORY ? D : 0)) * 4;
+  return (3 * C * (D + 4) + 2 * C * (C + 4) + 2 * SC_FLOATS + (D + C) / 2 * SLD + C * VLD + (KIND == MEMORY ? D : 0) +
+          (SPLIT > 2 ? HAND_FLOATS : 0)) * 4;
 }
 
-// D: keys' numbers at most.  Eight warps: four of 16 columns, twice, for the two halves of the sums over keys and tokens.
-template <int KIND, int D>
-__global__ void __launch_bounds__(THREADS, 2) state_chunks_kernel(const Args a) {
-  constexpr int LDD = D + 4, RT = D / 16;      // RT: the state's rows a thread updates, of four columns
+// D: keys' numbers at most.  SPLIT times four warps: four of 16 columns for each part of the sums over keys and tokens.  Two
+// parts, two blocks an SM; where no SM has a second block, four parts, which shortens a chunk's chain (128 blocks, 1,024 tokens
+// of four sequences of 16 heads of 128 x 128 with a matrix memory: 382 us in two parts, 244 in four; one sequence of 256
+// tokens 96 and 64).
+template <int KIND, int D, int SPLIT>
+__global__ void __launch_bounds__(128 * SPLIT, 4 / SPLIT) state_chunks_kernel(const Args a) {
+  constexpr int LDD = D + 4, THREADS = 128 * SPLIT, RT = D / (8 * SPLIT);  // RT: the state's rows a thread updates, of four columns
+  constexpr int VL = THREADS / C, OWN = 4 / SPLIT;                         // lanes of a token's values; tokens a thread keeps
   extern __shared__ __align__(16) float smem[];
   float* q_b = smem;                           // two buffers of q [C][LDD]
   float* k_s = q_b + 2 * C * LDD;              // k [C][LDD]
@@ -174,6 +180,7 @@ __global__ void __launch_bounds__(THREADS, 2) state_chunks_kernel(const Args a) 
   float* v_s = S_s + D / 2 * SLD;              // the values, laid out as more rows of the state
   float* vk_s = v_s + C / 2 * SLD;             // the values as they join the state [C][VLD]
   float* n_s = vk_s + C * VLD;                 // MEMORY: the normalizer [D], of the first column block
+  float* hand_s = n_s + (KIND == MEMORY ? D : 0);
   jb::pdl_launch_dependents();
   const int seq = blockIdx.z, h = blockIdx.y, c0 = blockIdx.x * COLS, H = a.H, d = a.d, e = a.e, j = h / (H / a.G);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -203,7 +210,7 @@ __global__ void __launch_bounds__(THREADS, 2) state_chunks_kernel(const Args a) 
     if (chunk < chunks) {
       load_rows(q_b + (chunk & 1) * C * LDD, chunk, a.q_col, 0);
       const float* P_g = scratch_g + chunk * per_chunk;
-      async16(P_b + (chunk & 1) * C * (C + 4) + (tid / 8) * (C + 4) + (tid % 8) * 4, P_g + tid * 4, true);     // 256 pieces
+      if (tid < P_FLOATS / 4) async16(P_b + (chunk & 1) * C * (C + 4) + (tid / 8) * (C + 4) + (tid % 8) * 4, P_g + tid * 4, true);     // 256 pieces
       if (tid < C) async16(reinterpret_cast<float*>(sc_b + (chunk & 1) * C + tid), P_g + P_FLOATS + 4 * tid, true);
     }
     commit();
@@ -212,17 +219,17 @@ __global__ void __launch_bounds__(THREADS, 2) state_chunks_kernel(const Args a) 
     if (chunk < chunks) load_rows(k_s, chunk, a.k_col, 1);
     commit();
   };
-  // values: a thread two neighbouring columns of every 16 of a token, and what the token's key is worth, a chunk ahead
-  const int vt = tid >> 3, vc = (tid & 7) * 2;
-  float2 v[COLS / 16];
+  // values: a thread two neighbouring columns of every 2 VL of a token, and what the token's key is worth, a chunk ahead
+  const int vt = tid / VL, vc = (tid % VL) * 2;
+  float2 v[COLS / (2 * VL)];
   float v_scale;
   auto fetch_v = [&](int chunk) {
     const bool in = vt < n_all - chunk * C;
     const float* row = a.proj + (size_t)(begin + chunk * C + (in ? vt : 0)) * a.ld + a.v_col + (size_t)h * e;
     v_scale = chunk < chunks ? scratch_g[chunk * per_chunk + P_FLOATS + 4 * vt + 1] : 0.0f;
 #pragma unroll
-    for (int i = 0; i < COLS / 16; ++i) {
-      const int c = c0 + 16 * i + vc;
+    for (int i = 0; i < COLS / (2 * VL); ++i) {
+      const int c = c0 + 2 * VL * i + vc;
       v[i] = make_float2(0.0f, 0.0f);
       if (in && pairs && c < e) v[i] = *reinterpret_cast<const float2*>(row + c);
       if (in && !pairs) v[i] = make_float2(c < e ? row[c] : 0.0f, c + 1 < e ? row[c + 1] : 0.0f);
@@ -230,11 +237,11 @@ __global__ void __launch_bounds__(THREADS, 2) state_chunks_kernel(const Args a) 
   };
   auto store_v = [&] {
 #pragma unroll
-    for (int i = 0; i < COLS / 16; ++i) {
+    for (int i = 0; i < COLS / (2 * VL); ++i) {
       if (KIND == LIGHTNING) v[i] = make_float2(silu(v[i].x), silu(v[i].y));
-      float* at = v_s + (vt >> 1) * SLD + 2 * (16 * i + vc) + (vt & 1);
+      float* at = v_s + (vt >> 1) * SLD + 2 * (2 * VL * i + vc) + (vt & 1);
       at[0] = v[i].x, at[2] = v[i].y;
-      *reinterpret_cast<float2*>(vk_s + vt * VLD + 16 * i + vc) = make_float2(v[i].x * v_scale, v[i].y * v_scale);
+      *reinterpret_cast<float2*>(vk_s + vt * VLD + 2 * VL * i + vc) = make_float2(v[i].x * v_scale, v[i].y * v_scale);
     }
   };
   load_qp(0);
@@ -247,8 +254,8 @@ __global__ void __launch_bounds__(THREADS, 2) state_chunks_kernel(const Args a) 
   if (has_n && tid < D) n_s[tid] = tid < d ? S_g[(size_t)d * e + tid] : 0.0f;
   store_v();
 
-  // outputs: a thread four tokens tg + 8 i and four columns, col[x] and the one after it, over one half of the sums
-  const int half = warp >> 2, tg = lane >> 2;
+  // outputs: a thread four tokens tg + 8 i and four columns, col[x] and the one after it, over one part of the sums
+  const int part = warp >> 2, tg = lane >> 2;
   const int col[2] = {16 * (warp & 3) + 2 * (lane & 3), 16 * (warp & 3) + 8 + 2 * (lane & 3)};
   // state's update: a thread RT rows, columns uc, uc + 1, uc + 16 and uc + 17
   const int ur = ((warp >> 1) * 4 + (lane >> 3)) * RT, uc = (warp & 1) * 32 + 2 * (lane & 7);
@@ -289,7 +296,7 @@ __global__ void __launch_bounds__(THREADS, 2) state_chunks_kernel(const Args a) 
           }
       };
 #pragma unroll 2
-      for (int k = half * (D / 2); k < (half + 1) * (D / 2); k += 4) step(q_s + k, LDD, S_s + (k >> 1) * SLD);
+      for (int k = part * (D / SPLIT); k < (part + 1) * (D / SPLIT); k += 4) step(q_s + k, LDD, S_s + (k >> 1) * SLD);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float s = sc_s[tg + 8 * i].x;
@@ -298,45 +305,49 @@ __global__ void __launch_bounds__(THREADS, 2) state_chunks_kernel(const Args a) 
         for (int x = 0; x < 4; ++x) acc[i][x] = jb::mul2(acc[i][x], ss);
       }
 #pragma unroll 2
-      for (int s = half * (C / 2); s < (half + 1) * (C / 2); s += 4) step(P_s + s, C + 4, v_s + (s >> 1) * SLD);
+      for (int s = part * (C / SPLIT); s < (part + 1) * (C / SPLIT); s += 4) step(P_s + s, C + 4, v_s + (s >> 1) * SLD);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int x = 0; x < 4; ++x) o[i][x] = jb::lo(acc[i][x]) + jb::hi(acc[i][x]);
     }
-    if (KIND == MAMBA) {                                                   // D x, by the half that keeps the token
+    if (KIND == MAMBA) {                                                   // D x, by the part that keeps the token
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        if ((i >> 1) == half) {
+        if (i / OWN == part) {
           const int t = tg + 8 * i;
 #pragma unroll
           for (int x = 0; x < 4; ++x) o[i][x] = fmaf(skip, v_s[(t >> 1) * SLD + 2 * (col[x >> 1] + (x & 1)) + (t & 1)], o[i][x]);
         }
     }
-    if (has_n) {                                                           // divisors: eight lanes a token
-      const int l = tid & 7;
+    if (has_n) {                                                           // divisors: VL lanes a token
+      const int l = tid % VL;
       float dot = 0.0f, ones = 0.0f;
 #pragma unroll
-      for (int r = 4 * l; r < D; r += 32) {
+      for (int r = 4 * l; r < D; r += 4 * VL) {
         const float4 x = *reinterpret_cast<const float4*>(q_s + vt * LDD + r), y = *reinterpret_cast<const float4*>(n_s + r);
         dot = fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, fmaf(x.w, y.w, dot))));
       }
-      const float4 p = *reinterpret_cast<const float4*>(P_s + vt * (C + 4) + 4 * l), sc = sc_s[vt];
-      ones = (p.x + p.y) + (p.z + p.w);
+      const float4 sc = sc_s[vt];
+      if (4 * l < C) {
+        const float4 p = *reinterpret_cast<const float4*>(P_s + vt * (C + 4) + 4 * l);
+        ones = (p.x + p.y) + (p.z + p.w);
+      }
       dot = fmaf(dot, sc.x, ones);
-      dot += __shfl_xor_sync(0xffffffffu, dot, 1);
-      dot += __shfl_xor_sync(0xffffffffu, dot, 2);
-      dot += __shfl_xor_sync(0xffffffffu, dot, 4);
+#pragma unroll
+      for (int w = 1; w < VL; w <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, w);
       if (l == 0 && vt < n) a.den[(size_t)(t0 + vt) * H + h] = fmaxf(fabsf(dot), sc.w) + DEN_FLOOR;
     }
     // in flight: k of this chunk, q and P of the next
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();                                                       // q, P, the values and the state have been read, k is there
-    // the halves meet: each keeps two tokens and hands the other its part of the rest, where q was
-    float4* hand = reinterpret_cast<float4*>(q_s) + (tid & 127);
+    // the parts meet: each keeps OWN tokens and hands the others its share of theirs (two parts: where q was)
+    float4* hand = reinterpret_cast<float4*>(SPLIT > 2 ? hand_s : q_s) + (tid & 127);
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if ((i >> 1) != half) hand[128 * i] = make_float4(o[i][0], o[i][1], o[i][2], o[i][3]);
+    for (int i = 0; i < 4; ++i) {
+      const int keeper = i / OWN;
+      if (keeper != part) hand[128 * (i * (SPLIT - 1) + part - (part > keeper))] = make_float4(o[i][0], o[i][1], o[i][2], o[i][3]);
+    }
     {
       jb::Pair S[RT / 2][4];
       const float decay = sc_s[0].z;
@@ -383,10 +394,14 @@ __global__ void __launch_bounds__(THREADS, 2) state_chunks_kernel(const Args a) 
     load_k(chunk + 1);
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-      if ((i >> 1) == half) {
-        const float4 part = hand[128 * i];
+      if (i / OWN == part) {
         const int t = tg + 8 * i;
-        const float y[4] = {o[i][0] + part.x, o[i][1] + part.y, o[i][2] + part.z, o[i][3] + part.w};
+        float y[4] = {o[i][0], o[i][1], o[i][2], o[i][3]};
+#pragma unroll
+        for (int w = 0; w < SPLIT - 1; ++w) {
+          const float4 more = hand[128 * (i * (SPLIT - 1) + w)];
+          y[0] += more.x, y[1] += more.y, y[2] += more.z, y[3] += more.w;
+        }
         if (t < n) {
           float* dst = a.out + ((size_t)(t0 + t) * H + h) * e + c0;
 #pragma unroll
@@ -411,10 +426,10 @@ __global__ void __launch_bounds__(THREADS, 2) state_chunks_kernel(const Args a) 
   if (has_n && tid < d) S_g[(size_t)d * e + tid] = n_s[tid];
 }
 
-template <int KIND, int D>
+template <int KIND, int D, int SPLIT>
 int launch(Args a, int n_seqs, int max_q_len, cudaStream_t stream) {
-  constexpr int smem = chunk_smem<KIND, D>();
-  cudaError_t e = cudaFuncSetAttribute(state_chunks_kernel<KIND, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  constexpr int smem = chunk_smem<KIND, D, SPLIT>();
+  cudaError_t e = cudaFuncSetAttribute(state_chunks_kernel<KIND, D, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return (int)e;
   const int group = a.H / a.G;
   // a block makes the products of a chunk and key head once for its group's heads, or for a share of them where that
@@ -427,8 +442,8 @@ int launch(Args a, int n_seqs, int max_q_len, cudaStream_t stream) {
     jb::Launch prepare(dim3(n_seqs * a.tiles, a.G, (group + a.heads_here - 1) / a.heads_here), dim3(THREADS), 0, stream);
     e = cudaLaunchKernelEx(&prepare.c, state_prepare_kernel<KIND>, a);
     if (e != cudaSuccess) return (int)e;
-    jb::Launch walk(dim3((a.e + COLS - 1) / COLS, a.H, n_seqs), dim3(THREADS), smem, stream);
-    e = cudaLaunchKernelEx(&walk.c, state_chunks_kernel<KIND, D>, a);
+    jb::Launch walk(dim3((a.e + COLS - 1) / COLS, a.H, n_seqs), dim3(128 * SPLIT), smem, stream);
+    e = cudaLaunchKernelEx(&walk.c, state_chunks_kernel<KIND, D, SPLIT>, a);
     if (e != cudaSuccess) return (int)e;
   }
   return 0;
@@ -450,9 +465,10 @@ JB_EXPORT int jb_state_chunks(int kind, const float* proj, int ld, int q_col, in
   JB_REFUSE(G < 1 || H % G != 0 || tiles < 1 || (kind == LIGHTNING && G != H), "state_chunks: %d heads, %d key heads, %d tiles", H, G, tiles);
   const Args a{proj, ld, q_col, k_col, v_col, gates, ld_gates, rate, bias, skip, scale, out, den, state, slot_stride, state_off,
                q_start, seq_slot, H, G, d, e, scratch, 0, tiles, 0};
-  const auto run = [&](auto small, auto large) { return (d <= 64 ? small : large)(a, n_seqs, max_q_len, stream); };
-  if (kind == MAMBA) return run(launch<MAMBA, 64>, launch<MAMBA, 128>);
-  if (kind == LIGHTNING) return run(launch<LIGHTNING, 64>, launch<LIGHTNING, 128>);
+  const bool few = (long long)n_seqs * H * ((e + COLS - 1) / COLS) <= 148;           // no SM has a second block
+  const auto run = [&](auto small, auto large, auto alone) { return (d <= 64 ? small : few ? alone : large)(a, n_seqs, max_q_len, stream); };
+  if (kind == MAMBA) return run(launch<MAMBA, 64, 2>, launch<MAMBA, 128, 2>, launch<MAMBA, 128, 4>);
+  if (kind == LIGHTNING) return run(launch<LIGHTNING, 64, 2>, launch<LIGHTNING, 128, 2>, launch<LIGHTNING, 128, 4>);
   JB_REFUSE(kind != MEMORY, "state_chunks: kind %d", kind);
-  return run(launch<MEMORY, 64>, launch<MEMORY, 128>);
+  return run(launch<MEMORY, 64, 2>, launch<MEMORY, 128, 2>, launch<MEMORY, 128, 4>);
 }

@@ -1136,7 +1136,7 @@ LIGHTNING_SEGMENT = 128       # tokens of a segment when a long prompt's recurre
 
 # -- recurrences with a matrix state and one decay a token and head, by chunks of tokens -----------------------------
 STATE_CHUNK = 32
-STATE_CHUNKS_FROM = 128               # longest sequence's tokens from which chunks are taken
+STATE_CHUNKS_FROM = (64, 128)         # longest sequence's tokens from which chunks are taken, keys of more than 64 numbers or less
 STATE_WALK_TOKENS = 256               # ... and up to which the walks have no segments
 STATE_SCRATCH_BYTES = 64 << 20        # at most: longer prompts go through it slab by slab
 _STATE_KINDS = {"mamba": (0, STATE_CHUNK * (STATE_CHUNK + 4)),
@@ -1145,17 +1145,18 @@ _STATE_KINDS = {"mamba": (0, STATE_CHUNK * (STATE_CHUNK + 4)),
 
 
 def state_chunks_pay(kind: str, n_seqs: int, heads: int, dim: int, vdim: int, max_q_len: int) -> bool:
-    """Whether chunks are the faster form.  A block (64 value columns of a head) walks its sequence's chunks, 5 to 9 us
-    each, so long prompts need blocks for all SMs; segments walked token by token make up for few sequences.  Walk and
-    chunks, microseconds: 16 heads of 128 x 128 with a matrix memory, one sequence, 128 tokens 82.7 and 49.9, 256 tokens 162
-    and 96, 1,024 tokens 151 and 349; four sequences of 1,024 tokens (128 blocks) 491 and 382, eight 1,342 and 421.
-    Lightning, the same heads, four sequences of 1,024 tokens 430 and 302, eight 817 and 461.  State space, 32 heads of 128
-    x 64, four sequences of 1,024 tokens (128 blocks) 317 and 328, eight 616 and 334; 128 heads, eight of 512 1,114 and 615.
-    At 64 tokens the two are even (24 and 21, 31 and 33)."""
-    if max_q_len < STATE_CHUNKS_FROM or dim > 128:
+    """Whether chunks are the faster form.  A block (64 value columns of a head) walks its sequence's chunks, 6 us each, so
+    long prompts need some blocks; for few, segments walked token by token make up.  Walk and chunks, microseconds: matrix
+    memory, 16 heads of 128 x 128, one sequence (32 blocks), 64 tokens 43 and 27, 256 tokens 162 and 64, 1,024 tokens 151
+    and 216; two sequences (64), 512 tokens 152 and 120, 4,000 tokens 870 and 844; four, 1,024 tokens 491 and 244; eight
+    1,342 and 421.  Lightning, the same heads, two sequences, 512 tokens 161 and 114, 2,048 tokens 441 and 444; four of 1,024
+    tokens 429 and 265.  State space, 32 heads of 128 x 64, two sequences (64), 1,024 tokens 164 and 205, three (96) 220 and
+    206, four 316 and 211.  Keys of at most 64 numbers, whose blocks stay small: 64 tokens 24 and 28, 128 tokens 60 and 47;
+    128 blocks of 2,048 tokens 474 and 504, 256 blocks 739 and 502."""
+    if max_q_len < STATE_CHUNKS_FROM[dim <= 64] or dim > 128:
         return False
     blocks = n_seqs * heads * -(-vdim // 64)
-    return max_q_len <= STATE_WALK_TOKENS or blocks >= (128 if dim > 64 and kind != "mamba" else 148)
+    return max_q_len <= STATE_WALK_TOKENS or blocks >= (148 if dim <= 64 else 96 if kind == "mamba" else 64)
 
 
 def _state_chunks(kind: str, workspace, proj: torch.Tensor, q_col: int, k_col: int, v_col: int, gates, ld_gates: int, rate,

@@ -383,7 +383,7 @@ class Scratch:
         return torch.full(shape, float("nan"), dtype=dtype, device=DEV)
 
 
-@pytest.mark.parametrize("H, G, d, e", [(2, 2, 128, 128), (4, 4, 64, 24), (3, 3, 20, 17), (2, 2, 4, 33), (6, 6, 128, 66), (2, 2, 68, 64), (2, 2, 64, 130)])
+@pytest.mark.parametrize("H, G, d, e", [(2, 2, 128, 128), (4, 4, 64, 24), (3, 3, 20, 17), (2, 2, 4, 33), (6, 6, 128, 66), (2, 2, 68, 64), (2, 2, 64, 130), (76, 76, 72, 66)])
 @pytest.mark.parametrize("lens", [[64], [65, 1, 31, 32, 33], [300, 3]])
 @pytest.mark.parametrize("kind", ["mamba", "lightning", "memory"])
 @pytest.mark.parametrize("slab", [0, 2])
