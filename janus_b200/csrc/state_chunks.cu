@@ -15,8 +15,9 @@
 // segments walked token by token, 1,188 so; 16 heads of 128 x 128 with a matrix memory 1,342 and 421; with 16 columns a
 // block, for which every q and k is read four times as often, 1,689 and 552.
 // All float32 but for the sums L and their differences, which are float64: a sum that has passed a strong decay is large, and
-// a difference of two of them would keep few digits in 32 bits.  Decays only appear as exponentials of differences that are
-// not positive.
+// a difference of two of them would keep few digits in 32 bits.  Decays only appear as exponentials of differences of L of a
+// later and an earlier token; L is of their sizes, the signs of those below zero are counted beside it (the walks take any
+// number as a decay, and so do the chunks).
 // Kinds: MAMBA   q = C, k = B, v = x, a = exp(-exp(A_log) dt), b = dt = softplus(raw + bias), y + D x
 //        LIGHTNING q, k, v through SiLU, a one number a head, b = 1
 //        MEMORY  a, b and exp(-m) as `exp_gates` leaves them; values of one make the normalizer n (the first block of a
@@ -114,6 +115,7 @@ __global__ void __launch_bounds__(THREADS) state_prepare_kernel(const Args a) {
   __syncthreads();
   for (int h = h_begin + warp; h < h_end; h += THREADS / 32) { // a head a warp, a token a lane
     float log_a = 0.0f, b = 0.0f, floor = 0.0f;
+    bool turns = false;                                        // a decay below zero turns the state's sign
     if (lane < n) {
       const size_t t = (size_t)(t0 + lane);
       if (KIND == MAMBA) {
@@ -122,10 +124,10 @@ __global__ void __launch_bounds__(THREADS) state_prepare_kernel(const Args a) {
         log_a = -expf(a.rate[h]) * b;
       } else if (KIND == LIGHTNING) {
         b = 1.0f;
-        log_a = logf(a.rate[h]);
+        turns = a.rate[h] < 0.0f, log_a = logf(fabsf(a.rate[h]));
       } else {
         const float* g = a.gates + (t * a.H + h) * 4;
-        log_a = logf(g[0]), b = g[1], floor = g[2];
+        turns = g[0] < 0.0f, log_a = logf(fabsf(g[0])), b = g[1], floor = g[2];
       }
       log_a = fmaxf(log_a, -10000.0f);                         // a decay of zero; the sums stay finite
     }
@@ -136,13 +138,17 @@ __global__ void __launch_bounds__(THREADS) state_prepare_kernel(const Args a) {
       if (lane >= o) L += before;
     }
     const double end = __shfl_sync(0xffffffffu, L, 31);
+    const unsigned turning = __ballot_sync(0xffffffffu, turns);
+    const int turned = __popc(turning & (0xffffffffu >> (31 - lane)));       // turns up to this token, of which an odd number
+    const auto decay = [](double log, int turns_in) { return turns_in & 1 ? -expf((float)log) : expf((float)log); };
     float* P_g = a.scratch + ((size_t)blockIdx.x * a.H + h) * scratch_floats(KIND);
     // per token: what multiplies q_t S, what multiplies k_t on its way into the state, the chunk's decay, exp(-m)
-    reinterpret_cast<float4*>(P_g + P_FLOATS)[lane] = make_float4(expf((float)L) * a.scale, expf((float)(end - L)) * b, expf((float)end), floor);
+    reinterpret_cast<float4*>(P_g + P_FLOATS)[lane] = make_float4(decay(L, turned) * a.scale, decay(end - L, __popc(turning) - turned) * b, decay(end, __popc(turning)), floor);
 #pragma unroll 8
     for (int t = 0; t < C; ++t) {
       const double Lt = __shfl_sync(0xffffffffu, L, t);
-      P_g[t * C + lane] = lane <= t ? expf((float)(Lt - L)) * b * a.scale * qk_s[t][lane] : 0.0f;
+      const int turned_t = __popc(turning & (0xffffffffu >> (31 - t)));
+      P_g[t * C + lane] = lane <= t ? decay(Lt - L, turned_t - turned) * b * a.scale * qk_s[t][lane] : 0.0f;
     }
   }
 }

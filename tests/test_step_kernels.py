@@ -485,3 +485,37 @@ def test_expert_down_blocks(ops, T, W, E):
             bound[t] += wd[e].double().abs() @ between.abs() * w
     # what stands between the products is rounded to bfloat16: half of 2^-8 of each number, and the float32 sums
     assert bool(((out.double() - want).abs() <= (2.0 ** -9 + 2.0 ** -12) * bound).all())
+
+
+def lightning_reference(q, k, v, decay, before, lens, slots):
+    """(outputs, states) of S <- decay S + k v^T, y = S^T q in float64; q, k, v [T, H, .] activated"""
+    out, after, at = torch.zeros(*v.shape, dtype=torch.float64, device=DEV), before.double().clone(), 0
+    for s, length in enumerate(lens):
+        S = before[slots[s].long()].double()
+        for t in range(at, at + length):
+            S = decay.double()[:, None, None] * S + k[t][:, :, None] * v[t][:, None, :]
+            out[t] = torch.einsum("hde,hd->he", S, q[t])
+        after[slots[s].long()] = S
+        at += length
+    return out, after
+
+
+@pytest.mark.parametrize("length", [64, 300])
+@pytest.mark.parametrize("d", [64, 128])
+def test_lightning_decays_of_any_sign(ops, monkeypatch, length, d):
+    """Decays below zero, above one and zero with either sign: chunks take them as the walk does."""
+    decay = torch.tensor([-0.5, 1.05, 0.9, -1.02, -0.0, -0.999], device=DEV)
+    H, e, lens = decay.numel(), 64, [length, 40]
+    T = sum(lens)
+    proj, before = rnd(T, H * (2 * d + e)), rnd(3, H, d, e, seed=4, s=0.3)
+    q_start, slots = ints(0, length, T), ints(2, 0)
+    q, k, v = (torch.nn.functional.silu(t.double()).view(T, H, -1) for t in proj.split([H * d, H * d, H * e], 1))
+    want, after = lightning_reference(q, k, v, decay, before, lens, slots)
+    for pays, asked in ((True, ["state_chunks"]), (False, [] if length <= 256 else ["lightning_segments"])):
+        monkeypatch.setattr(ops, "state_chunks_pay", lambda *_: pays)
+        out, state, workspace = torch.full((T, H * e), float("nan"), device=DEV), before.clone(), Scratch()
+        ops.lightning_scan(proj, 0, H * d, 2 * H * d, out, state, q_start, slots, decay, 2, H, d, e, length, workspace)
+        assert workspace.asked == asked
+        for h in range(H):                                   # some hundred roundings of 2^-24 against the head's mean size
+            assert worst(out.view(T, H, e)[:, h], want[:, h]) <= 4e-5, (pays, h)
+            assert worst(state[:, h], after[:, h]) <= 4e-5, (pays, h)
