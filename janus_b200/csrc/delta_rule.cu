@@ -537,20 +537,24 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) delta_chunks_kernel(
       float o[4];
 #pragma unroll
       for (int x = 0; x < 4; ++x) o[x] = m[x] * sc.x;
-#pragma unroll 2
-      for (int s = 0; s <= t_own; s += 4) {                                // P is zero past the diagonal
+      const auto four = [&](int s, int seen) {                             // four writes, of which `seen` come up to this token
         const float4 p = *reinterpret_cast<const float4*>(P_s + t_own * (C + 4) + s);
         const float ps[4] = {p.x, p.y, p.z, p.w};
 #pragma unroll
         for (int y = 0; y < 4; ++y) {
           const float2 wa = *reinterpret_cast<const float2*>(w_s + (s + y) * 20 + col[0]);
           const float2 wb = *reinterpret_cast<const float2*>(w_s + (s + y) * 20 + col[1]);
-          o[0] = fmaf(ps[y], wa.x, o[0]);
-          o[1] = fmaf(ps[y], wa.y, o[1]);
-          o[2] = fmaf(ps[y], wb.x, o[2]);
-          o[3] = fmaf(ps[y], wb.y, o[3]);
+          if (y < seen) {
+            o[0] = fmaf(ps[y], wa.x, o[0]);
+            o[1] = fmaf(ps[y], wa.y, o[1]);
+            o[2] = fmaf(ps[y], wb.x, o[2]);
+            o[3] = fmaf(ps[y], wb.y, o[3]);
+          }
         }
-      }
+      };
+#pragma unroll 2
+      for (int s = 0; s < (t_own & ~3); s += 4) four(s, 4);
+      four(t_own & ~3, ks + 1);                                            // (zero times a later write that is infinite would be NaN)
       if (t_own < n) {
 #pragma unroll
         for (int x = 0; x < 4; ++x)

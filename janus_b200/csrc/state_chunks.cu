@@ -138,17 +138,17 @@ __global__ void __launch_bounds__(THREADS) state_prepare_kernel(const Args a) {
       if (lane >= o) L += before;
     }
     const double end = __shfl_sync(0xffffffffu, L, 31);
-    const unsigned turning = __ballot_sync(0xffffffffu, turns);
-    const int turned = __popc(turning & (0xffffffffu >> (31 - lane)));       // turns up to this token, of which an odd number
-    const auto decay = [](double log, int turns_in) { return turns_in & 1 ? -expf((float)log) : expf((float)log); };
+    unsigned turned = KIND == MAMBA ? 0u : __ballot_sync(0xffffffffu, turns);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) turned ^= turned << o;                  // bit t: whether the turns up to token t are odd
+    const auto decay = [](double log, unsigned odd) { return __uint_as_float(__float_as_uint(expf((float)log)) ^ odd << 31); };
     float* P_g = a.scratch + ((size_t)blockIdx.x * a.H + h) * scratch_floats(KIND);
     // per token: what multiplies q_t S, what multiplies k_t on its way into the state, the chunk's decay, exp(-m)
-    reinterpret_cast<float4*>(P_g + P_FLOATS)[lane] = make_float4(decay(L, turned) * a.scale, decay(end - L, __popc(turning) - turned) * b, decay(end, __popc(turning)), floor);
+    reinterpret_cast<float4*>(P_g + P_FLOATS)[lane] = make_float4(decay(L, turned >> lane) * a.scale, decay(end - L, turned >> 31 ^ turned >> lane) * b, decay(end, turned >> 31), floor);
 #pragma unroll 8
     for (int t = 0; t < C; ++t) {
       const double Lt = __shfl_sync(0xffffffffu, L, t);
-      const int turned_t = __popc(turning & (0xffffffffu >> (31 - t)));
-      P_g[t * C + lane] = lane <= t ? decay(Lt - L, turned_t - turned) * b * a.scale * qk_s[t][lane] : 0.0f;
+      P_g[t * C + lane] = lane <= t ? decay(Lt - L, turned >> t ^ turned >> lane) * b * a.scale * qk_s[t][lane] : 0.0f;
     }
   }
 }
@@ -178,12 +178,13 @@ __global__ void __launch_bounds__(128 * SPLIT, 4 / SPLIT) state_chunks_kernel(co
   constexpr int LDD = D + 4, THREADS = 128 * SPLIT, RT = D / (8 * SPLIT);  // RT: the state's rows a thread updates, of four columns
   constexpr int VL = THREADS / C, OWN = 4 / SPLIT;                         // lanes of a token's values; tokens a thread keeps
   extern __shared__ __align__(16) float smem[];
+  __shared__ int wild_s;                       // whether a value was not finite
   float* q_b = smem;                           // two buffers of q [C][LDD]
   float* k_s = q_b + 2 * C * LDD;              // k [C][LDD]
   float* P_b = k_s + C * LDD;                  // two buffers of P [C][C + 4]
   float4* sc_b = reinterpret_cast<float4*>(P_b + 2 * C * (C + 4));         // two buffers of the scales [C]
   float* S_s = P_b + 2 * C * (C + 4) + 2 * SC_FLOATS;                      // [D / 2][SLD]: two rows of a column are neighbours
-  float* v_s = S_s + D / 2 * SLD;              // the values, laid out as more rows of the state
+  float* v_s = S_s + D / 2 * SLD;              // the values (the finite ones), laid out as more rows of the state
   float* vk_s = v_s + C / 2 * SLD;             // the values as they join the state [C][VLD]
   float* n_s = vk_s + C * VLD;                 // MEMORY: the normalizer [D], of the first column block
   float* hand_s = n_s + (KIND == MEMORY ? D : 0);
@@ -242,12 +243,23 @@ __global__ void __launch_bounds__(128 * SPLIT, 4 / SPLIT) state_chunks_kernel(co
     }
   };
   auto store_v = [&] {
+    float nothing = 0.0f;                      // zero, or NaN where a value is not finite
 #pragma unroll
     for (int i = 0; i < COLS / (2 * VL); ++i) {
       if (KIND == LIGHTNING) v[i] = make_float2(silu(v[i].x), silu(v[i].y));
       float* at = v_s + (vt >> 1) * SLD + 2 * (2 * VL * i + vc) + (vt & 1);
       at[0] = v[i].x, at[2] = v[i].y;
       *reinterpret_cast<float2*>(vk_s + vt * VLD + 2 * VL * i + vc) = make_float2(v[i].x * v_scale, v[i].y * v_scale);
+      nothing = fmaf(v[i].x, 0.0f, fmaf(v[i].y, 0.0f, nothing));
+    }
+    if (nothing != 0.0f) {                     // such values stay out of the product with P, see the end
+      wild_s = 1;
+#pragma unroll
+      for (int i = 0; i < COLS / (2 * VL); ++i) {
+        float* at = v_s + (vt >> 1) * SLD + 2 * (2 * VL * i + vc) + (vt & 1);
+        if (!isfinite(v[i].x)) at[0] = 0.0f;
+        if (!isfinite(v[i].y)) at[2] = 0.0f;
+      }
     }
   };
   load_qp(0);
@@ -258,6 +270,8 @@ __global__ void __launch_bounds__(128 * SPLIT, 4 / SPLIT) state_chunks_kernel(co
     S_s[(r >> 1) * SLD + 2 * c + (r & 1)] = (r < d && c0 + c < e) ? S_g[(size_t)r * e + c0 + c] : 0.0f;
   }
   if (has_n && tid < D) n_s[tid] = tid < d ? S_g[(size_t)d * e + tid] : 0.0f;
+  if (tid == 0) wild_s = 0;
+  __syncthreads();
   store_v();
 
   // outputs: a thread four tokens tg + 8 i and four columns, col[x] and the one after it, over one part of the sums
@@ -430,6 +444,20 @@ __global__ void __launch_bounds__(128 * SPLIT, 4 / SPLIT) state_chunks_kernel(co
     if (r < d && c0 + c < e) S_g[(size_t)r * e + c0 + c] = S_s[(r >> 1) * SLD + 2 * c + (r & 1)];
   }
   if (has_n && tid < d) S_g[(size_t)d * e + tid] = n_s[tid];
+  __syncthreads();
+  if (wild_s == 0) return;
+  // P's zeros for later tokens would not have kept a value that is not finite out of the sums, so it was left out: what it
+  // does to its own token and the later ones of its chunk is added here (to later chunks it came with the state)
+  for (int i = tid; i < n_all * COLS; i += THREADS) {
+    const int t = i / COLS, c = c0 + i % COLS, first = t / C * C;
+    if (c >= e) continue;
+    const float* P_g = scratch_g + (t / C) * per_chunk + (t % C) * C;
+    float* dst = a.out + ((size_t)(begin + t) * H + h) * e + c;
+    for (int s = first; s <= t; ++s) {
+      const float raw = a.proj[(size_t)(begin + s) * a.ld + a.v_col + (size_t)h * e + c], value = KIND == LIGHTNING ? silu(raw) : raw;
+      if (!isfinite(value)) *dst += P_g[s - first] * value;
+    }
+  }
 }
 
 template <int KIND, int D, int SPLIT>

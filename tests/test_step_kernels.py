@@ -519,3 +519,46 @@ def test_lightning_decays_of_any_sign(ops, monkeypatch, length, d):
         for h in range(H):                                   # some hundred roundings of 2^-24 against the head's mean size
             assert worst(out.view(T, H, e)[:, h], want[:, h]) <= 4e-5, (pays, h)
             assert worst(state[:, h], after[:, h]) <= 4e-5, (pays, h)
+
+
+@pytest.mark.parametrize("kind", ["mamba", "lightning", "memory", "delta"])
+def test_an_infinite_value_stays_behind_its_token(ops, monkeypatch, kind):
+    """An infinity among a token's values reaches its own column from that token on, whichever place of a chunk the token has:
+    everything else keeps every bit, by chunks as by the walk."""
+    H, d, e, lens, places = 2, 128, 64, [200, 70], [(64, 3), (66, 7), (77, 40), (94, 11), (95, 60), (201, 5)]
+    T, per = sum(lens), 128 * 64 + (128 if kind == "memory" else 0)
+    q_start, slots = ints(0, 200, T), ints(1, 0)
+    before, raw, bias, rate = rnd(2, H * per, seed=1, s=0.3), rnd(T, 2 * H, seed=2), rnd(H, seed=3), rnd(H, seed=4, mean=-1.0)
+    decay, gates = torch.tensor([0.9, 0.99], device=DEV), torch.rand(T, H, 4, generator=torch.Generator().manual_seed(5)).to(DEV)
+    monkeypatch.setattr(ops, "state_chunks_pay", lambda *_: True)
+    # the chunks by the size of a block (two or four parts share its sums), then the walk
+    for chunks, copies in ((True, 1), (True, 80), (False, 1)):
+        many, n = torch.arange(copies).repeat_interleave(2).mul(270).to(DEV), 2 * copies
+        starts = torch.cat([q_start[:2].repeat(copies) + many, many.new_full((1,), 270 * copies)]).int()
+        where = torch.arange(n, device=DEV).int()
+        results = []
+        for inf in (True, False):
+            one = rnd(T, H * (2 * d + e))
+            for t, c in places if inf else ():
+                one[t, 2 * H * d + c] = float("inf")
+            proj, out = one.repeat(copies, 1), torch.zeros(copies * T, H * e, device=DEV)
+            state, workspace = before[slots.long()].repeat(copies, 1), Scratch() if chunks else None
+            if kind == "mamba":
+                ops.mamba2_scan(torch.cat([proj[:, 2 * H * d:], proj[:, :2 * H * d]], 1), H * e, H * (e + d), raw.repeat(copies, 1)[:, :H], bias, rate,
+                                bias, out, state, 0, starts, where, n, H, H, d, e, 200, workspace)
+            elif kind == "lightning":
+                ops.lightning_scan(proj, 0, H * d, 2 * H * d, out, state.view(n, H, d, e), starts, where, decay, n, H, d, e, 200, workspace)
+            elif kind == "memory":
+                ops.gated_linear_scan(proj, 0, H * d, 2 * H * d, 1.0, gates.repeat(copies, 1, 1), out, state, starts, where, n, H, d, e, 200,
+                                      workspace, divisors=torch.empty(copies * T, H, device=DEV))
+            else:
+                floats = H * n * 7 * ops._DELTA_CHUNK_FLOATS
+                ops.delta_rule(proj, 0, H * d, 2 * H * d, raw.repeat(copies, 1), 0, H, rate, bias, 1e-6, out, state, 0, starts, where, n, H, H, d,
+                               e, torch.full((floats,), float("nan"), device=DEV) if chunks else None, 200)
+            results.append(out.view(copies, T, H, e))
+        got, clean = results
+        for t, c in places:
+            end = 200 if t < 200 else T
+            assert not bool(torch.isfinite(got[:, t:end, 0, c]).any()), (chunks, copies, t)
+            got[:, t:end, 0, c] = clean[:, t:end, 0, c]
+        assert torch.equal(got, clean), (chunks, copies)
