@@ -324,8 +324,9 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) delta_prepare_kernel(
     float b = 0.0f;
     if (lane < n) {
       const float z = raw[(size_t)(t0 + lane) * ld + a_col + h] + dt_bias[h];
-      // below -10,000 a decay is zero either way, and the sums stay finite
-      L = fmaxf(-expf(A_log[h]) * (z > 20.0f ? z : log1pf(expf(z))), -10000.0f);
+      // below -10,000 a decay is zero either way, and the sums stay finite (NaN stays NaN)
+      const float log_g = -expf(A_log[h]) * (z > 20.0f ? z : log1pf(expf(z)));
+      L = log_g < -10000.0f ? -10000.0f : log_g;
       b = 1.0f / (1.0f + expf(-raw[(size_t)(t0 + lane) * ld + b_col + h]));
     }
 #pragma unroll

@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(THREADS) state_prepare_kernel(const Args a) {
         const float* g = a.gates + (t * a.H + h) * 4;
         turns = g[0] < 0.0f, log_a = logf(fabsf(g[0])), b = g[1], floor = g[2];
       }
-      log_a = fmaxf(log_a, -10000.0f);                         // a decay of zero; the sums stay finite
+      log_a = log_a < -10000.0f ? -10000.0f : log_a;           // a decay of zero; the sums stay finite (and NaN stays NaN)
     }
     double L = log_a;
 #pragma unroll

@@ -562,3 +562,44 @@ def test_an_infinite_value_stays_behind_its_token(ops, monkeypatch, kind):
             assert not bool(torch.isfinite(got[:, t:end, 0, c]).any()), (chunks, copies, t)
             got[:, t:end, 0, c] = clean[:, t:end, 0, c]
         assert torch.equal(got, clean), (chunks, copies)
+
+
+@pytest.mark.parametrize("kind", ["mamba", "lightning", "memory", "delta"])
+def test_a_nan_decay_shows(ops, monkeypatch, kind):
+    """A decay that is not a number makes its head's outputs from that token on not a number, by chunks as by the walk; the
+    tokens before it, the other head and the other sequence keep every bit."""
+    H, d, e, lens, bad = 2, 128, 64, [200, 70], 77
+    T, per = sum(lens), 128 * 64 + (128 if kind == "memory" else 0)
+    q_start, slots = ints(0, 200, T), ints(1, 0)
+    proj, before = rnd(T, H * (2 * d + e)), rnd(2, H * per, seed=1, s=0.3)
+    raw, bias, rate = rnd(T, 2 * H, seed=2), rnd(H, seed=3), rnd(H, seed=4, mean=-1.0)
+    gates = torch.rand(T, H, 4, generator=torch.Generator().manual_seed(5)).to(DEV)
+    monkeypatch.setattr(ops, "state_chunks_pay", lambda *_: True)
+    results = {}
+    for chunks in (True, False):
+        for nan in (True, False):
+            out, state, workspace = torch.zeros(T, H * e, device=DEV), before.clone(), Scratch() if chunks else None
+            x, g, r = raw.clone(), gates.clone(), rate.clone()
+            first = 0 if kind == "lightning" else bad             # a lightning layer's decays are not a token's
+            if nan:
+                x[bad, 0] = x[bad, H] = g[bad, 0, 0] = float("nan")
+                r[0] = float("nan") if kind == "lightning" else r[0]
+            if kind == "mamba":
+                ops.mamba2_scan(proj, H * e, H * (e + d), x[:, :H], bias, r, bias, out, state, 0, q_start, slots, 2, H, H, d, e, 200, workspace)
+            elif kind == "lightning":
+                ops.lightning_scan(proj, 0, H * d, 2 * H * d, out, state.view(2, H, d, e), q_start, slots, r, 2, H, d, e, 200, workspace)
+            elif kind == "memory":
+                ops.gated_linear_scan(proj, 0, H * d, 2 * H * d, 1.0, g, out, state, q_start, slots, 2, H, d, e, 200, workspace,
+                                      divisors=torch.empty(T, H, device=DEV))
+            else:
+                floats = H * 2 * 7 * ops._DELTA_CHUNK_FLOATS
+                ops.delta_rule(proj, 0, H * d, 2 * H * d, x, 0, H, r, bias, 1e-6, out, state, 0, q_start, slots, 2, H, H, d, e,
+                               torch.full((floats,), float("nan"), device=DEV) if chunks else None, 200)
+            results[chunks, nan] = out.view(T, H, e), state.view(2, H, per)
+        (out, state), (clean, clean_state) = results[chunks, True], results[chunks, False]
+        sick = torch.zeros(T, H, dtype=torch.bool, device=DEV)
+        sick[first:200, 0] = True
+        if kind == "lightning":
+            sick[:, 0] = True
+        assert bool(torch.isnan(out[sick]).all()) and torch.equal(out[~sick], clean[~sick]), chunks
+        assert bool(torch.isnan(state[1, 0, :d * e]).all()) and torch.equal(state[:, 1], clean_state[:, 1]), chunks
