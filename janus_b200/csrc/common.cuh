@@ -157,6 +157,67 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// PARTS sums over the lanes, each bit for bit what `warp_sum` makes of it, in 5 (two parts) or 6 (four) shuffles instead of 5
+// a part: lane 32 / PARTS * p ends with part p's.
+template <int PARTS>
+__device__ __forceinline__ float warp_sums(const float (&v)[PARTS]) {
+  static_assert(PARTS == 1 || PARTS == 2 || PARTS == 4, "parts");
+  const int lane = threadIdx.x & 31;
+  float t = v[0];
+  int o = 16;
+  if constexpr (PARTS >= 2) {
+    const bool up = (lane & 16) != 0;
+    float keep[PARTS / 2];
+#pragma unroll
+    for (int p = 0; p < PARTS / 2; ++p) {
+      const float mine = up ? v[p + PARTS / 2] : v[p], other = up ? v[p] : v[p + PARTS / 2];
+      keep[p] = mine + __shfl_xor_sync(0xffffffffu, other, 16);
+    }
+    t = keep[0];
+    o = 8;
+    if constexpr (PARTS == 4) {
+      const bool odd = (lane & 8) != 0;
+      t = (odd ? keep[1] : keep[0]) + __shfl_xor_sync(0xffffffffu, odd ? keep[0] : keep[1], 8);
+      o = 4;
+    }
+  }
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1)
+    if (s <= o) t += __shfl_xor_sync(0xffffffffu, t, s);
+  return t;
+}
+
+// A row's sum in ONE order however many threads hold it, so that a row's result does not depend on how many rows a launch
+// has.  The row's vectors belong to THREADS x PARTS places (vector i to place i mod that number), thread x has places x,
+// x + THREADS, ... and in part[p] the sum over its p-th place in order; 32 neighbouring places meet as a warp's lanes do, and
+// so do these sums (in every warp).  `scratch`: THREADS * PARTS / 32 floats, no other sum's.
+template <int THREADS, int PARTS>
+__device__ __forceinline__ void row_put(const float (&part)[PARTS], float* scratch) {
+  const int lane = threadIdx.x & 31;
+  const float t = warp_sums<PARTS>(part);
+  if (lane % (32 / PARTS) == 0) scratch[lane / (32 / PARTS) * (THREADS / 32) + (threadIdx.x >> 5)] = t;
+}
+template <int PLACES>
+__device__ __forceinline__ float row_get(const float* scratch) {
+  constexpr int SUMS = PLACES / 32;
+  static_assert((SUMS & (SUMS - 1)) == 0 && SUMS <= 32, "places");
+  float t = scratch[threadIdx.x & (SUMS - 1)];
+#pragma unroll
+  for (int o = SUMS / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
+}
+template <int THREADS, int PARTS>
+__device__ __forceinline__ float row_sum(const float (&part)[PARTS], float* scratch) {
+  row_put<THREADS>(part, scratch);
+  __syncthreads();
+  return row_get<THREADS * PARTS>(scratch);
+}
+
+// sum + v . v, one multiply-add after another
+__device__ __forceinline__ float add_squares(float sum, float4 v) {
+  return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, fmaf(v.x, v.x, sum))));
+}
+
 // Block-wide sum; every thread gets the result.  `scratch` holds 33 floats.
 __device__ __forceinline__ float block_sum(float v, float* scratch) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

@@ -65,27 +65,18 @@ __device__ __forceinline__ void clear_slice(float4* __restrict__ clear, size_t n
 // ---- RMSNorm: one block per output row; y = (x / sqrt(mean(x^2) + eps)) * gamma -----
 // Rows of up to 2,048 floats take blocks of 128 threads, wider ones 256: what an SM has in flight is its
 // resident blocks' rows, and sixteen small blocks hold twice the bytes of eight (34,808 rows of 2,048: 166 us
-// with 256 threads).  The block's sum takes one barrier: every warp leaves its part, every thread adds the parts
-// in the same order.
+// with 256 threads).  The block's sum takes one barrier, and its order goes by the row's width alone (512 places,
+// `jb::row_sum`): a row's bits are the same alone, among a few rows and among many.
 // NORM_CACHE float4 per thread stay in registers between the two passes: 4 cover rows of 2,048 (128 threads)
 // and of 4,096 (256 threads) at 40 registers a thread, 8 cover rows of 8,192; wider rows are read twice.
 
-template <int THREADS>
-__device__ __forceinline__ float norm_block_sum(float v, float* scratch) {
-  v = jb::warp_sum(v);
-  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
-  __syncthreads();
-  float t = 0.0f;
-#pragma unroll
-  for (int w = 0; w < THREADS / 32; ++w) t += scratch[w];
-  return t;
-}
+constexpr int NORM_PLACES = 512;
 
 // A step of few rows (FEW: at most two a SM) is bound by the chain of latencies from the kernel before to the kernel
 // after: 512 threads a row, so that a thread has one or two loads to wait for, and the weight, which no kernel before
 // wrote, is in registers before the wait for that kernel ends (8 rows of 4,096: 4.8 -> 3.0 us in a decode step).
 
-constexpr int FEW_ROWS = 296, FEW_THREADS = 512;
+constexpr int FEW_ROWS = 296, FEW_THREADS = NORM_PLACES;
 
 template <typename TG, typename TO, int THREADS, int NORM_CACHE>
 __global__ void __launch_bounds__(THREADS, NORM_CACHE == 4 && THREADS != FEW_THREADS ? 1280 / THREADS : 1) rmsnorm_vec_kernel(const float* __restrict__ x,
@@ -94,7 +85,8 @@ __global__ void __launch_bounds__(THREADS, NORM_CACHE == 4 && THREADS != FEW_THR
                                                              TO* __restrict__ out, int H,
                                                              float4* __restrict__ clear, size_t clear_n4) {
   constexpr bool FEW = THREADS == FEW_THREADS;
-  __shared__ float scratch[THREADS / 32];
+  constexpr int PARTS = NORM_PLACES / THREADS;
+  __shared__ float scratch[NORM_PLACES / 32];
   jb::pdl_launch_dependents();
   const int n4 = H >> 2;
   float4 g[FEW ? NORM_CACHE : 1];
@@ -109,7 +101,7 @@ __global__ void __launch_bounds__(THREADS, NORM_CACHE == 4 && THREADS != FEW_THR
   const size_t src = row_index ? (size_t)row_index[r] : (size_t)r;
   const float* xr = x + src * H;
   float4 cache[NORM_CACHE];
-  float ss = 0.0f;
+  float part[PARTS] = {};
 #pragma unroll
   for (int c = 0; c < NORM_CACHE; ++c) {
     const int i = threadIdx.x + c * THREADS;
@@ -119,13 +111,13 @@ __global__ void __launch_bounds__(THREADS, NORM_CACHE == 4 && THREADS != FEW_THR
 #pragma unroll
   for (int c = 0; c < NORM_CACHE; ++c) {
     const int i = threadIdx.x + c * THREADS;
-    if (i < n4) ss += cache[c].x * cache[c].x + cache[c].y * cache[c].y + cache[c].z * cache[c].z + cache[c].w * cache[c].w;
+    if (i < n4) part[c % PARTS] = jb::add_squares(part[c % PARTS], cache[c]);
   }
-  for (int i = threadIdx.x + NORM_CACHE * THREADS; i < n4; i += THREADS) {
-    const float4 v = load4(xr + 4 * i);
-    ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-  }
-  ss = norm_block_sum<THREADS>(ss, scratch);
+  for (int i0 = threadIdx.x + NORM_CACHE * THREADS; i0 < n4; i0 += NORM_PLACES)
+#pragma unroll
+    for (int p = 0; p < PARTS; ++p)
+      if (i0 + p * THREADS < n4) part[p] = jb::add_squares(part[p], load4(xr + 4 * (i0 + p * THREADS)));
+  const float ss = jb::row_sum<THREADS>(part, scratch);
   const float rms = sqrtf(ss / (float)H + eps);
   TO* o = out + (size_t)r * H;
 #pragma unroll
@@ -570,7 +562,8 @@ __global__ void __launch_bounds__(THREADS) sublayer_norm_add_vec_kernel(float* _
                                                                          float4* __restrict__ clear, size_t clear_n4,
                                                                          float4* __restrict__ clear2, size_t clear2_n4) {
   constexpr bool FEW = THREADS == FEW_THREADS;
-  __shared__ float scratch[THREADS / 32];
+  constexpr int PARTS = NORM_PLACES / THREADS;
+  __shared__ float scratch[NORM_PLACES / 32];
   jb::pdl_launch_dependents();
   const size_t row = (size_t)blockIdx.x * H;
   float* res = residual + row;
@@ -590,7 +583,7 @@ __global__ void __launch_bounds__(THREADS) sublayer_norm_add_vec_kernel(float* _
   }
   float* yr = y + row;
   float4 cache[CACHE];
-  float ss = 0.0f;
+  float part[PARTS] = {};
 #pragma unroll
   for (int c = 0; c < CACHE; ++c) {
     const int i = threadIdx.x + c * THREADS;
@@ -604,13 +597,13 @@ __global__ void __launch_bounds__(THREADS) sublayer_norm_add_vec_kernel(float* _
 #pragma unroll
   for (int c = 0; c < CACHE; ++c) {
     const int i = threadIdx.x + c * THREADS;
-    if (i < n4) ss += cache[c].x * cache[c].x + cache[c].y * cache[c].y + cache[c].z * cache[c].z + cache[c].w * cache[c].w;
+    if (i < n4) part[c % PARTS] = jb::add_squares(part[c % PARTS], cache[c]);
   }
-  for (int i = threadIdx.x + CACHE * THREADS; i < n4; i += THREADS) {
-    const float4 v = load4(yr + 4 * i);
-    ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-  }
-  ss = norm_block_sum<THREADS>(ss, scratch);
+  for (int i0 = threadIdx.x + CACHE * THREADS; i0 < n4; i0 += NORM_PLACES)
+#pragma unroll
+    for (int p = 0; p < PARTS; ++p)
+      if (i0 + p * THREADS < n4) part[p] = jb::add_squares(part[p], load4(yr + 4 * (i0 + p * THREADS)));
+  const float ss = jb::row_sum<THREADS>(part, scratch);
   const float rms = sqrtf(ss / (float)H + eps);
   const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   auto finish = [&](int i, float4 v, float4 w, float4 old) {

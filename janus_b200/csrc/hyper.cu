@@ -10,8 +10,8 @@
 //   streams_mix:     the rewrite, in place, one thread per (token, column).
 //   streams_mix_rmsnorm: a sublayer's rewrite and the next sublayer's read in one launch.
 //
-// All sums run over s = 0, 1, ... in that order in float32, so a token's values do not depend
-// on what else is in the step.
+// All sums over streams run over s = 0, 1, ... in that order in float32, and the order of a row's sum of squares goes by
+// its width and alignment alone, so a token's values do not depend on what else is in the step.
 #include <stdio.h>
 
 #include "common.cuh"
@@ -56,7 +56,8 @@ __global__ void __launch_bounds__(THREADS) streams_rows_kernel(float* __restrict
                                                                const TG* __restrict__ gamma, float eps, TO* __restrict__ out,
                                                                int H, float* __restrict__ clear, float4* __restrict__ clear2,
                                                                size_t clear2_n4) {
-  __shared__ float scratch[THREADS / 32];
+  constexpr int PLACES = 512, PARTS = PLACES / THREADS;        // the order of the sum goes by the width alone
+  __shared__ float scratch[PLACES / 32];
   jb::pdl_launch_dependents();
   const int n4 = H >> 2;
   float mix[S][S], into[S], an[S];
@@ -75,7 +76,7 @@ __global__ void __launch_bounds__(THREADS) streams_rows_kernel(float* __restrict
   const size_t r = blockIdx.x, src = row_index != nullptr ? (size_t)row_index[r] : r;
   float* xr = x + src * S * H;
   float4 u[CACHE];
-  float ss = 0.0f;
+  float part[PARTS] = {};
   const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   float4 old[CACHE][S], yv[CACHE];
 #pragma unroll
@@ -104,19 +105,11 @@ __global__ void __launch_bounds__(THREADS) streams_rows_kernel(float* __restrict
       }
       fma4(u[c], an[to], v);
     }
-    ss += u[c].x * u[c].x;
-    ss += u[c].y * u[c].y;
-    ss += u[c].z * u[c].z;
-    ss += u[c].w * u[c].w;
+    part[c % PARTS] = jb::add_squares(part[c % PARTS], u[c]);
     if (y != nullptr) store4(y + r * H + i, zero);
     if (clear != nullptr) store4(clear + r * H + i, zero);
   }
-  ss = jb::warp_sum(ss);
-  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = ss;
-  __syncthreads();
-  ss = 0.0f;
-#pragma unroll
-  for (int w = 0; w < THREADS / 32; ++w) ss += scratch[w];
+  const float ss = jb::row_sum<THREADS>(part, scratch);
   const float rms = sqrtf(ss / (float)H + eps);
 #pragma unroll
   for (int c = 0; c < CACHE; ++c) {

@@ -53,38 +53,32 @@ __device__ __forceinline__ void store_out(bf16* p, const Vec<4>& x) {
   *reinterpret_cast<uint2*>(p) = u;
 }
 
-// One sum over the block with one barrier: `scratch` holds a float a warp, and no two sums of a launch share it.
-template <int THREADS>
-__device__ __forceinline__ float sum_once(float v, float* scratch) {
-  v = jb::warp_sum(v);
-  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
-  __syncthreads();
-  float t = 0.0f;
-#pragma unroll
-  for (int w = 0; w < THREADS / 32; ++w) t += scratch[w];
-  return t;
-}
-
 // The kernel below for rows of whole 16-byte vectors that THREADS threads hold CACHE float4 each of: every row is read
-// once, all its loads in flight together, into registers; the weights are asked for before the wait for the kernel
-// before.  (1,500 rows of 2,048 from two normed branches, 80 MB: 27 -> 11 us, one row 3.6 -> 1.9 us; before, the branches were
-// read twice and the row passed through shared memory four times.)
+// once, all its loads in flight together, into registers; few rows ask for the weights before the wait for the kernel
+// before.  A vector's sum is a place of its own (`jb::row_sum`), whichever thread has it: a row's bits go by its width alone.
+// (1,500 rows of 2,048 from two normed branches, 80 MB: 27 -> 11 us, one row 3.6 -> 1.9 us; before, the branches were
+// read twice and the row passed through shared memory four times.  2,532 rows of 4,096: 68 us with the weights in registers
+// all along, one block an SM, 50 without.)
 template <typename TO, int THREADS, int CACHE>
 __global__ void __launch_bounds__(THREADS) join_norm_rows_kernel(
     float* __restrict__ stream, float* __restrict__ ya, float* __restrict__ yb, const float* __restrict__ wa,
     const float* __restrict__ wb, float mult, float mult_b, const float* __restrict__ scale, const float* __restrict__ extra,
     const float* __restrict__ gamma, float eps, int center, TO* __restrict__ x_out, const int* __restrict__ row_index, int W,
     float4* __restrict__ clear, size_t clear_n4, float4* __restrict__ clear2, size_t clear2_n4) {
-  __shared__ float scratch[4][THREADS / 32];
+  __shared__ float scratch[4][THREADS * CACHE / 32];
   jb::pdl_launch_dependents();
   const bool joins = ya != nullptr, branches = yb != nullptr, normed = wa != nullptr;
+  constexpr bool EARLY = CACHE == 1;       // few rows; among many, other blocks hide the weights' latency, and their registers hold rows
   Vec<4> ga[CACHE], gb[CACHE], sc[CACHE], g[CACHE], v[CACHE], a[CACHE], b[CACHE];
+  const auto weights = [&](int c, int i) {
+    if (normed) ga[c].load(wa + i), gb[c].load(wb + i);
+    if (scale != nullptr) sc[c].load(scale + i);
+  };
 #pragma unroll
   for (int c = 0; c < CACHE; ++c) {
     const int i = 4 * ((int)threadIdx.x + c * THREADS);
-    if (i >= W) break;
-    if (normed) ga[c].load(wa + i), gb[c].load(wb + i);
-    if (scale != nullptr) sc[c].load(scale + i);
+    if (!EARLY || i >= W) break;
+    weights(c, i);
     if (x_out != nullptr) g[c].load(gamma + i);
   }
   jb::pdl_wait();
@@ -101,30 +95,28 @@ __global__ void __launch_bounds__(THREADS) join_norm_rows_kernel(
   clear_slice(clear2, clear2_n4);
   float inv_a = 1.0f, inv_b = 1.0f;
   if (normed) {
-    float sa = 0.0f, sb = 0.0f;
+    float sa[CACHE] = {}, sb[CACHE] = {};
 #pragma unroll
     for (int c = 0; c < CACHE; ++c) {
       if (4 * ((int)threadIdx.x + c * THREADS) >= W) break;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) sa = fmaf(a[c].v[j], a[c].v[j], sa), sb = fmaf(b[c].v[j], b[c].v[j], sb);
+      for (int j = 0; j < 4; ++j) sa[c] = fmaf(a[c].v[j], a[c].v[j], sa[c]), sb[c] = fmaf(b[c].v[j], b[c].v[j], sb[c]);
     }
-    sa = jb::warp_sum(sa), sb = jb::warp_sum(sb);
-    if ((threadIdx.x & 31) == 0) scratch[0][threadIdx.x >> 5] = sa, scratch[1][threadIdx.x >> 5] = sb;
+    jb::row_put<THREADS>(sa, scratch[0]);
+    jb::row_put<THREADS>(sb, scratch[1]);
     __syncthreads();
-    sa = sb = 0.0f;
-#pragma unroll
-    for (int w = 0; w < THREADS / 32; ++w) sa += scratch[0][w], sb += scratch[1][w];
-    inv_a = 1.0f / sqrtf(sa / (float)W + eps);
-    inv_b = 1.0f / sqrtf(sb / (float)W + eps);
+    inv_a = 1.0f / sqrtf(jb::row_get<THREADS * CACHE>(scratch[0]) / (float)W + eps);
+    inv_b = 1.0f / sqrtf(jb::row_get<THREADS * CACHE>(scratch[1]) / (float)W + eps);
   }
   Vec<4> zero;
 #pragma unroll
   for (int j = 0; j < 4; ++j) zero.v[j] = 0.0f;
-  float sum = 0.0f;
+  float sum[CACHE] = {};
 #pragma unroll
   for (int c = 0; c < CACHE; ++c) {
     const int i = 4 * ((int)threadIdx.x + c * THREADS);
     if (i >= W) break;
+    if (!EARLY) weights(c, i);
     if (joins) {
       Vec<4> y = a[c];
       zero.store(ya + at + i);
@@ -146,26 +138,27 @@ __global__ void __launch_bounds__(THREADS) join_norm_rows_kernel(
     }
     if (joins || extra != nullptr) v[c].store(stream + at + i);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) sum += v[c].v[j];
+    for (int j = 0; j < 4; ++j) sum[c] += v[c].v[j];
   }
   if (x_out == nullptr) return;
-  const float mean = center ? sum_once<THREADS>(sum, scratch[2]) / (float)W : 0.0f;
-  float sq = 0.0f;
+  const float mean = center ? jb::row_sum<THREADS>(sum, scratch[2]) / (float)W : 0.0f;
+  float sq[CACHE] = {};
 #pragma unroll
   for (int c = 0; c < CACHE; ++c) {
     if (4 * ((int)threadIdx.x + c * THREADS) >= W) break;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float d = v[c].v[j] - mean;
-      sq = fmaf(d, d, sq);
+      sq[c] = fmaf(d, d, sq[c]);
     }
   }
-  const float inv = 1.0f / sqrtf(sum_once<THREADS>(sq, scratch[3]) / (float)W + eps);
+  const float inv = 1.0f / sqrtf(jb::row_sum<THREADS>(sq, scratch[3]) / (float)W + eps);
   TO* x = x_out + (size_t)blockIdx.x * W;
 #pragma unroll
   for (int c = 0; c < CACHE; ++c) {
     const int i = 4 * ((int)threadIdx.x + c * THREADS);
     if (i >= W) break;
+    if (!EARLY) g[c].load(gamma + i);
 #pragma unroll
     for (int j = 0; j < 4; ++j) v[c].v[j] = ((v[c].v[j] - mean) * inv) * g[c].v[j];
     store_out(x + i, v[c]);

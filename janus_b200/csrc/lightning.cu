@@ -219,20 +219,21 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
   *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
 
-// gated_rmsnorm with the row in registers, CACHE vectors a thread, row and gate in flight together, the weight asked for
-// before the wait (4 rows of 2,048 in a decode step: 7.8 us with two scalar passes, 1.9 so; 2,623 rows, 54 MB: 31 and 12 us).
+// gated_rmsnorm with the row in registers, CACHE vectors a thread, row and gate in flight together, the weight of few rows
+// asked for before the wait (4 rows of 2,048 in a decode step: 7.8 us with two scalar passes, 1.9 so; 2,623 rows, 54 MB: 31 and 12 us).
 template <typename TG, typename TO, int THREADS_N, int CACHE>
-__global__ void __launch_bounds__(THREADS_N) gated_rmsnorm_rows_kernel(const float* __restrict__ o, const TG* __restrict__ w,
+__global__ void __launch_bounds__(THREADS_N, CACHE == 2 ? 6 : CACHE == 4 ? 4 : 1) gated_rmsnorm_rows_kernel(const float* __restrict__ o, const TG* __restrict__ w,
                                                                        const float* __restrict__ gate, int gate_ld, float eps,
                                                                        TO* __restrict__ out, int N) {
-  __shared__ float scratch[THREADS_N / 32];
+  __shared__ float scratch[THREADS_N * CACHE / 32];    // a vector's sum is a place of its own, whichever thread has it
   jb::pdl_launch_dependents();
   const size_t t = blockIdx.x;
+  constexpr bool EARLY = CACHE == 1;       // few rows; among many, other blocks hide the weight's latency, and its registers hold rows
   float4 x[CACHE], g[CACHE], ww[CACHE];
 #pragma unroll
   for (int c = 0; c < CACHE; ++c) {
     const int i = 4 * ((int)threadIdx.x + c * THREADS_N);
-    if (i < N) ww[c] = load4(w + i);
+    if (EARLY && i < N) ww[c] = load4(w + i);
   }
   jb::pdl_wait();
 #pragma unroll
@@ -240,23 +241,20 @@ __global__ void __launch_bounds__(THREADS_N) gated_rmsnorm_rows_kernel(const flo
     const int i = 4 * ((int)threadIdx.x + c * THREADS_N);
     if (i < N) x[c] = load4(o + t * N + i), g[c] = load4(gate + t * gate_ld + i);
   }
-  float ss = 0.0f;
+  float part[CACHE] = {};
 #pragma unroll
   for (int c = 0; c < CACHE; ++c)
-    if (4 * ((int)threadIdx.x + c * THREADS_N) < N) ss += x[c].x * x[c].x + x[c].y * x[c].y + x[c].z * x[c].z + x[c].w * x[c].w;
-  ss = jb::warp_sum(ss);
-  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = ss;
-  __syncthreads();
-  ss = 0.0f;
-#pragma unroll
-  for (int i = 0; i < THREADS_N / 32; ++i) ss += scratch[i];
+    if (4 * ((int)threadIdx.x + c * THREADS_N) < N) part[c] = jb::add_squares(0.0f, x[c]);
+  const float ss = jb::row_sum<THREADS_N>(part, scratch);
   const float rms = sqrtf(ss / (float)N + eps);
   const auto one = [&](float v, float weight, float z) { return (v / rms) * weight * (1.0f / (1.0f + expf(-z))); };
 #pragma unroll
   for (int c = 0; c < CACHE; ++c) {
     const int i = 4 * ((int)threadIdx.x + c * THREADS_N);
-    if (i < N) store4(out + t * N + i, make_float4(one(x[c].x, ww[c].x, g[c].x), one(x[c].y, ww[c].y, g[c].y),
-                                                   one(x[c].z, ww[c].z, g[c].z), one(x[c].w, ww[c].w, g[c].w)));
+    if (i >= N) continue;
+    if (!EARLY) ww[c] = load4(w + i);
+    store4(out + t * N + i, make_float4(one(x[c].x, ww[c].x, g[c].x), one(x[c].y, ww[c].y, g[c].y), one(x[c].z, ww[c].z, g[c].z),
+                                        one(x[c].w, ww[c].w, g[c].w)));
   }
 }
 

@@ -518,7 +518,8 @@ __global__ void __launch_bounds__(THREADS_G) gated_group_rmsnorm_rows_kernel(con
                                                                              const float* __restrict__ gate, int gate_ld,
                                                                              const float* __restrict__ w, float eps,
                                                                              TO* __restrict__ out, int N, int parts) {
-  __shared__ float scratch[THREADS_G / 32];
+  constexpr int PARTS = THREADS_G == 512 ? 2 : 1;               // pieces of up to 2,048 numbers have 256 places, wider ones 1,024
+  __shared__ float scratch[THREADS_G * PARTS / 32];
   jb::pdl_launch_dependents();
   const int t = blockIdx.x, n = N / parts, c0 = (int)blockIdx.y * n, n4 = n >> 2;
   const float4* row = reinterpret_cast<const float4*>(y + (size_t)t * N + c0);
@@ -532,19 +533,14 @@ __global__ void __launch_bounds__(THREADS_G) gated_group_rmsnorm_rows_kernel(con
 #pragma unroll
   for (int c = 0; c < CACHE; ++c)
     if ((int)threadIdx.x + c * THREADS_G < n4) a[c] = row[threadIdx.x + c * THREADS_G], z[c] = g[threadIdx.x + c * THREADS_G];
-  float ss = 0.0f;
+  float part[PARTS] = {};
 #pragma unroll
   for (int c = 0; c < CACHE; ++c) {
     if ((int)threadIdx.x + c * THREADS_G >= n4) break;
     a[c] = make_float4(a[c].x * silu_f(z[c].x), a[c].y * silu_f(z[c].y), a[c].z * silu_f(z[c].z), a[c].w * silu_f(z[c].w));
-    ss += a[c].x * a[c].x + a[c].y * a[c].y + a[c].z * a[c].z + a[c].w * a[c].w;
+    part[c % PARTS] = jb::add_squares(part[c % PARTS], a[c]);
   }
-  ss = jb::warp_sum(ss);
-  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = ss;
-  __syncthreads();
-  ss = 0.0f;
-#pragma unroll
-  for (int i = 0; i < THREADS_G / 32; ++i) ss += scratch[i];
+  const float ss = jb::row_sum<THREADS_G>(part, scratch);
   const float rms = sqrtf(ss / (float)n + eps);
 #pragma unroll
   for (int c = 0; c < CACHE; ++c) {

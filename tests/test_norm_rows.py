@@ -101,3 +101,69 @@ def test_join(ops, rows, W, form):
         assert not bool(ya.any())
     if form in ("two", "sum"):
         assert not bool(yb.any())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("W", [1024, 2048, 2052, 4096, 4100, 8192, 8200])
+def test_a_row_is_the_same_alone_and_among_many(ops, W, dtype):
+    """Bit for bit, whatever form the number of rows selects: a row alone, among 148 or 296 (few) and among 300 (many)."""
+    many, eps = 300, 1e-5
+    x, y, res, gate = rnd(many, W), rnd(many, W, seed=1), rnd(many, W, seed=2), rnd(many, W, seed=3)
+    streams, mix, into = rnd(many, 2 * W, seed=4), rnd(2, 2, seed=5), rnd(2, seed=6)
+    gamma, wa, wb = (rnd(W, seed=i, s=0.1, mean=1.0) for i in (7, 8, 9))
+
+    def norms(rows):
+        at = slice(many - rows, many)
+        made = []
+
+        def out():
+            made.append(torch.empty(rows, W, dtype=dtype, device=DEV))
+            return made[-1]
+        ops.rmsnorm(x[at].clone(), gamma, eps, out())
+        r = res[at].clone()
+        ops.sublayer_norm_add(y[at].clone(), gamma, eps, 0.7, r, out())
+        made.append(r)
+        ops.streams_rmsnorm(streams[at].clone(), 2, into, gamma, eps, out())
+        s = streams[at].clone()
+        ops.streams_mix_rmsnorm(s, y[at].clone(), mix, into, into, 2, gamma, eps, out())
+        made.append(s)
+        for center in (True, False):
+            r = res[at].clone()
+            ops.join_norm(r, gamma=gamma, eps=eps, center=center, x_out=out(), ya=y[at].clone(), yb=x[at].clone(), wa=wa, wb=wb, mult=0.5)
+            made.append(r)
+        ops.gated_rmsnorm(x[at].clone(), gamma, gate[at].clone(), eps, out())
+        ops.gated_group_rmsnorm(x[at].clone(), gate[at].clone(), gamma, eps, 1, out())
+        if W % 8 == 0:
+            ops.gated_group_rmsnorm(x[at].clone(), gate[at].clone(), gamma, eps, 2, out())
+        return [m[-1] for m in made]
+    want = norms(many)
+    for rows in (1, 100, 148, 296, 297):
+        assert [i for i, (a, b) in enumerate(zip(norms(rows), want)) if not torch.equal(a, b)] == [], rows
+
+
+def test_float32_logits_do_not_depend_on_the_step(ops):
+    """The 32-bit engine, bit for bit: a prompt of 400 tokens in one step, cut at 100, token after token at its end, and with
+    another sequence's tokens in the step."""
+    import janus_b200
+    from janus_b200.engine import StepEntry
+    config = dict(architectures=["LlamaForCausalLM"], hidden_size=1024, num_hidden_layers=2, num_attention_heads=8,
+                  num_key_value_heads=2, head_dim=128, intermediate_size=2048, vocab_size=1000, max_position_embeddings=1024,
+                  rms_norm_eps=1e-5, rope_theta=10000.0, tie_word_embeddings=False)
+    model = janus_b200.load_random(config, seed=3, dtype="float32", max_tokens=2048)
+    g = torch.Generator().manual_seed(0)
+    tokens, other = (torch.randint(0, 1000, (n,), generator=g).tolist() for n in (400, 77))
+
+    def logits(cuts, beside=None):
+        slots, at, rows = [model.alloc_slot(), model.alloc_slot()], 0, []
+        for end in cuts + [400]:
+            entries = [StepEntry(slots[0], tokens[at:end], range(end - at))]
+            if beside is not None and at == 0:
+                entries.insert(0, StepEntry(slots[1], beside, (0,)))
+            rows.append(model.step(entries)[-(end - at):].clone())
+            at = end
+        for s in slots:
+            model.free_slot(s)
+        return torch.cat(rows)
+    want = logits([])
+    for cuts, beside in (([100], None), ([296], None), ([397, 398, 399], None), ([100], other), ([], other)):
+        assert torch.equal(logits(cuts, beside), want), cuts
