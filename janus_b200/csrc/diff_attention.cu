@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(128) conv_rope_cache_walk_kernel(
   const bool turns = cos_sin != nullptr && i < rot;
   if (turns && i >= half) return;                        // written with the pair's first member
   const int parts = turns ? 2 : 1;
-  float w[2][WALK_TAPS][4];                              // [half][tokens back][channel]; taps that are not there weigh nothing
+  float w[2][WALK_TAPS][4];                              // [half][tokens back][channel]
 #pragma unroll
   for (int p = 0; p < 2; ++p)
 #pragma unroll
@@ -267,6 +267,7 @@ __global__ void __launch_bounds__(128) conv_rope_cache_walk_kernel(
         if (p >= parts) break;
 #pragma unroll
         for (int b = WALK_TAPS - 1; b >= 0; --b) {       // the oldest first
+          if (b >= taps) continue;                       // out of reach (a weight of zero would not keep an infinity out)
           const float4 v = b > 0 ? win[p][b - 1] : u[k][p];
           y[p].x = fmaf(w[p][b][0], v.x, y[p].x), y[p].y = fmaf(w[p][b][1], v.y, y[p].y);
           y[p].z = fmaf(w[p][b][2], v.z, y[p].z), y[p].w = fmaf(w[p][b][3], v.w, y[p].w);

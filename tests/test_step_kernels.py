@@ -603,3 +603,25 @@ def test_a_nan_decay_shows(ops, monkeypatch, kind):
             sick[:, 0] = True
         assert bool(torch.isnan(out[sick]).all()) and torch.equal(out[~sick], clean[~sick]), chunks
         assert bool(torch.isnan(state[1, 0, :d * e]).all()) and torch.equal(state[:, 1], clean_state[:, 1]), chunks
+
+
+@pytest.mark.parametrize("taps", [2, 3, 4])
+def test_conv_rope_cache_reaches_its_taps_only(ops, taps):
+    """An infinity at a token reaches `taps` tokens of its channel, no later one, in a prompt that walks (64 tokens and more)."""
+    T, H, G, d, e, bad = 80, 2, 1, 16, 16, [(20, 3), (33, 40), (47, 70)]
+    C = H * 2 * d + G * 2 * d + G * e
+    w, state, results = rnd(C, taps, seed=1), rnd(1, taps - 1, C, seed=2), []
+    for inf in (True, False):
+        proj = rnd(T, C)
+        for t, c in bad if inf else ():
+            proj[t, c] = float("inf")
+        k_cache, dest = pages_of(T, 2 * G, d, torch.float32)
+        v_cache, q = torch.zeros(k_cache.shape[0], G, PAGE, e, device=DEV), torch.empty(T, H * 2 * d, device=DEV)
+        ops.conv_rope_cache(proj, w, taps, state, torch.zeros(T, dtype=torch.int32, device=DEV), ints(0, T), ints(0),
+                            torch.arange(T, dtype=torch.int32, device=DEV), None, 0, q, dest, k_cache, v_cache, H, G, d, e, PAGE)
+        results.append(torch.cat([q, picked(k_cache, dest).reshape(T, -1), picked(v_cache, dest).reshape(T, -1)], 1))
+    got, clean = results
+    for t, c in bad:
+        assert not bool(torch.isfinite(got[t:t + taps, c]).any())
+        got[t:t + taps, c] = clean[t:t + taps, c]
+    assert torch.equal(got, clean)
