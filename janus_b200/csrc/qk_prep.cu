@@ -370,8 +370,9 @@ __global__ void head_norm_rope_cache_kernel(const float* __restrict__ proj, int 
 // half a rotation too): a head is one load a lane, pairs meet by shuffles, the shared weights are asked for before the wait.
 // (One token of 16 + 2 x 4 heads of 128: 7.1 us with one number a lane and access and three heads a warp one after another,
 // 2.7 so.)
+// Up to 32 warps a block: more than 64 registers a thread would not launch.
 template <typename TO>
-__global__ void head_norm_rope_rows_kernel(const float* __restrict__ proj, int ld, const float* __restrict__ wq,
+__global__ void __launch_bounds__(1024) head_norm_rope_rows_kernel(const float* __restrict__ proj, int ld, const float* __restrict__ wq,
                                            const float* __restrict__ wk, float eps, const float* __restrict__ table, int rot,
                                            const int* __restrict__ positions, TO* __restrict__ q_out,
                                            const int* __restrict__ dest, TO* __restrict__ k_cache, TO* __restrict__ v_cache,
