@@ -252,23 +252,38 @@ constexpr int V_FLOATS = C * DMAX, P_FLOATS = C * C, SC_FLOATS = C * 4;
 constexpr int SCRATCH_FLOATS = V_FLOATS + P_FLOATS + SC_FLOATS;           // of one chunk and head
 constexpr int PREPARE_HEADS = 8;               // heads of a group that a block prepares at most
 
+// Where the scratch of a sequence's first chunk lies, in chunks: `tiles` a sequence, or (packed) as many as it needs, one
+// sequence after another: floor(q_start / C) + seq begins at or past the end of the sequence before.
+__device__ __forceinline__ int first_slot(const int* q_start, int seq, int tiles, int packed) {
+  return packed ? q_start[seq] / C + seq : seq * tiles;
+}
+
 __global__ void __launch_bounds__(CHUNK_THREADS, 2) delta_prepare_kernel(
     const float* __restrict__ conv, int ldc, int q_col, int k_col, int v_col, const float* __restrict__ raw, int ld,
     int b_col, int a_col, const float* __restrict__ A_log, const float* __restrict__ dt_bias, float unit_eps,
-    float* __restrict__ out, float* __restrict__ scratch, const int* __restrict__ q_start, int H, int G, int d, int e,
-    int first_tile, int tiles, int heads_here) {
+    float* __restrict__ out, float* __restrict__ scratch, const int* __restrict__ q_start, int n_seqs, int H, int G, int d, int e,
+    int first_tile, int tiles, int packed, int heads_here) {
   // products of a chunk's keys with its keys and queries, which the heads of a group share
   __shared__ __align__(16) float q_s[C][LD], k_s[C][LD];
   __shared__ float kk_s[C][C + 1], qk_s[C][C + 1];
   __shared__ double L_s[PREPARE_HEADS][C];
   __shared__ float beta_s[PREPARE_HEADS][C], start_s[PREPARE_HEADS][C], iq_s[C], ik_s[C];
   jb::pdl_launch_dependents();
-  const int seq = blockIdx.x / tiles, tile = blockIdx.x % tiles, R = H / G, j = blockIdx.y;
+  const int R = H / G, j = blockIdx.y;
   const int h_begin = j * R + (int)blockIdx.z * heads_here, h_end = min((j + 1) * R, h_begin + heads_here);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const float q_mult = rsqrtf((float)d);
   jb::pdl_wait();
-  const int s0 = q_start[seq], t0 = s0 + (first_tile + tile) * C, n = min(C, q_start[seq + 1] - t0);
+  int seq = (int)blockIdx.x / tiles, tile = (int)blockIdx.x % tiles;
+  if (packed) {                                                            // the last sequence whose chunks begin up to here
+    seq = -1;
+    for (int s0 = 0; s0 < n_seqs; s0 += CHUNK_THREADS) {
+      const int s = s0 + (int)threadIdx.x;
+      seq += __syncthreads_count(s < n_seqs && first_slot(q_start, s, tiles, packed) <= (int)blockIdx.x);
+    }
+    tile = (int)blockIdx.x - first_slot(q_start, seq, tiles, packed);
+  }
+  const int t0 = q_start[seq] + (first_tile + tile) * C, n = min(C, q_start[seq + 1] - t0);
   if (n <= 0) return;
   // four tokens a warp: unit vectors of q and k, zero past the end of the chunk and of a row
   float4 qv[4], kv[4];
@@ -408,7 +423,7 @@ constexpr int CHUNK_SMEM = (5 * C * LD + C * (C + 4) + DMAX / 2 * SLD + 2 * C * 
 __global__ void __launch_bounds__(CHUNK_THREADS, 2) delta_chunks_kernel(
     const float* __restrict__ conv, int ldc, int q_col, int k_col, float* __restrict__ out, const float* __restrict__ scratch,
     float* __restrict__ state, long long slot_stride, long long state_off, const int* __restrict__ q_start,
-    const int* __restrict__ seq_slot, int H, int G, int d, int e, int first_tile, int tiles) {
+    const int* __restrict__ seq_slot, int H, int G, int d, int e, int first_tile, int tiles, int packed) {
   extern __shared__ __align__(16) float smem[];
   float* vq_b = smem;                          // two buffers of V [C][LD], then q [C][LD]: 64 rows to multiply with the state
   float* k_s = vq_b + 4 * C * LD;              // k [C][LD]
@@ -424,7 +439,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) delta_chunks_kernel(
   const int begin = q_start[seq] + first_tile * C, n_all = min(q_start[seq + 1] - begin, tiles * C);
   if (n_all <= 0) return;
   float* S_g = state + (size_t)seq_slot[seq] * slot_stride + state_off + (size_t)h * d * e;
-  const float* scratch_g = scratch + ((size_t)seq * tiles * H + h) * SCRATCH_FLOATS;
+  const float* scratch_g = scratch + ((size_t)first_slot(q_start, seq, tiles, packed) * H + h) * SCRATCH_FLOATS;
   const int chunks = (n_all + C - 1) / C;
 
   auto load_vq = [&](int chunk) {
@@ -629,34 +644,37 @@ JB_EXPORT int jb_delta_rule(const float* conv, int ldc, int q_col, int k_col, in
 
 // The same for prompts, by chunks: d <= 128, d, ldc, q_col and k_col multiples of 4, conv 16-byte aligned.  `scratch` holds
 // `tiles` chunks of every sequence; longer prompts go in slabs of as many, one after another from the state the last left.
+// tiles = 0: it holds tokens / 32 + n_seqs chunks, the whole step's, one sequence after another (`tokens`: of all sequences).
 JB_EXPORT int jb_delta_rule_chunks(const float* conv, int ldc, int q_col, int k_col, int v_col, const float* raw, int ld,
                                    int b_col, int a_col, const float* A_log, const float* dt_bias, float unit_eps, float* out,
                                    float* state, long long slot_stride, long long state_off, const int* q_start,
                                    const int* seq_slot, int n_seqs, int H, int G, int d, int e, int max_q_len, float* scratch,
-                                   int tiles, cudaStream_t stream) {
+                                   int tiles, int tokens, cudaStream_t stream) {
   if (n_seqs <= 0) return 0;
   JB_REFUSE(d < 1 || d > DMAX || e < 1 || ((d | ldc | q_col | k_col) & 3) != 0 || (((uintptr_t)conv | (uintptr_t)scratch) & 15) != 0,
             "delta_rule_chunks: keys of %d numbers in rows of %d at columns %d and %d", d, ldc, q_col, k_col);
-  JB_REFUSE(G < 1 || H % G != 0 || tiles < 1, "delta_rule_chunks: %d heads are not a multiple of %d key heads", H, G);
+  JB_REFUSE(G < 1 || H % G != 0 || tiles < 0 || max_q_len < 1, "delta_rule_chunks: %d heads are not a multiple of %d key heads", H, G);
   cudaError_t err = cudaFuncSetAttribute(delta_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CHUNK_SMEM);
   if (err != cudaSuccess) return (int)err;
-  const int all = (max_q_len + C - 1) / C;
+  const int all = (max_q_len + C - 1) / C, packed = tiles == 0;
+  if (packed) tiles = all;
+  const int slots = packed ? tokens / C + n_seqs : n_seqs * tiles;
   for (int first = 0; first < all; first += tiles) {
     // (the scratch of a slab is laid out for `tiles` chunks a sequence, whatever is left of it)
     // a block makes the products of a chunk and key head once for its group's heads, or for a share of them where that
     // leaves SMs without a block
-    const int group = H / G, chunks = n_seqs * tiles * G;
+    const int group = H / G, chunks = (packed ? tokens / C + 1 : slots) * G;         // that have tokens
     int parts = (2 * 148 + chunks - 1) / chunks;
     parts = parts < group ? parts : group;
     if (parts < (group + PREPARE_HEADS - 1) / PREPARE_HEADS) parts = (group + PREPARE_HEADS - 1) / PREPARE_HEADS;
     const int heads_here = (group + parts - 1) / parts;
-    jb::Launch prepare(dim3(n_seqs * tiles, G, (group + heads_here - 1) / heads_here), dim3(CHUNK_THREADS), 0, stream);
+    jb::Launch prepare(dim3(slots, G, (group + heads_here - 1) / heads_here), dim3(CHUNK_THREADS), 0, stream);
     err = cudaLaunchKernelEx(&prepare.c, delta_prepare_kernel, conv, ldc, q_col, k_col, v_col, raw, ld, b_col, a_col, A_log,
-                             dt_bias, unit_eps, out, scratch, q_start, H, G, d, e, first, tiles, heads_here);
+                             dt_bias, unit_eps, out, scratch, q_start, n_seqs, H, G, d, e, first, tiles, packed, heads_here);
     if (err != cudaSuccess) return (int)err;
     jb::Launch walk(dim3((e + 15) / 16, H, n_seqs), dim3(CHUNK_THREADS), CHUNK_SMEM, stream);
     err = cudaLaunchKernelEx(&walk.c, delta_chunks_kernel, conv, ldc, q_col, k_col, out, (const float*)scratch, state, slot_stride,
-                             state_off, q_start, seq_slot, H, G, d, e, first, tiles);
+                             state_off, q_start, seq_slot, H, G, d, e, first, tiles, packed);
     if (err != cudaSuccess) return (int)err;
   }
   return 0;

@@ -11,9 +11,9 @@
 // state in shared memory) walks the chunks: [exp(L) q, P] [S; v] is one product, whose sums two halves of the block share,
 // then the state's update.  A thread has four by four outputs and eight rows by four columns of the state; sums go in pairs
 // of neighbouring rows (packed multiply-adds).  Bound by what shared memory delivers (84% of its rate with all SMs full; the
-// multiply-adds, which would bound it next, 55%).  Eight sequences of 1,024 tokens, 128 heads of 128 x 64: 2,054 us as
-// segments walked token by token, 1,188 so; 16 heads of 128 x 128 with a matrix memory 1,342 and 421; with 16 columns a
-// block, for which every q and k is read four times as often, 1,689 and 552.
+// multiply-adds, which would bound it next, 55%).  Eight sequences of 1,024 tokens, 128 heads of 128 x 64: 2,035 us as
+// segments walked token by token, 1,131 so; 16 heads of 128 x 128 with a matrix memory 1,338 and 426; 16 columns a block,
+// for which every q and k is read four times as often, took 1.3 and 1.4 times as long.
 // All float32 but for the sums L and their differences, which are float64: a sum that has passed a strong decay is large, and
 // a difference of two of them would keep few digits in 32 bits.  Decays only appear as exponentials of differences of L of a
 // later and an earlier token; L is of their sizes, the signs of those below zero are counted beside it (the walks take any
@@ -55,18 +55,31 @@ struct Args {
   const int* seq_slot;
   int H, G, d, e;
   float* scratch;
-  int first_tile, tiles, heads_here;
+  int n_seqs, first_tile, tiles, heads_here, packed;
 };
+
+// Where the scratch of a sequence's first chunk lies, in chunks: `tiles` a sequence, or (packed) as many as it needs, one
+// sequence after another: floor(q_start / C) + seq begins at or past the end of the sequence before.
+__device__ __forceinline__ int first_slot(const Args& a, int seq) { return a.packed ? a.q_start[seq] / C + seq : seq * a.tiles; }
 
 template <int KIND>
 __global__ void __launch_bounds__(THREADS) state_prepare_kernel(const Args a) {
   __shared__ __align__(16) float q_s[C][LD], k_s[C][LD];
   __shared__ float qk_s[C][C + 1];
   jb::pdl_launch_dependents();
-  const int seq = blockIdx.x / a.tiles, tile = blockIdx.x % a.tiles, R = a.H / a.G, j = blockIdx.y;
+  const int R = a.H / a.G, j = blockIdx.y;
   const int h_begin = j * R + (int)blockIdx.z * a.heads_here, h_end = min((j + 1) * R, h_begin + a.heads_here);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   jb::pdl_wait();
+  int seq = (int)blockIdx.x / a.tiles, tile = (int)blockIdx.x % a.tiles;
+  if (a.packed) {                                              // the last sequence whose chunks begin up to here
+    seq = -1;
+    for (int s0 = 0; s0 < a.n_seqs; s0 += THREADS) {
+      const int s = s0 + (int)threadIdx.x;
+      seq += __syncthreads_count(s < a.n_seqs && first_slot(a, s) <= (int)blockIdx.x);
+    }
+    tile = (int)blockIdx.x - first_slot(a, seq);
+  }
   const int t0 = a.q_start[seq] + (a.first_tile + tile) * C, n = min(C, a.q_start[seq + 1] - t0);
   if (n <= 0) return;
   const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -193,11 +206,13 @@ __global__ void __launch_bounds__(128 * SPLIT, 4 / SPLIT) state_chunks_kernel(co
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool pairs = ((e | a.v_col) & 1) == 0 && ((uintptr_t)a.out & 7) == 0;          // columns go two at a time
   const bool has_n = KIND == MEMORY && blockIdx.x == 0;
+  if (tid == 0) wild_s = 0;
+  __syncthreads();
   jb::pdl_wait();
   const int begin = a.q_start[seq] + a.first_tile * C, n_all = min(a.q_start[seq + 1] - begin, a.tiles * C);
   if (n_all <= 0) return;
   float* S_g = a.state + (size_t)a.seq_slot[seq] * a.slot_stride + a.state_off + (size_t)h * d * (e + (KIND == MEMORY ? 1 : 0));
-  const float* scratch_g = a.scratch + ((size_t)seq * a.tiles * H + h) * scratch_floats(KIND);
+  const float* scratch_g = a.scratch + ((size_t)first_slot(a, seq) * H + h) * scratch_floats(KIND);
   const size_t per_chunk = (size_t)H * scratch_floats(KIND);
   const int chunks = (n_all + C - 1) / C;
 
@@ -270,8 +285,6 @@ __global__ void __launch_bounds__(128 * SPLIT, 4 / SPLIT) state_chunks_kernel(co
     S_s[(r >> 1) * SLD + 2 * c + (r & 1)] = (r < d && c0 + c < e) ? S_g[(size_t)r * e + c0 + c] : 0.0f;
   }
   if (has_n && tid < D) n_s[tid] = tid < d ? S_g[(size_t)d * e + tid] : 0.0f;
-  if (tid == 0) wild_s = 0;
-  __syncthreads();
   store_v();
 
   // outputs: a thread four tokens tg + 8 i and four columns, col[x] and the one after it, over one part of the sums
@@ -444,8 +457,8 @@ __global__ void __launch_bounds__(128 * SPLIT, 4 / SPLIT) state_chunks_kernel(co
     if (r < d && c0 + c < e) S_g[(size_t)r * e + c0 + c] = S_s[(r >> 1) * SLD + 2 * c + (r & 1)];
   }
   if (has_n && tid < d) S_g[(size_t)d * e + tid] = n_s[tid];
-  __syncthreads();
   if (wild_s == 0) return;
+  __syncthreads();
   // P's zeros for later tokens would not have kept a value that is not finite out of the sums, so it was left out: what it
   // does to its own token and the later ones of its chunk is added here (to later chunks it came with the state)
   for (int i = tid; i < n_all * COLS; i += THREADS) {
@@ -461,22 +474,23 @@ __global__ void __launch_bounds__(128 * SPLIT, 4 / SPLIT) state_chunks_kernel(co
 }
 
 template <int KIND, int D, int SPLIT>
-int launch(Args a, int n_seqs, int max_q_len, cudaStream_t stream) {
+int launch(Args a, int max_q_len, int tokens, cudaStream_t stream) {
   constexpr int smem = chunk_smem<KIND, D, SPLIT>();
   cudaError_t e = cudaFuncSetAttribute(state_chunks_kernel<KIND, D, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return (int)e;
   const int group = a.H / a.G;
   // a block makes the products of a chunk and key head once for its group's heads, or for a share of them where that
   // leaves SMs without a block
-  const long long chunks = (long long)n_seqs * a.tiles * a.G;
+  const int slots = a.packed ? tokens / C + a.n_seqs : a.n_seqs * a.tiles;
+  const long long chunks = (a.packed ? (long long)tokens / C + 1 : slots) * a.G;       // that have tokens
   int parts = (int)((2 * 148 + chunks - 1) / chunks);
   parts = parts < group ? parts : group;
   a.heads_here = (group + parts - 1) / parts;
   for (a.first_tile = 0; a.first_tile * C < max_q_len; a.first_tile += a.tiles) {
-    jb::Launch prepare(dim3(n_seqs * a.tiles, a.G, (group + a.heads_here - 1) / a.heads_here), dim3(THREADS), 0, stream);
+    jb::Launch prepare(dim3(slots, a.G, (group + a.heads_here - 1) / a.heads_here), dim3(THREADS), 0, stream);
     e = cudaLaunchKernelEx(&prepare.c, state_prepare_kernel<KIND>, a);
     if (e != cudaSuccess) return (int)e;
-    jb::Launch walk(dim3((a.e + COLS - 1) / COLS, a.H, n_seqs), dim3(128 * SPLIT), smem, stream);
+    jb::Launch walk(dim3((a.e + COLS - 1) / COLS, a.H, a.n_seqs), dim3(128 * SPLIT), smem, stream);
     e = cudaLaunchKernelEx(&walk.c, state_chunks_kernel<KIND, D, SPLIT>, a);
     if (e != cudaSuccess) return (int)e;
   }
@@ -486,21 +500,22 @@ int launch(Args a, int n_seqs, int max_q_len, cudaStream_t stream) {
 }  // namespace
 
 // kind: 0 state-space (MAMBA), 1 LIGHTNING, 2 matrix MEMORY, see the top.  d <= 128; d, ld, q_col and k_col multiples of 4,
-// proj and scratch 16-byte aligned.  `scratch` holds `tiles` chunks of every sequence (H * 1152 floats a chunk, LIGHTNING
-// H * 9344); longer prompts go in slabs of as many, one after another from the state the last left.
+// proj and scratch 16-byte aligned.  `scratch` (H * 1152 floats a chunk, LIGHTNING H * 9344) holds `tiles` chunks of every
+// sequence; longer prompts go in slabs of as many, one after another from the state the last left.  tiles = 0: it holds
+// tokens / 32 + n_seqs chunks, the whole step's, one sequence after another (`tokens`: of all sequences).
 JB_EXPORT int jb_state_chunks(int kind, const float* proj, int ld, int q_col, int k_col, int v_col, const float* gates,
                               int ld_gates, const float* rate, const float* bias, const float* skip, float scale, float* out,
                               float* den, float* state, long long slot_stride, long long state_off, const int* q_start,
                               const int* seq_slot, int n_seqs, int H, int G, int d, int e, int max_q_len, float* scratch,
-                              int tiles, cudaStream_t stream) {
+                              int tiles, int tokens, cudaStream_t stream) {
   if (n_seqs <= 0 || max_q_len <= 0) return 0;
   JB_REFUSE(d < 1 || d > DMAX || e < 1 || ((d | ld | q_col | k_col) & 3) != 0 || (((uintptr_t)proj | (uintptr_t)scratch) & 15) != 0,
             "state_chunks: keys of %d numbers in rows of %d at columns %d and %d", d, ld, q_col, k_col);
-  JB_REFUSE(G < 1 || H % G != 0 || tiles < 1 || (kind == LIGHTNING && G != H), "state_chunks: %d heads, %d key heads, %d tiles", H, G, tiles);
+  JB_REFUSE(G < 1 || H % G != 0 || tiles < 0 || (kind == LIGHTNING && G != H), "state_chunks: %d heads, %d key heads, %d tiles", H, G, tiles);
   const Args a{proj, ld, q_col, k_col, v_col, gates, ld_gates, rate, bias, skip, scale, out, den, state, slot_stride, state_off,
-               q_start, seq_slot, H, G, d, e, scratch, 0, tiles, 0};
+               q_start, seq_slot, H, G, d, e, scratch, n_seqs, 0, tiles > 0 ? tiles : (max_q_len + C - 1) / C, 0, tiles == 0};
   const bool few = (long long)n_seqs * H * ((e + COLS - 1) / COLS) <= 148;           // no SM has a second block
-  const auto run = [&](auto small, auto large, auto alone) { return (d <= 64 ? small : few ? alone : large)(a, n_seqs, max_q_len, stream); };
+  const auto run = [&](auto small, auto large, auto alone) { return (d <= 64 ? small : few ? alone : large)(a, max_q_len, tokens, stream); };
   if (kind == MAMBA) return run(launch<MAMBA, 64, 2>, launch<MAMBA, 128, 2>, launch<MAMBA, 128, 4>);
   if (kind == LIGHTNING) return run(launch<LIGHTNING, 64, 2>, launch<LIGHTNING, 128, 2>, launch<LIGHTNING, 128, 4>);
   JB_REFUSE(kind != MEMORY, "state_chunks: kind %d", kind);

@@ -67,10 +67,10 @@ _SIGNATURES = {
     "jb_attention_bf16_decode_capped": "ppppppppiiiiiiifiiffpppip",
     "jb_join_norm": "pppppffpppfipipiiplplp", "jb_head_norm_gate": "ppipipfipiiiip", "jb_sigmoid_gate": "pipiiiiip",
     "jb_head_norm_rope_cache": "pippfpippipppiiiiiiiiiifipifp",
-    "jb_delta_rule": "piiiipiiippfppllppiiiiip", "jb_delta_rule_chunks": "piiiipiiippfppllppiiiiiipip",
+    "jb_delta_rule": "piiiipiiippfppllppiiiiip", "jb_delta_rule_chunks": "piiiipiiippfppllppiiiiiipiip",
     "jb_route_topk": "piiippiiiipfip", "jb_experts_few_tokens": "pippipppippiiiiffip", "jb_expert_gather": "pippipiip", "jb_experts_few_tokens_tc": "pppipppppiiiiffip",
     "jb_expert_scatter": "pppipiip",
-    "jb_state_chunks": "ipiiiipipppfpppllppiiiiiipip",
+    "jb_state_chunks": "ipiiiipipppfpppllppiiiiiipiip",
     "jb_gla_decay": "piiippfpiip", "jb_exp_gates": "piiippfppllppiip",
     "jb_gated_linear_scan": "piiiifpiippplppiiiiiippp", "jb_scale_rows_sigmoid": "pipiiip",
     "jb_attention_tc_prefill": "pppppppiiiiiiiiiifpp", "jb_attention_tc_prefill_capped": "pppppppiiiiiiiiiiififfpppipp",
@@ -1137,26 +1137,56 @@ LIGHTNING_SEGMENT = 128       # tokens of a segment when a long prompt's recurre
 # -- recurrences with a matrix state and one decay a token and head, by chunks of tokens -----------------------------
 STATE_CHUNK = 32
 STATE_CHUNKS_FROM = (64, 128)         # longest sequence's tokens from which chunks are taken, keys of more than 64 numbers or less
-STATE_WALK_TOKENS = 256               # ... and up to which the walks have no segments
-STATE_SCRATCH_BYTES = 64 << 20        # at most: longer prompts go through it slab by slab
+STATE_WALK_TOKENS = (256, 512)        # ... and up to which a few blocks' chunks are faster than the walk, mamba and others
+# Scratch of a step whose chunks do not all fit, which then goes through them slab by slab (one chunk of every sequence is the
+# least, 600 KB of 128 heads).  At 18 KB a token of 128 heads it is one activation more of a prompt of 28,000 tokens.  With
+# 64 MB: eight sequences of 1,024 tokens of 128 state-space heads 1,230 us instead of 1,131, 64 of 128 tokens 1,942 instead of
+# 1,274, lightning 616 instead of 414 (the walks 1,529 and 490), delta rule 883 instead of 732.
+STATE_SCRATCH_BYTES = 512 << 20
+SINGLES_BLOCKS = 592                  # blocks up to which sequences of a token or two are no burden
 _STATE_KINDS = {"mamba": (0, STATE_CHUNK * (STATE_CHUNK + 4)),
                 "lightning": (1, STATE_CHUNK * (STATE_CHUNK + 4 + 256)),      # and the activated queries and keys
                 "memory": (2, STATE_CHUNK * (STATE_CHUNK + 4))}
 
 
-def state_chunks_pay(kind: str, n_seqs: int, heads: int, dim: int, vdim: int, max_q_len: int) -> bool:
-    """Whether chunks are the faster form.  A block (64 value columns of a head) walks its sequence's chunks, 6 us each, so
-    long prompts need some blocks; for few, segments walked token by token make up.  Walk and chunks, microseconds: matrix
-    memory, 16 heads of 128 x 128, one sequence (32 blocks), 64 tokens 43 and 27, 256 tokens 162 and 64, 1,024 tokens 151
-    and 216; two sequences (64), 512 tokens 152 and 120, 4,000 tokens 870 and 844; four, 1,024 tokens 491 and 244; eight
-    1,342 and 421.  Lightning, the same heads, two sequences, 512 tokens 161 and 114, 2,048 tokens 441 and 444; four of 1,024
-    tokens 429 and 265.  State space, 32 heads of 128 x 64, two sequences (64), 1,024 tokens 164 and 205, three (96) 220 and
-    206, four 316 and 211.  Keys of at most 64 numbers, whose blocks stay small: 64 tokens 24 and 28, 128 tokens 60 and 47;
-    128 blocks of 2,048 tokens 474 and 504, 256 blocks 739 and 502."""
+def _chunk_slots(n_seqs: int, tokens: int, max_q_len: int, chunk: int, bytes_per_slot: int, most: int):
+    """(chunks that the scratch holds, chunks a sequence and slab or 0: the whole step's one after another)."""
+    tiles, packed = -(-max_q_len // chunk), tokens // chunk + n_seqs      # (as many chunks as all sequences have, or more)
+    if n_seqs * tiles > 2 * packed and packed * bytes_per_slot <= most:     # a few long ones: a block looks its sequence up
+        return packed, 0
+    tiles = max(1, min(tiles, most // (bytes_per_slot * n_seqs)))
+    return n_seqs * tiles, tiles
+
+
+def _mostly_single_tokens(n_seqs: int, tokens: int, blocks: int) -> bool:
+    """Whether a chunked form would spend its time on sequences of a token or two, each of whose blocks costs what a chunk of
+    32 tokens costs, ten tokens of a walk: below eleven tokens a sequence, where the blocks come in several waves.  200 tokens
+    beside 63 single ones, walk and chunks, microseconds: state space of 128 heads 282 and 605, lightning 156 and 184, matrix
+    memory 163 and 155, delta rule 124 and 285; 100 beside 15 in 512 blocks: lightning 74 and 59, matrix memory 76 and 54."""
+    return tokens < 11 * n_seqs and blocks > SINGLES_BLOCKS
+
+
+def state_chunks_pay(kind: str, n_seqs: int, heads: int, dim: int, vdim: int, max_q_len: int, tokens: int) -> bool:
+    """Whether chunks are the faster form, from the work that a step has (`tokens`: of all sequences).  A block (64 value
+    columns of a head) walks its sequence's chunks, 6 us each, so long prompts need some blocks; for few, segments walked
+    token by token make up.  What counts is the sequences that are about as long as the longest: tokens / max_q_len.  Walk
+    and chunks, microseconds: matrix memory, 16 heads of 128 x 128, one sequence (32 blocks), 64 tokens 44 and 28, 256 tokens
+    162 and 64, 512 tokens 135 and 115, 1,024 tokens 150 and 214, 4,096 beside 31 single tokens 575 and 934; two sequences of
+    1,024 tokens 264 and 221, beside 30 single tokens 495 and 269; four 491 and 243; eight 1,338 and 426; 8 heads, 512 tokens
+    91 and 111.  Lightning, 16 heads: 512 tokens 161 and 113, 1,500 beside 7 single tokens 240 and 341; two sequences of 2,048
+    442 and 429, of 1,024 beside 30 334 and 366; four of 1,024 429 and 249.  State space, 32 heads of 128 x 64: 512 tokens 76
+    and 111; two sequences (64) of 1,024 tokens 165 and 207, three (96) 221 and 209, lengths of 1,000, 700, 400 and 100 201
+    and 212, two beside 30 single tokens 392 and 304; 128 heads, 4,096 beside 31 1,607 and 1,272.  Keys of at most 64
+    numbers, whose blocks stay small: 64 tokens 25 and 24, 128 tokens 46 and 31; 128 blocks of 2,048 tokens 388 and 453, 256
+    blocks 738 and 472."""
     if max_q_len < STATE_CHUNKS_FROM[dim <= 64] or dim > 128:
         return False
-    blocks = n_seqs * heads * -(-vdim // 64)
-    return max_q_len <= STATE_WALK_TOKENS or blocks >= (148 if dim <= 64 else 96 if kind == "mamba" else 64)
+    blocks, line = heads * -(-vdim // 64), 148 if dim <= 64 else 96 if kind == "mamba" else 64          # blocks of a sequence
+    if _mostly_single_tokens(n_seqs, tokens, n_seqs * blocks):
+        return False
+    if max_q_len <= STATE_WALK_TOKENS[kind != "mamba" and dim > 64 and n_seqs * blocks >= 32]:
+        return True
+    return n_seqs * blocks >= line and 3 * tokens * blocks >= 2 * line * max_q_len
 
 
 def _state_chunks(kind: str, workspace, proj: torch.Tensor, q_col: int, k_col: int, v_col: int, gates, ld_gates: int, rate,
@@ -1164,19 +1194,19 @@ def _state_chunks(kind: str, workspace, proj: torch.Tensor, q_col: int, k_col: i
                   heads: int, kv_heads: int, dim: int, vdim: int, max_q_len: int) -> bool:
     """Runs a prompt's recurrence by chunks of 32 tokens where that pays and is possible (scratch to be had, keys whose
     rows are whole 16-byte vectors); False: it was not."""
-    if workspace is None or not state_chunks_pay(kind, n_seqs, heads, dim, vdim, max_q_len):
+    tokens = proj.shape[0]
+    if workspace is None or not state_chunks_pay(kind, n_seqs, heads, dim, vdim, max_q_len, tokens):
         return False
     if any(x % 4 for x in (dim, proj.shape[1], q_col, k_col)) or proj.data_ptr() % 16:
         return False
     code, per_head = _STATE_KINDS[kind]
-    tiles = (max_q_len + STATE_CHUNK - 1) // STATE_CHUNK
-    slab = max(1, min(tiles, STATE_SCRATCH_BYTES // (4 * per_head * n_seqs * heads)))
-    scratch = workspace.get("state_chunks", (per_head * n_seqs * heads * slab,), torch.float32)
+    slots, tiles = _chunk_slots(n_seqs, tokens, max_q_len, STATE_CHUNK, 4 * per_head * heads, STATE_SCRATCH_BYTES)
+    scratch = workspace.get("state_chunks", (per_head * heads * slots,), torch.float32)
     _check(_lib("state_chunks").jb_state_chunks(
         code, _ptr(proj), proj.shape[1], int(q_col), int(k_col), int(v_col), _ptr(gates), int(ld_gates), _ptr(rate), _ptr(bias),
         _ptr(skip), float(scale), _ptr(out), _ptr(den), _ptr(state), int(slot_stride), int(state_off), _ptr(q_start),
-        _ptr(seq_slot), n_seqs, heads, kv_heads, dim, vdim, int(max_q_len), _ptr(scratch), slab, _stream()),
-        "state_chunks " + kind, kernels=2 * -(-tiles // slab))
+        _ptr(seq_slot), n_seqs, heads, kv_heads, dim, vdim, int(max_q_len), _ptr(scratch), tiles, tokens, _stream()),
+        "state_chunks " + kind, kernels=2 * -(-int(max_q_len) // (STATE_CHUNK * tiles)) if tiles else 2)
     return True
 
 
@@ -1708,34 +1738,42 @@ def delta_rule(conv: torch.Tensor, q_col: int, k_col: int, v_col: int, raw: torc
         _check(_lib("delta_rule").jb_delta_rule(*args, _stream()), "delta_rule")
         return
     _need(scratch, "delta rule scratch", torch.float32)
-    tiles = scratch.numel() // (n_seqs * heads * _DELTA_CHUNK_FLOATS)
-    if tiles < 1:
+    slots = scratch.numel() // (heads * _DELTA_CHUNK_FLOATS)
+    tiles = min(slots // n_seqs, -(-int(max_q_len) // DELTA_CHUNK))
+    if n_seqs * tiles * DELTA_CHUNK < n_seqs * int(max_q_len) and slots >= T // DELTA_CHUNK + n_seqs:
+        tiles = 0                                          # not every sequence has room for the longest's chunks, but all have for theirs
+    elif tiles < 1:
         raise KernelError("delta_rule: the scratch does not hold one chunk of every sequence")
-    _check(_lib("delta_rule").jb_delta_rule_chunks(*args, int(max_q_len), _ptr(scratch), tiles, _stream()), "delta_rule",
-           kernels=2 * -(-(-(-int(max_q_len) // DELTA_CHUNK)) // tiles))
+    _check(_lib("delta_rule").jb_delta_rule_chunks(*args, int(max_q_len), _ptr(scratch), tiles, T, _stream()), "delta_rule",
+           kernels=2 * -(-int(max_q_len) // (DELTA_CHUNK * tiles)) if tiles else 2)
 
 
 DELTA_CHUNK = 32                                            # tokens of a chunk
 _DELTA_CHUNK_FLOATS = DELTA_CHUNK * (128 + DELTA_CHUNK + 4)   # scratch of a chunk and head: rows of V and of P, four scales
-DELTA_SCRATCH_BYTES = 64 << 20                              # at most: longer prompts go through it slab by slab
+DELTA_SCRATCH_BYTES = 512 << 20                             # as STATE_SCRATCH_BYTES
 DELTA_CHUNKS_FROM = (64, 192)                               # longest sequence's tokens from which chunks are taken ...
 DELTA_CHUNKS_HEADS = 64                                     # ... with this many sequences x heads and more, and with fewer
 
 
-def delta_rule_scratch(n_seqs: int, heads: int, max_q_len: int, conv_width: int, q_col: int, k_col: int, dim: int) -> int:
+def delta_rule_scratch(n_seqs: int, heads: int, max_q_len: int, conv_width: int, q_col: int, k_col: int, dim: int,
+                       tokens: Optional[int] = None, vdim: int = 128) -> int:
     """Floats of scratch with which `delta_rule` goes by chunks; 0: it walks token by token.  Chunks take keys of 68 to 128
-    numbers whose rows are whole 16-byte vectors.  Walk and chunks, microseconds, heads of 128 x 128: one sequence of 16
-    heads, 64 tokens 20.6 and 26.8, 128 tokens 35.0 and 36.9, 192 tokens 49.2 and 45.8, 2,048 tokens 448 and 340; four
-    sequences, 64 tokens 50.9 and 41.1, 512 tokens 321 and 199; eight, 32 tokens 54.6 and 46.9, 2,048 tokens 2,339 and 1,384.
-    72 x 72 is much the same; keys of 64 would be padded to 128 (eight sequences of 32 heads of 64 x 64, 256 tokens: 211 and
-    236)."""
-    if not 64 < dim <= 128 or max_q_len < DELTA_CHUNKS_FROM[n_seqs * heads < DELTA_CHUNKS_HEADS]:
+    numbers whose rows are whole 16-byte vectors.  `tokens`: of all sequences (None: each is as long as the longest).  Walk
+    and chunks, microseconds, heads of 128 x 128: one sequence of 16 heads, 64 tokens 21 and 27, 128 tokens 35 and 37, 192
+    tokens 50 and 47, 2,048 tokens 447 and 347, 4,096 beside 31 single tokens 1,263 and 697; four sequences, 64 tokens 52 and
+    41, 512 tokens 321 and 202; eight, 32 tokens 56 and 47, 2,048 tokens 2,334 and 1,294; two of 1,024 beside 30 single tokens
+    318 and 310.  72 x 72 is much the same (eight of 256 tokens 216 and 144); keys of 64 would be padded to 128 (eight
+    sequences of 32 heads of 64 x 64, 256 tokens: 211 and 236)."""
+    if max_q_len < 1:
         return 0
-    if any(x % 4 for x in (dim, conv_width, q_col, k_col)):
+    if tokens is None:                                     # every sequence is as long as the longest
+        tokens = n_seqs * max_q_len
+    if not 64 < dim <= 128 or max_q_len < DELTA_CHUNKS_FROM[tokens * heads < max_q_len * DELTA_CHUNKS_HEADS]:
         return 0
-    per_tile = n_seqs * heads * _DELTA_CHUNK_FLOATS
-    tiles = (max_q_len + DELTA_CHUNK - 1) // DELTA_CHUNK
-    return per_tile * max(1, min(tiles, DELTA_SCRATCH_BYTES // (4 * per_tile)))
+    if any(x % 4 for x in (dim, conv_width, q_col, k_col)) or _mostly_single_tokens(n_seqs, tokens, n_seqs * heads * -(-vdim // 16)):
+        return 0
+    return heads * _DELTA_CHUNK_FLOATS * _chunk_slots(n_seqs, tokens, max_q_len, DELTA_CHUNK, 4 * heads * _DELTA_CHUNK_FLOATS,
+                                                      DELTA_SCRATCH_BYTES)[0]
 
 
 # -- experts of which a token uses a few ---------------------------------------------------------------------------

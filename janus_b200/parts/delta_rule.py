@@ -101,7 +101,7 @@ class GatedDeltaRule(Mixer):
                              ctx.token_seq, ctx.q_start, ctx.seq_slot, conv, ctx.n_seqs, single_tokens=ctx.is_decode)
         o = ws.get("delta_o", (T, self.v_width), torch.float32)
         floats = 0 if ctx.is_decode else ops.delta_rule_scratch(ctx.n_seqs, self.nh, ctx.max_q_len, self.channels, 0,
-                                                                self.qk_width, self.dim)
+                                                                self.qk_width, self.dim, ctx.n_tokens, self.vdim)
         scratch = ws.get("delta_scratch", (floats,), torch.float32) if floats else None
         ops.delta_rule(conv, 0, self.qk_width, 2 * self.qk_width, proj, self.b_col, self.a_col, self.a_log,
                        self.dt_bias, UNIT_EPS, o, state, 0, ctx.q_start, ctx.seq_slot, ctx.n_seqs, self.nh, self.nkv,

@@ -625,3 +625,43 @@ def test_conv_rope_cache_reaches_its_taps_only(ops, taps):
         assert not bool(torch.isfinite(got[t:t + taps, c]).any())
         got[t:t + taps, c] = clean[t:t + taps, c]
     assert torch.equal(got, clean)
+
+
+def test_chunks_of_many_sequences(ops, monkeypatch):
+    """A step of 300 sequences of one to 70 tokens, whose chunks lie one after another in the scratch: state space and delta
+    rule against the walk (the forms' own errors against float64 are tested above)."""
+    lens = [(1, 33, 2, 32, 64, 1, 70, 31)[i % 8] for i in range(300)]
+    n, T, H, d, e = 300, sum(lens), 2, 68, 20
+    q_start = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    slots = torch.arange(n - 1, -1, -1, dtype=torch.int32, device=DEV)
+    proj, raw, bias, rate = rnd(T, H * (2 * d + e)), rnd(T, 2 * H, seed=1), rnd(H, seed=2), rnd(H, seed=3, mean=-1.0)
+    before = rnd(n, H * d * e, seed=4, s=0.3)
+    monkeypatch.setattr(ops, "state_chunks_pay", lambda *_: True)
+    results = []
+    for workspace in (Scratch(), None):
+        out, state = torch.full((T, H * e), float("nan"), device=DEV), before.clone()
+        ops.mamba2_scan(proj, H * e, H * (e + d), raw[:, :H].contiguous(), bias, rate, bias, out, state, 0, q_start, slots, n, H, H, d, e, 70, workspace)
+        results.append((out, state))
+    assert worst(results[0][0], results[1][0]) <= 6e-5 and worst(results[0][1], results[1][1]) <= 6e-5
+    results = []
+    for slots_of in (T // 32 + n, 2 * n, 0):
+        out, state = torch.full((T, H * e), float("nan"), device=DEV), before.clone()
+        scratch = torch.full((slots_of * H * ops._DELTA_CHUNK_FLOATS,), float("nan"), device=DEV) if slots_of else None
+        ops.delta_rule(proj, 0, H * d, 2 * H * d, raw, 0, H, rate, bias, 1e-6, out, state, 0, q_start, slots, n, H, H, d, e, scratch, 70)
+        results.append((out, state))
+    for got in results[:2]:
+        assert worst(got[0], results[2][0]) <= 4e-5 and worst(got[1], results[2][1]) <= 4e-5
+
+
+@pytest.mark.parametrize("lens, chunks", [([4096] + [1] * 31, False), ([1024] * 8 + [1] * 24, True), ([200] + [1] * 63, False),
+                                          ([1024, 1024], True), ([1, 1, 1500, 1], False)])
+def test_mixed_steps_take_the_form_of_their_work(ops, lens, chunks):
+    """What decides between walk and chunks is the work that exists: one long prompt among single tokens has the blocks of
+    one sequence, and single tokens alone are no reason for chunks."""
+    n, T, H, d, e = len(lens), sum(lens), 16, 128, 128
+    q_start = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    proj, out = rnd(T, H * (2 * d + e)), torch.empty(T, H * e, device=DEV)
+    state, workspace = torch.zeros(n, H, d, e, device=DEV), Scratch()
+    ops.lightning_scan(proj, 0, H * d, 2 * H * d, out, state, q_start, torch.arange(n, dtype=torch.int32, device=DEV),
+                       torch.full((H,), 0.9, device=DEV), n, H, d, e, max(lens), workspace)
+    assert ("state_chunks" in workspace.asked) == chunks
