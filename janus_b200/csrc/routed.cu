@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(DN_WARPS * 32) expert_down_kernel(
 // are two steps' fragments under a permutation of the columns that the pairs' fragments share (a dot product does not
 // mind the order), so the weights stream once, 16 bytes a lane, and the pairs' rows come from L2 the same way.
 constexpr int TC_WARPS = 8, NG = 2;
-constexpr int DEEP_BLOCKS = 4 * 148;           // blocks of the second product up to which one wave holds them all: DEEP
+constexpr int DEEP_BLOCKS = 2 * 148;           // blocks of the second product that two an SM hold in one wave: up to here DEEP
 
 __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                           uint32_t b1) {
@@ -369,9 +369,11 @@ __device__ __forceinline__ uint4 stream16(const bf16* p) {
 // c a block.  K: the rows' width (a multiple of 32), R: the number of rows.
 // Bound by the weights' bytes, if enough of them are asked for.  DEEP: 256 bytes a lane at a time, two blocks an SM; else 64
 // bytes, and four blocks an SM, whose loads fill each other's waits for sums and stores.  The second product (few columns a
-// warp, then a sum and a store) gains from more blocks as soon as there are several an SM: 16 tokens, two of 8 experts,
-// 4096 -> 2048: 42.5 -> 27 us, 8 tokens 41 -> 32, 2 tokens of 7168 -> 4096: 64 -> 54; with one token (256 blocks) it takes
-// 17.7 us so and 13.5 DEEP.  The first product has enough in flight: 48.8, 46.3 and 82.7 us DEEP, 52.5, 52.9 and 92.3 else.
+// warp, then a sum and a store) gains from more blocks as soon as there are more than one wave of DEEP ones: 16 tokens, two of
+// 8 experts, 4096 -> 2048: 42.5 -> 27 us, 8 tokens 41 -> 32, 2 tokens of 7168 -> 4096: 64 -> 54; both products of two experts
+// from cold memory, DEEP and else: 256 blocks 34 and 32, 296 38 and 36 (four experts 26 and 26), 400 50 and 40, 512 54 and 46,
+// 592 60 and 52, 744 73 and 65.  In a decode step, behind the first product, one token's 256 blocks take 13.5 us DEEP and 17.7
+// else.  The first product has enough in flight: 48.8, 46.3 and 82.7 us DEEP, 52.5, 52.9 and 92.3 else.
 template <int MATS, bool DEEP>
 __global__ void __launch_bounds__(TC_WARPS * 32, DEEP ? 2 : 4) expert_tc_kernel(
     const bf16* __restrict__ x, const int* __restrict__ sel_e, const float* __restrict__ sel_w, int top, int n_pairs,

@@ -665,3 +665,9 @@ def test_mixed_steps_take_the_form_of_their_work(ops, lens, chunks):
     ops.lightning_scan(proj, 0, H * d, 2 * H * d, out, state, q_start, torch.arange(n, dtype=torch.int32, device=DEV),
                        torch.full((H,), 0.9, device=DEV), n, H, d, e, max(lens), workspace)
     assert ("state_chunks" in workspace.asked) == chunks
+
+
+@pytest.mark.parametrize("W, E", [(2368, 2), (2400, 2)])
+def test_expert_down_blocks_of_one_wave(ops, W, E):
+    """The second product at 296 blocks, two an SM, and at 300."""
+    test_expert_down_blocks(ops, 1, W, E)
