@@ -418,10 +418,15 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 // step's weights have passed through L2 (4 sequences x 16 heads over 516 keys: 26.6 -> 14.9 us; before, a lane's value rows came
 // eight at a time after the scores, one warp added up sixteen parts one after another, and two warps had a second chunk).
 constexpr int STAGED_PAIRS = 4096;         // more of them than the SMs hold at once have other blocks' loads to wait under
-constexpr int STAGED_WARPS = 20;           // the chunks of a window of 512 keys and of kept keys that it has left behind
+// Warps of a block at most: 16, which leaves a thread 128 registers for loads in flight.  17 to 20 chunks, a window of 512 keys
+// and the kept keys that it has left behind, are worth 20 warps where every SM has one block: one round instead of two (16
+// heads, cold pages, 600 keys of a window of 512: 20.5 us with 20 warps, 22.5 with 16; a window of 1,024, two rounds or three:
+// 32.7 either way; without a window 750 keys 28.6 and 26.6, 4,000 keys 94 and 86, 16,000 keys 305 and 289; 64 sequences in
+// a window of 512, blocks of 4 warps whichever it is: 100 and 86 by the registers alone).
+constexpr int STAGED_WARPS = 16, STAGED_ROUND = 20;
 
-template <int EJ>
-__global__ void __launch_bounds__(STAGED_WARPS * 32) diff_attention_staged_kernel(
+template <int EJ, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) diff_attention_staged_kernel(
     const float* __restrict__ q, const bf16* __restrict__ k_cache, const bf16* __restrict__ v_cache, bf16* __restrict__ out,
     const int* __restrict__ block_table, const int* __restrict__ token_seq, const int* __restrict__ positions, int H, int G,
     int d, int e, int page_size, int max_pages, int window, int keep_first, float scale, float lambda, float eps,
@@ -432,7 +437,7 @@ __global__ void __launch_bounds__(STAGED_WARPS * 32) diff_attention_staged_kerne
   bf16* vs = reinterpret_cast<bf16*>(staged_smem) + (size_t)warp * 32 * e;     // this warp's 32 value rows
   float* qw = reinterpret_cast<float*>(staged_smem + (size_t)warps * 64 * e);  // q [2 d], parts [warp][2][32 EJ], then m, l
   float* parts = qw + 2 * d;
-  float* ml = parts + warps * PART;                                            // [4][STAGED_WARPS]: m1, l1, m2, l2
+  float* ml = parts + warps * PART;                                            // [4][WARPS]: m1, l1, m2, l2
   jb::pdl_launch_dependents();
   jb::pdl_wait();
   const int t = blockIdx.x / H, h = blockIdx.x % H, g = h / (H / G);
@@ -534,16 +539,16 @@ __global__ void __launch_bounds__(STAGED_WARPS * 32) diff_attention_staged_kerne
     parts[warp * PART + 32 * j + lane] = a1[j];
     parts[warp * PART + 32 * EJ + 32 * j + lane] = a2[j];
   }
-  if (lane == 0) ml[warp] = m1, ml[STAGED_WARPS + warp] = l1, ml[2 * STAGED_WARPS + warp] = m2, ml[3 * STAGED_WARPS + warp] = l2;
+  if (lane == 0) ml[warp] = m1, ml[WARPS + warp] = l1, ml[2 * WARPS + warp] = m2, ml[3 * WARPS + warp] = l2;
   __syncthreads();
   if (warp != 0) return;
   const bool there = lane < warps && lane < chunks;                            // a warp without a chunk weighs nothing
   m1 = there ? ml[lane] : -CUDART_INF_F;
-  m2 = there ? ml[2 * STAGED_WARPS + lane] : -CUDART_INF_F;
+  m2 = there ? ml[2 * WARPS + lane] : -CUDART_INF_F;
   const float top1 = jb::warp_max(m1), top2 = jb::warp_max(m2);
   const float f1 = there && m1 != -CUDART_INF_F ? expf(m1 - top1) : 0.0f, f2 = there && m2 != -CUDART_INF_F ? expf(m2 - top2) : 0.0f;
-  l1 = jb::warp_sum(there ? ml[STAGED_WARPS + lane] * f1 : 0.0f);
-  l2 = jb::warp_sum(there ? ml[3 * STAGED_WARPS + lane] * f2 : 0.0f);
+  l1 = jb::warp_sum(there ? ml[WARPS + lane] * f1 : 0.0f);
+  l2 = jb::warp_sum(there ? ml[3 * WARPS + lane] * f2 : 0.0f);
 #pragma unroll
   for (int j = 0; j < EJ; ++j) a1[j] = a2[j] = 0.0f;
 #pragma unroll 4
@@ -833,11 +838,13 @@ JB_EXPORT int jb_diff_attention(const float* q, const void* k_cache, const void*
       page_size % 32 == 0 && (((uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0) {
     const int chunks = (int)((keys + 62) / 32 + (window > 0 && keep_first > 0 ? 1 : 0));     // of a query at most
     int w = warps;
-    if (w == max_warps(4) && (long long)T * H <= sms) w = STAGED_WARPS;        // one block an SM has room for all of them
-    if (w > STAGED_WARPS) w = STAGED_WARPS;
+    const bool round = w >= STAGED_WARPS && (long long)T * H <= sms && chunks > STAGED_WARPS && chunks <= STAGED_ROUND;
+    if (round) w = STAGED_ROUND;
+    else if (w > STAGED_WARPS) w = STAGED_WARPS;
     if (w > chunks) w = chunks;
-    const size_t bytes = (size_t)w * 64 * e + (size_t)(2 * d + w * 64 * EJ_ + 4 * STAGED_WARPS) * sizeof(float);
-    auto* fn = e <= 64 ? diff_attention_staged_kernel<2> : diff_attention_staged_kernel<4>;
+    const size_t bytes = (size_t)w * 64 * e + (size_t)(2 * d + w * 64 * EJ_ + 4 * (round ? STAGED_ROUND : STAGED_WARPS)) * sizeof(float);
+    auto* fn = e <= 64 ? (round ? diff_attention_staged_kernel<2, STAGED_ROUND> : diff_attention_staged_kernel<2, STAGED_WARPS>)
+                       : (round ? diff_attention_staged_kernel<4, STAGED_ROUND> : diff_attention_staged_kernel<4, STAGED_WARPS>);
     cudaError_t se = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (se != cudaSuccess) return (int)se;
     jb::Launch scfg(dim3((unsigned)(T * H)), dim3(w * 32), bytes, stream);

@@ -671,3 +671,24 @@ def test_mixed_steps_take_the_form_of_their_work(ops, lens, chunks):
 def test_expert_down_blocks_of_one_wave(ops, W, E):
     """The second product at 296 blocks, two an SM, and at 300."""
     test_expert_down_blocks(ops, 1, W, E)
+
+
+@pytest.mark.parametrize("e", [64, 128])
+@pytest.mark.parametrize("window, n", [(448, 600), (512, 600), (544, 640), (576, 640), (0, 512), (0, 513), (0, 640), (0, 641)])
+def test_diff_attention_rounds(ops, e, window, n):
+    """One sequence whose query sees 15 to 21 chunks of 32 keys: 16 warps, or one round of 17 to 20."""
+    H, G, d, kept, pages = 2, 1, 16, 4, (n + PAGE - 1) // PAGE
+    g = torch.Generator().manual_seed(n + window + e)
+    kc = torch.randn(pages, 2 * G, PAGE, d, generator=g).to(torch.bfloat16).to(DEV)
+    vc = torch.randn(pages, G, PAGE, e, generator=g).to(torch.bfloat16).to(DEV)
+    table = torch.randperm(pages, generator=g).int()[None].to(DEV)
+    q, out = rnd(1, H * 2 * d), torch.empty(1, H * e, dtype=torch.bfloat16, device=DEV)
+    ops.diff_attention(q, kc, vc, out, table, ints(0), ints(n - 1), H, G, d, e, PAGE, window, kept, 0.25, 0.4, 1e-5, 0.5)
+    k = kc[table[0].long()].double().permute(1, 0, 2, 3).reshape(G, 2, -1, d)[:, :, :n]
+    v = vc[table[0].long()].double().permute(1, 0, 2, 3).reshape(G, -1, e)[:, :n]
+    j = torch.arange(n, device=DEV)
+    seen = (n - 1 - j < window) | (j < kept) if window else torch.ones(n, dtype=torch.bool, device=DEV)
+    s = torch.einsum("hmd,hmnd->hmn", q.double().view(H, 2, d), k.repeat_interleave(H // G, 0)) * 0.25
+    maps = torch.einsum("hmn,hne->hme", torch.softmax(s.masked_fill(~seen, -math.inf), -1), v.repeat_interleave(H // G, 0))
+    # bfloat16, and a difference that nearly cancels, as above
+    assert worst(out.view(H, e), unit(maps[:, 0] - 0.4 * maps[:, 1], 1e-5) * 0.5) <= 4 * TOL[torch.bfloat16]
