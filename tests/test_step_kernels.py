@@ -673,6 +673,42 @@ def test_expert_down_blocks_of_one_wave(ops, W, E):
     test_expert_down_blocks(ops, 1, W, E)
 
 
+@pytest.mark.parametrize("H, G, lens, slab", [(8, 2, [1600, 1500], 0), (32, 2, [2400], 0), (20, 2, [70, 33], 0), (12, 12, [700, 650, 1], 3)])
+def test_delta_rule_chunks_of_many_heads(ops, H, G, lens, slab):
+    """Blocks that prepare several heads of a group (two to eight, and groups of more than eight in several blocks), with
+    decays that underflow to zero within a chunk and forget all before, against the walk and the walk against float64."""
+    T, n, d, e = sum(lens), len(lens), 128, 40
+    conv, raw = rnd(T, 2 * G * d + H * e), rnd(T, 2 * H, seed=1)
+    raw[13::29, H:] = 300.0                                   # a decay of exp(-100) and less at every 29th token
+    a_log, bias, before = rnd(H, seed=2, mean=-1.0), rnd(H, seed=3), rnd(n, H * d * e, seed=4, s=0.3)
+    q_start = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    slots = torch.arange(n - 1, -1, -1, dtype=torch.int32, device=DEV)
+    results = []
+    for floats in ((slab or (max(lens) + 31) // 32) * n * H * ops._DELTA_CHUNK_FLOATS, 0):
+        out, state = torch.full((T, H * e), float("nan"), device=DEV), before.clone()
+        ops.delta_rule(conv, 0, G * d, 2 * G * d, raw, 0, H, a_log, bias, 1e-6, out, state, 0, q_start, slots, n, H, G, d, e,
+                       torch.full((floats,), float("nan"), device=DEV) if floats else None, max(lens))
+        results.append((out, state))
+    x = conv.double()
+    norm = lambda t: (t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)).repeat_interleave(H // G, 1)      # noqa: E731
+    q, k = norm(x[:, :G * d].view(T, G, d)) * d ** -0.5, norm(x[:, G * d:2 * G * d].view(T, G, d))
+    v, beta, z = x[:, 2 * G * d:].reshape(T, H, e), torch.sigmoid(raw[:, :H].double()), raw[:, H:].double() + bias.double()
+    decay = torch.exp(-torch.exp(a_log.double()) * torch.logaddexp(z, torch.zeros_like(z)))
+    want, after, at = torch.zeros(T, H, e, dtype=torch.float64, device=DEV), before.double().clone(), 0
+    for s, length in enumerate(lens):
+        S = before[slots[s].long()].double().view(H, d, e)
+        for t in range(at, at + length):
+            S = decay[t][:, None, None] * S
+            w = beta[t][:, None] * (v[t] - torch.einsum("hde,hd->he", S, k[t]))
+            S = S + k[t][:, :, None] * w[:, None, :]
+            want[t] = torch.einsum("hde,hd->he", S, q[t])
+        after[slots[s].long()] = S.reshape(-1)
+        at += length
+    # as for the sizes above: a few hundred roundings of 2^-24 against the mean size of a result
+    err = [max(worst(o.view(T, H, e), want), worst(s, after)) for o, s in results]
+    assert err[0] <= 4e-5 and err[0] <= 4 * err[1] + 4e-6, err
+
+
 @pytest.mark.parametrize("e", [64, 128])
 @pytest.mark.parametrize("window, n", [(448, 600), (512, 600), (544, 640), (576, 640), (0, 512), (0, 513), (0, 640), (0, 641)])
 def test_diff_attention_rounds(ops, e, window, n):
