@@ -6,8 +6,8 @@
 // stored, where nothing is accumulated).
 // Even and odd k apart, because a packed multiply-add (`fma.rn.f32x2`) takes them as they lie in memory: the same 128
 // multiply-adds a cycle and SM in half the instructions (1,000 tokens x 16,384 rows x 2,048: 2,079 -> 1,855 us).
-// Short sums that meet in a shallow tree are also closer to the exact result than one chain over K (K = 8,192: 2.9e-7
-// against 1.6e-6 of the result).
+// Short sums that meet in a shallow tree are also closer to the exact result than one chain over K (K = 8,192: 1.4e-7
+// against 1.6e-6 of the result, 2-norms).
 // Formula: crates/janus-engine/src/compute/shaders/gemm_f32.wgsl:23-75
 // (weights [N, K] row-major, f32 accumulation over 16-wide k tiles).
 #include <cooperative_groups.h>
@@ -48,16 +48,17 @@ __device__ __forceinline__ void async_wait() {
 }
 
 // ---- few tokens: the product streams the weights -----------------------------------------------------------------
-// A block owns 8 or 16 weight rows at a time, each of its up to eight warps a range of k of them, walked by itself in
-// units of 256 k: lane (r, s) sums segment s of the unit for rows r (and 8 + r) and all tokens, so that 32 chains of 64
+// A block owns 16 weight rows at a time, each of its up to eight warps a range of k of them, walked by itself in
+// units of 256 k: lane (r, s) sums segment s of the unit for rows r and 8 + r and all tokens, so that 32 chains of 64
 // products run side by side.  A stage is half of a unit's segments, pieces of 128 contiguous bytes of every row and
 // token with 16 bytes of padding between them (the eight lanes of a shared-memory phase read eight different banks);
-// a warp's ring of 2 to 4 stages is its own, so nothing synchronises the block until the ranges meet, and it runs on
+// a warp's ring of two stages is its own, so nothing synchronises the block until the ranges meet, and it runs on
 // over the rows that a block works through one after another.  The first stages' weights are asked for before the
 // kernel that makes X has ended.
 constexpr int SUB = 32, PIECE = SUB + 4;       // numbers of a piece, and its pitch
+constexpr int RL = 2, STAGES = 2;              // rows of a lane, stages of a ring
 
-template <int TT, int RL, int STAGES>
+template <int TT>
 __global__ void __launch_bounds__(32 * RANGES) gemm_f32_stream_kernel(const float* __restrict__ X, const float* __restrict__ W,
                                                                       float* __restrict__ Y, int T, int N, int K, int ldx,
                                                                       int ldy, int accumulate) {
@@ -320,10 +321,10 @@ __global__ void __launch_bounds__(BT, 2) gemm_f32_tile_kernel(const float* __res
   }
 }
 
-template <int TT, int RL, int STAGES>
+template <int TT>
 int launch_stream(const float* X, const float* W, float* Y, int T, int N, int K, int ldx, int ldy, int accumulate,
                   cudaStream_t stream) {
-  auto* fn = gemm_f32_stream_kernel<TT, RL, STAGES>;
+  auto* fn = gemm_f32_stream_kernel<TT>;
   const int rows = 8 * RL, blocks = (N + rows - 1) / rows, range = range_of(K), ranges = (K + range - 1) / range;
   const size_t smem = 4 * (size_t)(RANGES * TT * rows + ranges * STAGES * (rows + TT) * SEGS * PIECE);
   const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -342,8 +343,12 @@ JB_EXPORT int jb_gemm_f32(const float* X, const float* W, float* Y, int T, int N
   // rows of whole 16-byte vectors (K and the rows' starts)
   const bool vec = K % 4 == 0 && ldx % 4 == 0 && (((uintptr_t)X | (uintptr_t)W) & 15) == 0;
   const int tiles = ((N + BN - 1) / BN) * ((T + BM - 1) / BM);
+  // The streaming kernel asks for the weights once for every 8 tokens, the tiles need some of them to fill the SMs.  Streamed and
+  // tiles from cold memory, microseconds, K = 2,048: 16 tokens 2,048 rows 20 and 39, 8,192 rows 50 and 82, 32,000 rows 172 and
+  // 233; 24 tokens 27 and 39, 72 and 82, 250 and 233 (16,384 rows 133 and 143, 4,096 rows 43 and 41); 32 tokens 33 and 39, 92
+  // and 82, 332 and 235 (2,560 rows 39 and 39; 2,048 rows of 8,192 90 and 123); 40 tokens of 2,048 rows 39 and 39.
   if (vec && (T <= 24 || (T <= 32 && N <= 20 * BN))) {
-#define JB_GO(TT) return launch_stream<TT, 2, 2>(X, W, Y, T, N, K, ldx, ldy, accumulate, stream)
+#define JB_GO(TT) return launch_stream<TT>(X, W, Y, T, N, K, ldx, ldy, accumulate, stream)
     if (T == 1) JB_GO(1);
     if (T == 2) JB_GO(2);
     if (T <= 4) JB_GO(4);

@@ -115,57 +115,57 @@ __global__ void causal_conv_silu_vec_kernel(const float* __restrict__ proj, int 
   int next_seq[AHEAD];
   for (int tb = t0; tb < t1; tb += AHEAD) {
 #pragma unroll
-  for (int k = 0; k < AHEAD; ++k) {
-    const int t = min(tb + k, t1 - 1);
-    next_seq[k] = token_seq[t];
-    next[k] = *reinterpret_cast<const float4*>(proj + (size_t)t * ld + col0 + c);
-  }
+    for (int k = 0; k < AHEAD; ++k) {
+      const int t = min(tb + k, t1 - 1);
+      next_seq[k] = token_seq[t];
+      next[k] = *reinterpret_cast<const float4*>(proj + (size_t)t * ld + col0 + c);
+    }
 #pragma unroll
-  for (int k = 0; k < AHEAD; ++k) {
-    const int t = tb + k;
-    if (t >= t1) break;
-    const int seq = next_seq[k];
-    if (seq != seq_before) {               // the tile's first token, or a sequence's first: fill the window
-      const int s0 = q_start[seq], li = t - s0;
-      const float* st = state + (size_t)seq_slot[seq] * slot_stride + state_off;
+    for (int k = 0; k < AHEAD; ++k) {
+      const int t = tb + k;
+      if (t >= t1) break;
+      const int seq = next_seq[k];
+      if (seq != seq_before) {               // the tile's first token, or a sequence's first: fill the window
+        const int s0 = q_start[seq], li = t - s0;
+        const float* st = state + (size_t)seq_slot[seq] * slot_stride + state_off;
+#pragma unroll
+        for (int j = 0; j < MAX - 1; ++j) {
+          if (j < taps - 1) {
+            const int src = li - (taps - 1) + j;
+            win[j] = src >= 0 ? *reinterpret_cast<const float4*>(proj + (size_t)(s0 + src) * ld + col0 + c)
+                              : *reinterpret_cast<const float4*>(st + (size_t)(taps - 1 + src) * C + c);
+          }
+        }
+        seq_before = seq;
+      }
+      const float4 u = next[k];
+      float4 acc = b4;
 #pragma unroll
       for (int j = 0; j < MAX - 1; ++j) {
         if (j < taps - 1) {
-          const int src = li - (taps - 1) + j;
-          win[j] = src >= 0 ? *reinterpret_cast<const float4*>(proj + (size_t)(s0 + src) * ld + col0 + c)
-                            : *reinterpret_cast<const float4*>(st + (size_t)(taps - 1 + src) * C + c);
+          acc.x = fmaf(wr[0][j], win[j].x, acc.x);
+          acc.y = fmaf(wr[1][j], win[j].y, acc.y);
+          acc.z = fmaf(wr[2][j], win[j].z, acc.z);
+          acc.w = fmaf(wr[3][j], win[j].w, acc.w);
         }
       }
-      seq_before = seq;
-    }
-    const float4 u = next[k];
-    float4 acc = b4;
 #pragma unroll
-    for (int j = 0; j < MAX - 1; ++j) {
-      if (j < taps - 1) {
-        acc.x = fmaf(wr[0][j], win[j].x, acc.x);
-        acc.y = fmaf(wr[1][j], win[j].y, acc.y);
-        acc.z = fmaf(wr[2][j], win[j].z, acc.z);
-        acc.w = fmaf(wr[3][j], win[j].w, acc.w);
+      for (int j = 0; j < MAX; ++j) {
+        if (j == taps - 1) {
+          acc.x = fmaf(wr[0][j], u.x, acc.x);
+          acc.y = fmaf(wr[1][j], u.y, acc.y);
+          acc.z = fmaf(wr[2][j], u.z, acc.z);
+          acc.w = fmaf(wr[3][j], u.w, acc.w);
+        }
       }
+      *reinterpret_cast<float4*>(out + (size_t)t * C + c) = silu4(acc);
+#pragma unroll
+      for (int j = 0; j < MAX - 2; ++j)
+        if (j < taps - 2) win[j] = win[j + 1];
+#pragma unroll
+      for (int j = 0; j < MAX - 1; ++j)
+        if (j == taps - 2) win[j] = u;
     }
-#pragma unroll
-    for (int j = 0; j < MAX; ++j) {
-      if (j == taps - 1) {
-        acc.x = fmaf(wr[0][j], u.x, acc.x);
-        acc.y = fmaf(wr[1][j], u.y, acc.y);
-        acc.z = fmaf(wr[2][j], u.z, acc.z);
-        acc.w = fmaf(wr[3][j], u.w, acc.w);
-      }
-    }
-    *reinterpret_cast<float4*>(out + (size_t)t * C + c) = silu4(acc);
-#pragma unroll
-    for (int j = 0; j < MAX - 2; ++j)
-      if (j < taps - 2) win[j] = win[j + 1];
-#pragma unroll
-    for (int j = 0; j < MAX - 1; ++j)
-      if (j == taps - 2) win[j] = u;
-  }
   }
 }
 
@@ -508,11 +508,10 @@ __device__ __forceinline__ void store4_out(bf16* p, float4 v) {
   *reinterpret_cast<uint2*>(p) = raw;
 }
 
-// Pieces made of whole 16-byte vectors: the gated values stay in shared memory between the two passes (the piece is
-// read once), 16 bytes a thread.
 // gated_group_rmsnorm with a piece's values in registers, CACHE vectors a thread, all loads in flight together and the
 // weight asked for before the wait: few rows take 1,024 threads a piece (8 rows of 8,192: 12 us through shared memory with
-// 256, 3.8 so; 2,532 rows: 53 and 47 to 53), many 512.
+// 256, 3.8 so; 2,532 rows: 53 and 47 to 53), many 512; whichever it is, a piece is summed in the same 1,024 places (256 up to
+// 2,048 numbers).
 template <typename TO, int THREADS_G, int CACHE>
 __global__ void __launch_bounds__(THREADS_G) gated_group_rmsnorm_rows_kernel(const float* __restrict__ y,
                                                                              const float* __restrict__ gate, int gate_ld,
@@ -551,6 +550,8 @@ __global__ void __launch_bounds__(THREADS_G) gated_group_rmsnorm_rows_kernel(con
   }
 }
 
+// Other pieces made of whole 16-byte vectors: the gated values stay in shared memory between the two passes (the piece is
+// read once), 16 bytes a thread.
 template <typename TO>
 __global__ void gated_group_rmsnorm_vec_kernel(const float* __restrict__ y, const float* __restrict__ gate, int gate_ld,
                                                const float* __restrict__ w, float eps, TO* __restrict__ out, int N,
