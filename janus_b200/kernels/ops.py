@@ -71,6 +71,7 @@ _SIGNATURES = {
     "jb_route_topk": "piiippiiiipfip", "jb_experts_few_tokens": "pippipppippiiiiffip", "jb_expert_gather": "pippipiip", "jb_experts_few_tokens_tc": "pppipppppiiiiffip",
     "jb_expert_scatter": "pppipiip",
     "jb_state_chunks": "ipiiiipipppfpppllppiiiiiipiip",
+    "jb_head_step": "ipiiiifpiiippfiplllpipiifpippiiiiip",
     "jb_gla_decay": "piiippfpiip", "jb_exp_gates": "piiippfppllppiip",
     "jb_gated_linear_scan": "piiiifpiippplppiiiiiippp", "jb_scale_rows_sigmoid": "pipiiip",
     "jb_attention_tc_prefill": "pppppppiiiiiiiiiifpp", "jb_attention_tc_prefill_capped": "pppppppiiiiiiiiiiififfpppipp",
@@ -1746,6 +1747,52 @@ def delta_rule(conv: torch.Tensor, q_col: int, k_col: int, v_col: int, raw: torc
         raise KernelError("delta_rule: the scratch does not hold one chunk of every sequence")
     _check(_lib("delta_rule").jb_delta_rule_chunks(*args, int(max_q_len), _ptr(scratch), tiles, T, _stream()), "delta_rule",
            kernels=2 * -(-int(max_q_len) // (DELTA_CHUNK * tiles)) if tiles else 2)
+
+
+HEAD_STEP_DIM, HEAD_STEP_VDIM = 128, 256                     # sizes that a block of `head_step` holds
+_HEAD_STEP_KINDS = {"delta": 0, "memory": 1, "channel": 2}
+
+
+def head_step_supported(dim: int, vdim: int, state: torch.Tensor, normalizer: bool = False) -> bool:
+    """Whether `head_step` takes heads of this size: a block holds a head's state, in whole 16-byte vectors."""
+    return (dim <= HEAD_STEP_DIM and vdim <= HEAD_STEP_VDIM and vdim % 4 == 0 and dim * (vdim + int(normalizer)) % 4 == 0
+            and state.shape[1] % 4 == 0 and state.data_ptr() % 16 == 0)
+
+
+def head_step(kind: str, rows: torch.Tensor, q_col: int, k_col: int, v_col: int, q_scale: float, raw: torch.Tensor, col_a: int,
+              col_b: int, p0: torch.Tensor, p1: torch.Tensor, scalar: float, state: torch.Tensor, gate: torch.Tensor,
+              weight: torch.Tensor, eps: float, out: torch.Tensor, q_start: torch.Tensor, seq_slot: torch.Tensor, heads: int,
+              kv_heads: int, dim: int, vdim: int, m_off: int = 0, sigmoid: bool = False) -> None:
+    """A step of one token a sequence through a recurrence, its heads' norm and their output gate, in one launch: q, k, v are
+    columns of the float32 `rows`; the state's heads begin a slot's row.  `kind` "delta": `delta_rule`, with beta's argument
+    at column col_a of `raw` and the decay's at col_b, p0 = A_log, p1 = dt_bias, scalar = the unit vectors' eps; "memory":
+    `exp_gates` and `gated_linear_scan` with divisors: col_a, col_b = the gates' columns, p0, p1 = their biases, scalar = the
+    cap, maxima at m_off; "channel": `gla_decay` and `gated_linear_scan`: col_a = the low-rank columns, p0 = the second
+    matrix, transposed [rank, heads dim], p1 = its bias, scalar = 1 / tau.  Then `head_norm_gate` with gate, weight and eps."""
+    T = rows.shape[0]
+    _need(rows, "projections", torch.float32)
+    _need(raw, "gates' arguments", torch.float32)
+    _need(state, "state", torch.float32)
+    _need(out, "gated heads", None, (T, heads * vdim))
+    _need(q_start, "q_start", torch.int32, (T + 1,))
+    _need(seq_slot, "sequence slots", torch.int32, (T,))
+    channel = kind == "channel"
+    _need(p0, "gates' parameters", torch.float32, (p0.shape[0], heads * dim) if channel else (heads,))
+    _need(p1, "gates' parameters", torch.float32, (heads * dim,) if channel else (heads,))
+    per_head = weight.numel() == heads * vdim and heads > 1
+    _need(weight, "head norm weight", torch.float32, (heads * vdim,) if per_head else (vdim,))
+    if gate.dtype != torch.float32 or gate.stride(1) != 1 or tuple(gate.shape) != (T, heads * vdim):
+        raise KernelError("head_step: the gate must be float32 columns of the heads' shape")
+    if raw.shape[0] != T or state.dim() != 2 or state.shape[1] < max(heads * dim * (vdim + (kind == "memory")), m_off):
+        raise KernelError("head_step: the rows or the state do not hold what the step reads")
+    if max(q_col + kv_heads * dim, k_col + kv_heads * dim, v_col + heads * vdim) > rows.shape[1]:
+        raise KernelError("head_step: the projections' columns reach past the rows")
+    _check(_lib("head_step").jb_head_step(
+        _HEAD_STEP_KINDS[kind], _ptr(rows), rows.shape[1], int(q_col), int(k_col), int(v_col), float(q_scale), _ptr(raw),
+        raw.shape[1], int(col_a), int(col_b), _ptr(p0), _ptr(p1), float(scalar), p0.shape[0] if channel else 0, _ptr(state),
+        state.shape[1], 0, int(m_off), _ptr(gate), gate.stride(0), _ptr(weight), vdim if per_head else 0, int(bool(sigmoid)),
+        float(eps), _ptr(out), dtype_code(out.dtype), _ptr(q_start), _ptr(seq_slot), T, heads, kv_heads, dim, vdim, _stream()),
+        "head_step " + kind)
 
 
 DELTA_CHUNK = 32                                            # tokens of a chunk

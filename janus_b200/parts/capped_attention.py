@@ -142,6 +142,11 @@ class CappedAttention(Mixer):
                 raise ValueError(f"a share of the first values of shape {tuple(vmix.shape)} is not one number")
             self.vmix = float(vmix)
 
+    @property
+    def shares_projection(self) -> bool:
+        """Whether `forward` takes the projections as the first columns of a wider matrix that lasts as long as the call."""
+        return self.value_mix != "first"
+
     def _projections(self, ctx, tokens: int) -> torch.Tensor:
         # the place whose values others mix in has a buffer of its own, which lasts as long as the step
         name = "capped_proj_first" if self.value_mix == "first" else "capped_proj"
@@ -164,20 +169,26 @@ class CappedAttention(Mixer):
         return buf if buf.numel() % 4 == 0 else None
 
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx, cache_view, writes_cache: bool = True,
-                scratch_cleared: bool = False) -> None:
+                scratch_cleared: bool = False, projected: Optional[tuple] = None) -> None:
+        """`projected` (matrix, 0): a float32 matrix whose first columns are this part's projections of x."""
         if not writes_cache:
             raise ValueError("this attention writes its own keys and values; it cannot read another place's")
         T = x.shape[0]
         ws = ctx.workspace
         group = cache_view.group
-        proj = self._projections(ctx, T)
-        self.proj.forward(x, proj, y_is_zero=scratch_cleared)
+        if projected is None:
+            proj = self._projections(ctx, T)
+            self.proj.forward(x, proj, y_is_zero=scratch_cleared)
+        else:
+            proj, col = projected
+            if col:
+                raise ValueError("this attention reads its projections from a matrix's first columns")
         if self.value_mix == "first":
             ctx.shared[FIRST_VALUES] = proj[:, self.v_col: self.gate_col]
         first = self._first_values(ctx, T)
         table = self.position.fused_rotary_table() if self.position is not None else None
         D, E = self.k_stored, self.v_stored
-        gate = proj[:, self.gate_col:] if self.gate else None
+        gate = proj[:, self.gate_col: self.gate_col + self.gate_width] if self.gate else None
         heads = dict(chunk=self.chunk, softcap=self.softcap, sink=self.sink, vd=E, slopes=self.slopes, sinks=self.sinks,
                      gate=gate if self.head_gate else None)
         attn = ws.get("capped_attn", (T, self.nh * E), self.dtype)

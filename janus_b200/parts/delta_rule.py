@@ -79,6 +79,8 @@ class GatedDeltaRule(Mixer):
         self.a_log, self.dt_bias = f32("A_log", A_log, (self.nh,)), f32("dt_bias", dt_bias, (self.nh,))
         self.norm_weight = f32("norm", norm, (self.vdim,))
 
+    shares_projection = True      # `forward` takes the projections as columns of a wider matrix
+
     def scratch_to_clear(self, ctx, tokens: int, writes_cache: bool = True) -> Optional[torch.Tensor]:
         """The projection's float32 buffer, if this step's product adds slices of K into it (decode-sized steps):
         the launch before this mixer clears it in passing."""
@@ -88,26 +90,37 @@ class GatedDeltaRule(Mixer):
         return buf if buf.numel() % 4 == 0 else None
 
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx, cache_view, writes_cache: bool = True,
-                scratch_cleared: bool = False) -> None:
+                scratch_cleared: bool = False, projected: Optional[tuple] = None) -> None:
+        """`projected` (matrix, column): a float32 matrix with this part's projections of x from that column on."""
         if not writes_cache:
             raise ValueError("a delta-rule mixer cannot read another place's state: its state is its own")
         T = x.shape[0]
         ws = ctx.workspace
         state = cache_view.state                                      # float32 [slots, state_floats]
-        proj = ws.get("delta_proj", (T, self.width), torch.float32)
-        self.proj.forward(x, proj, y_is_zero=scratch_cleared)
+        if projected is None:
+            proj, col = ws.get("delta_proj", (T, self.width), torch.float32), 0
+            self.proj.forward(x, proj, y_is_zero=scratch_cleared)
+        else:
+            proj, col = projected
         conv = ws.get("delta_conv", (T, self.channels), torch.float32)
-        ops.causal_conv_silu(proj, 0, self.channels, self.conv_w, None, self.taps, state, self.scan_floats,
+        ops.causal_conv_silu(proj, col, self.channels, self.conv_w, None, self.taps, state, self.scan_floats,
                              ctx.token_seq, ctx.q_start, ctx.seq_slot, conv, ctx.n_seqs, single_tokens=ctx.is_decode)
+        gate = proj[:, col + self.gate_col: col + self.gate_col + self.v_width]
+        gated = ws.get("delta_gated", (T, self.v_width), self.dtype)
+        if ctx.is_decode and ops.head_step_supported(self.dim, self.vdim, state):
+            ops.head_step("delta", conv, 0, self.qk_width, 2 * self.qk_width, float(self.dim) ** -0.5, proj, col + self.b_col,
+                          col + self.a_col, self.a_log, self.dt_bias, UNIT_EPS, state, gate, self.norm_weight, self.eps, gated,
+                          ctx.q_start, ctx.seq_slot, self.nh, self.nkv, self.dim, self.vdim)
+            self.o.forward_add(gated, residual)
+            return
         o = ws.get("delta_o", (T, self.v_width), torch.float32)
         floats = 0 if ctx.is_decode else ops.delta_rule_scratch(ctx.n_seqs, self.nh, ctx.max_q_len, self.channels, 0,
                                                                 self.qk_width, self.dim, ctx.n_tokens, self.vdim)
         scratch = ws.get("delta_scratch", (floats,), torch.float32) if floats else None
-        ops.delta_rule(conv, 0, self.qk_width, 2 * self.qk_width, proj, self.b_col, self.a_col, self.a_log,
+        ops.delta_rule(conv, 0, self.qk_width, 2 * self.qk_width, proj, col + self.b_col, col + self.a_col, self.a_log,
                        self.dt_bias, UNIT_EPS, o, state, 0, ctx.q_start, ctx.seq_slot, ctx.n_seqs, self.nh, self.nkv,
                        self.dim, self.vdim, scratch, ctx.max_q_len)
-        gated = ws.get("delta_gated", (T, self.v_width), self.dtype)
-        ops.head_norm_gate(o, proj[:, self.gate_col: self.gate_col + self.v_width], self.norm_weight, self.eps, gated,
+        ops.head_norm_gate(o, gate, self.norm_weight, self.eps, gated,
                            self.nh, self.vdim)
         self.o.forward_add(gated, residual)
 

@@ -40,6 +40,7 @@ class _GatedLinearBase(Mixer):
     """What the two mixers share: sizes, the stacked projection, the output product and the scratch to clear."""
 
     PROJ = "gated_linear_proj"
+    shares_projection = True      # `forward` takes the projections as columns of a wider matrix
 
     def __init__(self, hidden_size: int, num_heads: int, dim: int, vdim: int, eps: float, extra_rows: int,
                  dtype: torch.dtype, device: torch.device, name: str):
@@ -64,6 +65,15 @@ class _GatedLinearBase(Mixer):
             return None
         buf = ctx.workspace.get(self.PROJ, (tokens, self.width), torch.float32)
         return buf if buf.numel() % 4 == 0 else None
+
+
+    def _projections(self, x: torch.Tensor, ctx, scratch_cleared: bool, projected: Optional[tuple]):
+        """The matrix that holds this part's projections of x, and the column where they begin."""
+        if projected is not None:
+            return projected
+        proj = ctx.workspace.get(self.PROJ, (x.shape[0], self.width), torch.float32)
+        self.proj.forward(x, proj, y_is_zero=scratch_cleared)
+        return proj, 0
 
 
 class GatedLinearAttention(_GatedLinearBase):
@@ -96,21 +106,27 @@ class GatedLinearAttention(_GatedLinearBase):
         self.norm_weight = _f32("norm", norm, (self.vdim,), self.device)
 
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx, cache_view, writes_cache: bool = True,
-                scratch_cleared: bool = False) -> None:
+                scratch_cleared: bool = False, projected: Optional[tuple] = None) -> None:
         if not writes_cache:
             raise ValueError("a gated linear attention mixer cannot read another place's state: its state is its own")
         T = x.shape[0]
         ws = ctx.workspace
-        proj = ws.get(self.PROJ, (T, self.width), torch.float32)
-        self.proj.forward(x, proj, y_is_zero=scratch_cleared)
-        decays = ws.get("gla_decays", (T, self.qk_width), torch.float32)
-        ops.gla_decay(proj, self.extra_col, self.rank, self.a2t, self.a2_bias, self.tau, decays)
-        o = ws.get("gla_o", (T, self.v_width), torch.float32)
-        ops.gated_linear_scan(proj, 0, self.k_col, self.v_col, self.q_scale, decays, o, cache_view.state, ctx.q_start,
-                              ctx.seq_slot, ctx.n_seqs, self.nh, self.dim, self.vdim, ctx.max_q_len, ws,
-                              single_tokens=ctx.is_decode)
+        proj, col = self._projections(x, ctx, scratch_cleared, projected)
+        gate = proj[:, col + self.gate_col: col + self.gate_col + self.v_width]
         gated = ws.get("gla_gated", (T, self.v_width), self.dtype)
-        ops.head_norm_gate(o, proj[:, self.gate_col: self.gate_col + self.v_width], self.norm_weight, self.eps, gated,
+        if ctx.is_decode and ops.head_step_supported(self.dim, self.vdim, cache_view.state):
+            ops.head_step("channel", proj, col, col + self.k_col, col + self.v_col, self.q_scale, proj, col + self.extra_col, 0,
+                          self.a2t, self.a2_bias, 1.0 / self.tau, cache_view.state, gate, self.norm_weight, self.eps, gated,
+                          ctx.q_start, ctx.seq_slot, self.nh, self.nh, self.dim, self.vdim)
+            self.o.forward_add(gated, residual)
+            return
+        decays = ws.get("gla_decays", (T, self.qk_width), torch.float32)
+        ops.gla_decay(proj, col + self.extra_col, self.rank, self.a2t, self.a2_bias, self.tau, decays)
+        o = ws.get("gla_o", (T, self.v_width), torch.float32)
+        ops.gated_linear_scan(proj, col, col + self.k_col, col + self.v_col, self.q_scale, decays, o, cache_view.state,
+                              ctx.q_start, ctx.seq_slot, ctx.n_seqs, self.nh, self.dim, self.vdim, ctx.max_q_len, ws,
+                              single_tokens=ctx.is_decode)
+        ops.head_norm_gate(o, gate, self.norm_weight, self.eps, gated,
                            self.nh, self.vdim)
         self.o.forward_add(gated, residual)
 
@@ -147,24 +163,31 @@ class MatrixMemory(_GatedLinearBase):
         self.norm_weight = _f32("norm", norm, (self.v_width,), self.device)
 
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx, cache_view, writes_cache: bool = True,
-                scratch_cleared: bool = False) -> None:
+                scratch_cleared: bool = False, projected: Optional[tuple] = None) -> None:
         if not writes_cache:
             raise ValueError("a matrix memory mixer cannot read another place's state: its state is its own")
         T = x.shape[0]
         ws = ctx.workspace
         state = cache_view.state
-        proj = ws.get(self.PROJ, (T, self.width), torch.float32)
-        self.proj.forward(x, proj, y_is_zero=scratch_cleared)
+        proj, col = self._projections(x, ctx, scratch_cleared, projected)
+        gate = proj[:, col + self.gate_col: col + self.gate_col + self.v_width]
+        gated = ws.get("matrix_memory_gated", (T, self.v_width), self.dtype)
+        if ctx.is_decode and ops.head_step_supported(self.dim, self.vdim, state, normalizer=True):
+            ops.head_step("memory", proj, col, col + self.k_col, col + self.v_col, self.q_scale, proj, col + self.extra_col,
+                          col + self.extra_col + self.nh, self.bias_i, self.bias_f, self.cap, state, gate, self.norm_weight,
+                          self.eps, gated, ctx.q_start, ctx.seq_slot, self.nh, self.nh, self.dim, self.vdim, m_off=self.m_off,
+                          sigmoid=True)
+            self.o.forward_add(gated, residual)
+            return
         gates = ws.get("matrix_memory_gates", (T, self.nh, 4), torch.float32)
-        ops.exp_gates(proj, self.extra_col, self.extra_col + self.nh, self.bias_i, self.bias_f, self.cap, gates, state,
-                      self.m_off, ctx.q_start, ctx.seq_slot, ctx.n_seqs, self.nh)
+        ops.exp_gates(proj, col + self.extra_col, col + self.extra_col + self.nh, self.bias_i, self.bias_f, self.cap, gates,
+                      state, self.m_off, ctx.q_start, ctx.seq_slot, ctx.n_seqs, self.nh)
         o = ws.get("matrix_memory_o", (T, self.v_width), torch.float32)
         divisors = ws.get("matrix_memory_divisors", (T, self.nh), torch.float32)
-        ops.gated_linear_scan(proj, 0, self.k_col, self.v_col, self.q_scale, gates, o, state, ctx.q_start, ctx.seq_slot,
-                              ctx.n_seqs, self.nh, self.dim, self.vdim, ctx.max_q_len, ws, divisors=divisors,
+        ops.gated_linear_scan(proj, col, col + self.k_col, col + self.v_col, self.q_scale, gates, o, state, ctx.q_start,
+                              ctx.seq_slot, ctx.n_seqs, self.nh, self.dim, self.vdim, ctx.max_q_len, ws, divisors=divisors,
                               single_tokens=ctx.is_decode)
-        gated = ws.get("matrix_memory_gated", (T, self.v_width), self.dtype)
-        ops.head_norm_gate(o, proj[:, self.gate_col: self.gate_col + self.v_width], self.norm_weight, self.eps, gated,
+        ops.head_norm_gate(o, gate, self.norm_weight, self.eps, gated,
                            self.nh, self.vdim, sigmoid=True, denom=divisors)
         self.o.forward_add(gated, residual)
 
