@@ -68,8 +68,8 @@ _SIGNATURES = {
     "jb_join_norm": "pppppffpppfipipiiplplp", "jb_head_norm_gate": "ppipipfipiiiip", "jb_sigmoid_gate": "pipiiiiip",
     "jb_head_norm_rope_cache": "pippfpippipppiiiiiiiiiifipifp",
     "jb_delta_rule": "piiiipiiippfppllppiiiiip", "jb_delta_rule_chunks": "piiiipiiippfppllppiiiiiipiip",
-    "jb_route_topk": "piiippiiiipfip", "jb_experts_few_tokens": "pippipppippiiiiffip", "jb_expert_gather": "pippipiip", "jb_experts_few_tokens_tc": "pppipppppiiiiffip",
-    "jb_expert_scatter": "pppipiip",
+    "jb_route_topk": "piiippiiiipfip", "jb_route_tokens": "ppiipiippiiiipfip", "jb_experts_few_tokens": "pippipppippiiiiffip", "jb_expert_gather": "pippipiip", "jb_experts_few_tokens_tc": "pppipppppiiiiffip",
+    "jb_expert_scatter": "pppipiip", "jb_experts_stream": "pppipliplppppiiiiffipp",
     "jb_state_chunks": "ipiiiipipppfpppllppiiiiiipiip",
     "jb_head_step": "ipiiiifpiiippfiplllpipiifpippiiiiip",
     "jb_gla_decay": "piiippfpiip", "jb_exp_gates": "piiippfppllppiip",
@@ -1847,6 +1847,29 @@ def route_topk(logits: torch.Tensor, top: int, sel_e: torch.Tensor, sel_w: torch
                                         _stream()), "route_topk")
 
 
+ROUTE_MAX_NUMBERS = 1 << 16      # numbers of a router's matrix, and tokens, up to which product and choice are one launch
+ROUTE_MAX_TOKENS = 128
+
+
+def route_tokens(x: torch.Tensor, w: torch.Tensor, logits: torch.Tensor, top: int, sel_e: torch.Tensor, sel_w: torch.Tensor,
+                 softmax: bool = False, groups: int = 0, keep: int = 0, experts: Optional[int] = None,
+                 correction: Optional[torch.Tensor] = None, scale: float = 1.0, shares: bool = False) -> None:
+    """logits[t, r] = w[r] . x[t] (bfloat16 x [T, W] and w [R, W], W a multiple of 8; float32 [T, R]) and `route_topk` of
+    them, in one launch; for at most ROUTE_MAX_NUMBERS numbers in w, since every block reads all of it."""
+    (T, W), R = x.shape, w.shape[0]
+    E = R if experts is None else int(experts)
+    _need(x, "router in", torch.bfloat16)
+    _need(w, "router weight", torch.bfloat16, (R, W))
+    _need(logits, "router logits", torch.float32, (T, R))
+    _need(sel_e, "chosen experts", torch.int32, (T, top))
+    _need(sel_w, "experts' weights", torch.float32, (T, top))
+    if correction is not None:
+        _need(correction, "router's correction", torch.float32, (E,))
+    _check(_lib("routed").jb_route_tokens(_ptr(x), _ptr(w), W, R, _ptr(logits), E, int(top), _ptr(sel_e), _ptr(sel_w), T,
+                                          int(bool(softmax)), int(groups), int(keep), _ptr(correction), float(scale),
+                                          int(bool(shares)), _stream()), "route_tokens")
+
+
 def experts_few_tokens(h: torch.Tensor, sel_e: torch.Tensor, sel_w: torch.Tensor, w_gate: torch.Tensor,
                        w_up: torch.Tensor, w_down: torch.Tensor, act: torch.Tensor, out: torch.Tensor,
                        gate_limit: float = 0.0, gate_alpha: float = 1.0, weight_on_output: bool = False) -> None:
@@ -1889,6 +1912,40 @@ def experts_few_tokens_tc(h: torch.Tensor, sel_e: torch.Tensor, sel_w: torch.Ten
     _check(_lib("routed").jb_experts_few_tokens_tc(
         _ptr(h), _ptr(sel_e), _ptr(sel_w), top, _ptr(w_gate), _ptr(w_up), _ptr(w_down), _ptr(act), _ptr(out), T, W, F, E,
         float(gate_limit), float(gate_alpha), int(bool(weight_on_output)), _stream()), "experts_few_tokens_tc", kernels=2)
+
+
+EXPERTS_STREAM_TOKENS, EXPERTS_STREAM_EXPERTS, EXPERTS_STREAM_PLACES = 64, 512, 8192     # what `experts_stream` takes
+
+
+def experts_stream_supported(T: int, top: int, experts: int) -> bool:
+    """Whether `experts_stream` takes a step of T tokens.  Its slices of k meet by adds in the order in which they finish, so
+    deterministic runs stay with `experts_few_tokens_tc`."""
+    return (T <= EXPERTS_STREAM_TOKENS and experts <= EXPERTS_STREAM_EXPERTS
+            and min(T * top, experts) * T <= EXPERTS_STREAM_PLACES and not _deterministic[0])
+
+
+def experts_stream(x: torch.Tensor, sel_e: torch.Tensor, sel_w: torch.Tensor, gate_up: PackedWeight, down: PackedWeight,
+                   experts: int, z: torch.Tensor, act: torch.Tensor, pair_slot: torch.Tensor, out: torch.Tensor,
+                   gate_limit: float = 0.0, gate_alpha: float = 1.0, weight_on_output: bool = False) -> None:
+    """`experts_few_tokens` of up to 64 bfloat16 tokens, from the packed stacks of all experts' matrices (width and inner
+    width multiples of 128): z float32 scratch [T top, 2 F], zero; act bfloat16 scratch [min(experts, T top) T, F];
+    pair_slot int32 scratch [T top]."""
+    (T, W), top = x.shape, sel_e.shape[1]
+    E, F = int(experts), gate_up.rows // int(experts)
+    _need(x, "expert input", torch.bfloat16)
+    _need(sel_e, "chosen experts", torch.int32, (T, top))
+    _need(sel_w, "experts' weights", torch.float32, (T, top))
+    _need(z, "experts' sums", torch.float32, (T * top, 2 * F))
+    _need(act, "experts' scratch", torch.bfloat16, (min(E, T * top) * T, F))
+    _need(pair_slot, "experts' places", torch.int32, (T * top,))
+    _need(out, "experts' out", torch.float32, (T, W))
+    if gate_up.cols != W or down.cols != F or down.rows != E * W or gate_up.rows != E * F or not gate_up.up_tile_offset:
+        raise KernelError(f"experts_stream: stacks of {gate_up.rows} x {gate_up.cols} and {down.rows} x {down.cols} do not fit "
+                          f"{E} experts of {F} x {W}")
+    _check(_lib("experts_stream").jb_experts_stream(
+        _ptr(x), _ptr(sel_e), _ptr(sel_w), top, _ptr(gate_up.tiles), gate_up.n_tiles, gate_up.up_tile_offset, _ptr(down.tiles),
+        down.n_tiles, _ptr(z), _ptr(act), _ptr(pair_slot), _ptr(out), T, W, F, E, float(gate_limit), float(gate_alpha),
+        int(bool(weight_on_output)), _ptr(kernel_status(x.device)), _stream()), "experts_stream", kernels=3)
 
 
 EXPERT_PLAN_MAX_EXPERTS = 1024

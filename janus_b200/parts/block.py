@@ -99,12 +99,18 @@ class HyperConnectedBlock:
             self.mixer.forward(x, y, ctx, cache_view, writes_cache)
         last = self.mixer_connection
         if self.feed_forward is not None:
+            # so may a feed-forward
+            wants = getattr(self.feed_forward, "scratch_to_clear", None)
+            scratch = wants(ctx, T) if wants is not None else None
             if hasattr(last, "write_then_read"):
-                last.write_then_read(residual, y, self.feed_forward_connection, self.feed_forward_norm, x)
+                last.write_then_read(residual, y, self.feed_forward_connection, self.feed_forward_norm, x, clear2=scratch)
             else:
                 last.write(residual, y)
-                self.feed_forward_connection.read(residual, self.feed_forward_norm, x, clear=y)
-            self.feed_forward.forward(x, y, ctx)
+                self.feed_forward_connection.read(residual, self.feed_forward_norm, x, clear=y, clear2=scratch)
+            if scratch is not None:
+                self.feed_forward.forward(x, y, ctx, scratch_cleared=True)
+            else:
+                self.feed_forward.forward(x, y, ctx)
             last = self.feed_forward_connection
         ctx.pending_write = (last, y)
 

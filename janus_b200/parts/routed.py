@@ -5,10 +5,12 @@ float32 (the product's own accumulators), the scores s = sigmoid(z); a token's `
 largest scores (the lower index wins a tie) and their weights are those scores as they are, not renormalized.  The
 weight multiplies the expert's INPUT: out = sum over the chosen e of expert_e(s_e h).
 
-Steps of few (token, expert) pairs, every single-token step among them, stream each chosen expert's rows once for
-up to 16 of the tokens that chose it (`ops.experts_few_tokens_tc`: two launches with a block per (rows, expert),
-float32 sums, nothing read back by the host, so the step can be recorded into a CUDA graph; widths that are no multiples
-of 32, and the float32 engine, take up to four tokens at a time on the CUDA cores, `ops.experts_few_tokens`).  Prompt steps of the
+Steps of few (token, expert) pairs, every single-token step among them, stream the chosen experts' packed tiles once for
+up to 64 tokens (`ops.experts_stream`: width and inner width multiples of 128).  Other widths, more tokens and
+deterministic runs stream each chosen expert's rows once for up to 16 of the tokens that chose it
+(`ops.experts_few_tokens_tc`: two launches with a block per (rows, expert); widths that are no multiples
+of 32, and the float32 engine, take up to four tokens at a time on the CUDA cores, `ops.experts_few_tokens`).  Sums are
+float32 and nothing is read back by the host, so the step can be recorded into a CUDA graph.  Prompt steps of the
 bfloat16 engine with more pairs sort the (token, choice) pairs by expert, gather the weighted rows in that order and
 run the experts' two products on the tensor cores over their rows; the results are added back token by token in the
 order of the token's choices.  Where the sizes allow it (width and inner width multiples of 128) the sort is a kernel
@@ -68,8 +70,11 @@ class RoutedExperts(FeedForward):
         self.experts, self.top = int(experts), int(top)
         self.dtype, self.device = dtype, device
         # the router's product also makes the shared expert's gate: one more row
-        self.router = Linear(hidden_size, experts + (1 if self.shared_gate else 0), dtype, device, name="router",
-                             pad_width=True)
+        rows = experts + (1 if self.shared_gate else 0)
+        # few tokens of a small router: product and choice are one launch, which reads the matrix as it is
+        self.route_in_one = dtype == torch.bfloat16 and hidden_size % 8 == 0 and rows * hidden_size <= ops.ROUTE_MAX_NUMBERS
+        self.router_rows: Optional[torch.Tensor] = None
+        self.router = Linear(hidden_size, rows, dtype, device, name="router", pad_width=True)
         self.shared_gate_up = self.shared_down = None
         if self.shared_size is not None:
             self.shared_gate_up = GatedLinear(hidden_size, self.shared_size, dtype, device, name="shared_gate_up",
@@ -108,7 +113,10 @@ class RoutedExperts(FeedForward):
             if correction is None or tuple(correction.shape) != (self.experts,):
                 raise ValueError(f"the router needs a correction for each of its {self.experts} experts")
             self.correction = correction.to(device=self.device, dtype=torch.float32).contiguous()
-        self.router.load([router] + ([shared_sg] if self.shared_gate else []))
+        rows = [router] + ([shared_sg] if self.shared_gate else [])
+        self.router.load(rows)
+        if self.route_in_one:
+            self.router_rows = torch.cat([t.to(device=self.device, dtype=self.dtype) for t in rows]).contiguous()
         if self.shared_size is not None:
             self.shared_gate_up.load(shared_gate, shared_up)
             self.shared_down.load([shared_down])
@@ -135,31 +143,54 @@ class RoutedExperts(FeedForward):
                 self.gate_up.append(gu)
                 self.down.append(dn)
 
+    def _streams(self, ctx, tokens: int) -> bool:
+        """Whether the step streams the packed stacks of the experts' matrices."""
+        return (self.grouped and (ctx.is_decode or tokens * self.top <= FEW_PAIRS)
+                and ops.experts_stream_supported(tokens, self.top, self.experts))
+
     def scratch_to_clear(self, ctx, tokens: int) -> Optional[torch.Tensor]:
-        """The router's float32 logits, if this step's product adds slices of K into them: the launch before this part
-        may clear them in passing."""
-        if not self.router.meets_by_adds(tokens, torch.float32):
+        """The float32 sums of the streamed experts; else the router's logits, if this step's product adds slices of K into
+        them: the launch before this part may clear them in passing."""
+        if self._streams(ctx, tokens):
+            return ctx.workspace.get("experts_sums", (tokens * self.top, 2 * self.intermediate_size), torch.float32)
+        if self._routes_in_one(tokens) or not self.router.meets_by_adds(tokens, torch.float32):
             return None
         buf = ctx.workspace.get("router_logits", (tokens, self.router.out_features), torch.float32)
         return buf if buf.numel() % 4 == 0 else None
+
+    def _routes_in_one(self, tokens: int) -> bool:
+        return self.route_in_one and tokens <= ops.ROUTE_MAX_TOKENS
 
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx, scratch_cleared: bool = False) -> None:
         T = x.shape[0]
         ws = ctx.workspace
         logits = ws.get("router_logits", (T, self.router.out_features), torch.float32)
-        self.router.forward(x, logits, y_is_zero=scratch_cleared)
+        sel_e = ws.get("router_experts", (T, self.top), torch.int32)
+        sel_w = ws.get("router_weights", (T, self.top), torch.float32)
+        choice = dict(softmax=self.softmax, groups=self.groups, keep=self.keep, experts=self.experts,
+                      correction=self.correction, scale=self.weight_scale, shares=self.shares)
+        streams = self._streams(ctx, T)
+        if self._routes_in_one(T):
+            ops.route_tokens(x, self.router_rows, logits, self.top, sel_e, sel_w, **choice)
+        else:
+            self.router.forward(x, logits, y_is_zero=scratch_cleared and not streams)
+            ops.route_topk(logits, self.top, sel_e, sel_w, **choice)
         if self.shared_size is not None:
             shared = ws.get("shared_act", (T, self.shared_size), self.dtype)
             self.shared_gate_up.forward(x, shared, ctx)
             if self.shared_gate:
                 ops.scale_rows_sigmoid(shared, logits[:, self.experts])
             self.shared_down.forward_add(shared, residual)
-        sel_e = ws.get("router_experts", (T, self.top), torch.int32)
-        sel_w = ws.get("router_weights", (T, self.top), torch.float32)
-        ops.route_topk(logits, self.top, sel_e, sel_w, softmax=self.softmax, groups=self.groups, keep=self.keep,
-                       experts=self.experts, correction=self.correction, scale=self.weight_scale,
-                       shares=self.shares)
         pairs = T * self.top
+        if streams:
+            sums = ws.get("experts_sums", (pairs, 2 * self.intermediate_size), torch.float32)
+            if not scratch_cleared:
+                ops.zero_f32(sums)
+            act = ws.get("experts_act_rows", (min(self.experts, pairs) * T, self.intermediate_size), self.dtype)
+            ops.experts_stream(x, sel_e, sel_w, self.gate_up_stack, self.down_stack, self.experts, sums, act,
+                               ws.get("experts_places", (pairs,), torch.int32), residual,
+                               weight_on_output=self.weight_on_output)
+            return
         if self.dtype == torch.bfloat16 and not ctx.is_decode and pairs > FEW_PAIRS:
             if self.grouped:
                 self._grouped(x, sel_e, sel_w, residual, ctx)

@@ -100,3 +100,84 @@ def test_head_step(ops, kind, T, H, G, d, e):
         assert float(err) < 1e-6, float(err)
         untouched = [s for s in range(T + 2) if s not in slots.tolist()]
         assert torch.equal(got_state[untouched].cpu(), state[untouched])
+
+
+@pytest.mark.parametrize("T", [1, 5, 130])
+@pytest.mark.parametrize("W, E, extra, top, softmax, groups, keep", [(2048, 8, 0, 2, False, 0, 0), (264, 8, 1, 2, True, 4, 2), (8, 3, 1, 3, False, 0, 0),
+                                                                     (4096, 16, 0, 4, True, 0, 0), (1024, 40, 1, 6, False, 8, 3)])
+def test_route_tokens(ops, T, W, E, extra, top, softmax, groups, keep):
+    """The router's product and choice in one launch: logits against float64 (each half of a row is lanes' chains of at most
+    64 products and eight more sums: 72 roundings of 2^-24 of the sum of the products' sizes), the choice as `route_topk`
+    makes it from the same logits, and a token's row whatever the number of tokens."""
+    g = torch.Generator().manual_seed(W + E)
+    x, w = rnd(g, T, W).bfloat16().to(DEV), rnd(g, E + extra, W).bfloat16().to(DEV)
+    corr = rnd(g, E).to(DEV) if groups == 0 else None
+    logits = torch.full((T, E + extra), float("nan"), device=DEV)
+    sel_e, sel_w = torch.full((T, top), -1, dtype=torch.int32, device=DEV), torch.full((T, top), float("nan"), device=DEV)
+    how = dict(softmax=softmax, groups=groups, keep=keep, experts=E, correction=corr, scale=1.5, shares=True)
+    ops.route_tokens(x, w, logits, top, sel_e, sel_w, **how)
+    ref, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert bool(((logits.double() - ref).abs() <= 72 * 2.0 ** -24 * size).all())
+    e2, w2 = torch.empty_like(sel_e), torch.empty_like(sel_w)
+    ops.route_topk(logits, top, e2, w2, **how)
+    assert torch.equal(sel_e, e2) and torch.equal(sel_w, w2)
+    one = torch.empty(1, E + extra, device=DEV)
+    ops.route_tokens(x[T // 2: T // 2 + 1].contiguous(), w, one, top, e2[:1], w2[:1], **how)
+    assert torch.equal(one[0], logits[T // 2]) and torch.equal(e2[0], sel_e[T // 2])
+
+
+def plain_experts(x, sel_e, sel_w, wg, wu, wd, base, on_output):
+    out = base.double().clone()
+    x, wg, wu, wd = x.double(), wg.double(), wu.double(), wd.double()
+    for t in range(x.shape[0]):
+        for k in range(sel_e.shape[1]):
+            e, s = int(sel_e[t, k]), float(sel_w[t, k])
+            h = x[t] if on_output else x[t] * s
+            a = (F.silu(wg[e] @ h) * (wu[e] @ h)).bfloat16().double()
+            out[t] += (wd[e] @ a) * (s if on_output else 1.0)
+    return out
+
+
+@pytest.mark.parametrize("T, top, E, W, Fi, on_output", [(1, 2, 8, 256, 384, False), (1, 1, 1, 128, 128, True), (5, 3, 4, 384, 256, True),
+                                                         (16, 2, 5, 128, 640, False), (17, 2, 40, 256, 128, True),
+                                                         (33, 4, 3 + 4, 128, 256, False), (64, 2, 64, 128, 128, True),
+                                                         (64, 8, 120, 128, 128, False), (2, 2, 8, 2048, 1024, True)])
+def test_experts_stream(ops, T, top, E, W, Fi, on_output):
+    """The streamed experts against float64 (their activations rounded to bfloat16, as the kernel's are), with slices of k
+    that begin and end anywhere, experts nobody chose, one that all chose, and tokens on both sides of a tile.  An activation
+    may round the other way (2^-8 of itself, in few of them): 2^-8 of the largest result bounds what that does to a sum."""
+    g = torch.Generator().manual_seed(T * 100 + E)
+    x = rnd(g, T, W).bfloat16()
+    wg, wu, wd = (rnd(g, E, *s, s=W ** -0.5).bfloat16() for s in ((Fi, W), (Fi, W), (W, Fi)))
+    sel_e = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(T)]).int()
+    sel_e[:, 0] = torch.where((sel_e == 0).any(1), sel_e[:, 0], torch.zeros(T, dtype=torch.int32))     # all choose expert 0
+    sel_w = torch.rand(T, top, generator=g) + 0.1
+    base = rnd(g, T, W)
+    assert ops.experts_stream_supported(T, top, E)
+    gu = ops.pack_gated(wg.reshape(E * Fi, W).to(DEV), wu.reshape(E * Fi, W).to(DEV))
+    dn = ops.pack_weight(wd.reshape(E * W, Fi).to(DEV))
+    z = torch.zeros(T * top, 2 * Fi, device=DEV)
+    act = torch.full((min(E, T * top) * T, Fi), float("nan"), dtype=torch.bfloat16, device=DEV)
+    out, places = base.to(DEV), torch.empty(T * top, dtype=torch.int32, device=DEV)
+    ops.experts_stream(x.to(DEV), sel_e.to(DEV), sel_w.to(DEV), gu, dn, E, z, act, places, out, weight_on_output=on_output)
+    ops.check_kernel_status(torch.device(DEV))
+    used = torch.unique(sel_e).tolist()
+    assert places.tolist() == [used.index(e) for e in sel_e.reshape(-1).tolist()]
+    want = plain_experts(x, sel_e, sel_w, wg, wu, wd, base, on_output)
+    err = float((out.double().cpu() - want).abs().max() / (want - base.double()).abs().max())
+    assert err < 2.0 ** -8, err
+    for t in range(T):                     # the sums themselves, in float32
+        for k in range(top):
+            e = int(sel_e[t, k])
+            ref = torch.cat([wg[e].double() @ x[t].double(), wu[e].double() @ x[t].double()])
+            assert float((z[t * top + k].double().cpu() - ref).abs().max()) < 1e-5 * float(ref.abs().max()) + 1e-6
+
+
+def test_experts_stream_refuses(ops):
+    assert not ops.experts_stream_supported(65, 2, 8) and not ops.experts_stream_supported(1, 2, 513)
+    assert not ops.experts_stream_supported(64, 8, 200)             # 200 experts x 64 tokens
+    ops.set_deterministic(True)
+    try:
+        assert not ops.experts_stream_supported(1, 2, 8)
+    finally:
+        ops.set_deterministic(False)
