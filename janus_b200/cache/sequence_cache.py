@@ -22,6 +22,7 @@ from typing import Dict, List, Optional, Sequence
 import numpy as np
 import torch
 
+from ..kernels import ops
 from ..parts.base import CacheSpec, KVSpec, StateSpec, split_cache_spec
 from .pages import PAGE_SIZE, CacheFull, PagePool
 
@@ -143,8 +144,12 @@ class SequenceCache:
         self._live[slot] = True
         self.lengths[slot] = 0
         self.epochs[slot] += 1
-        for st in self.states.values():
-            st[slot].zero_()
+        if self.states:
+            if self.device.type == "cuda":
+                ops.clear_rows(list(self.states.values()), slot)
+            else:
+                for st in self.states.values():
+                    st[slot].zero_()
         return slot
 
     def free_slot(self, slot: int) -> None:

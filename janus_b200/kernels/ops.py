@@ -8,7 +8,7 @@ import contextlib
 import ctypes
 import functools
 import os
-from typing import Optional, Tuple
+from typing import Optional, Sequence, Tuple
 
 import torch
 
@@ -54,7 +54,7 @@ def stream_scope():
 # plain Python integers and floats (a pointer is `tensor.data_ptr()`, None is a null pointer).
 _SIGNATURES = {
     "jb_embed_gather": "pippiippfp", "jb_rmsnorm": "pppifpiiiplp", "jb_residual_add": "ppilp",
-    "jb_swiglu": "ppiiip", "jb_swiglu_f32_to_bf16": "piipiip", "jb_zero_f32": "plp",
+    "jb_swiglu": "ppiiip", "jb_swiglu_f32_to_bf16": "piipiip", "jb_zero_f32": "plp", "jb_clear_rows": "ppip",
     "jb_pack_weight_bf16": "piipp", "jb_rope_cache_write": "piipipppppiiiiiiip",
     "jb_gemm_f32": "pppiiiiiip", "jb_attention_f32": "pppppppiiiiiiiififfipppip",
     "jb_gemm_bf16": "pplipiiiiiiplpiffpp", "jb_gemm_bf16_pair": "pplipiiiiiiiffpp",
@@ -260,6 +260,24 @@ def zero_f32(t: torch.Tensor) -> None:
 
 
 # -- rotary positions + cache append --------------------------------------------
+CLEAR_ROWS = 16      # rows that one launch of `clear_rows` takes
+
+
+def clear_rows(matrices: Sequence[torch.Tensor], row: int) -> None:
+    """Set row `row` of every float32 tensor (its first axis) to zero, up to CLEAR_ROWS of them in one launch."""
+    for first in range(0, len(matrices), CLEAR_ROWS):
+        some = matrices[first: first + CLEAR_ROWS]
+        for m in some:
+            _need(m, "rows to clear", torch.float32)
+            if not 0 <= row < m.shape[0]:
+                raise KernelError(f"clear_rows: row {row} of {m.shape[0]}")
+        n = [m.numel() // m.shape[0] for m in some]
+        at = (ctypes.c_void_p * len(some))(*(m.data_ptr() + 4 * row * k for m, k in zip(some, n)))
+        _check(_lib("elementwise").jb_clear_rows(ctypes.cast(at, ctypes.c_void_p),
+                                                 ctypes.cast((ctypes.c_longlong * len(some))(*n), ctypes.c_void_p), len(some),
+                                                 _stream()), "clear_rows")
+
+
 def rope_cache_write(qkv: torch.Tensor, q_out: torch.Tensor, cos_sin: Optional[torch.Tensor],
                      positions: torch.Tensor, dest: Optional[torch.Tensor], k_cache: Optional[torch.Tensor],
                      v_cache: Optional[torch.Tensor], nh: int, nkv: int, hd: int, page_size: int,

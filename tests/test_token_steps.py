@@ -181,3 +181,12 @@ def test_experts_stream_refuses(ops):
         assert not ops.experts_stream_supported(1, 2, 8)
     finally:
         ops.set_deterministic(False)
+
+
+def test_clear_rows(ops):
+    """A row of many matrices at once: sizes that are whole vectors and sizes that are not, more matrices than a launch takes."""
+    sizes = [4, 1, 7, 4096, 5000, 2 ** 20] + [8 + i for i in range(14)]
+    m = [torch.ones(3, n, device=DEV) for n in sizes] + [torch.ones(3, 2, 5, device=DEV)]
+    ops.clear_rows(m, 1)
+    for t in m:
+        assert float(t[1].abs().sum()) == 0.0 and bool((t[0] == 1).all()) and bool((t[2] == 1).all())
