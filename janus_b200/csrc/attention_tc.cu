@@ -907,12 +907,15 @@ int tc_prefill_launch(const void* q, const void* k_cache, const void* v_cache, v
       return JB_ERR_TENSORMAP;
   }
   // Two row tiles per CTA over blocks of 128 keys are the faster kernel once there are CTAs enough for every
-  // SM; below that the finer one-tile CTAs spread better.
+  // SM (of those that have tokens: about half a pair a sequence is empty); below that the finer one-tile CTAs spread better.
+  // So they do for sequences of less than two pairs of tiles, of which a CTA's start and end are the most: two one-tile CTAs
+  // share an SM (64 sequences of 5 to 130 tokens, 32 + 8 heads of 64: 53 us in pairs, 37 not; six of 65 to 400, 16 + 4 heads of
+  // 128, 99 CTAs: 16.8 and 14.9; eight of 150 to 701, 32 + 8 heads of 128, 458 CTAs: 52 and 65).
   const int n_tiles = (max_q_len + tpt - 1) / tpt;
-  const long long ctas_of_pairs = (long long)((n_tiles + 1) / 2) * nkv * n_seqs;
+  const long long ctas_of_pairs = (T / (2 * tpt) + (n_seqs + 1) / 2ll) * nkv;
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  [[maybe_unused]] bool pairs = ctas_of_pairs >= sms;
+  [[maybe_unused]] bool pairs = ctas_of_pairs >= sms && T > 4ll * tpt * n_seqs;
   if (const char* e = getenv("JANUS_ATTN_TC_TILES")) {   // 1 or 2: tiles per CTA whatever the size (for tests and measurements)
     if (e[0] == '1') pairs = false;
     if (e[0] == '2') pairs = true;
