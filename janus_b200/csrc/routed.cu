@@ -549,7 +549,7 @@ __global__ void __launch_bounds__(TC_WARPS * 32, DEEP ? 2 : 4) expert_tc_kernel(
   }
 }
 
-constexpr int PLAN_THREADS = 1024, PLAN_MAX_EXPERTS = 1024;
+constexpr int PLAN_THREADS = 1024, PLAN_MAX_EXPERTS = 1024, PLAN_AHEAD = 8;
 
 // Sorts the (token, choice) pairs by expert and lists the tiles of the two grouped products, in one block, so that
 // the host never learns the router's choice.  order[place] = pair and where[pair] = place, an expert's pairs next
@@ -557,7 +557,9 @@ constexpr int PLAN_THREADS = 1024, PLAN_MAX_EXPERTS = 1024;
 // its count of items in [0] and item i as (t0, t_end, wf0, f0) at [4 + 4 i]: rows [t0, t_end) of the sorted pairs,
 // weight rows from wf0 on in the stack of the experts' matrices, output columns from f0 on.  Tiles are 256 rows;
 // `gu` tiles are 128 features of F wide, `dn` tiles 256 features of W.  Inside an expert the row tiles run fastest,
-// so CTAs that run side by side share a weight tile.
+// so CTAs that run side by side share a weight tile.  What bounds it is that one block does it: a warp's pairs count with
+// one atomic an expert, a warp writes an expert's tiles (8 experts, two a token: 1,500 tokens of 4,096 x 2,048 13.1 us with an atomic
+// a pair and a thread an expert, 8.4 so; 3,072 tokens of 7,168 x 4,096 18.8 and 6.8).
 __global__ void __launch_bounds__(PLAN_THREADS) expert_plan_kernel(const int* __restrict__ sel_e, int n_pairs, int E,
                                                                    int F, int W, int* __restrict__ order,
                                                                    int* __restrict__ where, int* __restrict__ gu,
@@ -565,9 +567,30 @@ __global__ void __launch_bounds__(PLAN_THREADS) expert_plan_kernel(const int* __
   __shared__ int count[PLAN_MAX_EXPERTS], start[PLAN_MAX_EXPERTS], cursor[PLAN_MAX_EXPERTS], tiles_before[PLAN_MAX_EXPERTS];
   jb::pdl_launch_dependents();
   jb::pdl_wait();
-  for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // a warp's lanes that chose the same expert count together: its places are its first lane's and the lanes before
+  const auto add = [&](int* counter, int e, bool in) {
+    const unsigned same = __match_any_sync(0xffffffffu, in ? e : -1);
+    const int first = __ffs(same) - 1;
+    int at = 0;
+    if (in && lane == first) at = atomicAdd(&counter[e], __popc(same));
+    return __shfl_sync(0xffffffffu, at, first) + __popc(same & ((1u << lane) - 1u));
+  };
+  for (int e = threadIdx.x; e < E; e += PLAN_THREADS) count[e] = 0;
+  int mine[PLAN_AHEAD];                                      // the first pairs, kept for the second pass
+#pragma unroll
+  for (int k = 0; k < PLAN_AHEAD; ++k) {
+    const int i = k * PLAN_THREADS + threadIdx.x;
+    mine[k] = i < n_pairs ? sel_e[i] : -1;
+  }
   __syncthreads();
-  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) atomicAdd(&count[sel_e[i]], 1);
+#pragma unroll
+  for (int k = 0; k < PLAN_AHEAD; ++k)
+    if (k * PLAN_THREADS < n_pairs) add(count, mine[k], mine[k] >= 0);
+  for (int i0 = PLAN_AHEAD * PLAN_THREADS; i0 < n_pairs; i0 += PLAN_THREADS) {
+    const int i = i0 + threadIdx.x;
+    add(count, i < n_pairs ? sel_e[i] : 0, i < n_pairs);
+  }
   __syncthreads();
   const int gu_per = (F + 127) / 128, dn_per = (W + 255) / 256;
   if (threadIdx.x == 0) {
@@ -582,19 +605,29 @@ __global__ void __launch_bounds__(PLAN_THREADS) expert_plan_kernel(const int* __
     dn[0] = tiles * dn_per;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
-    const int place = atomicAdd(&cursor[sel_e[i]], 1);
-    order[place] = i;
-    where[i] = place;
+  const auto put = [&](int i, int e, bool in) {
+    const int place = add(cursor, e, in);
+    if (in) order[place] = i, where[i] = place;
+  };
+#pragma unroll
+  for (int k = 0; k < PLAN_AHEAD; ++k)
+    if (k * PLAN_THREADS < n_pairs) put(k * PLAN_THREADS + threadIdx.x, mine[k], mine[k] >= 0);
+  for (int i0 = PLAN_AHEAD * PLAN_THREADS; i0 < n_pairs; i0 += PLAN_THREADS) {
+    const int i = i0 + threadIdx.x;
+    put(i, i < n_pairs ? sel_e[i] : 0, i < n_pairs);
   }
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+  for (int e = warp; e < E; e += PLAN_THREADS / 32) {        // a warp an expert's tiles
     const int n_tt = (count[e] + 255) / 256, end = start[e] + count[e];
     int4* g = reinterpret_cast<int4*>(gu + 4) + (size_t)tiles_before[e] * gu_per;
-    for (int ft = 0; ft < gu_per; ++ft)
-      for (int tt = 0; tt < n_tt; ++tt) g[ft * n_tt + tt] = make_int4(start[e] + tt * 256, end, e * F + ft * 128, ft * 128);
+    for (int i = lane; i < gu_per * n_tt; i += 32) {
+      const int ft = i / n_tt, t0 = start[e] + i % n_tt * 256;
+      g[i] = make_int4(t0, end, e * F + ft * 128, ft * 128);
+    }
     int4* d = reinterpret_cast<int4*>(dn + 4) + (size_t)tiles_before[e] * dn_per;
-    for (int ft = 0; ft < dn_per; ++ft)
-      for (int tt = 0; tt < n_tt; ++tt) d[ft * n_tt + tt] = make_int4(start[e] + tt * 256, end, e * W + ft * 256, ft * 256);
+    for (int i = lane; i < dn_per * n_tt; i += 32) {
+      const int ft = i / n_tt, t0 = start[e] + i % n_tt * 256;
+      d[i] = make_int4(t0, end, e * W + ft * 256, ft * 256);
+    }
   }
 }
 

@@ -190,3 +190,46 @@ def test_clear_rows(ops):
     ops.clear_rows(m, 1)
     for t in m:
         assert float(t[1].abs().sum()) == 0.0 and bool((t[0] == 1).all()) and bool((t[2] == 1).all())
+
+
+@pytest.mark.parametrize("T, H, e", [(1, 3, 128), (5, 1, 4), (7, 16, 100), (33, 2, 128), (300, 5, 64)])
+@pytest.mark.parametrize("per_head, sigmoid, divided", [(False, False, False), (True, True, True)])
+def test_head_norm_gate_in_vectors(ops, T, H, e, per_head, sigmoid, divided):
+    """Heads in whole vectors against float64 and against the general form (a gate whose rows are off a 16-byte boundary)."""
+    g = torch.Generator().manual_seed(T + e)
+    o, wide, w = rnd(g, T, H * e), rnd(g, T, H * e + 4), rnd(g, H * e if per_head else e)
+    den = rnd(g, T, H).abs() + 0.5 if divided else None
+    odd = torch.zeros(T, H * e + 5)
+    odd[:, 1: H * e + 1] = wide[:, :H * e]
+    x = o.double().view(T, H, e) / (1.0 if den is None else den.double()[:, :, None])
+    z = wide[:, :H * e].double().view(T, H, e)
+    want = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5) * w.double().view(-1, e) * (torch.sigmoid(z) if sigmoid else F.silu(z))
+    for dtype, tol in ((torch.float32, 1e-6), (torch.bfloat16, 2.0 ** -8)):
+        outs = []
+        for gate in (wide.to(DEV)[:, :H * e], odd.to(DEV)[:, 1: H * e + 1]):
+            out = torch.full((T, H * e), float("nan"), dtype=dtype, device=DEV)
+            ops.head_norm_gate(o.to(DEV), gate, w.to(DEV), 1e-5, out, H, e, sigmoid=sigmoid, denom=None if den is None else den.to(DEV))
+            outs.append(out.double().cpu().view(T, H, e))
+            assert float(((outs[-1] - want).abs() / (want.abs() + want.abs().mean())).max()) < tol
+
+
+@pytest.mark.parametrize("pairs, E", [(1, 1), (7, 3), (1024, 8), (8192, 8), (8193, 70), (20000, 1024)])
+def test_expert_plan_counts(ops, pairs, E):
+    """Pairs sorted by expert and the tiles of both products, at the edges of what a thread keeps and of warps."""
+    g = torch.Generator().manual_seed(pairs)
+    sel = torch.randint(0, E, (pairs, 1), generator=g).int()
+    Fi, W = 384, 512
+    mg, md = ops.grouped_max_items(pairs, E, Fi, "swiglu"), ops.grouped_max_items(pairs, E, W, "store")
+    order, where = (torch.full((pairs,), -1, dtype=torch.int32, device=DEV) for _ in range(2))
+    tg, td = (torch.full((4 + 4 * n,), -1, dtype=torch.int32, device=DEV) for n in (mg, md))
+    ops.expert_plan(sel.to(DEV), E, Fi, W, order, where, tg, td)
+    o, wh, s = order.cpu().long(), where.cpu().long(), sel[:, 0].long()
+    assert torch.equal(torch.sort(o).values, torch.arange(pairs)) and torch.equal(wh[o], torch.arange(pairs))
+    assert bool((s[o][1:] >= s[o][:-1]).all())
+    counts = torch.bincount(s, minlength=E)
+    starts = torch.cumsum(counts, 0) - counts
+    for table, per, rows in ((tg.cpu(), 128, Fi), (td.cpu(), 256, W)):
+        want = [(int(starts[e]) + 256 * tt, int(starts[e] + counts[e]), e * rows + per * ft, per * ft)
+                for e in range(E) for ft in range(rows // per) for tt in range((int(counts[e]) + 255) // 256)]
+        assert int(table[0]) == len(want)
+        assert table[4: 4 + 4 * len(want)].view(-1, 4).tolist() == [list(w) for w in want]
