@@ -133,6 +133,43 @@ class Engine:
 
     # -- the step --------------------------------------------------------------
     def _validate(self, entries: Sequence[StepEntry], device_tokens: bool = False) -> None:
+        """Raises StepError for a step that cannot run.  The whole step is looked over at once; only one that does not pass
+        is gone through entry by entry, which says what is wrong with the first that cannot run."""
+        if not self._passes(entries, device_tokens):
+            self._validate_each(entries, device_tokens)
+
+    def _passes(self, entries: Sequence[StepEntry], device_tokens: bool) -> bool:
+        lengths, live, parts = self.cache.lengths, self.cache.is_live, []
+        slots = [e.slot for e in entries]
+        if not entries or len(set(slots)) < len(slots):
+            return False
+        for e in entries:
+            tokens, want, n = e.tokens, e.want, len(e.tokens)
+            if n == 0 or not live(e.slot) or lengths[e.slot] + n > self.max_seq_len:
+                return False
+            if n > 1:
+                # the array stays with the entry for the step's index buffer (a batch's prompts are tens of thousands)
+                tokens = np.asarray(tokens, dtype=np.int64)
+                if tokens.ndim != 1:
+                    return False
+                e.tokens = tokens
+                parts.append(tokens)
+            else:
+                t = int(tokens[0])
+                if not (0 <= t < self.model.vocab_size or (device_tokens and t == FROM_DEVICE)):
+                    return False
+            if type(want) is range:
+                if len(want) and not (0 <= min(want[0], want[-1]) and max(want[0], want[-1]) < n):
+                    return False
+            elif any(not 0 <= int(w) < n for w in want):
+                return False
+        if parts:
+            tokens = parts[0] if len(parts) == 1 else np.concatenate(parts)
+            low = FROM_DEVICE if device_tokens else 0
+            return low <= int(tokens.min()) and int(tokens.max()) < self.model.vocab_size
+        return True
+
+    def _validate_each(self, entries: Sequence[StepEntry], device_tokens: bool) -> None:
         if not entries:
             raise StepError("a step needs at least one sequence")
         seen = set()
@@ -187,8 +224,9 @@ class Engine:
         device once, and hand out views.  Returns (ctx, want_rows)."""
         cache = self.cache
         S = len(entries)
+        slots = [e.slot for e in entries]
         lens = [len(e.tokens) for e in entries]
-        starts = [cache.lengths[e.slot] for e in entries]
+        starts = [cache.lengths[s] for s in slots]
         T = sum(lens)
         after = [s + n for s, n in zip(starts, lens)]
         P = max((a + PAGE_SIZE - 1) // PAGE_SIZE for a in after)
@@ -196,11 +234,13 @@ class Engine:
             if P > pages_capacity:
                 raise StepError("a sequence outgrew the page capacity this step was laid out for")
             P = pages_capacity
-        wants: List[int] = []
-        q_start = [0]
+        wants, q_start = [], [0]
         for e, n in zip(entries, lens):
-            wants.extend(q_start[-1] + int(w) for w in e.want)
+            w = e.want
+            w = np.arange(w.start, w.stop, w.step) if type(w) is range else np.array([int(x) for x in w], dtype=np.int64)
+            wants.append(w + q_start[-1])
             q_start.append(q_start[-1] + n)
+        wants = np.concatenate(wants)
         W = len(wants)
         G = len(cache.groups)
         sizes = [T, T, T, S + 1, S, S, W] + [T, S * P] * G + [S + 1]
@@ -209,22 +249,24 @@ class Engine:
             offsets.append(offsets[-1] + _pad4(s))
         host = np.zeros(offsets[-1], dtype=np.int32)
         o = offsets
-        host[o[0]:o[0] + T] = np.concatenate([np.asarray(e.tokens, dtype=np.int32) for e in entries])
-        host[o[1]:o[1] + T] = np.concatenate([np.arange(s, s + n, dtype=np.int32) for s, n in zip(starts, lens)])
-        host[o[2]:o[2] + T] = np.repeat(np.arange(S, dtype=np.int32), lens)
+        of_seq = np.repeat(np.arange(S), lens)                  # each token's sequence
+        positions = np.arange(T) - np.repeat(np.subtract(q_start[:-1], starts), lens)
+        page, row = positions // PAGE_SIZE, positions % PAGE_SIZE
+        host[o[0]:o[0] + T] = np.concatenate([e.tokens for e in entries])
+        host[o[1]:o[1] + T] = positions
+        host[o[2]:o[2] + T] = of_seq
         host[o[3]:o[3] + S + 1] = q_start
         host[o[4]:o[4] + S] = after
-        host[o[5]:o[5] + S] = [e.slot for e in entries]
+        host[o[5]:o[5] + S] = slots
         host[o[6]:o[6] + W] = wants
         for gi, g in enumerate(cache.groups):
             base = 7 + 2 * gi
-            host[o[base]:o[base] + T] = np.concatenate(
-                [g.dest_rows(e.slot, s, n) for e, s, n in zip(entries, starts, lens)])
-            bt = np.full((S, P), -1, dtype=np.int32)
-            for i, e in enumerate(entries):
-                pages = g.pages[e.slot]
+            bt = host[o[base + 1]:o[base + 1] + S * P].reshape(S, P)
+            bt[:] = -1
+            for i, s in enumerate(slots):
+                pages = g.pages[s]
                 bt[i, :len(pages)] = pages
-            host[o[base + 1]:o[base + 1] + S * P] = bt.reshape(-1)
+            host[o[base]:o[base] + T] = bt[of_seq, page] * PAGE_SIZE + row
         host[o[7 + 2 * G] + 1:o[7 + 2 * G] + S + 1] = np.cumsum(after)
         total = offsets[-1]
         self.last_step_h2d_bytes = 4 * total
