@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(THREADS) delta_rule_kernel(
 // sequence, head and 16 value columns, the state in shared memory) is three small products a chunk.  All in float32 but for the
 // sums L and their differences (float64: past a strong decay a difference of two large sums would keep few digits in 32
 // bits); the decays only ever appear as exponentials of differences that are not positive.  One sequence of 1,500 tokens, 16 heads of 128 x
-// 128: 460 us as the walk above, a chain of 307 ns a token; 39 us of prepare and 221 of chunks so.
+// 128: 460 us as the walk above, a chain of 307 ns a token; 39 us of prepare and 153 of chunks so.
 constexpr int C = 32, DMAX = 128, LD = DMAX + 4, CHUNK_THREADS = 256;
 constexpr int V_FLOATS = C * DMAX, P_FLOATS = C * C, SC_FLOATS = C * 4;
 constexpr int SCRATCH_FLOATS = V_FLOATS + P_FLOATS + SC_FLOATS;           // of one chunk and head
@@ -420,10 +420,16 @@ __device__ __forceinline__ void async16(float* dst, const float* src, bool in) {
 constexpr int SLD = 40;                        // floats of a pair of the state's rows: 16 columns of two, and padding
 constexpr int CHUNK_SMEM = (5 * C * LD + C * (C + 4) + DMAX / 2 * SLD + 2 * C * 20 + C * 4) * 4;
 
-__global__ void __launch_bounds__(CHUNK_THREADS, 2) delta_chunks_kernel(
+// SPLIT times 256 threads, which share the first product's sums over k.  Once, two blocks an SM; twice where no SM has a second
+// block, which shortens a chunk's chain (prepare and chunks, one sequence of 16 heads of 128 x 128, 128 blocks: 1,500
+// tokens 265 and 192 us, 192 tokens 48 and 38; 8 heads of 72 x 72, 1,500 tokens 249 and 175).
+template <int SPLIT>
+__global__ void __launch_bounds__(CHUNK_THREADS * SPLIT, 2 / SPLIT) delta_chunks_kernel(
     const float* __restrict__ conv, int ldc, int q_col, int k_col, float* __restrict__ out, const float* __restrict__ scratch,
     float* __restrict__ state, long long slot_stride, long long state_off, const int* __restrict__ q_start,
     const int* __restrict__ seq_slot, int H, int G, int d, int e, int first_tile, int tiles, int packed) {
+  constexpr int THREADS = CHUNK_THREADS * SPLIT, KS = 4 * SPLIT;             // lanes that share a thread's sums
+  constexpr int OWN = 4 / SPLIT, RP = 2 / SPLIT;                             // columns of a row, pairs of the state's rows a thread keeps
   extern __shared__ __align__(16) float smem[];
   float* vq_b = smem;                          // two buffers of V [C][LD], then q [C][LD]: 64 rows to multiply with the state
   float* k_s = vq_b + 4 * C * LD;              // k [C][LD]
@@ -446,7 +452,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) delta_chunks_kernel(
     float* vq_s = vq_b + (chunk & 1) * 2 * C * LD;
     const int t0 = begin + chunk * C, n = min(C, n_all - chunk * C);
     const float* V_g = scratch_g + (size_t)chunk * H * SCRATCH_FLOATS;
-    for (int i = tid; i < C * DMAX / 4; i += CHUNK_THREADS) {
+    for (int i = tid; i < C * DMAX / 4; i += THREADS) {
       const int t = i / (DMAX / 4), r = (i % (DMAX / 4)) * 4;
       async16(vq_s + t * LD + r, V_g + t * DMAX + r, true);
       const bool in = t < n && r < d;
@@ -457,12 +463,12 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) delta_chunks_kernel(
   auto load_kp = [&](int chunk) {
     const int t0 = begin + chunk * C, n = min(C, n_all - chunk * C);
     const float* P_g = scratch_g + (size_t)chunk * H * SCRATCH_FLOATS + V_FLOATS;
-    for (int i = tid; i < C * DMAX / 4; i += CHUNK_THREADS) {
+    for (int i = tid; i < C * DMAX / 4; i += THREADS) {
       const int t = i / (DMAX / 4), r = (i % (DMAX / 4)) * 4;
       const bool in = t < n && r < d;
       async16(k_s + t * LD + r, conv + (size_t)(t0 + (in ? t : 0)) * ldc + k_col + (size_t)j * d + (in ? r : 0), in);
     }
-    async16(P_s + (tid / 8) * (C + 4) + (tid % 8) * 4, P_g + tid * 4, true);           // 256 threads, 256 pieces
+    if (tid < P_FLOATS / 4) async16(P_s + (tid / 8) * (C + 4) + (tid % 8) * 4, P_g + tid * 4, true);
     if (tid < C) async16(reinterpret_cast<float*>(sc_s + tid), P_g + P_FLOATS + 4 * tid, true);
     asm volatile("cp.async.commit_group;");
   };
@@ -470,28 +476,28 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) delta_chunks_kernel(
   load_kp(0);
   if (chunks > 1) load_vq(1);
   else asm volatile("cp.async.commit_group;");
-  for (int i = tid; i < DMAX * 16; i += CHUNK_THREADS) {
+  for (int i = tid; i < DMAX * 16; i += THREADS) {
     const int r = i >> 4, c = i & 15;
     S_s[(r >> 1) * SLD + 2 * c + (r & 1)] = (r < d && c0 + c < e) ? S_g[(size_t)r * e + c0 + c] : 0.0f;
   }
 
-  // first product: a thread four of the 64 rows, four columns, every fourth group of four k
-  const int cg = lane & 3, ks = (lane >> 2) & 3, rg = (warp << 1) | (lane >> 4);
-  const int t_own = (rg * 4 + ks) & (C - 1);                               // the row that is this thread's after the sums meet
+  // first product: a thread four of the 64 rows, four columns, every KS-th group of four k
+  const int cg = lane & 3, ks = (lane >> 2) & (KS - 1), rg = SPLIT == 1 ? (warp << 1) | (lane >> 4) : warp;
+  const int t_own = (rg * 4 + (ks & 3)) & (C - 1);                         // the row that is this thread's after the sums meet
   const bool is_q = rg >= C / 4;
-  // its columns: 2 cg, 2 cg + 1, 8 + 2 cg, 9 + 2 cg
-  const int col[2] = {2 * cg, 8 + 2 * cg};
-  // state's update, by the threads without queries: two pairs of rows, four columns
-  const int uc = (tid & 3) * 4, ur = ((tid & 127) >> 2) * 2;
+  // its columns: 2 cg, 2 cg + 1, 8 + 2 cg, 9 + 2 cg; after the sums meet the OWN of them from own[0] on
+  const int col[2] = {2 * cg, 8 + 2 * cg}, own[2] = {SPLIT == 1 || ks < 4 ? col[0] : col[1], col[1]};
+  // state's update, by the threads without queries: RP pairs of rows, four columns
+  const int uc = (tid & 3) * 4, ur = ((tid & (THREADS / 2 - 1)) >> 2) * RP;
 
   for (int chunk = 0; chunk < chunks; ++chunk) {
     const int t0 = begin + chunk * C, n = min(C, n_all - chunk * C);
     float* mine = out + ((size_t)(t0 + t_own) * H + h) * e + c0;
-    float u[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (!is_q && t_own < n) {
+    float u[OWN];
 #pragma unroll
-      for (int x = 0; x < 4; ++x)
-        if (c0 + col[x >> 1] + (x & 1) < e) u[x] = mine[col[x >> 1] + (x & 1)];
+    for (int x = 0; x < OWN; ++x) {
+      const int c = own[x >> 1] + (x & 1);
+      u[x] = !is_q && t_own < n && c0 + c < e ? mine[c] : 0.0f;
     }
     // groups in flight, oldest first: V and q of this chunk, k and P of it, V and q of the next
     asm volatile("cp.async.wait_group 2;" ::: "memory");
@@ -503,8 +509,8 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) delta_chunks_kernel(
 #pragma unroll
       for (int x = 0; x < 4; ++x) acc[i][x] = 0;
 #pragma unroll 2
-    for (int it = 0; it < DMAX / 16; ++it) {
-      const int k4 = 4 * it + ks;                                          // group of four rows of the state
+    for (int it = 0; it < DMAX / (4 * KS); ++it) {
+      const int k4 = KS * it + ks;                                         // group of four rows of the state
       ulonglong2 a[4], b[2][2];
 #pragma unroll
       for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(vq_s + (rg * 4 + i) * LD + 4 * k4);
@@ -522,18 +528,30 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) delta_chunks_kernel(
         }
       }
     }
-    // the four lanes of a row group and column group add up; lane ks keeps row ks
-    float m[4];
+    // the KS lanes of a row group and column group add up; lane ks keeps row ks % 4, of eight lanes two columns each
+    float r[4][OWN];
 #pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      float r[4];
+    for (int i = 0; i < 4; ++i) {
+      if (SPLIT == 1) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) r[i] = jb::lo(acc[i][x]) + jb::hi(acc[i][x]);
+        for (int x = 0; x < OWN; ++x) r[i][x] = jb::lo(acc[i][x]) + jb::hi(acc[i][x]);
+      } else {
+        const bool right = ks >= 4;
+#pragma unroll
+        for (int x = 0; x < OWN; ++x) {
+          const float a = jb::lo(acc[i][x]) + jb::hi(acc[i][x]), b = jb::lo(acc[i][2 + x]) + jb::hi(acc[i][2 + x]);
+          r[i][x] = (right ? b : a) + __shfl_xor_sync(0xffffffffu, right ? a : b, 16);
+        }
+      }
+    }
+    float m[OWN];
+#pragma unroll
+    for (int x = 0; x < OWN; ++x) {
       // rows 0, 1 go to the lanes with bit 1 of ks clear, rows 2, 3 to the others; then one row each
       const bool up = (ks & 2) != 0, odd = (ks & 1) != 0;
-      float a = up ? r[2] : r[0], b = up ? r[3] : r[1];
-      a += __shfl_xor_sync(0xffffffffu, up ? r[0] : r[2], 8);
-      b += __shfl_xor_sync(0xffffffffu, up ? r[1] : r[3], 8);
+      float a = up ? r[2][x] : r[0][x], b = up ? r[3][x] : r[1][x];
+      a += __shfl_xor_sync(0xffffffffu, up ? r[0][x] : r[2][x], 8);
+      b += __shfl_xor_sync(0xffffffffu, up ? r[1][x] : r[3][x], 8);
       m[x] = odd ? b : a;
       m[x] += __shfl_xor_sync(0xffffffffu, odd ? a : b, 4);
     }
@@ -542,46 +560,45 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) delta_chunks_kernel(
     const float4 sc = sc_s[t_own];
     if (!is_q) {
 #pragma unroll
-      for (int x = 0; x < 4; ++x) {
+      for (int x = 0; x < OWN; ++x) {
         const float w = u[x] - m[x];
-        w_s[t_own * 20 + col[x >> 1] + (x & 1)] = w;
-        wk_s[t_own * 20 + col[x >> 1] + (x & 1)] = w * sc.y;
+        w_s[t_own * 20 + own[x >> 1] + (x & 1)] = w;
+        wk_s[t_own * 20 + own[x >> 1] + (x & 1)] = w * sc.y;
       }
     }
     __syncthreads();
     if (is_q) {
-      float o[4];
+      float o[OWN];
 #pragma unroll
-      for (int x = 0; x < 4; ++x) o[x] = m[x] * sc.x;
+      for (int x = 0; x < OWN; ++x) o[x] = m[x] * sc.x;
       const auto four = [&](int s, int seen) {                             // four writes, of which `seen` come up to this token
         const float4 p = *reinterpret_cast<const float4*>(P_s + t_own * (C + 4) + s);
         const float ps[4] = {p.x, p.y, p.z, p.w};
 #pragma unroll
         for (int y = 0; y < 4; ++y) {
-          const float2 wa = *reinterpret_cast<const float2*>(w_s + (s + y) * 20 + col[0]);
-          const float2 wb = *reinterpret_cast<const float2*>(w_s + (s + y) * 20 + col[1]);
+          float2 w[OWN / 2];
+#pragma unroll
+          for (int x = 0; x < OWN / 2; ++x) w[x] = *reinterpret_cast<const float2*>(w_s + (s + y) * 20 + own[x]);
           if (y < seen) {
-            o[0] = fmaf(ps[y], wa.x, o[0]);
-            o[1] = fmaf(ps[y], wa.y, o[1]);
-            o[2] = fmaf(ps[y], wb.x, o[2]);
-            o[3] = fmaf(ps[y], wb.y, o[3]);
+#pragma unroll
+            for (int x = 0; x < OWN / 2; ++x) o[2 * x] = fmaf(ps[y], w[x].x, o[2 * x]), o[2 * x + 1] = fmaf(ps[y], w[x].y, o[2 * x + 1]);
           }
         }
       };
 #pragma unroll 2
       for (int s = 0; s < (t_own & ~3); s += 4) four(s, 4);
-      four(t_own & ~3, ks + 1);                                            // (zero times a later write that is infinite would be NaN)
+      four(t_own & ~3, (ks & 3) + 1);                                          // (zero times a later write that is infinite would be NaN)
       if (t_own < n) {
 #pragma unroll
-        for (int x = 0; x < 4; ++x)
-          if (c0 + col[x >> 1] + (x & 1) < e) mine[col[x >> 1] + (x & 1)] = o[x];
+        for (int x = 0; x < OWN; ++x)
+          if (c0 + own[x >> 1] + (x & 1) < e) mine[own[x >> 1] + (x & 1)] = o[x];
       }
     }
     if (!is_q) {
-      jb::Pair S[2][4];
+      jb::Pair S[RP][4];
       const jb::Pair g = jb::pair(sc.z, sc.z);
 #pragma unroll
-      for (int y = 0; y < 2; ++y)
+      for (int y = 0; y < RP; ++y)
 #pragma unroll
         for (int x = 0; x < 4; x += 2) {
           const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(S_s + (ur + y) * SLD + 2 * (uc + x));
@@ -590,17 +607,22 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) delta_chunks_kernel(
         }
 #pragma unroll 8
       for (int t = 0; t < C; ++t) {
-        const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(k_s + t * LD + 2 * ur);
+        jb::Pair k[RP];
+        if constexpr (RP == 2) {
+          const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(k_s + t * LD + 2 * ur);
+          k[0] = v.x, k[1] = v.y;
+        } else {
+          k[0] = *reinterpret_cast<const jb::Pair*>(k_s + t * LD + 2 * ur);
+        }
         const float4 w = *reinterpret_cast<const float4*>(wk_s + t * 20 + uc);
         const jb::Pair ws[4] = {jb::pair(w.x, w.x), jb::pair(w.y, w.y), jb::pair(w.z, w.z), jb::pair(w.w, w.w)};
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          S[0][x] = jb::fma2(k.x, ws[x], S[0][x]);
-          S[1][x] = jb::fma2(k.y, ws[x], S[1][x]);
-        }
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+          for (int y = 0; y < RP; ++y) S[y][x] = jb::fma2(k[y], ws[x], S[y][x]);
       }
 #pragma unroll
-      for (int y = 0; y < 2; ++y)
+      for (int y = 0; y < RP; ++y)
 #pragma unroll
         for (int x = 0; x < 4; x += 2)
           *reinterpret_cast<ulonglong2*>(S_s + (ur + y) * SLD + 2 * (uc + x)) = make_ulonglong2(S[y][x], S[y][x + 1]);
@@ -612,7 +634,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) delta_chunks_kernel(
     else asm volatile("cp.async.commit_group;");
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  for (int i = tid; i < DMAX * 16; i += CHUNK_THREADS) {
+  for (int i = tid; i < DMAX * 16; i += THREADS) {
     const int r = i >> 4, c = i & 15;
     if (r < d && c0 + c < e) S_g[(size_t)r * e + c0 + c] = S_s[(r >> 1) * SLD + 2 * c + (r & 1)];
   }
@@ -654,7 +676,9 @@ JB_EXPORT int jb_delta_rule_chunks(const float* conv, int ldc, int q_col, int k_
   JB_REFUSE(d < 1 || d > DMAX || e < 1 || ((d | ldc | q_col | k_col) & 3) != 0 || (((uintptr_t)conv | (uintptr_t)scratch) & 15) != 0,
             "delta_rule_chunks: keys of %d numbers in rows of %d at columns %d and %d", d, ldc, q_col, k_col);
   JB_REFUSE(G < 1 || H % G != 0 || tiles < 0 || max_q_len < 1, "delta_rule_chunks: %d heads are not a multiple of %d key heads", H, G);
-  cudaError_t err = cudaFuncSetAttribute(delta_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CHUNK_SMEM);
+  const bool few = (long long)n_seqs * H * ((e + 15) / 16) <= 148;                   // no SM has a second block
+  auto* const walk_kernel = few ? delta_chunks_kernel<2> : delta_chunks_kernel<1>;
+  cudaError_t err = cudaFuncSetAttribute(walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CHUNK_SMEM);
   if (err != cudaSuccess) return (int)err;
   const int all = (max_q_len + C - 1) / C, packed = tiles == 0;
   if (packed) tiles = all;
@@ -672,8 +696,8 @@ JB_EXPORT int jb_delta_rule_chunks(const float* conv, int ldc, int q_col, int k_
     err = cudaLaunchKernelEx(&prepare.c, delta_prepare_kernel, conv, ldc, q_col, k_col, v_col, raw, ld, b_col, a_col, A_log,
                              dt_bias, unit_eps, out, scratch, q_start, n_seqs, H, G, d, e, first, tiles, packed, heads_here);
     if (err != cudaSuccess) return (int)err;
-    jb::Launch walk(dim3((e + 15) / 16, H, n_seqs), dim3(CHUNK_THREADS), CHUNK_SMEM, stream);
-    err = cudaLaunchKernelEx(&walk.c, delta_chunks_kernel, conv, ldc, q_col, k_col, out, (const float*)scratch, state, slot_stride,
+    jb::Launch walk(dim3((e + 15) / 16, H, n_seqs), dim3(few ? 2 * CHUNK_THREADS : CHUNK_THREADS), CHUNK_SMEM, stream);
+    err = cudaLaunchKernelEx(&walk.c, walk_kernel, conv, ldc, q_col, k_col, out, (const float*)scratch, state, slot_stride,
                              state_off, q_start, seq_slot, H, G, d, e, first, tiles, packed);
     if (err != cudaSuccess) return (int)err;
   }
