@@ -117,12 +117,19 @@ __global__ void __launch_bounds__(32 * RANGES) gemm_f32_stream_kernel(const floa
   load_step = 0, load_slot = 0, load_n0 = (int)blockIdx.x * ROWS;
   for (int i = 0; i < loaded; ++i) load_x(true), next();
 
+  // A unit's sums, one for each (row, token) and segment, join the range in the order of the segments: the four lanes of a row
+  // exchange theirs so that each ends with all four segments of its share of the (row, token) pairs, in as many shuffles as a
+  // lane has pairs (every lane asking the others for every pair took four times as many: 8 tokens, 16,384 rows of 2,048, 46.6 us
+  // and 44.5 so, 16 tokens 88 and 83.5, 8 tokens of 128,256 rows of 1,536 242 and 230; up to 4 tokens level).
+  constexpr int PAIRS = RL * TT, MINE = PAIRS >= 4 ? PAIRS / 4 : PAIRS;
   Pair acc[RL][TT];
-  float sum[RL][TT];
+  float sum[MINE];
 #pragma unroll
   for (int r = 0; r < RL; ++r)
 #pragma unroll
-    for (int t = 0; t < TT; ++t) acc[r][t] = 0, sum[r][t] = 0.0f;
+    for (int t = 0; t < TT; ++t) acc[r][t] = 0;
+#pragma unroll
+  for (int i = 0; i < MINE; ++i) sum[i] = 0.0f;
   const int row = lane >> 2, seg = lane & 3;
   int step = 0, n0 = (int)blockIdx.x * ROWS, slot = 0;
 
@@ -155,28 +162,49 @@ __global__ void __launch_bounds__(32 * RANGES) gemm_f32_stream_kernel(const floa
     slot = slot + 1 == STAGES ? 0 : slot + 1;
     if (step & 1) {                                            // the unit's segments join the range in order
       const int u0 = k0 - SUB;
+      float one[PAIRS];
 #pragma unroll
-      for (int r = 0; r < RL; ++r)
+      for (int i = 0; i < PAIRS; ++i) one[i] = even_and_odd(acc[i / TT][i % TT]), acc[i / TT][i % TT] = 0;
+      if constexpr (PAIRS >= 4) {
+        const bool odd = seg & 1, late = seg & 2;
+        float two[PAIRS / 2][2];                               // half of the pairs, segments seg & ~1 and seg | 1
 #pragma unroll
-        for (int t = 0; t < TT; ++t) {
-          const float mine = even_and_odd(acc[r][t]);
-          acc[r][t] = 0;
-#pragma unroll
-          for (int s = 0; s < SEGS; ++s) {
-            const float v = __shfl_sync(0xffffffffu, mine, (lane & ~3) | s);
-            if (u0 + s * SEG < k_end) sum[r][t] += v;
-          }
+        for (int i = 0; i < PAIRS / 2; ++i) {
+          const float keep = odd ? one[PAIRS / 2 + i] : one[i];
+          const float got = __shfl_xor_sync(0xffffffffu, odd ? one[i] : one[PAIRS / 2 + i], 1);
+          two[i][0] = odd ? got : keep, two[i][1] = odd ? keep : got;
         }
+#pragma unroll
+        for (int i = 0; i < MINE; ++i) {
+          float four[SEGS];
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const float keep = late ? two[MINE + i][x] : two[i][x];
+            const float got = __shfl_xor_sync(0xffffffffu, late ? two[i][x] : two[MINE + i][x], 2);
+            four[x] = late ? got : keep, four[2 + x] = late ? keep : got;
+          }
+#pragma unroll
+          for (int x = 0; x < SEGS; ++x)
+            if (u0 + x * SEG < k_end) sum[i] += four[x];
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < PAIRS; ++i)
+#pragma unroll
+          for (int x = 0; x < SEGS; ++x) {
+            const float v = __shfl_sync(0xffffffffu, one[i], (lane & ~3) | x);
+            if (u0 + x * SEG < k_end) sum[i] += v;
+          }
+      }
     }
     if (++step < steps) continue;
     step = 0;
 #pragma unroll
-    for (int r = 0; r < RL; ++r)
-#pragma unroll
-      for (int t = 0; t < TT; ++t) {
-        if ((t & 3) == seg) met[(warp * TT + t) * ROWS + r * 8 + row] = sum[r][t];
-        sum[r][t] = 0.0f;
-      }
+    for (int i = 0; i < MINE; ++i) {
+      const int pair = PAIRS >= 4 ? (seg & 1) * (PAIRS / 2) + (seg >> 1) * MINE + i : i;
+      if (PAIRS >= 4 || seg == i) met[(warp * TT + pair % TT) * ROWS + pair / TT * 8 + row] = sum[i];
+      sum[i] = 0.0f;
+    }
     __syncthreads();
     for (int e = threadIdx.x; e < tokens * ROWS; e += blockDim.x) {
       const int t = e / ROWS, n = n0 + e % ROWS;
@@ -344,8 +372,8 @@ JB_EXPORT int jb_gemm_f32(const float* X, const float* W, float* Y, int T, int N
   const bool vec = K % 4 == 0 && ldx % 4 == 0 && (((uintptr_t)X | (uintptr_t)W) & 15) == 0;
   const int tiles = ((N + BN - 1) / BN) * ((T + BM - 1) / BM);
   // The streaming kernel asks for the weights once for every 8 tokens, the tiles need some of them to fill the SMs.  Streamed and
-  // tiles from cold memory, microseconds, K = 2,048: 16 tokens 2,048 rows 20 and 39, 8,192 rows 50 and 82, 32,000 rows 172 and
-  // 233; 24 tokens 27 and 39, 72 and 82, 250 and 233 (16,384 rows 133 and 143, 4,096 rows 43 and 41); 32 tokens 33 and 39, 92
+  // tiles from cold memory, microseconds, K = 2,048: 16 tokens 2,048 rows 20 and 39, 8,192 rows 48 and 82, 32,000 rows 162 and
+  // 233; 24 tokens 27 and 39, 70 and 82, 240 and 233 (16,384 rows 133 and 143, 4,096 rows 43 and 41); 32 tokens 33 and 39, 92
   // and 82, 332 and 235 (2,560 rows 39 and 39; 2,048 rows of 8,192 90 and 123); 40 tokens of 2,048 rows 39 and 39.
   if (vec && (T <= 24 || (T <= 32 && N <= 20 * BN))) {
 #define JB_GO(TT) return launch_stream<TT>(X, W, Y, T, N, K, ldx, ldy, accumulate, stream)
