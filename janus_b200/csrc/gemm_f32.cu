@@ -372,9 +372,10 @@ JB_EXPORT int jb_gemm_f32(const float* X, const float* W, float* Y, int T, int N
   const bool vec = K % 4 == 0 && ldx % 4 == 0 && (((uintptr_t)X | (uintptr_t)W) & 15) == 0;
   const int tiles = ((N + BN - 1) / BN) * ((T + BM - 1) / BM);
   // The streaming kernel asks for the weights once for every 8 tokens, the tiles need some of them to fill the SMs.  Streamed and
-  // tiles from cold memory, microseconds, K = 2,048: 16 tokens 2,048 rows 20 and 39, 8,192 rows 48 and 82, 32,000 rows 162 and
-  // 233; 24 tokens 27 and 39, 70 and 82, 240 and 233 (16,384 rows 133 and 143, 4,096 rows 43 and 41); 32 tokens 33 and 39, 92
+  // tiles from cold memory, microseconds, K = 2,048: 16 tokens 2,048 rows 20 and 39, 8,192 rows 50 and 82, 32,000 rows 172 and
+  // 233; 24 tokens 27 and 39, 72 and 82, 250 and 233 (16,384 rows 133 and 143, 4,096 rows 43 and 41); 32 tokens 33 and 39, 92
   // and 82, 332 and 235 (2,560 rows 39 and 39; 2,048 rows of 8,192 90 and 123); 40 tokens of 2,048 rows 39 and 39.
+  // (Streamed ones of 8 tokens and more take 5 % less since their sums meet in fewer shuffles.)
   if (vec && (T <= 24 || (T <= 32 && N <= 20 * BN))) {
 #define JB_GO(TT) return launch_stream<TT>(X, W, Y, T, N, K, ldx, ldy, accumulate, stream)
     if (T == 1) JB_GO(1);

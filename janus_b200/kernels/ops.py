@@ -1824,9 +1824,10 @@ def delta_rule_scratch(n_seqs: int, heads: int, max_q_len: int, conv_width: int,
                        tokens: Optional[int] = None, vdim: int = 128) -> int:
     """Floats of scratch with which `delta_rule` goes by chunks; 0: it walks token by token.  Chunks take keys of 68 to 128
     numbers whose rows are whole 16-byte vectors.  `tokens`: of all sequences (None: each is as long as the longest).  Walk
-    and chunks, microseconds, heads of 128 x 128: one sequence of 16 heads, 192 tokens 50 and 38,
-    2,048 tokens 447 and 251 (before the chunks' blocks of few got more threads 64 tokens 21 and 27, 128 tokens 35 and 37), 4,096 beside 31 single tokens 1,263 and 697; four sequences, 64 tokens 52 and
-    41, 512 tokens 321 and 202; eight, 32 tokens 56 and 47, 2,048 tokens 2,334 and 1,294; two of 1,024 beside 30 single tokens
+    and chunks, microseconds, heads of 128 x 128: one sequence of 16 heads, 64 tokens 21 and 27, 128 tokens 35 and 37 (with
+    256 threads a block), 192 tokens 50 and 38, 2,048 tokens 447 and 251, 4,096 beside 31 single tokens 1,263 and 697; four
+    sequences, 64 tokens 52 and 41, 512 tokens 321 and 202; eight, 32 tokens 56 and 47, 2,048 tokens 2,334 and 1,294; two of
+    1,024 beside 30 single tokens
     318 and 310.  72 x 72 is much the same (eight of 256 tokens 216 and 144); keys of 64 would be padded to 128 (eight
     sequences of 32 heads of 64 x 64, 256 tokens: 211 and 236)."""
     if max_q_len < 1:
