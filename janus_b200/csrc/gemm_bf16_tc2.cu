@@ -352,6 +352,35 @@ __global__ void __launch_bounds__(THREADS) gemm_tc2_kernel(const __grid_constant
     TileCoord tc;
     for (; walk.next(tc); ++j) {
       const int buf = j & 1;
+      // A rotating epilogue has its token's place and the angles of its first pairs by the time the products are there: asked
+      // for in the epilogue, eight bytes a pair and after the positions, with half of the warps idle at heads of 64, they were
+      // what a tile's end waited for (4,351 tokens, 32 + 2 x 8 heads of 64, width 2,048: 65 -> 44 us; 1,395 tokens, 16 + 2 x 4
+      // heads of 128 28 -> 19.5; 3,407 tokens, 32 + 2 x 8 heads of 128, width 4,096 139 -> 129).
+      int t = 0, dst = 0, hd = 32, half = 16, turned = 0;
+      bool t_ok = false;
+      float4 cs[MODE == QKV_ROPE ? 8 : 1];
+      const float* angles = nullptr;
+      const auto turn = [&](int i) {
+        turned = i;
+        if (((uintptr_t)rope.cos_sin & 15) == 0) {
+#pragma unroll
+          for (int x = 0; x < (MODE == QKV_ROPE ? 8 : 0); ++x) cs[x] = *reinterpret_cast<const float4*>(angles + 2 * i + 4 * x);
+        } else {
+#pragma unroll
+          for (int x = 0; x < (MODE == QKV_ROPE ? 8 : 0); ++x) {
+            const float2 a = *reinterpret_cast<const float2*>(angles + 2 * i + 4 * x), b = *reinterpret_cast<const float2*>(angles + 2 * i + 4 * x + 2);
+            cs[x] = make_float4(a.x, a.y, b.x, b.y);
+          }
+        }
+      };
+      if (MODE == QKV_ROPE) {
+        t = tc.t0 + (int)rank * BM + quarter * 32 + lane;
+        t_ok = t < T;
+        hd = rope.hd, half = hd >> 1;
+        dst = t_ok ? rope.dest[t] : 0;
+        angles = rope.cos_sin + (size_t)(t_ok ? rope.positions[t] : 0) * hd;
+        turn(part % (half / 16) * 16);
+      }
       if (!mbar_wait(acc_full0 + 8 * buf, (j >> 1) & 1, status, 23)) break;
       tc_fence_after();
       const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * ACC_COLS;
@@ -391,16 +420,11 @@ __global__ void __launch_bounds__(THREADS) gemm_tc2_kernel(const __grid_constant
           }
         }
       } else if (MODE == QKV_ROPE) {
-        // this lane is a token; the 256 columns are whole heads of q, k or v
-        const int t = tc.t0 + (int)rank * BM + quarter * 32 + lane;
-        const bool t_ok = t < T;
-        const int hd = rope.hd, half = hd >> 1;
-        const int pos = t_ok ? rope.positions[t] : 0;
-        const int dst = t_ok ? rope.dest[t] : 0;
-        const float* cs = rope.cos_sin + (size_t)pos * hd;
+        // this lane is a token; the 256 columns are whole heads of q, k or v, eight times sixteen pairs (x, x + hd / 2), of which
+        // every EPI_PARTS-th are this warp's
 #pragma unroll 1
-        for (int c = 0; c < BN; c += hd) {
-          const int f = tc.f0 + c;
+        for (int n = part; n < BN / 32; n += EPI_PARTS) {
+          const int c = n / (half / 16) * hd, i = n % (half / 16) * 16, f = tc.f0 + c;
           if (f >= N_out) break;
           const int head = f / hd;
           __nv_bfloat16* out;
@@ -412,40 +436,33 @@ __global__ void __launch_bounds__(THREADS) gemm_tc2_kernel(const __grid_constant
             __nv_bfloat16* base = head < rope.nh + rope.nkv ? rope.k_cache : rope.v_cache;
             out = base + (((size_t)(dst / rope.page_size) * rope.nkv + kvh) * rope.page_size + dst % rope.page_size) * hd;
           }
-#pragma unroll 1
-          for (int i = 16 * part; i < half; i += 16 * EPI_PARTS) {   // (half is a multiple of 16 * EPI_PARTS or the parts idle)
-            uint32_t lo[16], hi[16];
-            tmem_ld16(lane_base + c + i, lo);
-            tmem_ld16(lane_base + c + half + i, hi);
-            tmem_ld_wait();
-            if (t_ok) {
-              uint32_t plo[8], phi[8];
+          if (n > part && i != turned) turn(i);
+          uint32_t lo[16], hi[16];
+          tmem_ld16(lane_base + c + i, lo);
+          tmem_ld16(lane_base + c + half + i, hi);
+          tmem_ld_wait();
+          if (t_ok) {
+            uint32_t plo[8], phi[8];
 #pragma unroll
-              for (int jj = 0; jj < 16; jj += 2) {
-                float y0[2], y1[2];
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                  const float x0 = __uint_as_float(lo[jj + e]), x1 = __uint_as_float(hi[jj + e]);
-                  if (rotate) {
-                    const float2 k = *reinterpret_cast<const float2*>(cs + 2 * (i + jj + e));   // (cos, sin)
-                    y0[e] = x0 * k.x - x1 * k.y;
-                    y1[e] = x0 * k.y + x1 * k.x;
-                  } else {
-                    y0[e] = x0;
-                    y1[e] = x1;
-                  }
-                }
-                const __nv_bfloat162 a = __floats2bfloat162_rn(y0[0], y0[1]), b = __floats2bfloat162_rn(y1[0], y1[1]);
-                plo[jj / 2] = *(const uint32_t*)&a;
-                phi[jj / 2] = *(const uint32_t*)&b;
+            for (int jj = 0; jj < 16; jj += 2) {
+              float x0 = __uint_as_float(lo[jj]), x1 = __uint_as_float(hi[jj]);
+              float y0 = __uint_as_float(lo[jj + 1]), y1 = __uint_as_float(hi[jj + 1]);
+              if (rotate) {
+                const float4 k = cs[jj / 2];                       // (cos, sin) of two pairs
+                const float x = x0, y = y0;
+                x0 = x * k.x - x1 * k.y, x1 = x * k.y + x1 * k.x;
+                y0 = y * k.z - y1 * k.w, y1 = y * k.w + y1 * k.z;
               }
-              uint4* d0 = (uint4*)(out + i);
-              uint4* d1 = (uint4*)(out + half + i);
-              d0[0] = make_uint4(plo[0], plo[1], plo[2], plo[3]);
-              d0[1] = make_uint4(plo[4], plo[5], plo[6], plo[7]);
-              d1[0] = make_uint4(phi[0], phi[1], phi[2], phi[3]);
-              d1[1] = make_uint4(phi[4], phi[5], phi[6], phi[7]);
+              const __nv_bfloat162 a = __floats2bfloat162_rn(x0, y0), b = __floats2bfloat162_rn(x1, y1);
+              plo[jj / 2] = *(const uint32_t*)&a;
+              phi[jj / 2] = *(const uint32_t*)&b;
             }
+            uint4* d0 = (uint4*)(out + i);
+            uint4* d1 = (uint4*)(out + half + i);
+            d0[0] = make_uint4(plo[0], plo[1], plo[2], plo[3]);
+            d0[1] = make_uint4(plo[4], plo[5], plo[6], plo[7]);
+            d1[0] = make_uint4(phi[0], phi[1], phi[2], phi[3]);
+            d1[1] = make_uint4(phi[4], phi[5], phi[6], phi[7]);
           }
         }
       } else {
