@@ -191,9 +191,10 @@ __global__ void conv_rope_cache_vec_kernel(const float* __restrict__ proj, int l
 
 // The same for prompts with up to four taps: a thread owns four channels (both halves of four rotated pairs) and walks
 // WALK_TOKENS tokens, its last three inputs in registers, so an input is read once instead of `taps` times, and its taps
-// once a walk; WALK_AHEAD tokens' inputs and places are in flight before the first is used.  (2,623 tokens x 3,072
-// channels, 59 MB: 87 us a token a thread, 37 so.)
-constexpr int WALK_TOKENS = 16, WALK_AHEAD = 4, WALK_TAPS = 4;
+// once a walk; WALK_AHEAD tokens' inputs, places and angles are in flight before the first is used.  What is left is a walk's
+// start (taps, first window) and its chain of loads.  (2,623 tokens x 3,072 channels, 59 MB: 87 us a token a thread; 37.5 with
+// angles asked for token by token, taps number by number and divisions for every number's place; 25 so.)
+constexpr int WALK_TOKENS = 8, WALK_AHEAD = 2, WALK_TAPS = 4, WALK_FROM = 64;
 
 template <typename TC>
 __global__ void __launch_bounds__(128) conv_rope_cache_walk_kernel(
@@ -211,31 +212,40 @@ __global__ void __launch_bounds__(128) conv_rope_cache_walk_kernel(
   if (turns && i >= half) return;                        // written with the pair's first member
   const int parts = turns ? 2 : 1;
   float w[2][WALK_TAPS][4];                              // [half][tokens back][channel]
+  if (taps == WALK_TAPS && ((uintptr_t)conv_w & 15) == 0) {
 #pragma unroll
-  for (int p = 0; p < 2; ++p)
+    for (int p = 0; p < 2; ++p)
 #pragma unroll
-    for (int b = 0; b < WALK_TAPS; ++b)
+      for (int x = 0; x < 4; ++x) {
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (p < parts) v = *reinterpret_cast<const float4*>(conv_w + (size_t)(c + p * half + x) * WALK_TAPS);
+        w[p][3][x] = v.x, w[p][2][x] = v.y, w[p][1][x] = v.z, w[p][0][x] = v.w;
+      }
+  } else {
 #pragma unroll
-      for (int x = 0; x < 4; ++x)
-        w[p][b][x] = p < parts && b < taps ? conv_w[(size_t)(c + p * half + x) * taps + taps - 1 - b] : 0.0f;
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+      for (int b = 0; b < WALK_TAPS; ++b)
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+          w[p][b][x] = p < parts && b < taps ? conv_w[(size_t)(c + p * half + x) * taps + taps - 1 - b] : 0.0f;
+  }
   jb::pdl_wait();
   const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   float4 win[2][WALK_TAPS - 1];                          // win[.][b]: the input b + 1 tokens back
   const int t0 = blockIdx.x * WALK_TOKENS, t1 = min(T, t0 + WALK_TOKENS);
-  const auto put = [&](int c0, float4 y, int t, size_t page, int off) {
-    if (c0 < Cq) {
-      *reinterpret_cast<float4*>(q_out + (size_t)t * Cq + c0) = y;
-    } else if (c0 < Cq + Ck) {
-      const int kc = c0 - Cq;
-      store4c<TC>(k_cache + ((page * 2 * G + kc / d) * page_size + off) * d + kc % d, y);
-    } else {
-      const int vc = c0 - Cq - Ck;
-      store4c<TC>(v_cache + ((page * G + vc / e) * page_size + off) * e + vc % e, y);
-    }
+  // where a channel's numbers go: queries by token, keys and values by page and row
+  const bool is_q = c < Cq, is_k = c < Cq + Ck;
+  const int at = is_q ? c : is_k ? c - Cq : c - Cq - Ck, size = is_k ? d : e, heads = is_k ? 2 * G : G;
+  TC* const cache = (is_k ? k_cache : v_cache) + (is_q ? 0 : (size_t)(at / size) * page_size * size + at % size);
+  const size_t page_numbers = (size_t)heads * page_size * size;
+  const auto put = [&](int shift, float4 y, int t, unsigned row) {
+    if (is_q) *reinterpret_cast<float4*>(q_out + (size_t)t * Cq + c + shift) = y;
+    else store4c<TC>(cache + (row / (unsigned)page_size) * page_numbers + (row % (unsigned)page_size) * size + shift, y);
   };
   int before = -1;
   for (int tb = t0; tb < t1; tb += WALK_AHEAD) {
-    float4 u[WALK_AHEAD][2];
+    float4 u[WALK_AHEAD][2], angles[WALK_AHEAD][2];
     int seqs[WALK_AHEAD], pos[WALK_AHEAD], dst[WALK_AHEAD];
 #pragma unroll
     for (int k = 0; k < WALK_AHEAD; ++k) {
@@ -244,6 +254,13 @@ __global__ void __launch_bounds__(128) conv_rope_cache_walk_kernel(
 #pragma unroll
       for (int p = 0; p < 2; ++p)
         u[k][p] = p < parts ? *reinterpret_cast<const float4*>(proj + (size_t)t * ld + c + p * half) : zero;
+    }
+    if (turns) {
+#pragma unroll
+      for (int k = 0; k < WALK_AHEAD; ++k) {
+        const float* cs = cos_sin + (size_t)pos[k] * half * 2 + 2 * i;
+        angles[k][0] = *reinterpret_cast<const float4*>(cs), angles[k][1] = *reinterpret_cast<const float4*>(cs + 4);
+      }
     }
 #pragma unroll
     for (int k = 0; k < WALK_AHEAD; ++k) {
@@ -274,17 +291,13 @@ __global__ void __launch_bounds__(128) conv_rope_cache_walk_kernel(
         }
         win[p][2] = win[p][1], win[p][1] = win[p][0], win[p][0] = u[k][p];
       }
-      const size_t page = (size_t)(dst[k] / page_size);
-      const int off = dst[k] % page_size;
       if (!turns) {
-        put(c, y[0], t, page, off);
+        put(0, y[0], t, dst[k]);
         continue;
       }
-      const float* cs = cos_sin + (size_t)pos[k] * half * 2 + 2 * i;
-      const float4 a0 = *reinterpret_cast<const float4*>(cs), a1 = *reinterpret_cast<const float4*>(cs + 4);
-      const float4 a = y[0], b = y[1];
-      put(c, make_float4(a.x * a0.x - b.x * a0.y, a.y * a0.z - b.y * a0.w, a.z * a1.x - b.z * a1.y, a.w * a1.z - b.w * a1.w), t, page, off);
-      put(c + half, make_float4(b.x * a0.x + a.x * a0.y, b.y * a0.z + a.y * a0.w, b.z * a1.x + a.z * a1.y, b.w * a1.z + a.w * a1.w), t, page, off);
+      const float4 a0 = angles[k][0], a1 = angles[k][1], a = y[0], b = y[1];
+      put(0, make_float4(a.x * a0.x - b.x * a0.y, a.y * a0.z - b.y * a0.w, a.z * a1.x - b.z * a1.y, a.w * a1.z - b.w * a1.w), t, dst[k]);
+      put(half, make_float4(b.x * a0.x + a.x * a0.y, b.y * a0.z + a.y * a0.w, b.z * a1.x + a.z * a1.y, b.w * a1.z + a.w * a1.w), t, dst[k]);
     }
   }
 }
@@ -760,7 +773,7 @@ JB_EXPORT int jb_conv_rope_cache(const float* proj, int ld, const float* conv_w,
   const bool vec = d % 4 == 0 && e % 4 == 0 && rot % 8 == 0 && ld % 4 == 0 &&
                    (((uintptr_t)proj | (uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)conv_state |
                      (uintptr_t)cos_sin) & 15) == 0;
-  if (vec && conv_w != nullptr && taps >= 2 && taps <= WALK_TAPS && !update_state && T >= 4 * WALK_TOKENS) {
+  if (vec && conv_w != nullptr && taps >= 2 && taps <= WALK_TAPS && !update_state && T >= WALK_FROM) {
     jb::Launch wcfg(dim3((T + WALK_TOKENS - 1) / WALK_TOKENS, (C / 4 + 127) / 128), dim3(128), 0, stream);
     if (cache_dtype == JB_F32)
       return (int)cudaLaunchKernelEx(&wcfg.c, conv_rope_cache_walk_kernel<float>, proj, ld, conv_w, taps, (const float*)conv_state,

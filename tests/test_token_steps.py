@@ -233,3 +233,24 @@ def test_expert_plan_counts(ops, pairs, E):
                 for e in range(E) for ft in range(rows // per) for tt in range((int(counts[e]) + 255) // 256)]
         assert int(table[0]) == len(want)
         assert table[4: 4 + 4 * len(want)].view(-1, 4).tolist() == [list(w) for w in want]
+
+
+@pytest.mark.parametrize("T", [64, 65, 71, 137])
+def test_conv_taps_off_their_vectors(ops, T):
+    """A prompt's taps are read four to a load where they begin on 16 bytes, else one by one: the same numbers either way."""
+    g = torch.Generator().manual_seed(T)
+    H, G, d, e, page, rot = 2, 1, 16, 12, 16, 8
+    C = (2 * H + 2 * G) * d + G * e
+    proj, loose, state = rnd(g, T, C).to(DEV), rnd(g, 4 * C + 1).to(DEV), rnd(g, 1, 3, C).to(DEV)
+    angles = rnd(g, T, rot // 2)
+    table = torch.stack([angles.cos(), angles.sin()], dim=-1).contiguous().to(DEV)
+    ints = lambda *v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    pos, seq = torch.arange(T, dtype=torch.int32, device=DEV), torch.zeros(T, dtype=torch.int32, device=DEV)
+    pages = -(-T // page)
+    results = []
+    for w in (loose[1:].view(C, 4), loose[1:].clone().view(C, 4)):
+        q = torch.empty(T, 2 * H * d, device=DEV)
+        k_cache, v_cache = torch.zeros(pages, 2 * G, page, d, device=DEV), torch.zeros(pages, G, page, e, device=DEV)
+        ops.conv_rope_cache(proj, w, 4, state, seq, ints(0, T), ints(0), pos, table, rot, q, pos, k_cache, v_cache, H, G, d, e, page)
+        results.append((q, k_cache, v_cache))
+    assert all(torch.equal(a, b) for a, b in zip(*results)) and results[0][0].abs().max() > 0
