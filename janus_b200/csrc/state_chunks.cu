@@ -20,6 +20,7 @@
 // number as a decay, and so do the chunks).
 // Kinds: MAMBA   q = C, k = B, v = x, a = exp(-exp(A_log) dt), b = dt = softplus(raw + bias), y + D x
 //        LIGHTNING q, k, v through SiLU, a one number a head, b = 1
+//        CHANNEL a decay for each of a head's d key channels, b = 1 (see `channel_prepare_kernel`)
 //        MEMORY  a, b and exp(-m) as `exp_gates` leaves them; values of one make the normalizer n (the first block of a
 //                head has it beside its columns), of which the divisor max(|scale n . q|, exp(-m)) + 1e-6 is kept
 #include <stdio.h>
@@ -31,9 +32,12 @@ namespace {
 constexpr int C = 32, DMAX = 128, LD = DMAX + 4, THREADS = 256;
 constexpr int P_FLOATS = C * C, SC_FLOATS = 4 * C, QK_FLOATS = 2 * C * DMAX;
 constexpr float DEN_FLOOR = 1e-6f;
-enum { MAMBA = 0, LIGHTNING = 1, MEMORY = 2 };
-// scratch of a chunk and head: P, the scales, and for LIGHTNING the activated q and k
-__host__ __device__ constexpr int scratch_floats(int kind) { return P_FLOATS + SC_FLOATS + (kind == LIGHTNING ? QK_FLOATS : 0); }
+enum { MAMBA = 0, LIGHTNING = 1, MEMORY = 2, CHANNEL = 3 };
+// scratch of a chunk and head: P, the scales, and for LIGHTNING the activated q and k; CHANNEL: P, the chunk's decay of every
+// channel, and the weighted q and k
+__host__ __device__ constexpr bool keeps_qk(int kind) { return kind == LIGHTNING || kind == CHANNEL; }
+__host__ __device__ constexpr int scratch_floats(int kind) { return P_FLOATS + SC_FLOATS + (keeps_qk(kind) ? QK_FLOATS : 0); }
+static_assert(SC_FLOATS == DMAX, "a chunk's decays of all channels take the place of the scales");
 
 __device__ __forceinline__ float silu(float z) { return z / (1.0f + expf(-z)); }
 __device__ __forceinline__ float4 silu4(float4 z) { return make_float4(silu(z.x), silu(z.y), silu(z.z), silu(z.w)); }
@@ -41,7 +45,7 @@ __device__ __forceinline__ float4 silu4(float4 z) { return make_float4(silu(z.x)
 struct Args {
   const float* proj;      // rows of ld: q, k and v at their columns
   int ld, q_col, k_col, v_col;
-  const float* gates;     // MAMBA: raw dt, rows of ld_gates; MEMORY: [T][H][4] of a, b, exp(-m)
+  const float* gates;     // MAMBA: raw dt, rows of ld_gates; MEMORY: [T][H][4] of a, b, exp(-m); CHANNEL: [T][H d] of a
   int ld_gates;
   const float* rate;      // MAMBA: A_log [H]; LIGHTNING: a [H]
   const float* bias;      // MAMBA: dt_bias [H]
@@ -62,15 +66,8 @@ struct Args {
 // sequence after another: floor(q_start / C) + seq begins at or past the end of the sequence before.
 __device__ __forceinline__ int first_slot(const Args& a, int seq) { return a.packed ? a.q_start[seq] / C + seq : seq * a.tiles; }
 
-template <int KIND>
-__global__ void __launch_bounds__(THREADS) state_prepare_kernel(const Args a) {
-  __shared__ __align__(16) float q_s[C][LD], k_s[C][LD];
-  __shared__ float qk_s[C][C + 1];
-  jb::pdl_launch_dependents();
-  const int R = a.H / a.G, j = blockIdx.y;
-  const int h_begin = j * R + (int)blockIdx.z * a.heads_here, h_end = min((j + 1) * R, h_begin + a.heads_here);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  jb::pdl_wait();
+// The chunk of a block of a prepare kernel: its first token and how many it has (none: n <= 0).
+__device__ __forceinline__ void find_chunk(const Args& a, int& t0, int& n) {
   int seq = (int)blockIdx.x / a.tiles, tile = (int)blockIdx.x % a.tiles;
   if (a.packed) {                                              // the last sequence whose chunks begin up to here
     seq = -1;
@@ -80,7 +77,20 @@ __global__ void __launch_bounds__(THREADS) state_prepare_kernel(const Args a) {
     }
     tile = (int)blockIdx.x - first_slot(a, seq);
   }
-  const int t0 = a.q_start[seq] + (a.first_tile + tile) * C, n = min(C, a.q_start[seq + 1] - t0);
+  t0 = a.q_start[seq] + (a.first_tile + tile) * C, n = min(C, a.q_start[seq + 1] - t0);
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(THREADS) state_prepare_kernel(const Args a) {
+  __shared__ __align__(16) float q_s[C][LD], k_s[C][LD];
+  __shared__ float qk_s[C][C + 1];
+  jb::pdl_launch_dependents();
+  const int R = a.H / a.G, j = blockIdx.y;
+  const int h_begin = j * R + (int)blockIdx.z * a.heads_here, h_end = min((j + 1) * R, h_begin + a.heads_here);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  jb::pdl_wait();
+  int t0, n;
+  find_chunk(a, t0, n);
   if (n <= 0) return;
   const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   float4 qv[4], kv[4];
@@ -166,6 +176,109 @@ __global__ void __launch_bounds__(THREADS) state_prepare_kernel(const Args a) {
   }
 }
 
+// CHANNEL.  Products of decays stand where the other kinds have exponentials of sums: along the tokens, as a walk makes them, so
+// that decays of zero, below zero and not a number need no case, and nothing is divided by.  q_t goes with the product from
+// the chunk's start to its own token, k_t with the one from the next token to the chunk's end, both products in float64.
+// P[t][s] = scale q_t . (k_s times what lies between): half a warp owns a token s (and then 31 - s, so that all warps have as
+// much to do), eight channels a lane, and takes its k along the later tokens; from the end of its four tokens on by products of
+// the four and of their first ones, made in float64 too, which leaves twelve roundings where token by token there were 31.
+// Four tokens' sums meet in five shuffles.  Eight sequences of 40 to 511 tokens, 16 heads of 128 x 128: 435 us as segments walked
+// token by token, 214 by chunks, one of 256 tokens 104 and 62; errors against float64, relative to all outputs and to the state,
+// 1.14e-7 and 7.8e-8 by the walk, 1.10e-7 to 1.12e-7 and 7.2e-8 to 7.9e-8 so (1.21e-7 and 9.9e-8 with float32 products throughout).
+constexpr int CHANNEL_SMEM = (3 * C * DMAX + C * (C + 4)) * 4;
+__global__ void __launch_bounds__(THREADS) channel_prepare_kernel(const Args a) {
+  extern __shared__ __align__(16) float smem[];
+  float(*q_s)[DMAX] = reinterpret_cast<float(*)[DMAX]>(smem), (*k_s)[DMAX] = q_s + C, (*a_s)[DMAX] = k_s + C;
+  float* P_s = smem + 3 * C * DMAX;
+  jb::pdl_launch_dependents();
+  const int h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  jb::pdl_wait();
+  int t0, n;
+  find_chunk(a, t0, n);
+  if (n <= 0) return;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {                                // past the sequence's end and the keys': nothing, kept as it is
+    const int t = 4 * warp + u;
+    const bool in = t < n && 4 * lane < a.d;
+    const size_t row = (size_t)(t0 + (in ? t : 0)), c = (size_t)h * a.d + (in ? 4 * lane : 0);
+    float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f), k = q, w = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    if (in) {
+      q = *reinterpret_cast<const float4*>(a.proj + row * a.ld + a.q_col + c);
+      k = *reinterpret_cast<const float4*>(a.proj + row * a.ld + a.k_col + c);
+      w = *reinterpret_cast<const float4*>(a.gates + row * a.ld_gates + c);
+    }
+    *reinterpret_cast<float4*>(&q_s[t][4 * lane]) = make_float4(q.x * a.scale, q.y * a.scale, q.z * a.scale, q.w * a.scale);
+    *reinterpret_cast<float4*>(&k_s[t][4 * lane]) = k;
+    *reinterpret_cast<float4*>(&a_s[t][4 * lane]) = w;
+  }
+  __syncthreads();
+  float* P_g = a.scratch + ((size_t)blockIdx.x * a.H + h) * scratch_floats(CHANNEL);
+  float* Q_g = P_g + P_FLOATS + SC_FLOATS;
+  const int g = lane & 15, half = lane >> 4;
+  const int first[2] = {2 * warp, 30 - 2 * warp}, own[2] = {2 * warp + half, 31 - 2 * warp - half};
+  ulonglong2 r[2][2];                                          // k of the two tokens: channels 4 g and on, 64 + 4 g and on
+#pragma unroll
+  for (int p = 0; p < 2; ++p)
+#pragma unroll
+    for (int y = 0; y < 2; ++y) r[p][y] = *reinterpret_cast<const ulonglong2*>(&k_s[own[p]][64 * y + 4 * g]);
+  __syncthreads();                                             // k's place is taken below
+  {
+    const int c = threadIdx.x & (DMAX - 1);
+    double w = 1.0;
+    if (threadIdx.x < DMAX) {
+#pragma unroll 8
+      for (int t = 0; t < C; ++t) w *= a_s[t][c], Q_g[t * DMAX + c] = (float)(q_s[t][c] * w);
+      P_g[P_FLOATS + c] = (float)w;
+    } else {
+#pragma unroll 2
+      for (int t = C - 4; t >= 0; t -= 4) {
+        double four[4];                                        // decays, then their products from the first of the four
+#pragma unroll
+        for (int u = 3; u >= 0; --u) four[u] = a_s[t + u][c], Q_g[(C + t + u) * DMAX + c] = (float)(k_s[t + u][c] * w), w *= four[u];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) four[u] = u > 0 ? four[u - 1] * four[u] : four[0], k_s[t + u][c] = (float)four[u];
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    const int s = own[p];
+    for (int tb = first[p] & ~3; tb < C; tb += 4) {
+      float sum[4];
+      const bool here = tb <= s;                               // s is one of the four (of all the warp, or of none)
+      ulonglong2 now[2] = {r[p][0], r[p][1]};
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int t = tb + u;
+        jb::Pair acc = 0;
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+          const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(&(here ? a_s : k_s)[t][64 * y + 4 * g]);
+          const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(&q_s[t][64 * y + 4 * g]);
+          const ulonglong2 from = here ? now[y] : r[p][y];
+          if (t > s) now[y] = make_ulonglong2(jb::mul2(from.x, w.x), jb::mul2(from.y, w.y));
+          acc = jb::fma2(q.y, now[y].y, jb::fma2(q.x, now[y].x, acc));
+        }
+        sum[u] = jb::lo(acc) + jb::hi(acc);
+      }
+      r[p][0] = now[0], r[p][1] = now[1];
+      const bool up8 = g & 8, up4 = g & 4;
+      float x = (up8 ? sum[2] : sum[0]) + __shfl_xor_sync(0xffffffffu, up8 ? sum[0] : sum[2], 8);
+      const float y = (up8 ? sum[3] : sum[1]) + __shfl_xor_sync(0xffffffffu, up8 ? sum[1] : sum[3], 8);
+      x = (up4 ? y : x) + __shfl_xor_sync(0xffffffffu, up4 ? x : y, 4);
+      x += __shfl_xor_sync(0xffffffffu, x, 2);
+      x += __shfl_xor_sync(0xffffffffu, x, 1);
+      if ((g & 3) == 0) P_s[(tb + (g >> 2)) * (C + 4) + s] = x;
+    }
+  }
+  __syncthreads();
+  const int t = threadIdx.x >> 3, s = (threadIdx.x & 7) * 4;   // what lies above the diagonal is not there (and may be old)
+  float4 x = *reinterpret_cast<const float4*>(P_s + t * (C + 4) + s);
+  x.x = s <= t ? x.x : 0.0f, x.y = s + 1 <= t ? x.y : 0.0f, x.z = s + 2 <= t ? x.z : 0.0f, x.w = s + 3 <= t ? x.w : 0.0f;
+  *reinterpret_cast<float4*>(P_g + t * C + s) = x;
+}
+
 // copies 16 bytes, or zeros
 __device__ __forceinline__ void async16(float* dst, const float* src, bool in) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
@@ -220,7 +333,7 @@ __global__ void __launch_bounds__(128 * SPLIT, 4 / SPLIT) state_chunks_kernel(co
     const int t0 = begin + chunk * C, n = min(C, n_all - chunk * C);
     for (int i = tid; i < C * D / 4; i += THREADS) {
       const int t = i / (D / 4), r = (i % (D / 4)) * 4;
-      if (KIND == LIGHTNING) {
+      if (keeps_qk(KIND)) {
         async16(dst + t * LDD + r, scratch_g + chunk * per_chunk + P_FLOATS + SC_FLOATS + (which * C + t) * DMAX + r, true);
       } else {
         const bool in = t < n && r < d;
@@ -248,7 +361,7 @@ __global__ void __launch_bounds__(128 * SPLIT, 4 / SPLIT) state_chunks_kernel(co
   auto fetch_v = [&](int chunk) {
     const bool in = vt < n_all - chunk * C;
     const float* row = a.proj + (size_t)(begin + chunk * C + (in ? vt : 0)) * a.ld + a.v_col + (size_t)h * e;
-    v_scale = chunk < chunks ? scratch_g[chunk * per_chunk + P_FLOATS + 4 * vt + 1] : 0.0f;
+    v_scale = KIND == CHANNEL ? 1.0f : chunk < chunks ? scratch_g[chunk * per_chunk + P_FLOATS + 4 * vt + 1] : 0.0f;
 #pragma unroll
     for (int i = 0; i < COLS / (2 * VL); ++i) {
       const int c = c0 + 2 * VL * i + vc;
@@ -331,7 +444,7 @@ __global__ void __launch_bounds__(128 * SPLIT, 4 / SPLIT) state_chunks_kernel(co
 #pragma unroll 2
       for (int k = part * (D / SPLIT); k < (part + 1) * (D / SPLIT); k += 4) step(q_s + k, LDD, S_s + (k >> 1) * SLD);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < 4 && KIND != CHANNEL; ++i) {                     // (CHANNEL: q has its scale)
         const float s = sc_s[tg + 8 * i].x;
         const jb::Pair ss = jb::pair(s, s);
 #pragma unroll
@@ -390,8 +503,8 @@ __global__ void __launch_bounds__(128 * SPLIT, 4 / SPLIT) state_chunks_kernel(co
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
           const ulonglong2 old = *reinterpret_cast<const ulonglong2*>(S_s + ((ur >> 1) + p) * SLD + 2 * (uc + 16 * x));
-          S[p][2 * x] = jb::mul2(old.x, g);
-          S[p][2 * x + 1] = jb::mul2(old.y, g);
+          S[p][2 * x] = KIND == CHANNEL ? 0 : jb::mul2(old.x, g);          // (CHANNEL: the chunk's sum by itself, see the end)
+          S[p][2 * x + 1] = KIND == CHANNEL ? 0 : jb::mul2(old.y, g);
         }
 #pragma unroll 4
       for (int t = 0; t < C; ++t) {
@@ -414,8 +527,15 @@ __global__ void __launch_bounds__(128 * SPLIT, 4 / SPLIT) state_chunks_kernel(co
 #pragma unroll
       for (int p = 0; p < RT / 2; ++p)
 #pragma unroll
-        for (int x = 0; x < 2; ++x)
-          *reinterpret_cast<ulonglong2*>(S_s + ((ur >> 1) + p) * SLD + 2 * (uc + 16 * x)) = make_ulonglong2(S[p][2 * x], S[p][2 * x + 1]);
+        for (int x = 0; x < 2; ++x) {
+          ulonglong2* at = reinterpret_cast<ulonglong2*>(S_s + ((ur >> 1) + p) * SLD + 2 * (uc + 16 * x));
+          if (KIND == CHANNEL) {                                           // two channels' decays
+            const jb::Pair both = reinterpret_cast<const jb::Pair*>(sc_s)[(ur >> 1) + p];
+            const ulonglong2 old = *at;
+            S[p][2 * x] = jb::fma2(old.x, both, S[p][2 * x]), S[p][2 * x + 1] = jb::fma2(old.y, both, S[p][2 * x + 1]);
+          }
+          *at = make_ulonglong2(S[p][2 * x], S[p][2 * x + 1]);
+        }
     }
     if (has_n && tid < D) {                                                // n <- decay n + the sum of b k
       float s = n_s[tid] * sc_s[0].z;
@@ -477,6 +597,9 @@ template <int KIND, int D, int SPLIT>
 int launch(Args a, int max_q_len, int tokens, cudaStream_t stream) {
   constexpr int smem = chunk_smem<KIND, D, SPLIT>();
   cudaError_t e = cudaFuncSetAttribute(state_chunks_kernel<KIND, D, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  constexpr int prepare_smem = KIND == CHANNEL ? CHANNEL_SMEM : 0;
+  if (e == cudaSuccess && KIND == CHANNEL)
+    e = cudaFuncSetAttribute(channel_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CHANNEL_SMEM);
   if (e != cudaSuccess) return (int)e;
   const int group = a.H / a.G;
   // a block makes the products of a chunk and key head once for its group's heads, or for a share of them where that
@@ -487,8 +610,8 @@ int launch(Args a, int max_q_len, int tokens, cudaStream_t stream) {
   parts = parts < group ? parts : group;
   a.heads_here = (group + parts - 1) / parts;
   for (a.first_tile = 0; a.first_tile * C < max_q_len; a.first_tile += a.tiles) {
-    jb::Launch prepare(dim3(slots, a.G, (group + a.heads_here - 1) / a.heads_here), dim3(THREADS), 0, stream);
-    e = cudaLaunchKernelEx(&prepare.c, state_prepare_kernel<KIND>, a);
+    jb::Launch prepare(dim3(slots, a.G, (group + a.heads_here - 1) / a.heads_here), dim3(THREADS), prepare_smem, stream);
+    e = cudaLaunchKernelEx(&prepare.c, KIND == CHANNEL ? channel_prepare_kernel : state_prepare_kernel<KIND == CHANNEL ? MAMBA : KIND>, a);
     if (e != cudaSuccess) return (int)e;
     jb::Launch walk(dim3((a.e + COLS - 1) / COLS, a.H, a.n_seqs), dim3(128 * SPLIT), smem, stream);
     e = cudaLaunchKernelEx(&walk.c, state_chunks_kernel<KIND, D, SPLIT>, a);
@@ -499,8 +622,8 @@ int launch(Args a, int max_q_len, int tokens, cudaStream_t stream) {
 
 }  // namespace
 
-// kind: 0 state-space (MAMBA), 1 LIGHTNING, 2 matrix MEMORY, see the top.  d <= 128; d, ld, q_col and k_col multiples of 4,
-// proj and scratch 16-byte aligned.  `scratch` (H * 1152 floats a chunk, LIGHTNING H * 9344) holds `tiles` chunks of every
+// kind: 0 state-space (MAMBA), 1 LIGHTNING, 2 matrix MEMORY, 3 a decay a CHANNEL, see the top.  d <= 128; d, ld, q_col and k_col multiples of 4,
+// proj and scratch 16-byte aligned.  `scratch` (H * 1152 floats a chunk, LIGHTNING and CHANNEL H * 9344) holds `tiles` chunks of every
 // sequence; longer prompts go in slabs of as many, one after another from the state the last left.  tiles = 0: it holds
 // tokens / 32 + n_seqs chunks, the whole step's, one sequence after another (`tokens`: of all sequences).
 JB_EXPORT int jb_state_chunks(int kind, const float* proj, int ld, int q_col, int k_col, int v_col, const float* gates,
@@ -511,13 +634,15 @@ JB_EXPORT int jb_state_chunks(int kind, const float* proj, int ld, int q_col, in
   if (n_seqs <= 0 || max_q_len <= 0) return 0;
   JB_REFUSE(d < 1 || d > DMAX || e < 1 || ((d | ld | q_col | k_col) & 3) != 0 || (((uintptr_t)proj | (uintptr_t)scratch) & 15) != 0,
             "state_chunks: keys of %d numbers in rows of %d at columns %d and %d", d, ld, q_col, k_col);
-  JB_REFUSE(G < 1 || H % G != 0 || tiles < 0 || (kind == LIGHTNING && G != H), "state_chunks: %d heads, %d key heads, %d tiles", H, G, tiles);
+  JB_REFUSE(G < 1 || H % G != 0 || tiles < 0 || (keeps_qk(kind) && G != H), "state_chunks: %d heads, %d key heads, %d tiles", H, G, tiles);
   const Args a{proj, ld, q_col, k_col, v_col, gates, ld_gates, rate, bias, skip, scale, out, den, state, slot_stride, state_off,
                q_start, seq_slot, H, G, d, e, scratch, n_seqs, 0, tiles > 0 ? tiles : (max_q_len + C - 1) / C, 0, tiles == 0};
   const bool few = (long long)n_seqs * H * ((e + COLS - 1) / COLS) <= 148;           // no SM has a second block
   const auto run = [&](auto small, auto large, auto alone) { return (d <= 64 ? small : few ? alone : large)(a, max_q_len, tokens, stream); };
   if (kind == MAMBA) return run(launch<MAMBA, 64, 2>, launch<MAMBA, 128, 2>, launch<MAMBA, 128, 4>);
   if (kind == LIGHTNING) return run(launch<LIGHTNING, 64, 2>, launch<LIGHTNING, 128, 2>, launch<LIGHTNING, 128, 4>);
+  JB_REFUSE(kind == CHANNEL && ((ld_gates & 3) != 0 || ((uintptr_t)gates & 15) != 0), "state_chunks: decays in rows of %d", ld_gates);
+  if (kind == CHANNEL) return run(launch<CHANNEL, 64, 2>, launch<CHANNEL, 128, 2>, launch<CHANNEL, 128, 4>);
   JB_REFUSE(kind != MEMORY, "state_chunks: kind %d", kind);
   return run(launch<MEMORY, 64, 2>, launch<MEMORY, 128, 2>, launch<MEMORY, 128, 4>);
 }

@@ -1165,7 +1165,8 @@ STATE_SCRATCH_BYTES = 512 << 20
 SINGLES_BLOCKS = 592                  # blocks up to which sequences of a token or two are no burden
 _STATE_KINDS = {"mamba": (0, STATE_CHUNK * (STATE_CHUNK + 4)),
                 "lightning": (1, STATE_CHUNK * (STATE_CHUNK + 4 + 256)),      # and the activated queries and keys
-                "memory": (2, STATE_CHUNK * (STATE_CHUNK + 4))}
+                "memory": (2, STATE_CHUNK * (STATE_CHUNK + 4)),
+               "channel": (3, STATE_CHUNK * (STATE_CHUNK + 4 + 256))}         # and the weighted queries and keys
 
 
 def _chunk_slots(n_seqs: int, tokens: int, max_q_len: int, chunk: int, bytes_per_slot: int, most: int):
@@ -1197,7 +1198,9 @@ def state_chunks_pay(kind: str, n_seqs: int, heads: int, dim: int, vdim: int, ma
     and 111; two sequences (64) of 1,024 tokens 165 and 207, three (96) 221 and 209, lengths of 1,000, 700, 400 and 100 201
     and 212, two beside 30 single tokens 392 and 304; 128 heads, 4,096 beside 31 1,607 and 1,272.  Keys of at most 64
     numbers, whose blocks stay small: 64 tokens 25 and 24, 128 tokens 46 and 31; 128 blocks of 2,048 tokens 388 and 453, 256
-    blocks 738 and 472."""
+    blocks 738 and 472.  A decay a channel has the same lines; 16 heads of 128 x 128: one sequence of 64 tokens 31 and 28, 256
+    104 and 62, 512 113 and 108, 1,024 141 and 200; two of 512 147 and 116, four of 1,024 462 and 251, eight 1,222 and 445, of
+    40 to 511 tokens 435 and 214; 64 of 16 tokens 84 and 157."""
     if max_q_len < STATE_CHUNKS_FROM[dim <= 64] or dim > 128:
         return False
     blocks, line = heads * -(-vdim // 64), 148 if dim <= 64 else 96 if kind == "mamba" else 64          # blocks of a sequence
@@ -1217,6 +1220,8 @@ def _state_chunks(kind: str, workspace, proj: torch.Tensor, q_col: int, k_col: i
     if workspace is None or not state_chunks_pay(kind, n_seqs, heads, dim, vdim, max_q_len, tokens):
         return False
     if any(x % 4 for x in (dim, proj.shape[1], q_col, k_col)) or proj.data_ptr() % 16:
+        return False
+    if kind == "channel" and gates.data_ptr() % 16:
         return False
     code, per_head = _STATE_KINDS[kind]
     slots, tiles = _chunk_slots(n_seqs, tokens, max_q_len, STATE_CHUNK, 4 * per_head * heads, STATE_SCRATCH_BYTES)
@@ -2075,8 +2080,8 @@ def gated_linear_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, q_
     [T, heads dim], a decay per key channel, b = 1, and a slot's state row holds [heads, dim, vdim].  With `divisors`
     (float32 [T, heads], written), `decays` is what `exp_gates` left ([T, heads, 4]: a_t and b_t one number a head),
     a normalizer n <- a_t n + b_t k_t walks along, divisors[t, h] = max(|n . q|, exp(-m_t)) + 1e-6, and a slot's state
-    row holds per head [dim, vdim] then [dim] of n.  With a workspace, prompts with `divisors` go by chunks of tokens where
-    that pays; else steps whose longest sequence brings more than 256 tokens run in passes over segments of 64 to 256
+    row holds per head [dim, vdim] then [dim] of n.  With a workspace, prompts go by chunks of tokens where that
+    pays; else steps whose longest sequence brings more than 256 tokens run in passes over segments of 64 to 256
     tokens (4 launches); else one launch.  `single_tokens`: every
     sequence brings one token (the state is read and written once)."""
     T = proj.shape[0]
@@ -2096,9 +2101,9 @@ def gated_linear_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, q_
         raise KernelError("gated_linear_scan: the projections' columns reach past the rows")
     if single_tokens and T != n_seqs:
         raise KernelError("gated_linear_scan: single_tokens needs one token per sequence")
-    if scalar and not single_tokens and _state_chunks("memory", workspace, proj, q_col, k_col, v_col, decays, 0, None, None, None,
-                                                      q_scale, out, divisors, state, state.shape[1], 0, q_start, seq_slot,
-                                                      n_seqs, heads, heads, dim, vdim, max_q_len):
+    if not single_tokens and _state_chunks("memory" if scalar else "channel", workspace, proj, q_col, k_col, v_col, decays,
+                                           0 if scalar else heads * dim, None, None, None, q_scale, out, divisors, state,
+                                           state.shape[1], 0, q_start, seq_slot, n_seqs, heads, heads, dim, vdim, max_q_len):
         return
     seg, scratch, seg_decay = -1 if single_tokens else 0, None, None
     if workspace is not None and max_q_len > 2 * GATED_LINEAR_SEGMENT and not single_tokens:

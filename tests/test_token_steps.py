@@ -254,3 +254,95 @@ def test_conv_taps_off_their_vectors(ops, T):
         ops.conv_rope_cache(proj, w, 4, state, seq, ints(0, T), ints(0), pos, table, rot, q, pos, k_cache, v_cache, H, G, d, e, page)
         results.append((q, k_cache, v_cache))
     assert all(torch.equal(a, b) for a, b in zip(*results)) and results[0][0].abs().max() > 0
+
+
+class Scratch:
+    """A workspace whose buffers come filled with NaN, and what was asked for."""
+
+    def __init__(self):
+        self.asked = []
+
+    def get(self, name, shape, dtype):
+        self.asked.append(name)
+        return torch.full(shape, float("nan"), dtype=dtype, device=DEV)
+
+
+def channel_walk(q, k, v, a, lens, S):
+    """The recurrence with a decay a channel in the numbers' own type: (outputs [T, H, e], states [n, H, d, e])."""
+    out, states, at = [], [], 0
+    for n, s in zip(lens, S):
+        for t in range(at, at + n):
+            s = a[t, :, :, None] * s + k[t, :, :, None] * v[t, :, None, :]
+            out.append(torch.einsum("hde,hd->he", s, q[t]))
+        states.append(s)
+        at += n
+    return torch.stack(out), torch.stack(states)
+
+
+@pytest.mark.parametrize("H, d, e, lens", [(2, 128, 64, [64]), (3, 100, 68, [33, 1, 130]), (1, 4, 10, [31, 65, 32]), (2, 64, 128, [97, 200]),
+                                           (16, 128, 128, [70] * 10), (5, 128, 65, [1] * 40 + [161])])
+@pytest.mark.parametrize("decays", ["mild", "strong", "any"])
+def test_channel_chunks(ops, monkeypatch, H, d, e, lens, decays):
+    """Prompts by chunks of 32 tokens with a decay a key channel: parts of a chunk, several sequences, one block an SM and two,
+    columns that are no pairs, decays that are zero or below it, and the scratch in slabs.  An output's error is at most a
+    rounding for each factor on the way to it, of the sum of its terms' sizes."""
+    g = torch.Generator().manual_seed(H * 1000 + d + e)
+    T, n, col = sum(lens), len(lens), 8
+    proj = rnd(g, T, col + H * (2 * d + e) + (-(2 * H * d + H * e)) % 4)
+    a = torch.rand(T, H * d, generator=g)
+    a = 1 - 0.05 * a if decays == "mild" else a
+    if decays == "any":
+        a = (a * 2 - 1) * (torch.rand(T, H * d, generator=g) > 0.02)
+    before, scale = rnd(g, n + 1, H * d * e), d ** -0.5
+    slots = torch.randperm(n + 1, generator=g)[:n]
+    q_start = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist())
+    parts = [proj[:, col: col + H * d].view(T, H, d) * scale, proj[:, col + H * d: col + 2 * H * d].view(T, H, d),
+             proj[:, col + 2 * H * d: col + 2 * H * d + H * e].view(T, H, e), a.view(T, H, d)]
+    S = before[slots].view(n, H, d, e)
+    want, states = channel_walk(*(x.double() for x in parts), lens, S.double())
+    size, state_size = channel_walk(*(x.double().abs() for x in parts), lens, S.double().abs())
+    monkeypatch.setattr(ops, "state_chunks_pay", lambda *_: True)
+    for most in (ops.STATE_SCRATCH_BYTES, 1):                           # all chunks at once, and one of every sequence after another
+        monkeypatch.setattr(ops, "STATE_SCRATCH_BYTES", most)
+        out, state, ws = torch.full((T, H * e), float("nan"), device=DEV), before.to(DEV), Scratch()
+        ops.gated_linear_scan(proj.to(DEV), col, col + H * d, col + 2 * H * d, scale, a.to(DEV), out, state, q_start.int().to(DEV),
+                              slots.int().to(DEV), n, H, d, e, max(lens), ws)
+        assert ws.asked == ["state_chunks"]
+        bound = (d + 2 * max(lens) + 40) * 2.0 ** -24
+        assert ((out.cpu().double().view(T, H, e) - want).abs() <= bound * size + 1e-30).all()
+        got = state.cpu()[slots].double().view(n, H, d, e)
+        assert ((got - states).abs() <= bound * state_size + 1e-30).all()
+        rest = [s for s in range(n + 1) if s not in slots.tolist()]
+        assert torch.equal(state.cpu()[rest], before[rest])
+
+
+@pytest.mark.parametrize("what", ["value", "decay", "key"])
+def test_channel_chunks_that_are_not_finite(ops, monkeypatch, what):
+    """A value, a decay or a key that is not finite shows from its token on, in its column or its head, and nowhere else, by
+    chunks as by the walk."""
+    g = torch.Generator().manual_seed(3)
+    H, d, e, lens, bad = 2, 128, 64, [200, 70], 77
+    T, per = sum(lens), 128 * 64
+    ints = lambda *v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    proj, before, a = rnd(g, T, H * (2 * d + e)).to(DEV), rnd(g, 2, H * per).to(DEV), torch.rand(T, H * d, generator=g).to(DEV)
+    monkeypatch.setattr(ops, "state_chunks_pay", lambda *_: True)
+    for ws in (Scratch(), None):
+        results = []
+        for sick in (True, False):
+            x, w, out, state = proj.clone(), a.clone(), torch.zeros(T, H * e, device=DEV), before.clone()
+            if sick:
+                if what == "value":
+                    x[bad, 2 * H * d + 3] = float("inf")
+                elif what == "key":
+                    x[bad, H * d + 5] = float("inf")
+                else:
+                    w[bad, 5] = float("nan")
+            ops.gated_linear_scan(x, 0, H * d, 2 * H * d, 1.0, w, out, state, ints(0, 200, T), ints(1, 0), 2, H, d, e, 200, ws)
+            results.append((out.view(T, H, e), state.view(2, H, d, e)))
+        (got, state), (clean, clean_state) = results
+        columns = slice(3, 4) if what == "value" else slice(0, e)
+        assert not torch.isfinite(got[bad:200, 0, columns]).any()
+        got[bad:200, 0, columns] = clean[bad:200, 0, columns]
+        assert torch.equal(got, clean)
+        assert not torch.isfinite(state[1, 0, :, columns] if what == "value" else state[1, 0, 5]).any()
+        assert torch.equal(state[0], clean_state[0]) and torch.equal(state[1, 1], clean_state[1, 1])
