@@ -100,7 +100,7 @@ class ParallelMixers(Mixer):
 
     def _buffers(self, ctx, tokens: int):
         """The branches' buffers [2, tokens, hidden_size], the shared product's result or None, and what of both has to
-        be zero."""
+        be zero: the product's result too where it lies behind the buffers on a 16-byte boundary, else it is cleared by itself."""
         out = 2 * tokens * self.hidden_size
         if self.proj is None:
             buf = ctx.workspace.get("parallel_branches", (out,), torch.float32)
@@ -126,7 +126,7 @@ class ParallelMixers(Mixer):
             for i, b in enumerate(self.branches.values()):
                 b.forward(x, buf[i], ctx, cache_view, writes_cache)
         else:
-            self.proj.forward(x, proj, y_is_zero=True)          # (zero only where slices of K meet in it)
+            self.proj.forward(x, proj, y_is_zero=to_clear.numel() > buf.numel())
             col = 0
             for i, b in enumerate(self.branches.values()):
                 b.forward(x, buf[i], ctx, cache_view, writes_cache, projected=(proj, col))
