@@ -142,6 +142,8 @@ class CappedAttention(Mixer):
                 raise ValueError(f"a share of the first values of shape {tuple(vmix.shape)} is not one number")
             self.vmix = float(vmix)
 
+    projects_first = True         # a wider matrix has this part's projections as its first columns
+
     @property
     def shares_projection(self) -> bool:
         """Whether `forward` takes the projections as the first columns of a wider matrix that lasts as long as the call."""

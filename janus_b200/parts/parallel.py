@@ -10,7 +10,8 @@ state of fixed size, so that a place of the cache serves both.  Each adds its ou
 its own; one launch norms, weighs and adds both into the sublayer's output and leaves the buffers zeroed.
 
 Where both branches can read their projections from columns of a wider matrix (`shares_projection`), one product makes
-the rows of both: their weights are stacked, the left branch's first.  A single token's step of a width of 2,048 spends
+the rows of both: their weights are stacked, the left branch's first unless the right one reads a matrix's first columns
+only (`projects_first`).  A single token's step of a width of 2,048 spends
 as long on the start, the end and the cleared result of such a product as on its weights (16 heads of attention beside
 16 of the delta rule, four layers: 12 launches and 12 us of 375 less a step).  The branches' buffers and, where the
 product adds slices of K, its result lie side by side, so that the launch before this mixer clears all of it at once.
@@ -54,10 +55,13 @@ class ParallelMixers(Mixer):
         self.w = {"left": None, "right": None}
         self.proj: Optional[Linear] = None
         branches = list(self.branches.values())
+        heads_the_rows = [getattr(b, "projects_first", False) for b in branches]
         # (rows and both branches' first columns on whole 16-byte vectors, as if the matrix were each one's own)
-        if all(getattr(b, "shares_projection", False) and b.proj.out_features % 4 == 0 for b in branches):
-            rows = sum(b.proj.out_features for b in branches)
-            self.proj = Linear(hidden_size, rows, dtype, device, name="both", pad_width=True)
+        if (all(getattr(b, "shares_projection", False) and b.proj.out_features % 4 == 0 for b in branches)
+                and not all(heads_the_rows)):
+            n = [b.proj.out_features for b in branches]
+            self.columns = [n[1], 0] if heads_the_rows[1] else [0, n[0]]       # where each branch's rows begin
+            self.proj = Linear(hidden_size, sum(n), dtype, device, name="both", pad_width=True)
             for b in branches:
                 b.proj = _StackedRows(b.proj)
 
@@ -93,7 +97,7 @@ class ParallelMixers(Mixer):
                 raise TypeError("mixers side by side without branch norms take no branch weights")
             self.branches[side].load(**{n[len(side) + 1:]: v for n, v in tensors.items() if n.startswith(side + ".")})
         if self.proj is not None:
-            stacked = [b.proj for b in self.branches.values()]
+            stacked = [b.proj for _, b in sorted(zip(self.columns, self.branches.values()), key=lambda p: p[0])]
             self.proj.load([t for rows in stacked for t in rows.tensors])
             for rows in stacked:
                 rows.tensors = None
@@ -127,10 +131,8 @@ class ParallelMixers(Mixer):
                 b.forward(x, buf[i], ctx, cache_view, writes_cache)
         else:
             self.proj.forward(x, proj, y_is_zero=to_clear.numel() > buf.numel())
-            col = 0
             for i, b in enumerate(self.branches.values()):
-                b.forward(x, buf[i], ctx, cache_view, writes_cache, projected=(proj, col))
-                col += b.proj.out_features
+                b.forward(x, buf[i], ctx, cache_view, writes_cache, projected=(proj, self.columns[i]))
         ops.join_norm(residual, ya=buf[0], yb=buf[1], wa=self.w["left"], wb=self.w["right"], mult=self.left_mult,
                       mult_b=self.right_mult, eps=self.eps)
 
