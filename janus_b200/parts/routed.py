@@ -7,7 +7,7 @@ weight multiplies the expert's INPUT: out = sum over the chosen e of expert_e(s_
 
 Steps of few (token, expert) pairs, every single-token step among them, stream the chosen experts' packed tiles once for
 up to 64 tokens (`ops.experts_stream`: width and inner width multiples of 128).  Other widths, more tokens and
-deterministic runs stream each chosen expert's rows once for up to 16 of the tokens that chose it
+deterministic runs (in which a token's experts are added in order) stream each chosen expert's rows once for up to 16 of the tokens that chose it
 (`ops.experts_few_tokens_tc`: two launches with a block per (rows, expert); widths that are no multiples
 of 32, and the float32 engine, take up to four tokens at a time on the CUDA cores, `ops.experts_few_tokens`).  Sums are
 float32 and nothing is read back by the host, so the step can be recorded into a CUDA graph.  Prompt steps of the
@@ -42,6 +42,7 @@ from .linear import GatedLinear, Linear
 
 FEW_PAIRS = 64           # up to this many (token, expert) pairs a bfloat16 prompt step streams the experts' rows
 MAX_STREAM_PAIRS = 65535  # pairs of one launch of the streaming kernels
+IN_ORDER_PAIRS = 8192    # pairs whose results deterministic runs keep at a time
 
 
 class RoutedExperts(FeedForward):
@@ -197,18 +198,42 @@ class RoutedExperts(FeedForward):
             else:
                 self._by_expert(x, sel_e, sel_w, residual, ctx)
             return
+        if ops.is_deterministic() and self.top > 1:
+            self._in_order(x, sel_e, sel_w, residual, ctx)
+        else:
+            self._few(x, sel_e, sel_w, residual, ctx)
+
+    def _few(self, x: torch.Tensor, sel_e: torch.Tensor, sel_w: torch.Tensor, out: torch.Tensor, ctx) -> None:
+        """Each chosen expert's rows streamed once for several of its tokens; a token's experts add into `out` as they finish."""
+        ws = ctx.workspace
+        (T, top), F = sel_e.shape, self.intermediate_size
         if self.streams_on_tensor_cores:
-            act = ws.get("experts_act_rows", (pairs, self.intermediate_size), self.dtype)
-            ops.experts_few_tokens_tc(x, sel_e, sel_w, self.w_gate, self.w_up, self.w_down, act, residual,
+            act = ws.get("experts_act_rows", (T * top, F), self.dtype)
+            ops.experts_few_tokens_tc(x, sel_e, sel_w, self.w_gate, self.w_up, self.w_down, act, out,
                                       weight_on_output=self.weight_on_output)
             return
-        act = ws.get("experts_act", (pairs, self.intermediate_size), torch.float32)
-        rows = max(1, MAX_STREAM_PAIRS // self.top)
+        act = ws.get("experts_act", (T * top, F), torch.float32)
+        rows = max(1, MAX_STREAM_PAIRS // top)
         for t0 in range(0, T, rows):
             t1 = min(T, t0 + rows)
             ops.experts_few_tokens(x[t0:t1], sel_e[t0:t1], sel_w[t0:t1], self.w_gate, self.w_up, self.w_down,
-                                   act[t0 * self.top: t1 * self.top], residual[t0:t1],
-                                   weight_on_output=self.weight_on_output)
+                                   act[t0 * top: t1 * top], out[t0:t1], weight_on_output=self.weight_on_output)
+
+    def _in_order(self, x: torch.Tensor, sel_e: torch.Tensor, sel_w: torch.Tensor, residual: torch.Tensor, ctx) -> None:
+        """The same with an order: every pair is a token of its own with a single expert and a row of its own for the result,
+        and a token's rows are added in the order of its choices."""
+        (T, W), top, ws = x.shape, self.top, ctx.workspace
+        most = min(T, max(1, IN_ORDER_PAIRS // top))
+        places = torch.arange(most * top, out=ws.get("experts_order", (most * top,), torch.int32))
+        for t0 in range(0, T, most):
+            t1 = min(T, t0 + most)
+            pairs = (t1 - t0) * top
+            rows = ws.get("experts_rows", (pairs, W), self.dtype)
+            ops.expert_gather(x[t0:t1], places[:pairs], None, top, rows)
+            results = ws.get("experts_results", (pairs, W), torch.float32)
+            results.zero_()
+            self._few(rows, sel_e[t0:t1].view(pairs, 1), sel_w[t0:t1].view(pairs, 1), results, ctx)
+            ops.expert_scatter(results, places[:pairs], top, residual[t0:t1])
 
     def _grouped(self, x: torch.Tensor, sel_e: torch.Tensor, sel_w: torch.Tensor, residual: torch.Tensor, ctx) -> None:
         """The tensor-core path of a prompt step without the host: sort, gather, two grouped products, add back."""

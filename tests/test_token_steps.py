@@ -346,3 +346,46 @@ def test_channel_chunks_that_are_not_finite(ops, monkeypatch, what):
         assert torch.equal(got, clean)
         assert not torch.isfinite(state[1, 0, :, columns] if what == "value" else state[1, 0, 5]).any()
         assert torch.equal(state[0], clean_state[0]) and torch.equal(state[1, 1], clean_state[1, 1])
+
+
+@pytest.mark.parametrize("dtype, W, Fi", [(torch.bfloat16, 256, 128), (torch.bfloat16, 96, 64), (torch.bfloat16, 40, 24), (torch.float32, 64, 48)])
+@pytest.mark.parametrize("T, top, on_output", [(1, 2, False), (5, 1, False), (16, 4, True), (40, 3, False)])
+def test_deterministic_experts_are_added_in_order(ops, dtype, W, Fi, T, top, on_output):
+    """Deterministic mode: a token's experts are added up in the order of its choices and the sum goes to the residual, whatever
+    finishes first, so every run gives the same bits; and they are the bits of the experts' own results in that order."""
+    from types import SimpleNamespace
+
+    from janus_b200.engine.workspace import Workspace
+    from janus_b200.parts.routed import RoutedExperts
+    g, E = torch.Generator().manual_seed(T + W), 8
+    ops.set_deterministic(True)
+    try:
+        part = RoutedExperts(W, Fi, E, top, weight_on="output" if on_output else "input", dtype=dtype,
+                             device=torch.device(DEV))
+        wts = {n: rnd(g, *s[0], s=s[0][-1] ** -0.5).to(dtype) for n, s in part.weight_shapes().items()}
+        part.load(**wts)
+        x, base = rnd(g, T, W).to(dtype).to(DEV), rnd(g, T, W).to(DEV)
+        ctx = SimpleNamespace(is_decode=True, workspace=Workspace(torch.device(DEV)))
+
+        def run(p):
+            out = base.clone()
+            p.forward(x, out, ctx)
+            return out
+
+        first = run(part)
+        for _ in range(50):
+            assert torch.equal(run(part), first)
+        sel_e, sel_w = (ctx.workspace.get(n, (T, top), t).clone() for n, t in (("router_experts", torch.int32), ("router_weights", torch.float32)))
+        sums = torch.zeros(T, W, device=DEV)
+        for k in range(top):                     # the experts' results one by one, into zeros
+            one, e, s = torch.zeros(T, W, device=DEV), sel_e[:, k:k + 1].contiguous(), sel_w[:, k:k + 1].contiguous()
+            if dtype == torch.bfloat16 and W % 32 == 0 and Fi % 32 == 0:
+                ops.experts_few_tokens_tc(x, e, s, part.w_gate, part.w_up, part.w_down, torch.empty(T, Fi, dtype=dtype, device=DEV), one,
+                                          weight_on_output=on_output)
+            else:
+                ops.experts_few_tokens(x, e, s, part.w_gate, part.w_up, part.w_down, torch.empty(T, Fi, device=DEV), one,
+                                       weight_on_output=on_output)
+            sums += one
+        assert torch.equal(first, base + sums)
+    finally:
+        ops.set_deterministic(False)
