@@ -214,7 +214,16 @@ int launch(const Args& p, void* out, int out_dtype, int n_seqs, cudaStream_t str
   JB_REFUSE(p.d < 1 || p.d > MAX_D || p.e < 4 || p.e > MAX_E || p.e % 4 || ((long long)p.d * ex) % 4 || p.slot_stride % 4 ||
                 p.state_off % 4 || ((uintptr_t)p.state & 15),
             "head_step: heads of %d x %d are not whole 16-byte vectors of at most %d x %d", p.d, p.e, MAX_D, MAX_E);
-  JB_REFUSE(p.H < 1 || p.H > 65535 || p.G < 1 || p.H % p.G, "head_step: %d heads of %d", p.H, p.G);
+  JB_REFUSE(p.H < 1 || p.H > 65535 || p.G < 1 || p.H % p.G || (KIND != DELTA && p.G != p.H), "head_step: %d heads of %d", p.H, p.G);
+  const long long keys = (long long)p.G * p.d, values = (long long)p.H * p.e, from_a = KIND == CHANNEL ? p.rank : p.H;
+  JB_REFUSE(p.q_col < 0 || p.k_col < 0 || p.v_col < 0 || p.q_col + keys > p.ld || p.k_col + keys > p.ld || p.v_col + values > p.ld ||
+                p.col_a < 0 || from_a < 0 || p.col_a + from_a > p.ld_raw ||
+                (KIND != CHANNEL && (p.col_b < 0 || p.col_b + (long long)p.H > p.ld_raw)),
+            "head_step: columns %d, %d, %d of %d and %d, %d of %d do not hold %d heads of %d x %d", p.q_col, p.k_col, p.v_col, p.ld,
+            p.col_a, p.col_b, p.ld_raw, p.H, p.d, p.e);
+  JB_REFUSE(p.state_off < 0 || p.state_off + (long long)p.H * p.d * ex > p.slot_stride ||
+                (KIND == MEMORY && (p.m_off < 0 || p.m_off + p.H > p.slot_stride)),
+            "head_step: slots of %lld numbers do not hold the state", p.slot_stride);
   jb::Launch cfg(dim3(n_seqs, p.H), dim3(THREADS), 0, stream);
 #define JB_GO(CG)                                                                                                 \
   return out_dtype == JB_F32 ? (int)cudaLaunchKernelEx(&cfg.c, head_step_kernel<KIND, CG, float>, p, (float*)out) \

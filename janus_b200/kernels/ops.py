@@ -1806,10 +1806,14 @@ def head_step(kind: str, rows: torch.Tensor, q_col: int, k_col: int, v_col: int,
     _need(weight, "head norm weight", torch.float32, (heads * vdim,) if per_head else (vdim,))
     if gate.dtype != torch.float32 or gate.stride(1) != 1 or tuple(gate.shape) != (T, heads * vdim):
         raise KernelError("head_step: the gate must be float32 columns of the heads' shape")
-    if raw.shape[0] != T or state.dim() != 2 or state.shape[1] < max(heads * dim * (vdim + (kind == "memory")), m_off):
+    if kind != "delta" and kv_heads != heads:
+        raise KernelError(f"head_step: '{kind}' has a key head for each of its {heads} heads, not {kv_heads}")
+    memory, low = kind == "memory", p0.shape[0] if channel else heads
+    if raw.shape[0] != T or state.dim() != 2 or state.shape[1] < max(heads * dim * (vdim + memory), m_off + heads * memory):
         raise KernelError("head_step: the rows or the state do not hold what the step reads")
-    if max(q_col + kv_heads * dim, k_col + kv_heads * dim, v_col + heads * vdim) > rows.shape[1]:
-        raise KernelError("head_step: the projections' columns reach past the rows")
+    if (max(q_col + kv_heads * dim, k_col + kv_heads * dim, v_col + heads * vdim) > rows.shape[1]
+            or max(col_a + low, 0 if channel else col_b + heads) > raw.shape[1]):
+        raise KernelError("head_step: the columns of the projections or of the gates' arguments reach past the rows")
     _check(_lib("head_step").jb_head_step(
         _HEAD_STEP_KINDS[kind], _ptr(rows), rows.shape[1], int(q_col), int(k_col), int(v_col), float(q_scale), _ptr(raw),
         raw.shape[1], int(col_a), int(col_b), _ptr(p0), _ptr(p1), float(scalar), p0.shape[0] if channel else 0, _ptr(state),
