@@ -54,7 +54,8 @@ __global__ void __launch_bounds__(THREADS, CG <= 32 ? 2 : 1) head_step_kernel(co
   constexpr int ROWS = THREADS / CG, RI = MAX_D / ROWS, COLS = 4 * CG;
   __shared__ float q_s[MAX_D], k_s[MAX_D], a_s[MAX_D], parts_s[4][MAX_D];
   __shared__ __align__(16) float sums_s[KIND == DELTA ? 2 : 1][ROWS][COLS];
-  __shared__ float w_s[COLS], o_s[COLS], nq_s[THREADS / 32];
+  __shared__ __align__(16) float w_s[COLS];
+  __shared__ float o_s[COLS], nq_s[THREADS / 32];
   jb::pdl_launch_dependents();
   const int seq = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int d = p.d, e = p.e, ex = e + (KIND == MEMORY ? 1 : 0);
