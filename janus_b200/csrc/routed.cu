@@ -128,7 +128,7 @@ __global__ void route_topk_kernel(const float* __restrict__ logits, int ld, Choi
 // L2 and from memory, 8 experts: 2,048 wide, 1 token 6.1, 6.8 and 3.6, 4.2; 16 tokens 6.6, 7.4 and 3.6, 5.3; 4,096 wide, 2
 // tokens 6.3, 6.9 and 4.8, 7.0; 16 experts, 64 tokens 6.9, 7.6 and 5.4, 7.9; 592 tokens 9.6, 10.8 and 7.7, 10.5 (1,500
 // tokens 9.8 and 15, in blocks of four tokens).
-constexpr int ROUTE_WARPS = 16, ROUTE_AHEAD = 4, ROUTE_MAX_NUMBERS = 1 << 16;
+constexpr int ROUTE_WARPS = 16, ROUTE_AHEAD = 4, ROUTE_MAX_NUMBERS = 1 << 16, ROUTE_MAX_ROWS = 4096;   // (rows: 48 KB of sums)
 __global__ void __launch_bounds__(ROUTE_WARPS * 32) route_tokens_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
                                                                         int W, int R, float* __restrict__ logits, Choice c,
                                                                         int* __restrict__ sel_e, float* __restrict__ sel_w) {
@@ -716,7 +716,8 @@ JB_EXPORT int jb_route_tokens(const void* x, const void* w, int W, int R, float*
   if (T <= 0) return 0;
   const Choice c{E, top, softmax, groups, keep, correction, scale, shares};
   if (const int e = check_choice(c)) return e;
-  JB_REFUSE(R < E || W < 8 || W % 8 || (long long)R * W > ROUTE_MAX_NUMBERS, "route_tokens: %d rows of %d (%d experts)", R, W, E);
+  JB_REFUSE(R < E || R > ROUTE_MAX_ROWS || W < 8 || W % 8 || (long long)R * W > ROUTE_MAX_NUMBERS,
+            "route_tokens: %d rows of %d (%d experts)", R, W, E);
   JB_REFUSE(((uintptr_t)x | (uintptr_t)w) & 15, "route_tokens: operands must be 16-byte aligned");
   jb::Launch cfg(dim3(T), dim3(ROUTE_WARPS * 32), 3 * (size_t)R * sizeof(float), stream);
   return (int)cudaLaunchKernelEx(&cfg.c, route_tokens_kernel, (const bf16*)x, (const bf16*)w, W, R, logits, c, sel_e, sel_w);

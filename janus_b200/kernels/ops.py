@@ -1875,15 +1875,16 @@ def route_topk(logits: torch.Tensor, top: int, sel_e: torch.Tensor, sel_w: torch
                                         _stream()), "route_topk")
 
 
-ROUTE_MAX_NUMBERS = 1 << 16      # numbers of a router's matrix, and tokens, up to which product and choice are one launch
-ROUTE_MAX_TOKENS = 128
+# numbers and rows of a router's matrix, and tokens, up to which product and choice are one launch (a block keeps three numbers a
+# row in shared memory, of which 48 KB need no leave)
+ROUTE_MAX_NUMBERS, ROUTE_MAX_ROWS, ROUTE_MAX_TOKENS = 1 << 16, 4096, 128
 
 
 def route_tokens(x: torch.Tensor, w: torch.Tensor, logits: torch.Tensor, top: int, sel_e: torch.Tensor, sel_w: torch.Tensor,
                  softmax: bool = False, groups: int = 0, keep: int = 0, experts: Optional[int] = None,
                  correction: Optional[torch.Tensor] = None, scale: float = 1.0, shares: bool = False) -> None:
     """logits[t, r] = w[r] . x[t] (bfloat16 x [T, W] and w [R, W], W a multiple of 8; float32 [T, R]) and `route_topk` of
-    them, in one launch; for at most ROUTE_MAX_NUMBERS numbers in w, since every block reads all of it."""
+    them, in one launch; for at most ROUTE_MAX_NUMBERS numbers in w, since every block reads all of it, and ROUTE_MAX_ROWS rows."""
     (T, W), R = x.shape, w.shape[0]
     E = R if experts is None else int(experts)
     _need(x, "router in", torch.bfloat16)

@@ -73,7 +73,8 @@ class RoutedExperts(FeedForward):
         # the router's product also makes the shared expert's gate: one more row
         rows = experts + (1 if self.shared_gate else 0)
         # few tokens of a small router: product and choice are one launch, which reads the matrix as it is
-        self.route_in_one = dtype == torch.bfloat16 and hidden_size % 8 == 0 and rows * hidden_size <= ops.ROUTE_MAX_NUMBERS
+        self.route_in_one = (dtype == torch.bfloat16 and hidden_size % 8 == 0 and rows * hidden_size <= ops.ROUTE_MAX_NUMBERS
+                             and rows <= ops.ROUTE_MAX_ROWS)
         self.router_rows: Optional[torch.Tensor] = None
         self.router = Linear(hidden_size, rows, dtype, device, name="router", pad_width=True)
         self.shared_gate_up = self.shared_down = None

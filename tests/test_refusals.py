@@ -69,3 +69,12 @@ def test_the_c_entry_of_head_step_refuses_them_too(kind, changed):
     assert set(changed) <= set(a)
     a.update(changed)
     assert ops._lib("head_step").jb_head_step(*a.values()) == BAD_SIZE
+
+
+def test_a_router_of_more_rows_than_a_launch_holds():
+    """3 numbers a row lie in shared memory, of which a launch has 48 KB: 8,192 rows of 8 numbers go in two launches."""
+    from janus_b200.parts.routed import RoutedExperts
+    part = RoutedExperts(8, 8, 8192, 2, dtype=torch.bfloat16, device=torch.device("cpu"))
+    assert not part.route_in_one
+    assert ops._lib("routed").jb_route_tokens(0, 0, 8, 8192, 0, 8192, 2, 0, 0, 1, 0, 0, 0, 0, 1.0, 0, 0) == BAD_SIZE
+    assert ops._lib("routed").jb_route_tokens(0, 0, 8, 4097, 0, 4097, 2, 0, 0, 1, 0, 0, 0, 0, 1.0, 0, 0) == BAD_SIZE

@@ -104,7 +104,8 @@ def test_head_step(ops, kind, T, H, G, d, e):
 
 @pytest.mark.parametrize("T", [1, 5, 130])
 @pytest.mark.parametrize("W, E, extra, top, softmax, groups, keep", [(2048, 8, 0, 2, False, 0, 0), (264, 8, 1, 2, True, 4, 2), (8, 3, 1, 3, False, 0, 0),
-                                                                     (4096, 16, 0, 4, True, 0, 0), (1024, 40, 1, 6, False, 8, 3)])
+                                                                     (4096, 16, 0, 4, True, 0, 0), (1024, 40, 1, 6, False, 8, 3),
+                                                                     (16, 4095, 1, 2, False, 0, 0)])
 def test_route_tokens(ops, T, W, E, extra, top, softmax, groups, keep):
     """The router's product and choice in one launch: logits against float64 (each half of a row is lanes' chains of at most
     64 products and eight more sums: 72 roundings of 2^-24 of the sum of the products' sizes), the choice as `route_topk`
