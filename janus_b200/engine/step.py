@@ -139,14 +139,14 @@ class Engine:
             self._validate_each(entries, device_tokens)
 
     def _passes(self, entries: Sequence[StepEntry], device_tokens: bool) -> bool:
-        lengths, live, parts = self.cache.lengths, self.cache.is_live, []
-        slots = [e.slot for e in entries]
-        if not entries or len(set(slots)) < len(slots):
-            return False
+        lengths, live, longest, V = self.cache.lengths, self.cache.is_live, self.max_seq_len, self.model.vocab_size
+        parts, seen, low = [], set(), FROM_DEVICE if device_tokens else 0
         for e in entries:
-            tokens, want, n = e.tokens, e.want, len(e.tokens)
-            if n == 0 or not live(e.slot) or lengths[e.slot] + n > self.max_seq_len:
+            slot, tokens, want = e.slot, e.tokens, e.want
+            n = len(tokens)
+            if n == 0 or slot in seen or not live(slot) or lengths[slot] + n > longest:
                 return False
+            seen.add(slot)
             if n > 1:
                 # the array stays with the entry for the step's index buffer (a batch's prompts are tens of thousands)
                 tokens = np.asarray(tokens, dtype=np.int64)
@@ -154,20 +154,19 @@ class Engine:
                     return False
                 e.tokens = tokens
                 parts.append(tokens)
-            else:
-                t = int(tokens[0])
-                if not (0 <= t < self.model.vocab_size or (device_tokens and t == FROM_DEVICE)):
-                    return False
+            elif not low <= int(tokens[0]) < V:
+                return False
             if type(want) is range:
                 if len(want) and not (0 <= min(want[0], want[-1]) and max(want[0], want[-1]) < n):
                     return False
-            elif any(not 0 <= int(w) < n for w in want):
-                return False
+                continue
+            for w in want:
+                if not 0 <= int(w) < n:
+                    return False
         if parts:
             tokens = parts[0] if len(parts) == 1 else np.concatenate(parts)
-            low = FROM_DEVICE if device_tokens else 0
-            return low <= int(tokens.min()) and int(tokens.max()) < self.model.vocab_size
-        return True
+            return low <= int(tokens.min()) and int(tokens.max()) < V
+        return len(entries) > 0
 
     def _validate_each(self, entries: Sequence[StepEntry], device_tokens: bool) -> None:
         if not entries:
