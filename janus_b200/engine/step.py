@@ -233,13 +233,19 @@ class Engine:
             if P > pages_capacity:
                 raise StepError("a sequence outgrew the page capacity this step was laid out for")
             P = pages_capacity
-        wants, q_start = [], [0]
-        for e, n in zip(entries, lens):
-            w = e.want
-            w = np.arange(w.start, w.stop, w.step) if type(w) is range else np.array([int(x) for x in w], dtype=np.int64)
-            wants.append(w + q_start[-1])
+        q_start = [0]
+        for n in lens:
             q_start.append(q_start[-1] + n)
-        wants = np.concatenate(wants)
+        # wanted rows: places one by one in a list, which costs less than an array an entry; ranges as arrays
+        wants, places = [], []
+        for e, first in zip(entries, q_start):
+            w = e.want
+            if type(w) is range:
+                wants += [np.array(places, dtype=np.int64), np.arange(first + w.start, first + w.stop, w.step)]
+                places = []
+            else:
+                places += [first + int(x) for x in w]
+        wants = np.concatenate(wants + [np.array(places, dtype=np.int64)])
         W = len(wants)
         G = len(cache.groups)
         sizes = [T, T, T, S + 1, S, S, W] + [T, S * P] * G + [S + 1]
