@@ -19,7 +19,6 @@ from __future__ import annotations
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence
 
-import numpy as np
 import torch
 
 from ..kernels import ops
@@ -77,11 +76,6 @@ class KVGroup:
             if p >= 0:
                 self.pool.give_back(p)
         self.pages[slot] = []
-
-    def dest_rows(self, slot: int, start: int, n: int) -> np.ndarray:
-        pos = np.arange(start, start + n, dtype=np.int64)
-        pages = np.asarray(self.pages[slot], dtype=np.int64)
-        return (pages[pos // PAGE_SIZE] * PAGE_SIZE + pos % PAGE_SIZE).astype(np.int32)
 
 
 @dataclass
