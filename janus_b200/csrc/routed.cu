@@ -126,8 +126,8 @@ __global__ void route_topk_kernel(const float* __restrict__ logits, int ld, Choi
 // chain of loads, sums and comparisons that a token's choice is, and with many tokens that every block reads the whole
 // matrix.  Product (its result cleared first) and choice in launches of their own, and here, microseconds with weights from
 // L2 and from memory, 8 experts: 2,048 wide, 1 token 6.1, 6.8 and 3.6, 4.2; 16 tokens 6.6, 7.4 and 3.6, 5.3; 4,096 wide, 2
-// tokens 6.3, 6.9 and 4.8, 7.0; 16 experts, 64 tokens 6.9, 7.6 and 5.4, 7.9; 592 tokens 9.6, 10.8 and 7.7, 10.5 (1,500
-// tokens 9.8 and 15, in blocks of four tokens).
+// tokens 6.3, 6.9 and 4.8, 7.0; 592 tokens 9.6, 10.8 and 7.7, 10.5 (1,500 tokens 9.8 and 15, in blocks of four tokens).  Two
+// warps a row make many rows dear: the callers' lines, measured on both sides, are beside ROUTE_MAX_NUMBERS in ops.py.
 constexpr int ROUTE_WARPS = 16, ROUTE_AHEAD = 4, ROUTE_MAX_NUMBERS = 1 << 16, ROUTE_MAX_ROWS = 4096;   // (rows: 48 KB of sums)
 __global__ void __launch_bounds__(ROUTE_WARPS * 32) route_tokens_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
                                                                         int W, int R, float* __restrict__ logits, Choice c,

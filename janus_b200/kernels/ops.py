@@ -1875,16 +1875,19 @@ def route_topk(logits: torch.Tensor, top: int, sel_e: torch.Tensor, sel_w: torch
                                         _stream()), "route_topk")
 
 
-# numbers and rows of a router's matrix, and tokens, up to which product and choice are one launch (a block keeps three numbers a
-# row in shared memory, of which 48 KB need no leave)
-ROUTE_MAX_NUMBERS, ROUTE_MAX_ROWS, ROUTE_MAX_TOKENS = 1 << 16, 4096, 128
+# Numbers and rows of a router's matrix, and tokens, up to which product and choice in one launch are the faster form: every block
+# reads the whole matrix, two warps a row.  Two launches and one in a captured step, weights from memory, microseconds, 4 to 64
+# tokens: 8 x 2,048 6.9 to 7.9 and 4.3 to 4.9; 8 x 4,096 7.2 to 7.7 and 5.6 to 5.9; 16 x 2,048 8.4 to 8.8 and 7.3 to 8.1; 24 x 2,048 7.1
+# to 8.0 and 7.1 to 7.8; 9 x 4,096 7.1 to 7.8 and 7.4 to 7.3; beyond the line 8 x 8,192 7.9 to 8.2 and 8.0 to 8.8, 16 x 4,096 8.6 to 9.0 and
+# 9.8 to 10.3, 32 x 1,024 8.2 to 9.1 and 8.8 to 9.8, 64 x 512 10.4 to 11.8 and 15, 128 x 512 15 and 28, 512 x 128 32 and 90.
+ROUTE_MAX_NUMBERS, ROUTE_MAX_ROWS, ROUTE_MAX_TOKENS = 24 * 2048, 24, 128
 
 
 def route_tokens(x: torch.Tensor, w: torch.Tensor, logits: torch.Tensor, top: int, sel_e: torch.Tensor, sel_w: torch.Tensor,
                  softmax: bool = False, groups: int = 0, keep: int = 0, experts: Optional[int] = None,
                  correction: Optional[torch.Tensor] = None, scale: float = 1.0, shares: bool = False) -> None:
     """logits[t, r] = w[r] . x[t] (bfloat16 x [T, W] and w [R, W], W a multiple of 8; float32 [T, R]) and `route_topk` of
-    them, in one launch; for at most ROUTE_MAX_NUMBERS numbers in w, since every block reads all of it, and ROUTE_MAX_ROWS rows."""
+    them, in one launch, of at most 65,536 numbers and 4,096 rows in w (three numbers a row lie in 48 KB of shared memory)."""
     (T, W), R = x.shape, w.shape[0]
     E = R if experts is None else int(experts)
     _need(x, "router in", torch.bfloat16)

@@ -78,3 +78,14 @@ def test_a_router_of_more_rows_than_a_launch_holds():
     assert not part.route_in_one
     assert ops._lib("routed").jb_route_tokens(0, 0, 8, 8192, 0, 8192, 2, 0, 0, 1, 0, 0, 0, 0, 1.0, 0, 0) == BAD_SIZE
     assert ops._lib("routed").jb_route_tokens(0, 0, 8, 4097, 0, 4097, 2, 0, 0, 1, 0, 0, 0, 0, 1.0, 0, 0) == BAD_SIZE
+
+
+@pytest.mark.parametrize("rows, width, one", [(8, 2048, True), (16, 2048, True), (24, 2048, True), (9, 4096, True), (12, 4096, True), (8, 264, True),
+                                              (24, 8, True), (25, 8, False), (13, 4096, False), (8, 8192, False), (64, 512, False)])
+def test_which_routers_choose_in_the_product_s_launch(rows, width, one):
+    """On both sides of the lines in rows and in numbers; a shared expert's gate is a row too."""
+    from janus_b200.parts.routed import RoutedExperts
+    for gate in (False, True):
+        part = RoutedExperts(width, 8, rows - gate, 2, shared_size=8 if gate else None, shared_gate=gate, dtype=torch.bfloat16,
+                             device=torch.device("cpu"))
+        assert part.route_in_one is one
