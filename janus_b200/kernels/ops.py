@@ -1782,6 +1782,21 @@ def head_step_supported(dim: int, vdim: int, state: torch.Tensor, normalizer: bo
             and state.shape[1] % 4 == 0 and state.data_ptr() % 16 == 0)
 
 
+HEAD_STEP_BLOCKS, HEAD_STEP_NUMBERS = 1536, 128 * 64
+
+
+def head_step_pays(kind: str, n_seqs: int, heads: int, dim: int, vdim: int) -> bool:
+    """Whether one launch is faster than gates, recurrence, norm and gate in launches of their own.  A block a (sequence, head)
+    computes its gates again and, with small states, is more start and end than work, so many blocks lose.  Launches of
+    their own and one launch, microseconds in a captured step; the delta rule gains everywhere (one sequence to 256, heads of 32 x 32
+    to 128 x 256: 1.2 to 3.5 times).  Matrix memory, 16 heads of 32 x 32: 64 sequences 12.7 and 10.9, 128 17.2 and 19.8, 256 26 and
+    38; 64 heads of 32 x 64, 16 sequences 12.7 and 10.3, 32 18.0 and 18.7, 64 27 and 36; from 128 x 64 on it gains or is level (16 heads
+    of 128 x 128, 256 sequences 128 and 98; 12 of 128 x 64, 256 54 and 54).  A decay a channel: 1,024 blocks 1.0 to 1.6 times as
+    fast, 1,536 of 128 x 64 31 and 23; 2,048 of 64 x 64 24 and 24, of 64 x 128 35 and 48, of 128 x 128 77 and 78; 4,096 of 32 x 32 28 and 40,
+    of 128 x 128 137 and 147."""
+    return kind == "delta" or n_seqs * heads <= HEAD_STEP_BLOCKS or (kind == "memory" and dim * vdim >= HEAD_STEP_NUMBERS)
+
+
 def head_step(kind: str, rows: torch.Tensor, q_col: int, k_col: int, v_col: int, q_scale: float, raw: torch.Tensor, col_a: int,
               col_b: int, p0: torch.Tensor, p1: torch.Tensor, scalar: float, state: torch.Tensor, gate: torch.Tensor,
               weight: torch.Tensor, eps: float, out: torch.Tensor, q_start: torch.Tensor, seq_slot: torch.Tensor, heads: int,

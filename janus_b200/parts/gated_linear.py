@@ -114,7 +114,8 @@ class GatedLinearAttention(_GatedLinearBase):
         proj, col = self._projections(x, ctx, scratch_cleared, projected)
         gate = proj[:, col + self.gate_col: col + self.gate_col + self.v_width]
         gated = ws.get("gla_gated", (T, self.v_width), self.dtype)
-        if ctx.is_decode and ops.head_step_supported(self.dim, self.vdim, cache_view.state):
+        if (ctx.is_decode and ops.head_step_supported(self.dim, self.vdim, cache_view.state)
+                and ops.head_step_pays("channel", T, self.nh, self.dim, self.vdim)):
             ops.head_step("channel", proj, col, col + self.k_col, col + self.v_col, self.q_scale, proj, col + self.extra_col, 0,
                           self.a2t, self.a2_bias, 1.0 / self.tau, cache_view.state, gate, self.norm_weight, self.eps, gated,
                           ctx.q_start, ctx.seq_slot, self.nh, self.nh, self.dim, self.vdim)
@@ -172,7 +173,8 @@ class MatrixMemory(_GatedLinearBase):
         proj, col = self._projections(x, ctx, scratch_cleared, projected)
         gate = proj[:, col + self.gate_col: col + self.gate_col + self.v_width]
         gated = ws.get("matrix_memory_gated", (T, self.v_width), self.dtype)
-        if ctx.is_decode and ops.head_step_supported(self.dim, self.vdim, state, normalizer=True):
+        if (ctx.is_decode and ops.head_step_supported(self.dim, self.vdim, state, normalizer=True)
+                and ops.head_step_pays("memory", T, self.nh, self.dim, self.vdim)):
             ops.head_step("memory", proj, col, col + self.k_col, col + self.v_col, self.q_scale, proj, col + self.extra_col,
                           col + self.extra_col + self.nh, self.bias_i, self.bias_f, self.cap, state, gate, self.norm_weight,
                           self.eps, gated, ctx.q_start, ctx.seq_slot, self.nh, self.nh, self.dim, self.vdim, m_off=self.m_off,

@@ -89,3 +89,11 @@ def test_which_routers_choose_in_the_product_s_launch(rows, width, one):
         part = RoutedExperts(width, 8, rows - gate, 2, shared_size=8 if gate else None, shared_gate=gate, dtype=torch.bfloat16,
                              device=torch.device("cpu"))
         assert part.route_in_one is one
+
+
+@pytest.mark.parametrize("kind, n, heads, dim, vdim, one", [
+    ("delta", 256, 64, 32, 32, True), ("channel", 1, 16, 128, 128, True), ("channel", 96, 16, 128, 128, True), ("channel", 97, 16, 128, 128, False),
+    ("channel", 64, 32, 64, 64, False), ("memory", 24, 64, 32, 64, True), ("memory", 25, 64, 32, 64, False), ("memory", 256, 32, 128, 64, True),
+    ("memory", 256, 32, 64, 128, True), ("memory", 256, 32, 64, 124, False)])
+def test_which_single_token_steps_are_one_launch(kind, n, heads, dim, vdim, one):
+    assert ops.head_step_pays(kind, n, heads, dim, vdim) is one
