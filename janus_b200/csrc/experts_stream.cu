@@ -11,10 +11,11 @@
 // expert, row tile by row tile, k tile by k tile, and each of 148 CTAs takes one run of them, as long as every other's to a
 // tile.  A run ends and begins in the middle of a row tile; the parts meet in z or out.  All tokens of the step are columns
 // of every expert's product (16, 32 or 64 of them): a column that did not choose the expert is computed and left out.
-// Before, blocks of 16 rows with mma.sync read the weights row by row, for two tokens of 8 experts of 7,168 x 4,096 6.05 waves
-// of them.  Both products of a layer in a captured step, microseconds, before and now (the activation's launch included):
-// these two tokens 150 and 116 (their experts' bytes at the copy rate: 108); 16 tokens of 8 experts of 4,096 x 2,048 78 and 76
-// (62); 8 tokens 80 and 68; one token 41 and 28 (16).
+// Blocks of 16 rows with mma.sync (expert_tc_kernel) read the weights row by row, for two tokens of 8 experts of 7,168 x 4,096
+// in 6.05 waves.  Both products of a layer in a captured step, microseconds, by such blocks and here (the activation's launch
+// included): these two tokens 114 and 106 (their experts' bytes at the copy rate: 99), 64 tokens 381 and 228 (215); of 4,096 x
+// 2,048, one token 29 and 28 (15), 16 tokens 74 and 74 (61), 64 tokens 129 and 84; of 1,536 x 1,024, where start and end are the
+// most of it, 8 tokens 19 and 23 (10): the callers' line is `experts_stream_pays` in ops.py.
 #include <stdio.h>
 
 #include "tc_common.cuh"

@@ -1971,6 +1971,25 @@ def experts_stream_supported(T: int, top: int, experts: int) -> bool:
             and min(T * top, experts) * T <= EXPERTS_STREAM_PLACES and not _deterministic[0])
 
 
+@functools.lru_cache(maxsize=4096)
+def experts_stream_pays(T: int, top: int, experts: int, F: int, W: int) -> bool:
+    """Whether `experts_stream` is faster than `experts_few_tokens_tc`, by an estimate of both in microseconds from how many
+    experts T tokens choose when every one is as likely, and how long their weights take at the copy rate.  Row blocks
+    start for every expert, chosen or not, go again over an expert's rows for every 16 of its tokens and read their tokens' rows from L2;
+    tiles cost two more launches' worth of start, all tokens as columns and the adds of their sums.  The constants were fitted to
+    238 cases in captured steps with weights from memory (4 to 512 experts of 128 x 128 to 7,168 x 4,096, 1 to 16 a token, 1 to 64
+    tokens): the pick is 0.5 % slower than the better form on average, at worst 12 %, where always tiles were 13 % and row blocks 16 %.
+    Row blocks and tiles: two of 8 experts of 4,096 x 2,048, 1 token 29 and 28, 16 tokens 74 and 74, 64 tokens 129 and 84; of
+    1,536 x 1,024, 8 tokens 19 and 23; of 128 x 128 6 and 11; six of 64 of 1,408 x 2,048, 1 token 41 and 31; one of 4 of 1,024 x
+    1,024, 16 tokens 12 and 18."""
+    pairs, chosen = T * top, experts * (1.0 - (1.0 - top / experts) ** T)
+    stream = chosen * 6 * F * W / 6548e3
+    rows = (5.8 + experts * (F + W) / 12700 + 0.87 * stream + 0.66 * stream ** 0.5 + 0.074 * stream * max(0.0, pairs / chosen - 8)
+            + pairs * F * W / 56e6 + 0.053 * T + 0.79e-3 * F)
+    tiles = 9.9 + 0.164 * T + pairs * (2 * F + W) / 276e3 + 0.84 * stream + 1.17 * stream ** 0.5
+    return tiles < rows
+
+
 def experts_stream(x: torch.Tensor, sel_e: torch.Tensor, sel_w: torch.Tensor, gate_up: PackedWeight, down: PackedWeight,
                    experts: int, z: torch.Tensor, act: torch.Tensor, pair_slot: torch.Tensor, out: torch.Tensor,
                    gate_limit: float = 0.0, gate_alpha: float = 1.0, weight_on_output: bool = False) -> None:

@@ -6,8 +6,9 @@ largest scores (the lower index wins a tie) and their weights are those scores a
 weight multiplies the expert's INPUT: out = sum over the chosen e of expert_e(s_e h).
 
 Steps of few (token, expert) pairs, every single-token step among them, stream the chosen experts' packed tiles once for
-up to 64 tokens (`ops.experts_stream`: width and inner width multiples of 128).  Other widths, more tokens and
-deterministic runs (in which a token's experts are added in order) stream each chosen expert's rows once for up to 16 of the tokens that chose it
+up to 64 tokens (`ops.experts_stream`: width and inner width multiples of 128) where that is the faster form
+(`ops.experts_stream_pays`: large experts, many of them, or many tokens an expert).  Other sizes, more tokens and deterministic
+runs (in which a token's experts are added in order) stream each chosen expert's rows once for up to 16 of the tokens that chose it
 (`ops.experts_few_tokens_tc`: two launches with a block per (rows, expert); widths that are no multiples
 of 32, and the float32 engine, take up to four tokens at a time on the CUDA cores, `ops.experts_few_tokens`).  Sums are
 float32 and nothing is read back by the host, so the step can be recorded into a CUDA graph.  Prompt steps of the
@@ -148,7 +149,8 @@ class RoutedExperts(FeedForward):
     def _streams(self, ctx, tokens: int) -> bool:
         """Whether the step streams the packed stacks of the experts' matrices."""
         return (self.grouped and (ctx.is_decode or tokens * self.top <= FEW_PAIRS)
-                and ops.experts_stream_supported(tokens, self.top, self.experts))
+                and ops.experts_stream_supported(tokens, self.top, self.experts)
+                and ops.experts_stream_pays(tokens, self.top, self.experts, self.intermediate_size, self.hidden_size))
 
     def scratch_to_clear(self, ctx, tokens: int) -> Optional[torch.Tensor]:
         """The float32 sums of the streamed experts; else the router's logits, if this step's product adds slices of K into

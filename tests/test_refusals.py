@@ -97,3 +97,13 @@ def test_which_routers_choose_in_the_product_s_launch(rows, width, one):
     ("memory", 256, 32, 64, 128, True), ("memory", 256, 32, 64, 124, False)])
 def test_which_single_token_steps_are_one_launch(kind, n, heads, dim, vdim, one):
     assert ops.head_step_pays(kind, n, heads, dim, vdim) is one
+
+
+@pytest.mark.parametrize("T, top, experts, F, W, tiles", [
+    (1, 2, 8, 4096, 2048, True), (64, 2, 8, 4096, 2048, True), (2, 2, 8, 7168, 4096, True), (16, 2, 8, 7168, 4096, True), (1, 6, 64, 1408, 2048, True),
+    (64, 8, 128, 768, 2048, True), (32, 8, 256, 512, 1024, True), (8, 10, 512, 512, 2048, True), (64, 16, 16, 512, 1024, True),
+    (1, 1, 512, 128, 256, True), (1, 2, 8, 1536, 1024, False), (64, 2, 8, 1536, 1024, False), (1, 1, 1, 128, 128, False),
+    (64, 2, 8, 128, 128, False), (16, 1, 4, 1024, 1024, False), (32, 4, 40, 256, 384, False), (8, 2, 16, 1024, 2048, False)])
+def test_which_experts_stream_their_tiles(T, top, experts, F, W, tiles):
+    """Sizes whose forms were measured more than 3 % apart, or that are a model's own."""
+    assert ops.experts_stream_pays(T, top, experts, F, W) is tiles

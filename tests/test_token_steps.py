@@ -390,3 +390,40 @@ def test_deterministic_experts_are_added_in_order(ops, dtype, W, Fi, T, top, on_
         assert torch.equal(first, base + sums)
     finally:
         ops.set_deterministic(False)
+
+
+@pytest.mark.parametrize("tiles", [True, False])
+@pytest.mark.parametrize("T, E, top, on_output", [(1, 8, 2, False), (17, 5, 1, True), (64, 40, 3, False)])
+def test_routed_part_by_tiles_and_by_rows(ops, monkeypatch, tiles, T, E, top, on_output):
+    """The whole part in a step of few tokens, in either form, with scratch that comes filled with NaN and with scratch that the
+    launch before has cleared, against float64 (bound as in `test_experts_stream`; an input's weight is rounded with it by rows,
+    2^-9 of a sum's terms more)."""
+    from types import SimpleNamespace
+
+    from janus_b200.engine.workspace import Workspace
+    from janus_b200.parts.routed import RoutedExperts
+    g, W, Fi = torch.Generator().manual_seed(T + E), 256, 128
+    monkeypatch.setattr(ops, "experts_stream_pays", lambda *_: tiles)
+    part = RoutedExperts(W, Fi, E, top, weight_on="output" if on_output else "input", device=torch.device(DEV))
+    wts = {n: rnd(g, *s[0], s=s[0][-1] ** -0.5).bfloat16() for n, s in part.weight_shapes().items()}
+    part.load(**wts)
+    x, base = rnd(g, T, W).bfloat16(), rnd(g, T, W)
+    ws = Workspace(torch.device(DEV))
+    ctx = SimpleNamespace(is_decode=True, workspace=ws)
+    for cleared in (False, True, True):
+        out = base.to(DEV)
+        scratch = part.scratch_to_clear(ctx, T)
+        assert not tiles or tuple(scratch.shape) == (T * top, 2 * Fi)
+        for buf in ws._buffers.values():
+            if buf.is_floating_point():
+                buf.fill_(float("nan"))
+        if cleared and scratch is not None:
+            scratch.zero_()
+        part.forward(x.to(DEV), out, ctx, scratch_cleared=cleared)
+        ops.check_kernel_status(torch.device(DEV))
+        sel_e, sel_w = (ws.get(n, (T, top), t).cpu() for n, t in (("router_experts", torch.int32), ("router_weights", torch.float32)))
+        wg, wu, wd = (torch.stack([wts[f"e{e}_{kind}"] for e in range(E)]) for kind in ("gate", "up", "down"))
+        want = plain_experts(x, sel_e, sel_w, wg, wu, wd, base, on_output)
+        err = float((out.double().cpu() - want).abs().max() / (want - base.double()).abs().max())
+        assert err < 2.0 ** -8 + 2.0 ** -9, err
+    assert ("experts_sums", torch.float32) in ws._buffers or not tiles
