@@ -25,7 +25,7 @@
 // The tensor core computes S_{j+1} and the P.V product of block j-1 while the softmax of block j runs.
 // Its MMA lane waits 750 of 900 cycles per page for K and V (the copy engine gives about 80 GB/s per SM for
 // such boxes), so prefill_tc128_kernel (below) lets two tiles share what is loaded and takes two pages at a
-// time; it runs whenever it has CTAs enough for every SM.
+// time; which of the two runs, and why, is at `pairs_pay`.
 // Every mbarrier wait is bounded in time and reports through `*status` (codes 11-13).
 // Formulas: crates/janus-engine/src/compute/shaders/attention.wgsl:96-115,170-185,
 // softmax.wgsl:29-50; kv head of query head h is floor(h * nkv / nh).
@@ -866,6 +866,59 @@ JB_EXPORT int jb_attention_tc_head_dim() { return HD; }
 // q, out: [T, nh * hd] bf16; caches: [n_pages, nkv, 64, hd] bf16.  Needs nh / nkv <= 128 and a head size
 // that is a multiple of 8 (rows of 16 bytes for the tensor maps) up to the build's row.
 namespace {
+// ---- one row tile a CTA, or two ----------------------------------------------------------------------------------
+// Two tiles over blocks of 128 keys load keys once for both, but a CTA has an SM to itself and its second tile may be empty; of
+// one-tile CTAs an SM holds two, whose starts and ends fill each other's waits.  Heads of up to 64 numbers go by one tile: it was
+// the faster form, or within 4 % of it, in all of 740 cases (32 + 8 heads of 64: one sequence of 8,190 tokens 381 and 440 us, 64 of
+// 5 to 130 32 and 49).  Larger heads go by an estimate of both forms' times, from how many CTAs there are, the blocks of 128
+// keys that they see, and the longest CTA's.  What is known of a step is its tokens, its sequences, the longest one's tokens and the
+// longest cache: the others are taken to be equal, so one long prompt beside many single tokens is seen for what it is.  One tile
+// and two, 32 + 8 heads of 128: 2,000 tokens beside 63 single ones 335 and 209 us, 64 sequences of 5 to 130 65 and 57, eight of 150
+// to 701 55 and 46; 16 + 4 heads, six of 65 to 400 13.7 and 16.6.  The constants (microseconds) were fitted to 920 cases (1 to
+// 16 query heads a key head, 1 to 64 sequences, up to 16,384 tokens, cached keys, windows, chunks, caps, gates, slopes; heads of 72, 96 and
+// 128): the pick is 0.7 % slower than the better form on average, 43 cases by more than 5 %, the worst by 27 % (24 + 2 heads,
+// eight of 100 tokens behind 4,000 cached keys).  By the longest length it was 4 and 59 %, by the mean length 7 and 69 %.
+struct Step {
+  int T, n_seqs, max_q_len, max_kv, nkv, tpt, hd, window, chunk;
+  bool capped;
+};
+struct FormCost {
+  int tiles;                                        // of a CTA
+  // a launch, a CTA, a block of keys (of all CTAs; in the longest one), 1,000 CTAs of the grid, and what a cap adds to a block
+  double start, cta, block, chain, launched, capped;
+};
+double estimate_us(const Step& s, const FormCost& f, int sms) {
+  const double rows = (double)f.tiles * s.tpt, past = s.max_kv > s.max_q_len ? s.max_kv - s.max_q_len : 0;
+  double see = 1e9;                                 // keys that a CTA's rows can see at most
+  if (s.window > 0) see = s.window + rows;
+  if (s.chunk > 0 && s.chunk < see) see = s.chunk;
+  double ctas = 0.0, blocks = 0.0, longest = 0.0;
+  for (int which = 0; which < (s.n_seqs > 1 ? 2 : 1); ++which) {       // the longest sequence, the others
+    const double n = which ? s.n_seqs - 1 : 1;
+    const int rest = which ? (s.T - s.max_q_len) / (s.n_seqs - 1) : 0;
+    const double l = which ? (rest > 1 ? rest : 1) : s.max_q_len, full = past + l;
+    double reach = past + (l + rows) / 2;           // of a CTA, on average
+    if (s.chunk > 0 && full > s.chunk && (s.chunk + rows) / 2 < reach) reach = (s.chunk + rows) / 2;
+    if (s.window > 0 && full > see) {
+      const double ramp = see > past ? see - past : 0.0;               // tokens before the window begins to move
+      reach = ((past + ramp / 2) * ramp + see * (l - ramp)) / l;
+    }
+    if (reach > see) reach = see;
+    const double mine = (double)(long long)((l + rows - 1) / rows) * n;
+    ctas += mine;
+    blocks += mine * (reach / 128 + 0.5);
+    if (which == 0) longest = (full < see ? full : see) / 128 + 0.5;
+  }
+  const double work = s.capped ? 1.0 + f.capped : 1.0;
+  const double all = s.nkv * (ctas * f.cta + blocks * f.block * work) / sms, chain = longest * f.chain * work + f.cta;
+  const double grid = (double)((s.max_q_len + (int)rows - 1) / (int)rows) * s.nkv * s.n_seqs;
+  return f.start + (all > chain ? all : chain) + f.launched * grid / 1000;
+}
+bool pairs_pay(const Step& s, int sms) {
+  static constexpr FormCost one{1, 2.1, 2.7, 1.84, 1.7, 8.1, 0.65}, two{2, 2.7, 4.5, 2.58, 2.42, 7.5, 0.9};
+  return s.hd > 64 && estimate_us(s, two, sms) < estimate_us(s, one, sms);
+}
+
 // kv_rows > 0: keys and values are the matrix at k_cache ([kv_rows] rows of nkv (hd + vd) numbers), see `Keys`
 int tc_prefill_launch(const void* q, const void* k_cache, const void* v_cache, void* out, const int* block_table,
                       const int* q_start, const int* kv_len, int T, int n_pages, int n_seqs, int max_q_len, int nh,
@@ -906,16 +959,11 @@ int tc_prefill_launch(const void* q, const void* k_cache, const void* v_cache, v
             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return JB_ERR_TENSORMAP;
   }
-  // Two row tiles per CTA over blocks of 128 keys are the faster kernel once there are CTAs enough for every
-  // SM (of those that have tokens: about half a pair a sequence is empty); below that the finer one-tile CTAs spread better.
-  // So they do for sequences of less than two pairs of tiles, of which a CTA's start and end are the most: two one-tile CTAs
-  // share an SM (64 sequences of 5 to 130 tokens, 32 + 8 heads of 64: 53 us in pairs, 37 not; six of 65 to 400, 16 + 4 heads of
-  // 128, 99 CTAs: 16.8 and 14.9; eight of 150 to 701, 32 + 8 heads of 128, 458 CTAs: 52 and 65).
   const int n_tiles = (max_q_len + tpt - 1) / tpt;
-  const long long ctas_of_pairs = (T / (2 * tpt) + (n_seqs + 1) / 2ll) * nkv;
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  [[maybe_unused]] bool pairs = ctas_of_pairs >= sms && T > 4ll * tpt * n_seqs;
+  [[maybe_unused]] bool pairs = pairs_pay(Step{T, n_seqs, max_q_len, max_pages * PAGE, nkv, tpt, hd, window, cap.chunk, cap.cap_s != 0.0f},
+                                           sms);
   if (const char* e = getenv("JANUS_ATTN_TC_TILES")) {   // 1 or 2: tiles per CTA whatever the size (for tests and measurements)
     if (e[0] == '1') pairs = false;
     if (e[0] == '2') pairs = true;
@@ -956,6 +1004,13 @@ JB_EXPORT int jb_attention_tc_prefill(const void* q, const void* k_cache, const 
                                       cudaStream_t stream) {
   return tc_prefill_launch(q, k_cache, v_cache, out, block_table, q_start, kv_len, T, n_pages, n_seqs, max_q_len, nh,
                            nkv, hd, page_size, max_pages, window, scale, Cap{}, status, stream, Keys{nullptr, hd});
+}
+
+// Whether a step of such sizes goes by CTAs of two row tiles (148 SMs), without launching anything.
+JB_EXPORT int jb_attention_tc_two_tiles(int T, int n_seqs, int max_q_len, int max_kv_len, int nh, int nkv, int hd, int window,
+                                        int chunk, int capped) {
+  return n_seqs > 0 && nkv > 0 && nh >= nkv && HD <= 128 &&
+         pairs_pay(Step{T, n_seqs, max_q_len, max_kv_len, nkv, BM / (nh / nkv), hd, window, chunk, capped != 0}, 148);
 }
 
 // As jb_attention_tc_prefill, with a chunked mask (chunk > 0: a query sees only the keys of its own chunk of

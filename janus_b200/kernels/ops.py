@@ -74,7 +74,7 @@ _SIGNATURES = {
     "jb_head_step": "ipiiiifpiiippfiplllpipiifpippiiiiip",
     "jb_gla_decay": "piiippfpiip", "jb_exp_gates": "piiippfppllppiip",
     "jb_gated_linear_scan": "piiiifpiippplppiiiiiippp", "jb_scale_rows_sigmoid": "pipiiip",
-    "jb_attention_tc_prefill": "pppppppiiiiiiiiiifpp", "jb_attention_tc_prefill_capped": "pppppppiiiiiiiiiiififfpppipp",
+    "jb_attention_tc_prefill": "pppppppiiiiiiiiiifpp", "jb_attention_tc_two_tiles": "iiiiiiiiii", "jb_attention_tc_prefill_capped": "pppppppiiiiiiiiiiififfpppipp",
     "jb_streams_rmsnorm": "pppipifpiiipplp", "jb_streams_mix": "ppppiiip", "jb_streams_mix_rmsnorm": "pppppipifpiiiplp", "jb_embed_streams": "pippiiippp",
     "jb_lightning_scan": "piiiipppppiiiiiipp", "jb_gated_rmsnorm": "ppipifpiiip",
     "jb_conv_rope_cache": "pipipipppppippppiiiiiiip", "jb_conv_state_update": "pipippiip",
