@@ -119,9 +119,13 @@ __global__ void __launch_bounds__(32 * RANGES) gemm_f32_stream_kernel(const floa
 
   // A unit's sums, one for each (row, token) and segment, join the range in the order of the segments: the four lanes of a row
   // exchange theirs so that each ends with all four segments of its share of the (row, token) pairs, in as many shuffles as a
-  // lane has pairs (every lane asking the others for every pair took four times as many: 8 tokens, 16,384 rows of 2,048, 46.6 us
-  // and 44.5 so, 16 tokens 88 and 83.5, 8 tokens of 128,256 rows of 1,536 242 and 230; up to 4 tokens level).
-  constexpr int PAIRS = RL * TT, MINE = PAIRS >= 4 ? PAIRS / 4 : PAIRS;
+  // lane has pairs (every lane asking the others for every pair took four times as many: 8 tokens, 16,384 rows of 2,048, 44.0 us
+  // and 41.4 so, 16 tokens 86 and 81, 8 tokens of 50,257 rows of 1,536 97 and 92, 4 tokens 68 and 66).  One or two tokens have too
+  // few pairs for the selections to pay: each lane asks for each (one token, 1,536 rows of 1,536, 3.48 us, 3.63 exchanged; two
+  // 3.77 and 3.88).
+  constexpr int PAIRS = RL * TT;
+  constexpr bool EXCHANGED = TT >= 4;
+  constexpr int MINE = EXCHANGED ? PAIRS / 4 : PAIRS;
   Pair acc[RL][TT];
   float sum[MINE];
 #pragma unroll
@@ -165,7 +169,7 @@ __global__ void __launch_bounds__(32 * RANGES) gemm_f32_stream_kernel(const floa
       float one[PAIRS];
 #pragma unroll
       for (int i = 0; i < PAIRS; ++i) one[i] = even_and_odd(acc[i / TT][i % TT]), acc[i / TT][i % TT] = 0;
-      if constexpr (PAIRS >= 4) {
+      if constexpr (EXCHANGED) {
         const bool odd = seg & 1, late = seg & 2;
         float two[PAIRS / 2][2];                               // half of the pairs, segments seg & ~1 and seg | 1
 #pragma unroll
@@ -201,8 +205,8 @@ __global__ void __launch_bounds__(32 * RANGES) gemm_f32_stream_kernel(const floa
     step = 0;
 #pragma unroll
     for (int i = 0; i < MINE; ++i) {
-      const int pair = PAIRS >= 4 ? (seg & 1) * (PAIRS / 2) + (seg >> 1) * MINE + i : i;
-      if (PAIRS >= 4 || seg == i) met[(warp * TT + pair % TT) * ROWS + pair / TT * 8 + row] = sum[i];
+      const int pair = EXCHANGED ? (seg & 1) * (PAIRS / 2) + (seg >> 1) * MINE + i : i;
+      if (EXCHANGED || i % TT == seg) met[(warp * TT + pair % TT) * ROWS + pair / TT * 8 + row] = sum[i];
       sum[i] = 0.0f;
     }
     __syncthreads();
@@ -372,10 +376,9 @@ JB_EXPORT int jb_gemm_f32(const float* X, const float* W, float* Y, int T, int N
   const bool vec = K % 4 == 0 && ldx % 4 == 0 && (((uintptr_t)X | (uintptr_t)W) & 15) == 0;
   const int tiles = ((N + BN - 1) / BN) * ((T + BM - 1) / BM);
   // The streaming kernel asks for the weights once for every 8 tokens, the tiles need some of them to fill the SMs.  Streamed and
-  // tiles from cold memory, microseconds, K = 2,048: 16 tokens 2,048 rows 20 and 39, 8,192 rows 50 and 82, 32,000 rows 172 and
-  // 233; 24 tokens 27 and 39, 72 and 82, 250 and 233 (16,384 rows 133 and 143, 4,096 rows 43 and 41); 32 tokens 33 and 39, 92
+  // tiles from cold memory, microseconds, K = 2,048, before the sums met in fewer shuffles (5 % less since, from 5 tokens on): 16
+  // tokens 2,048 rows 20 and 39, 8,192 rows 50 and 82, 32,000 rows 172 and 233; 24 tokens 27 and 39, 72 and 82, 250 and 233 (16,384 rows 133 and 143, 4,096 rows 43 and 41); 32 tokens 33 and 39, 92
   // and 82, 332 and 235 (2,560 rows 39 and 39; 2,048 rows of 8,192 90 and 123); 40 tokens of 2,048 rows 39 and 39.
-  // (Streamed ones of 8 tokens and more take 5 % less since their sums meet in fewer shuffles.)
   if (vec && (T <= 24 || (T <= 32 && N <= 20 * BN))) {
 #define JB_GO(TT) return launch_stream<TT>(X, W, Y, T, N, K, ldx, ldy, accumulate, stream)
     if (T == 1) JB_GO(1);
