@@ -128,12 +128,16 @@ __global__ void route_topk_kernel(const float* __restrict__ logits, int ld, Choi
 // L2 and from memory, 8 experts: 2,048 wide, 1 token 6.1, 6.8 and 3.6, 4.2; 16 tokens 6.6, 7.4 and 3.6, 5.3; 4,096 wide, 2
 // tokens 6.3, 6.9 and 4.8, 7.0; 592 tokens 9.6, 10.8 and 7.7, 10.5 (1,500 tokens 9.8 and 15, in blocks of four tokens).  Two
 // warps a row make many rows dear: the callers' lines, measured on both sides, are beside ROUTE_MAX_NUMBERS in ops.py.
-constexpr int ROUTE_WARPS = 16, ROUTE_AHEAD = 4, ROUTE_MAX_NUMBERS = 1 << 16, ROUTE_MAX_ROWS = 4096;   // (rows: 48 KB of sums)
+// Up to ROUTE_EARLY tokens the launch behind may begin early; with more, its first blocks would share the SMs with these large ones,
+// fewer on some SMs than on others, and the experts' products, whose rows come in several waves, stay out of step for all of
+// their run: a decode step of two routed layers (8 experts of 2,656 x 2,048), 24 sequences 339 and 320 us, 64 sequences 502 and
+// 446, 16 sequences 318 and 299; 8 sequences level.
+constexpr int ROUTE_EARLY = 8, ROUTE_WARPS = 16, ROUTE_AHEAD = 4, ROUTE_MAX_NUMBERS = 1 << 16, ROUTE_MAX_ROWS = 4096;   // (rows: 48 KB of sums)
 __global__ void __launch_bounds__(ROUTE_WARPS * 32) route_tokens_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
                                                                         int W, int R, float* __restrict__ logits, Choice c,
                                                                         int* __restrict__ sel_e, float* __restrict__ sel_w) {
   extern __shared__ float z[];                     // [R] logits, then [2][R] sums of half a row
-  jb::pdl_launch_dependents();
+  if (gridDim.x <= ROUTE_EARLY) jb::pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.x;
   float* halves = z + R;
   const int chunks = W / 8, per = (chunks + 1) / 2;              // 16-byte pieces of a row, and of its first half
