@@ -128,16 +128,16 @@ __global__ void route_topk_kernel(const float* __restrict__ logits, int ld, Choi
 // L2 and from memory, 8 experts: 2,048 wide, 1 token 6.1, 6.8 and 3.6, 4.2; 16 tokens 6.6, 7.4 and 3.6, 5.3; 4,096 wide, 2
 // tokens 6.3, 6.9 and 4.8, 7.0; 592 tokens 9.6, 10.8 and 7.7, 10.5 (1,500 tokens 9.8 and 15, in blocks of four tokens).  Two
 // warps a row make many rows dear: the callers' lines, measured on both sides, are beside ROUTE_MAX_NUMBERS in ops.py.
-// Up to ROUTE_EARLY tokens the launch behind may begin early; with more, its first blocks would share the SMs with these large ones,
-// fewer on some SMs than on others, and the experts' products, whose rows come in several waves, stay out of step for all of
-// their run: a decode step of two routed layers (8 experts of 2,656 x 2,048), 24 sequences 339 and 320 us, 64 sequences 502 and
-// 446, 16 sequences 318 and 299; 8 sequences level.
-constexpr int ROUTE_EARLY = 8, ROUTE_WARPS = 16, ROUTE_AHEAD = 4, ROUTE_MAX_NUMBERS = 1 << 16, ROUTE_MAX_ROWS = 4096;   // (rows: 48 KB of sums)
+// early: the launch behind may begin at once.  Not where it is expert_tc_kernel: its first blocks would share the SMs with these
+// large ones, fewer on some SMs than on others, and products of several waves stay out of step for all of their run: a decode step of two
+// routed layers (8 experts of 2,656 x 2,048), 24 sequences 339 and 320 us, 64 sequences 502 and 446, 16 sequences 318 and 299.
+constexpr int ROUTE_WARPS = 16, ROUTE_AHEAD = 4, ROUTE_MAX_NUMBERS = 1 << 16, ROUTE_MAX_ROWS = 4096;   // (rows: 48 KB of sums)
 __global__ void __launch_bounds__(ROUTE_WARPS * 32) route_tokens_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
                                                                         int W, int R, float* __restrict__ logits, Choice c,
-                                                                        int* __restrict__ sel_e, float* __restrict__ sel_w) {
+                                                                        int* __restrict__ sel_e, float* __restrict__ sel_w,
+                                                                        int early) {
   extern __shared__ float z[];                     // [R] logits, then [2][R] sums of half a row
-  if (gridDim.x <= ROUTE_EARLY) jb::pdl_launch_dependents();
+  if (early) jb::pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.x;
   float* halves = z + R;
   const int chunks = W / 8, per = (chunks + 1) / 2;              // 16-byte pieces of a row, and of its first half
@@ -713,10 +713,10 @@ JB_EXPORT int jb_route_topk(const float* logits, int ld, int E, int top, int* se
 }
 
 // x: [T, W], w: [R, W], both bfloat16 row-major, W a multiple of 8; logits: float32 [T, R], written; the choice goes by the
-// first E of a row's logits.
+// first E of a row's logits.  early: see the kernel.
 JB_EXPORT int jb_route_tokens(const void* x, const void* w, int W, int R, float* logits, int E, int top, int* sel_e,
                               float* sel_w, int T, int softmax, int groups, int keep, const float* correction, float scale,
-                              int shares, cudaStream_t stream) {
+                              int shares, int early, cudaStream_t stream) {
   if (T <= 0) return 0;
   const Choice c{E, top, softmax, groups, keep, correction, scale, shares};
   if (const int e = check_choice(c)) return e;
@@ -724,7 +724,8 @@ JB_EXPORT int jb_route_tokens(const void* x, const void* w, int W, int R, float*
             "route_tokens: %d rows of %d (%d experts)", R, W, E);
   JB_REFUSE(((uintptr_t)x | (uintptr_t)w) & 15, "route_tokens: operands must be 16-byte aligned");
   jb::Launch cfg(dim3(T), dim3(ROUTE_WARPS * 32), 3 * (size_t)R * sizeof(float), stream);
-  return (int)cudaLaunchKernelEx(&cfg.c, route_tokens_kernel, (const bf16*)x, (const bf16*)w, W, R, logits, c, sel_e, sel_w);
+  return (int)cudaLaunchKernelEx(&cfg.c, route_tokens_kernel, (const bf16*)x, (const bf16*)w, W, R, logits, c, sel_e, sel_w,
+                                 early);
 }
 
 // h: [T, W] in x_dtype; the experts' weights ([E] of them) in w_dtype; act: float32 scratch [T top, F]; out: float32

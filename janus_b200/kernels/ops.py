@@ -68,7 +68,7 @@ _SIGNATURES = {
     "jb_join_norm": "pppppffpppfipipiiplplp", "jb_head_norm_gate": "ppipipfipiiiip", "jb_sigmoid_gate": "pipiiiiip",
     "jb_head_norm_rope_cache": "pippfpippipppiiiiiiiiiifipifp",
     "jb_delta_rule": "piiiipiiippfppllppiiiiip", "jb_delta_rule_chunks": "piiiipiiippfppllppiiiiiipiip",
-    "jb_route_topk": "piiippiiiipfip", "jb_route_tokens": "ppiipiippiiiipfip", "jb_experts_few_tokens": "pippipppippiiiiffip", "jb_expert_gather": "pippipiip", "jb_experts_few_tokens_tc": "pppipppppiiiiffip",
+    "jb_route_topk": "piiippiiiipfip", "jb_route_tokens": "ppiipiippiiiipfiip", "jb_experts_few_tokens": "pippipppippiiiiffip", "jb_expert_gather": "pippipiip", "jb_experts_few_tokens_tc": "pppipppppiiiiffip",
     "jb_expert_scatter": "pppipiip", "jb_experts_stream": "pppipliplppppiiiiffipp",
     "jb_state_chunks": "ipiiiipipppfpppllppiiiiiipiip",
     "jb_head_step": "ipiiiifpiiippfiplllpipiifpippiiiiip",
@@ -1900,9 +1900,10 @@ ROUTE_MAX_NUMBERS, ROUTE_MAX_ROWS, ROUTE_MAX_TOKENS = 24 * 2048, 24, 128
 
 def route_tokens(x: torch.Tensor, w: torch.Tensor, logits: torch.Tensor, top: int, sel_e: torch.Tensor, sel_w: torch.Tensor,
                  softmax: bool = False, groups: int = 0, keep: int = 0, experts: Optional[int] = None,
-                 correction: Optional[torch.Tensor] = None, scale: float = 1.0, shares: bool = False) -> None:
+                 correction: Optional[torch.Tensor] = None, scale: float = 1.0, shares: bool = False, early: bool = True) -> None:
     """logits[t, r] = w[r] . x[t] (bfloat16 x [T, W] and w [R, W], W a multiple of 8; float32 [T, R]) and `route_topk` of
-    them, in one launch, of at most 65,536 numbers and 4,096 rows in w (three numbers a row lie in 48 KB of shared memory)."""
+    them, in one launch, of at most 65,536 numbers and 4,096 rows in w (three numbers a row lie in 48 KB of shared memory).
+    `early`: the launch behind may begin before this one ends; off before `experts_few_tokens_tc`, which that sets out of step."""
     (T, W), R = x.shape, w.shape[0]
     E = R if experts is None else int(experts)
     _need(x, "router in", torch.bfloat16)
@@ -1914,7 +1915,7 @@ def route_tokens(x: torch.Tensor, w: torch.Tensor, logits: torch.Tensor, top: in
         _need(correction, "router's correction", torch.float32, (E,))
     _check(_lib("routed").jb_route_tokens(_ptr(x), _ptr(w), W, R, _ptr(logits), E, int(top), _ptr(sel_e), _ptr(sel_w), T,
                                           int(bool(softmax)), int(groups), int(keep), _ptr(correction), float(scale),
-                                          int(bool(shares)), _stream()), "route_tokens")
+                                          int(bool(shares)), int(bool(early)), _stream()), "route_tokens")
 
 
 def experts_few_tokens(h: torch.Tensor, sel_e: torch.Tensor, sel_w: torch.Tensor, w_gate: torch.Tensor,
@@ -1978,7 +1979,8 @@ def experts_stream_pays(T: int, top: int, experts: int, F: int, W: int) -> bool:
     start for every expert, chosen or not, go again over an expert's rows for every 16 of its tokens and read their tokens' rows from L2;
     tiles cost two more launches' worth of start, all tokens as columns and the adds of their sums.  The constants were fitted to
     238 cases in captured steps with weights from memory (4 to 512 experts of 128 x 128 to 7,168 x 4,096, 1 to 16 a token, 1 to 64
-    tokens): the pick is 0.5 % slower than the better form on average, at worst 12 %, where always tiles were 13 % and row blocks 16 %.
+    tokens): the pick is 0.5 % slower than the better form on average, at worst 12 %, where always tiles were 13 % and row blocks 16 %;
+    of whole decode steps with three such layers (346 cases) 0.3 and 8 %, where either form alone was 4 %.
     Row blocks and tiles: two of 8 experts of 4,096 x 2,048, 1 token 29 and 28, 16 tokens 74 and 74, 64 tokens 129 and 84; of
     1,536 x 1,024, 8 tokens 19 and 23; of 128 x 128 6 and 11; six of 64 of 1,408 x 2,048, 1 token 41 and 31; one of 4 of 1,024 x
     1,024, 16 tokens 12 and 18."""

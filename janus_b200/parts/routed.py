@@ -173,9 +173,11 @@ class RoutedExperts(FeedForward):
         sel_w = ws.get("router_weights", (T, self.top), torch.float32)
         choice = dict(softmax=self.softmax, groups=self.groups, keep=self.keep, experts=self.experts,
                       correction=self.correction, scale=self.weight_scale, shares=self.shares)
-        streams = self._streams(ctx, T)
+        streams, pairs = self._streams(ctx, T), T * self.top
+        by_tiles = streams or (self.dtype == torch.bfloat16 and not ctx.is_decode and pairs > FEW_PAIRS)
         if self._routes_in_one(T):
-            ops.route_tokens(x, self.router_rows, logits, self.top, sel_e, sel_w, **choice)
+            ops.route_tokens(x, self.router_rows, logits, self.top, sel_e, sel_w, early=by_tiles or self.shared_size is not None,
+                             **choice)
         else:
             self.router.forward(x, logits, y_is_zero=scratch_cleared and not streams)
             ops.route_topk(logits, self.top, sel_e, sel_w, **choice)
@@ -185,7 +187,6 @@ class RoutedExperts(FeedForward):
             if self.shared_gate:
                 ops.scale_rows_sigmoid(shared, logits[:, self.experts])
             self.shared_down.forward_add(shared, residual)
-        pairs = T * self.top
         if streams:
             sums = ws.get("experts_sums", (pairs, 2 * self.intermediate_size), torch.float32)
             if not scratch_cleared:
@@ -195,7 +196,7 @@ class RoutedExperts(FeedForward):
                                ws.get("experts_places", (pairs,), torch.int32), residual,
                                weight_on_output=self.weight_on_output)
             return
-        if self.dtype == torch.bfloat16 and not ctx.is_decode and pairs > FEW_PAIRS:
+        if by_tiles:
             if self.grouped:
                 self._grouped(x, sel_e, sel_w, residual, ctx)
             else:

@@ -76,8 +76,8 @@ def test_a_router_of_more_rows_than_a_launch_holds():
     from janus_b200.parts.routed import RoutedExperts
     part = RoutedExperts(8, 8, 8192, 2, dtype=torch.bfloat16, device=torch.device("cpu"))
     assert not part.route_in_one
-    assert ops._lib("routed").jb_route_tokens(0, 0, 8, 8192, 0, 8192, 2, 0, 0, 1, 0, 0, 0, 0, 1.0, 0, 0) == BAD_SIZE
-    assert ops._lib("routed").jb_route_tokens(0, 0, 8, 4097, 0, 4097, 2, 0, 0, 1, 0, 0, 0, 0, 1.0, 0, 0) == BAD_SIZE
+    assert ops._lib("routed").jb_route_tokens(0, 0, 8, 8192, 0, 8192, 2, 0, 0, 1, 0, 0, 0, 0, 1.0, 0, 1, 0) == BAD_SIZE
+    assert ops._lib("routed").jb_route_tokens(0, 0, 8, 4097, 0, 4097, 2, 0, 0, 1, 0, 0, 0, 0, 1.0, 0, 1, 0) == BAD_SIZE
 
 
 @pytest.mark.parametrize("rows, width, one", [(8, 2048, True), (16, 2048, True), (24, 2048, True), (9, 4096, True), (12, 4096, True), (8, 264, True),
