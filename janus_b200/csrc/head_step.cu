@@ -9,8 +9,9 @@
 // What bounds it: the state's bytes for many heads, else a chain of loads and sums, which the launches of its parts made three
 // times.  In a captured step of 8 sequences, 16 heads of 128 x 128 (17 MB of state, 2.7 us): matrix memory, gates 3.0 +
 // recurrence 4.1 + norm 4.1 us, here 6.9; channel decays 11.8 + 4.1 + 4.1 us, here 6.9.  One sequence of the delta rule is
-// level with its walk and norm, a launch less.  512 threads hold a head's state of up to 128 x 256 numbers in registers: a thread four columns of
-// every ROWS-th row, all of its loads in flight before the gates are known.
+// level with its walk and norm, a launch less.  Where many small heads lose by it is at `head_step_pays` in ops.py.  512 threads
+// hold a head's state of up to 128 x 256 numbers in registers: a thread four columns of every ROWS-th row, all of its loads in
+// flight before the gates are known.
 #include <math_constants.h>
 #include <stdio.h>
 

@@ -453,7 +453,8 @@ def pack_gated(gate: torch.Tensor, up: torch.Tensor) -> PackedWeight:
 # JANUS_DETERMINISTIC=1 (or `set_deterministic(True)` before a model is built): the slices of a cut K are
 # summed in the fixed order of the slices instead of by atomic adds in the order they happen to finish, so the
 # same requests give the same bits.  Every slice leaves its tile in scratch; the one that arrives last at the
-# output tile's ticket adds them up (single-CTA kernel; CTA pairs then run uncut).
+# output tile's ticket adds them up (single-CTA kernel; CTA pairs then run uncut).  Experts of few tokens go by
+# `experts_few_tokens_tc` (no slices), a row for every pair's result, added in the order of a token's choices.
 _deterministic = [os.environ.get("JANUS_DETERMINISTIC", "0") == "1"]
 
 
