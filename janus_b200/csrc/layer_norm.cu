@@ -308,30 +308,37 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o, const float* 
 }
 
 // The same for heads of at most 128 numbers in whole, aligned groups of four: a lane has four numbers of a head, a warp ITEMS
-// heads whose loads are all in flight before the first sum (1,500 tokens of 16 heads of 128, 30 MB: 16.5 us with
-// one number a lane and access and a head a warp, 12.5 so; 2,207 tokens 23.9 and 15.7).
+// heads whose loads are all in flight before the first sum.  One number a lane and access and a head a warp, and so, microseconds
+// with operands in L2: 1,500 tokens of 16 heads of 128 10.3 and 8.2, 4,000 27 and 18, of 32 heads of 64 45 and 34.  Below some
+// 1.3 million numbers the longer chain of a warp is what shows: 600 tokens of 16 heads of 128 5.4 and 5.6, of 4 heads 3.5 and 3.7,
+// 40 tokens 2.7 and 3.5.
 constexpr int GATE_ITEMS = 4;
+constexpr long long GATE_VEC_FROM = 5 << 18;
 template <typename TO>
 __global__ void __launch_bounds__(128) head_norm_gate_vec_kernel(const float* __restrict__ o, const float* __restrict__ gate, int ld_gate,
                                                                  const float* __restrict__ weight, int w_stride,
                                                                  const float* __restrict__ denom, float eps, int act,
-                                                                 TO* __restrict__ out, long long items, int heads, int e) {
+                                                                 TO* __restrict__ out, unsigned items, int heads, int e) {
   jb::pdl_launch_dependents();
   jb::pdl_wait();
-  const long long first = ((long long)blockIdx.x * 4 + (threadIdx.x >> 5)) * GATE_ITEMS;
+  const unsigned first = (blockIdx.x * 4 + (threadIdx.x >> 5)) * GATE_ITEMS;
   const int j = 4 * (threadIdx.x & 31);
   const bool in = j < e;
-  float4 v[GATE_ITEMS], g[GATE_ITEMS];
+  float4 v[GATE_ITEMS], g[GATE_ITEMS], w[GATE_ITEMS];
   float under[GATE_ITEMS];
+  unsigned t = first / (unsigned)heads;
+  int h = (int)(first - t * heads);
 #pragma unroll
-  for (int k = 0; k < GATE_ITEMS; ++k) {
-    const long long item = first + k < items ? first + k : items - 1;
-    v[k] = g[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (in) {
+  for (int k = 0; k < GATE_ITEMS; ++k, ++h) {
+    if (h == heads) h = 0, ++t;
+    const unsigned item = first + k;
+    v[k] = g[k] = w[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (in && item < items) {
       v[k] = *reinterpret_cast<const float4*>(o + (size_t)item * e + j);
-      g[k] = *reinterpret_cast<const float4*>(gate + (size_t)(item / heads) * ld_gate + (size_t)(item % heads) * e + j);
+      g[k] = *reinterpret_cast<const float4*>(gate + (size_t)t * ld_gate + (size_t)h * e + j);
+      w[k] = *reinterpret_cast<const float4*>(weight + (size_t)h * w_stride + j);
     }
-    under[k] = denom != nullptr ? denom[item] : 1.0f;
+    under[k] = denom != nullptr && item < items ? denom[item] : 1.0f;
   }
 #pragma unroll
   for (int k = 0; k < GATE_ITEMS; ++k) {
@@ -341,14 +348,13 @@ __global__ void __launch_bounds__(128) head_norm_gate_vec_kernel(const float* __
     const float ss = jb::warp_sum(fmaf(a, a, fmaf(b, b, fmaf(c, c, d * d))));
     const float inv = u / sqrtf(ss / (float)e + eps);
     if (!in) continue;
-    const float4 w = *reinterpret_cast<const float4*>(weight + (size_t)((first + k) % heads) * w_stride + j);
     const auto gated = [&](float x, float y, float z) {
       const float s = 1.0f / (1.0f + expf(-z));
       return ((x * inv) * y) * (act == 0 ? z * s : s);
     };
     Vec<4> r;
-    r.v[0] = gated(v[k].x, w.x, g[k].x), r.v[1] = gated(v[k].y, w.y, g[k].y);
-    r.v[2] = gated(v[k].z, w.z, g[k].z), r.v[3] = gated(v[k].w, w.w, g[k].w);
+    r.v[0] = gated(v[k].x, w[k].x, g[k].x), r.v[1] = gated(v[k].y, w[k].y, g[k].y);
+    r.v[2] = gated(v[k].z, w[k].z, g[k].z), r.v[3] = gated(v[k].w, w[k].w, g[k].w);
     store_out(out + (size_t)(first + k) * e + j, r);
   }
 }
@@ -474,14 +480,14 @@ JB_EXPORT int jb_head_norm_gate(const float* o, const float* gate, int ld_gate, 
                                 int e, cudaStream_t stream) {
   if (T <= 0) return 0;
   const long long items = (long long)T * heads;
-  if (e <= 128 && ((e | ld_gate | w_stride) & 3) == 0 && (out_dtype == JB_F32 || out_dtype == JB_BF16) &&
+  if (e <= 128 && items < (1ll << 31) && items * e >= GATE_VEC_FROM && ((e | ld_gate | w_stride) & 3) == 0 && (out_dtype == JB_F32 || out_dtype == JB_BF16) &&
       (((uintptr_t)o | (uintptr_t)gate | (uintptr_t)weight | (uintptr_t)out) & 15) == 0) {
     jb::Launch vcfg(dim3((unsigned)((items + 4 * GATE_ITEMS - 1) / (4 * GATE_ITEMS))), dim3(128), 0, stream);
     if (out_dtype == JB_F32)
       return (int)cudaLaunchKernelEx(&vcfg.c, head_norm_gate_vec_kernel<float>, o, gate, ld_gate, weight, w_stride, denom, eps, act,
-                                     (float*)out, items, heads, e);
+                                     (float*)out, (unsigned)items, heads, e);
     return (int)cudaLaunchKernelEx(&vcfg.c, head_norm_gate_vec_kernel<bf16>, o, gate, ld_gate, weight, w_stride, denom, eps, act,
-                                   (bf16*)out, items, heads, e);
+                                   (bf16*)out, (unsigned)items, heads, e);
   }
   jb::Launch cfg(dim3((unsigned)((items + 3) / 4)), dim3(128), 0, stream);
   cudaError_t err;

@@ -193,7 +193,8 @@ def test_clear_rows(ops):
         assert float(t[1].abs().sum()) == 0.0 and bool((t[0] == 1).all()) and bool((t[2] == 1).all())
 
 
-@pytest.mark.parametrize("T, H, e", [(1, 3, 128), (5, 1, 4), (7, 16, 100), (33, 2, 128), (300, 5, 64)])
+@pytest.mark.parametrize("T, H, e", [(1, 3, 128), (5, 1, 4), (7, 16, 100), (33, 2, 128), (300, 5, 64), (700, 15, 128), (1311, 10, 100),
+                                     (4097, 5, 64), (3277, 100, 4)])
 @pytest.mark.parametrize("per_head, sigmoid, divided", [(False, False, False), (True, True, True)])
 def test_head_norm_gate_in_vectors(ops, T, H, e, per_head, sigmoid, divided):
     """Heads in whole vectors against float64 and against the general form (a gate whose rows are off a 16-byte boundary)."""
