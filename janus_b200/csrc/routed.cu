@@ -561,9 +561,11 @@ constexpr int PLAN_THREADS = 1024, PLAN_MAX_EXPERTS = 1024, PLAN_AHEAD = 8;
 // its count of items in [0] and item i as (t0, t_end, wf0, f0) at [4 + 4 i]: rows [t0, t_end) of the sorted pairs,
 // weight rows from wf0 on in the stack of the experts' matrices, output columns from f0 on.  Tiles are 256 rows;
 // `gu` tiles are 128 features of F wide, `dn` tiles 256 features of W.  Inside an expert the row tiles run fastest,
-// so CTAs that run side by side share a weight tile.  What bounds it is that one block does it: a warp's pairs count with
-// one atomic an expert, a warp writes an expert's tiles (8 experts, two a token: 1,500 tokens of 4,096 x 2,048 13.1 us with an atomic
-// a pair and a thread an expert, 8.4 so; 3,072 tokens of 7,168 x 4,096 18.8 and 6.8).
+// so CTAs that run side by side share a weight tile.  What bounds it is that one block does it: all its threads write tiles, a
+// group of them an expert's, and a thread's first pairs are asked for at once.  With a thread an expert, and so, microseconds: 8
+// experts of 2,048 x 4,096, 1,500 pairs 5.4 and 3.4, 4,000 7.5 and 3.9; of 4,096 x 7,168, 6,144 pairs 15.5 and 4.3; 64 of 1,408 x 2,048,
+// 4,000 pairs 7.6 and 6.3; 256 of 512 x 1,024, 1,500 pairs 10.2 and 9.9.  (A warp's pairs of one expert counted together by match
+// were slower everywhere: 12.1 and 22.7 with 256 experts and 4,000 pairs.)
 __global__ void __launch_bounds__(PLAN_THREADS) expert_plan_kernel(const int* __restrict__ sel_e, int n_pairs, int E,
                                                                    int F, int W, int* __restrict__ order,
                                                                    int* __restrict__ where, int* __restrict__ gu,
@@ -571,17 +573,8 @@ __global__ void __launch_bounds__(PLAN_THREADS) expert_plan_kernel(const int* __
   __shared__ int count[PLAN_MAX_EXPERTS], start[PLAN_MAX_EXPERTS], cursor[PLAN_MAX_EXPERTS], tiles_before[PLAN_MAX_EXPERTS];
   jb::pdl_launch_dependents();
   jb::pdl_wait();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // a warp's lanes that chose the same expert count together: its places are its first lane's and the lanes before
-  const auto add = [&](int* counter, int e, bool in) {
-    const unsigned same = __match_any_sync(0xffffffffu, in ? e : -1);
-    const int first = __ffs(same) - 1;
-    int at = 0;
-    if (in && lane == first) at = atomicAdd(&counter[e], __popc(same));
-    return __shfl_sync(0xffffffffu, at, first) + __popc(same & ((1u << lane) - 1u));
-  };
   for (int e = threadIdx.x; e < E; e += PLAN_THREADS) count[e] = 0;
-  int mine[PLAN_AHEAD];                                      // the first pairs, kept for the second pass
+  int mine[PLAN_AHEAD];                                      // the first pairs' experts, kept for the second pass
 #pragma unroll
   for (int k = 0; k < PLAN_AHEAD; ++k) {
     const int i = k * PLAN_THREADS + threadIdx.x;
@@ -589,12 +582,11 @@ __global__ void __launch_bounds__(PLAN_THREADS) expert_plan_kernel(const int* __
   }
   __syncthreads();
 #pragma unroll
-  for (int k = 0; k < PLAN_AHEAD; ++k)
-    if (k * PLAN_THREADS < n_pairs) add(count, mine[k], mine[k] >= 0);
-  for (int i0 = PLAN_AHEAD * PLAN_THREADS; i0 < n_pairs; i0 += PLAN_THREADS) {
-    const int i = i0 + threadIdx.x;
-    add(count, i < n_pairs ? sel_e[i] : 0, i < n_pairs);
+  for (int k = 0; k < PLAN_AHEAD; ++k) {
+    if (k * PLAN_THREADS >= n_pairs) break;
+    if (mine[k] >= 0) atomicAdd(&count[mine[k]], 1);
   }
+  for (int i = PLAN_AHEAD * PLAN_THREADS + threadIdx.x; i < n_pairs; i += PLAN_THREADS) atomicAdd(&count[sel_e[i]], 1);
   __syncthreads();
   const int gu_per = (F + 127) / 128, dn_per = (W + 255) / 256;
   if (threadIdx.x == 0) {
@@ -609,29 +601,27 @@ __global__ void __launch_bounds__(PLAN_THREADS) expert_plan_kernel(const int* __
     dn[0] = tiles * dn_per;
   }
   __syncthreads();
-  const auto put = [&](int i, int e, bool in) {
-    const int place = add(cursor, e, in);
-    if (in) order[place] = i, where[i] = place;
+  const auto put = [&](int i, int e) {
+    const int place = atomicAdd(&cursor[e], 1);
+    order[place] = i, where[i] = place;
   };
 #pragma unroll
-  for (int k = 0; k < PLAN_AHEAD; ++k)
-    if (k * PLAN_THREADS < n_pairs) put(k * PLAN_THREADS + threadIdx.x, mine[k], mine[k] >= 0);
-  for (int i0 = PLAN_AHEAD * PLAN_THREADS; i0 < n_pairs; i0 += PLAN_THREADS) {
-    const int i = i0 + threadIdx.x;
-    put(i, i < n_pairs ? sel_e[i] : 0, i < n_pairs);
+  for (int k = 0; k < PLAN_AHEAD; ++k) {
+    if (k * PLAN_THREADS >= n_pairs) break;
+    if (mine[k] >= 0) put(k * PLAN_THREADS + threadIdx.x, mine[k]);
   }
-  for (int e = warp; e < E; e += PLAN_THREADS / 32) {        // a warp an expert's tiles
+  for (int i = PLAN_AHEAD * PLAN_THREADS + threadIdx.x; i < n_pairs; i += PLAN_THREADS) put(i, sel_e[i]);
+  const int shift = 31 - __clz(PLAN_THREADS / E), e = threadIdx.x >> shift, per = 1 << shift;   // threads that share an expert's tiles
+  if (e < E) {
     const int n_tt = (count[e] + 255) / 256, end = start[e] + count[e];
-    int4* g = reinterpret_cast<int4*>(gu + 4) + (size_t)tiles_before[e] * gu_per;
-    for (int i = lane; i < gu_per * n_tt; i += 32) {
-      const int ft = i / n_tt, t0 = start[e] + i % n_tt * 256;
-      g[i] = make_int4(t0, end, e * F + ft * 128, ft * 128);
-    }
-    int4* d = reinterpret_cast<int4*>(dn + 4) + (size_t)tiles_before[e] * dn_per;
-    for (int i = lane; i < dn_per * n_tt; i += 32) {
-      const int ft = i / n_tt, t0 = start[e] + i % n_tt * 256;
-      d[i] = make_int4(t0, end, e * W + ft * 256, ft * 256);
-    }
+    const auto list = [&](int4* at, int n, int size, int step) {
+      for (int i = threadIdx.x & (per - 1); i < n * n_tt; i += per) {
+        const int ft = n_tt == 1 ? i : i / n_tt;
+        at[i] = make_int4(start[e] + (i - ft * n_tt) * 256, end, e * size + ft * step, ft * step);
+      }
+    };
+    list(reinterpret_cast<int4*>(gu + 4) + (size_t)tiles_before[e] * gu_per, gu_per, F, 128);
+    list(reinterpret_cast<int4*>(dn + 4) + (size_t)tiles_before[e] * dn_per, dn_per, W, 256);
   }
 }
 
