@@ -422,7 +422,9 @@ constexpr int CHUNK_SMEM = (5 * C * LD + C * (C + 4) + DMAX / 2 * SLD + 2 * C * 
 
 // SPLIT times 256 threads, which share the first product's sums over k.  Once, two blocks an SM; twice where no SM has a second
 // block, which shortens a chunk's chain (prepare and chunks, one sequence of 16 heads of 128 x 128, 128 blocks: 1,500
-// tokens 265 and 192 us, 192 tokens 48 and 38; 8 heads of 72 x 72, 1,500 tokens 249 and 175).
+// tokens 265 and 192 us, 192 tokens 48 and 38; 8 heads of 72 x 72, 1,500 tokens 249 and 175; 1,000 tokens, 4 heads of 128 x 128,
+// 32 blocks, 164 and 117).  Very few blocks have the chip's clock and memory to themselves and are faster with 256 (3 heads, 24 blocks,
+// 106 and 115; one head, 2,000 tokens, 190 and 210; 28 blocks level).
 template <int SPLIT>
 __global__ void __launch_bounds__(CHUNK_THREADS * SPLIT, 2 / SPLIT) delta_chunks_kernel(
     const float* __restrict__ conv, int ldc, int q_col, int k_col, float* __restrict__ out, const float* __restrict__ scratch,
@@ -676,7 +678,8 @@ JB_EXPORT int jb_delta_rule_chunks(const float* conv, int ldc, int q_col, int k_
   JB_REFUSE(d < 1 || d > DMAX || e < 1 || ((d | ldc | q_col | k_col) & 3) != 0 || (((uintptr_t)conv | (uintptr_t)scratch) & 15) != 0,
             "delta_rule_chunks: keys of %d numbers in rows of %d at columns %d and %d", d, ldc, q_col, k_col);
   JB_REFUSE(G < 1 || H % G != 0 || tiles < 0 || max_q_len < 1, "delta_rule_chunks: %d heads are not a multiple of %d key heads", H, G);
-  const bool few = (long long)n_seqs * H * ((e + 15) / 16) <= 148;                   // no SM has a second block
+  const long long blocks = (long long)n_seqs * H * ((e + 15) / 16);
+  const bool few = blocks > 28 && blocks <= 148;                                     // no SM has a second block, many have one
   auto* const walk_kernel = few ? delta_chunks_kernel<2> : delta_chunks_kernel<1>;
   cudaError_t err = cudaFuncSetAttribute(walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CHUNK_SMEM);
   if (err != cudaSuccess) return (int)err;
