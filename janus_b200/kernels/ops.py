@@ -1201,12 +1201,18 @@ def state_chunks_pay(kind: str, n_seqs: int, heads: int, dim: int, vdim: int, ma
     numbers, whose blocks stay small: 64 tokens 25 and 24, 128 tokens 46 and 31; 128 blocks of 2,048 tokens 388 and 453, 256
     blocks 738 and 472.  A decay a channel has the same lines; 16 heads of 128 x 128: one sequence of 64 tokens 31 and 28, 256
     104 and 62, 512 113 and 108, 1,024 141 and 200; two of 512 147 and 116, four of 1,024 462 and 251, eight 1,222 and 445, of
-    40 to 511 tokens 435 and 214; 64 of 16 tokens 84 and 157."""
+    40 to 511 tokens 435 and 214; 64 of 16 tokens 84 and 157.  Its walk is cheaper for many short sequences (32 of 20 to 90 tokens, 32
+    heads of 128 x 128 231 and 258, 16 heads 132 and 139, of 96 x 64 79 and 88) and for narrow values (four of 700, 16 heads of 96 x 64,
+    64 blocks, 152 and 172; eight of 40 to 511, 128 blocks, 221 and 131)."""
     if max_q_len < STATE_CHUNKS_FROM[dim <= 64] or dim > 128:
         return False
     blocks, line = heads * -(-vdim // 64), 148 if dim <= 64 else 96 if kind == "mamba" else 64          # blocks of a sequence
     if _mostly_single_tokens(n_seqs, tokens, n_seqs * blocks):
         return False
+    if kind == "channel" and dim > 64:
+        if max_q_len < 128 and n_seqs * blocks >= (512 if vdim <= 64 else 1024):
+            return False
+        line = 96 if vdim <= 64 else line
     if max_q_len <= STATE_WALK_TOKENS[kind != "mamba" and dim > 64 and n_seqs * blocks >= 32]:
         return True
     return n_seqs * blocks >= line and 3 * tokens * blocks >= 2 * line * max_q_len
