@@ -107,3 +107,12 @@ def test_which_single_token_steps_are_one_launch(kind, n, heads, dim, vdim, one)
 def test_which_experts_stream_their_tiles(T, top, experts, F, W, tiles):
     """Sizes whose forms were measured more than 3 % apart, or that are a model's own."""
     assert ops.experts_stream_pays(T, top, experts, F, W) is tiles
+
+
+@pytest.mark.parametrize("heads, dim, vdim, lens, chunks", [
+    (16, 128, 128, [64], True), (16, 128, 128, [300, 300], True), (16, 128, 128, [400] * 8, True), (32, 128, 128, [1000, 1000], True),
+    (32, 128, 128, [55] * 32, False), (16, 128, 128, [55] * 32, False), (16, 96, 64, [55] * 32, False), (16, 128, 128, [64] * 16, True),
+    (16, 96, 64, [700] * 4, False), (16, 96, 64, [275] * 8, True), (16, 128, 128, [1000], False), (16, 64, 64, [55] * 32, False)])
+def test_which_prompts_of_channel_decays_go_by_chunks(heads, dim, vdim, lens, chunks):
+    """On both sides of the lines in blocks, tokens and width of the values."""
+    assert ops.state_chunks_pay("channel", len(lens), heads, dim, vdim, max(lens), sum(lens)) is chunks
