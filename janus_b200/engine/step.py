@@ -236,16 +236,20 @@ class Engine:
         q_start = [0]
         for n in lens:
             q_start.append(q_start[-1] + n)
-        # wanted rows: places one by one in a list, which costs less than an array an entry; ranges as arrays
+        # wanted rows: places one by one in a list, which costs less than an array an entry; long ranges as arrays
         wants, places = [], []
         for e, first in zip(entries, q_start):
             w = e.want
-            if type(w) is range:
-                wants += [np.array(places, dtype=np.int64), np.arange(first + w.start, first + w.stop, w.step)]
-                places = []
+            if type(w) is range and len(w) > 32:
+                if places:
+                    wants.append(np.array(places, dtype=np.int64))
+                    places = []
+                wants.append(np.arange(first + w.start, first + w.stop, w.step))
             else:
                 places += [first + int(x) for x in w]
-        wants = np.concatenate(wants + [np.array(places, dtype=np.int64)])
+        if places or not wants:
+            wants.append(np.array(places, dtype=np.int64))
+        wants = wants[0] if len(wants) == 1 else np.concatenate(wants)
         W = len(wants)
         G = len(cache.groups)
         sizes = [T, T, T, S + 1, S, S, W] + [T, S * P] * G + [S + 1]
